@@ -9,10 +9,10 @@
 //   input grad     dX = dY * W        A K-major,  B N-major     (reference mm_nn_bf16o, kernels.cu:55-60)
 //   weight grad    dW = dY^T * X      A M-major,  B N-major     (reference mm_tn_bf16[_acc], kernels.cu:41-53)
 //
-// Structure: persistent CTAs (one per SM), 6 warps.  Warp 0 streams operand tiles with TMA
+// Structure: persistent CTAs (one per SM), 10 warps.  Warp 0 streams operand tiles with TMA
 // into a ring of 128-byte-swizzled shared-memory stages; one lane of warp 1 issues
 // tcgen05.mma (128 x BN x 16 per instruction) into one of two TMEM accumulator buffers and
-// commits stage-release / accumulator-ready mbarriers; warps 2-5 drain the other
+// commits stage-release / accumulator-ready mbarriers; warps 2-9 drain the other
 // accumulator with tcgen05.ld and run the fused epilogue, so the epilogue of tile i
 // overlaps the main loop of tile i+1.
 //
@@ -20,8 +20,8 @@
 // (add_bias_k kernels.cu:174, bias_gelu_k :292, bias_residual_k :274, gelu_bwd_k :431,
 // add_k :262) and the beta=1 weight-gradient accumulation.
 //
-// Bias gradients: with `colsum` set (weight-gradient products, A = dY in M-major form) four more
-// warps add up the columns of the A tiles while they sit in shared memory and the CTAs that own
+// Bias gradients: with `colsum` set (weight-gradient products, A = dY in M-major form) four of the
+// epilogue warps add up the columns of the A tiles while they sit in shared memory and the CTAs that own
 // the first column of output tiles add the sums into colsum[M] -- the reference's separate
 // colsum_k pass over dY (kernels.cu:511-524) disappears.  A stage is handed back to the TMA
 // producer only after both the MMAs and these warps are done with it.
@@ -248,13 +248,12 @@ struct GemmParams {
   const bf16* bias;        // [N]
   bf16* aux; int ldaux;    // EPI_BIAS_GELU: pre-activation out; EPI_BIAS_RESID/EPI_RESID: residual in; EPI_DGELU: pre-activation in
   float alpha;             // scales the accumulator before the epilogue
-  float* colsum;           // [M] fp32 or null: colsum[m] (+)= sum_k op(A)[m, k]  (needs a_mn; launch with CSUM_THREADS)
+  float* colsum;           // [M] fp32 or null: colsum[m] (+)= sum_k op(A)[m, k]  (needs a_mn)
   int* err;                // library error word
 };
 
 constexpr int BM = 128, BK = 64, UMMA_K = 16;
-constexpr int GEMM_THREADS = 192;
-constexpr int CSUM_THREADS = 320;          // + four column-sum warps
+constexpr int GEMM_THREADS = 320;          // TMA, MMA and eight epilogue warps (or four and four column-sum warps)
 
 // PAIR: two CTAs of a cluster form one 256 x BN tile (tcgen05 cta_group::2).  Each CTA stages its
 // own 128 rows of A and its own half of B, so a pair moves and re-reads 2/3 of the shared-memory
@@ -270,7 +269,7 @@ template <int BN, bool PAIR = false> struct GemmCfg {
 };
 
 template <int BN, bool PAIR>
-__global__ void __launch_bounds__(CSUM_THREADS, 1)
+__global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b, const GemmParams p) {
   using Cfg = GemmCfg<BN, PAIR>;
   constexpr int TM = PAIR ? 2 * BM : BM;                       // rows of one scheduled tile
@@ -301,7 +300,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ C
       mbar_init(bar_full + 8 * s, 1); mbar_init(bar_empty + 8 * s, 1); mbar_init(bar_free + 8 * s, 4);
     }
     // accumulator-free barrier: one arrival per epilogue warp of every CTA that reads the accumulator
-    for (int a = 0; a < 2; a++) { mbar_init(bar_tfull + 8 * a, 1); mbar_init(bar_tempty + 8 * a, PAIR ? 8 : 4); }
+    for (int a = 0; a < 2; a++) { mbar_init(bar_tfull + 8 * a, 1); mbar_init(bar_tempty + 8 * a, (PAIR ? 2 : 1) * (csum ? 4 : 8)); }
     *abort_flag = 0;
     mbar_fence_init();
   }
@@ -404,9 +403,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ C
         if (ok) { if (PAIR) umma_commit_pair(bar_tfull + 8 * acc, 3); else umma_commit(bar_tfull + 8 * acc); }
       }
     }
-  } else if (warp >= 6) {
+  } else if (csum && warp >= 6) {
     // ------------------------------------------------------------------ column sums of A (bias gradient)
-    // Present only in launches with CSUM_THREADS.  A stage is read after the MMAs that consume it
+    // Present only in launches with column sums.  A stage is read after the MMAs that consume it
     // have retired (its "empty" barrier, which also reaches the second CTA of a pair) and before the
     // producer may refill it (the "free" barrier).  Warp cw owns columns [32 cw, 32 cw + 32) of the
     // 128-column A tile: four 16-byte chunks of one 64-column slab.  Lane = 8 p + 4 h + c4 reads
@@ -464,7 +463,11 @@ gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ C
     }
   } else {
     // ------------------------------------------------------------------ epilogue warps
+    // Eight warps, two per TMEM quadrant, each with half of the tile's columns (four with all columns where the other four
+    // form column sums).  With four warps the epilogue of a 256-wide tile outlasts a main loop of K = 512 and bounds the
+    // products of narrow models.
     const int q = warp & 3;                    // TMEM lane quadrant this warp may access
+    const int col_lo = (!csum && warp >= 6) ? BN / 2 : 0, col_hi = (!csum && warp < 6) ? BN / 2 : BN;
     int tcount = 0;
     bool ok = true;
     for (int t = worker; ok && t < num_tiles; t += n_workers, tcount++) {
@@ -481,7 +484,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ C
       uint4 nb[4], nx[4];
       auto fetch = [&](int c0) {
         const int col = tn * BN + c0;
-        if (c0 >= BN || col + 32 > p.N) return;
+        if (c0 >= col_hi || col + 32 > p.N) return;
         if (use_bias) {
           const uint4* bp = reinterpret_cast<const uint4*>(p.bias + col);
 #pragma unroll
@@ -495,15 +498,15 @@ gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ C
       };
       if (use_aux && row_ok) {
         const char* ap = reinterpret_cast<const char*>(p.aux + (size_t)row * p.ldaux + tn * BN);
-        const int nbytes = min(BN, p.N - tn * BN) * 2;
-        for (int b = 128; b < nbytes; b += 128) prefetch_l2(ap + b);
+        const int nbytes = min(col_hi, p.N - tn * BN) * 2;
+        for (int b = col_lo * 2 + 128; b < nbytes; b += 128) prefetch_l2(ap + b);
       }
-      fetch(0);
+      fetch(col_lo);
       if (!mbar_wait(bar_tfull + 8 * acc, aph, abort_flag, 3, p.err)) { ok = false; break; }
       tc_fence_after();
       const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + acc * BN;
 #pragma unroll 1
-      for (int c0 = 0; c0 < BN; c0 += 32) {
+      for (int c0 = col_lo; c0 < col_hi; c0 += 32) {
         const int col = tn * BN + c0;
         if (col >= p.N) break;                 // uniform across the warp
         uint32_t r[32];
@@ -622,6 +625,226 @@ gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ C
   }
 }
 
+// ------------------------------------------------------------------------------- split-K kernel
+// Products whose output has too few tiles for the chip and whose K is long (weight gradients of narrow layers: K is the number
+// of tokens; input gradients and forward products of few rows): a k-block costs a CTA 0.4-0.5 us whatever its tile width (the
+// chain TMA -> tcgen05.mma -> release), so one CTA per tile takes K / 64 of them one after the other while most SMs idle.
+// Here the 2, 4 or 8 CTAs of a cluster share one 128 x BN tile: CTA r multiplies the r-th slice of K, leaves its fp32
+// partial tile in its own shared memory (the operand stages are free by then), and after a cluster barrier every CTA adds
+// its 128 / split rows over the CTAs in rank order through distributed shared memory and runs the epilogue on them.  No
+// workspace and no atomics; the order of the additions is fixed, so results are reproducible.
+// Measured (dW with column sums, K = 9216): 512 x 512 62.2 -> 21.1 us, 1536 x 512 63.6 -> 37.3, 256 x 512 62.1 -> 14.9;
+// K = 4096: 1024 x 256 30.2 -> 15.6; forward 128 x 1024 x 4096: 27.9 -> 13.8.
+__device__ __forceinline__ float4 ld_cluster_v4(uint32_t a) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a));
+  return v;
+}
+__device__ __forceinline__ uint32_t ld_cluster_u32(uint32_t a) {
+  uint32_t v;
+  asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(a));
+  return v;
+}
+// Epilogue of four adjacent columns (col % 4 == 0) of one row; the arithmetic and rounding points of gemm_kernel.
+__device__ __forceinline__ void epilogue4(const GemmParams& p, int row, int col, float (&v)[4]) {
+  const int n = min(4, p.N - col);
+  const bool use_bias = (p.epi == EPI_BIAS || p.epi == EPI_BIAS_GELU || p.epi == EPI_BIAS_RESID);
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    v[i] *= p.alpha;
+    if (use_bias && i < n) v[i] += __bfloat162float(p.bias[col + i]);
+  }
+  if (p.epi == EPI_BIAS_GELU) {
+    bf16* ap = p.aux + (size_t)row * p.ldaux + col;
+    if (n == 4) *reinterpret_cast<uint2*>(ap) = make_uint2(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]));
+    else for (int i = 0; i < n; i++) ap[i] = __float2bfloat16(v[i]);
+#pragma unroll
+    for (int i = 0; i < 4; i++) v[i] = gelu_tanh(__bfloat162float(__float2bfloat16(v[i])));
+  } else if (p.epi == EPI_BIAS_RESID || p.epi == EPI_RESID || p.epi == EPI_DGELU) {
+    const bf16* ap = p.aux + (size_t)row * p.ldaux + col;
+    float x[4] = {0.f, 0.f, 0.f, 0.f};
+    if (n == 4) {
+      const uint2 u = *reinterpret_cast<const uint2*>(ap);
+      const float2 a = unpack_bf16(u.x), b = unpack_bf16(u.y);
+      x[0] = a.x; x[1] = a.y; x[2] = b.x; x[3] = b.y;
+    } else for (int i = 0; i < n; i++) x[i] = __bfloat162float(ap[i]);
+#pragma unroll
+    for (int i = 0; i < 4; i++) v[i] = p.epi == EPI_DGELU ? v[i] * gelu_tanh_grad(x[i]) : v[i] + x[i];
+  }
+  if (p.out_fp32) {
+    float* cp = reinterpret_cast<float*>(p.C) + (size_t)row * p.ldc + col;
+    if (n == 4) {
+      if (p.accumulate) red_add_v4_f32(cp, v[0], v[1], v[2], v[3]);
+      else *reinterpret_cast<float4*>(cp) = make_float4(v[0], v[1], v[2], v[3]);
+    } else for (int i = 0; i < n; i++) cp[i] = p.accumulate ? cp[i] + v[i] : v[i];
+  } else {
+    bf16* cp = reinterpret_cast<bf16*>(p.C) + (size_t)row * p.ldc + col;
+    if (n == 4) *reinterpret_cast<uint2*>(cp) = make_uint2(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]));
+    else for (int i = 0; i < n; i++) cp[i] = __float2bfloat16(v[i]);
+  }
+}
+
+template <int BN>
+__global__ void __launch_bounds__(GEMM_THREADS, 1)
+gemm_splitk_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b, const GemmParams p,
+                   int split) {
+  using Cfg = GemmCfg<BN>;
+  constexpr int PITCH = BN + 4;                      // floats per row of the partial tile: conflict-free 16-byte rows
+  static_assert((BM * PITCH + BM) * 4 <= Cfg::STAGES * Cfg::STAGE_BYTES, "the partial tile reuses the operand stages");
+  const uint32_t rank = cluster_ctarank();
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+  uint8_t* smem_al = smem_raw + (smem_base - smem_u32(smem_raw));
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem_al + Cfg::STAGES * Cfg::STAGE_BYTES);
+  const uint32_t bar_full = smem_u32(bars), bar_empty = bar_full + 8 * Cfg::STAGES, bar_free = bar_empty + 8 * Cfg::STAGES,
+                 bar_tfull = bar_free + 8 * Cfg::STAGES;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 3 * Cfg::STAGES + 1);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  const bool csum = p.colsum != nullptr;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tiles_m = (p.M + BM - 1) / BM, tile = (int)blockIdx.x / split;
+  const int m0 = (tile % tiles_m) * BM, tn = tile / tiles_m, n0 = tn * BN;
+  const int num_kb = (p.K + BK - 1) / BK, per = (num_kb + split - 1) / split;
+  const int kb0 = min(num_kb, (int)rank * per), nkb = min(num_kb, kb0 + per) - kb0;       // the launcher leaves no slice empty
+
+  if (tid == 0) {
+    for (int s = 0; s < Cfg::STAGES; s++) { mbar_init(bar_full + 8 * s, 1); mbar_init(bar_empty + 8 * s, 1); mbar_init(bar_free + 8 * s, 4); }
+    mbar_init(bar_tfull, 1);
+    *abort_flag = 0;
+    mbar_fence_init();
+    tma_prefetch_desc(&tma_a);
+    tma_prefetch_desc(&tma_b);
+  }
+  if (warp == 1) { tmem_alloc(smem_u32(tmem_slot), BN); tmem_relinquish(); }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *tmem_slot;
+  pdl_wait();
+  pdl_launch_dependents();
+
+  bool ok = true;
+  float cs[8];
+#pragma unroll
+  for (int j = 0; j < 8; j++) cs[j] = 0.f;
+  if (warp == 0) {
+    if (lane == 0) {
+      for (int i = 0; i < nkb; i++) {
+        const int s = i % Cfg::STAGES, kb = kb0 + i;
+        const uint32_t ph = (i / Cfg::STAGES) & 1;
+        if (!mbar_wait(bar_empty + 8 * s, ph ^ 1, abort_flag, 2, p.err)) break;
+        if (csum && !mbar_wait(bar_free + 8 * s, ph ^ 1, abort_flag, 2, p.err)) break;
+        const uint32_t sa = smem_base + s * Cfg::STAGE_BYTES, sb = sa + Cfg::A_BYTES;
+        mbar_expect_tx(bar_full + 8 * s, Cfg::STAGE_BYTES);
+        if (!p.a_mn) tma_load_2d(sa, &tma_a, bar_full + 8 * s, kb * BK, m0);
+        else
+          for (int j = 0; j < BM / 64; j++) tma_load_2d(sa + j * (BK * 128), &tma_a, bar_full + 8 * s, m0 + j * 64, kb * BK);
+        if (!p.b_mn) tma_load_2d(sb, &tma_b, bar_full + 8 * s, kb * BK, n0);
+        else
+          for (int j = 0; j < BN / 64; j++) tma_load_2d(sb + j * (BK * 128), &tma_b, bar_full + 8 * s, n0 + j * 64, kb * BK);
+      }
+    }
+  } else if (warp == 1) {
+    if (lane == 0) {
+      const uint32_t idesc = umma_idesc_bf16(BM, BN, p.a_mn, p.b_mn);
+      const uint32_t a_lbo = p.a_mn ? BK * 128 : 16, b_lbo = p.b_mn ? BK * 128 : 16;
+      const uint32_t a_kstep = p.a_mn ? (UMMA_K * 128) >> 4 : (UMMA_K * 2) >> 4;
+      const uint32_t b_kstep = p.b_mn ? (UMMA_K * 128) >> 4 : (UMMA_K * 2) >> 4;
+      for (int i = 0; ok && i < nkb; i++) {
+        const int s = i % Cfg::STAGES;
+        if (!mbar_wait(bar_full + 8 * s, (i / Cfg::STAGES) & 1, abort_flag, 1, p.err)) { ok = false; break; }
+        tc_fence_after();
+        const uint32_t sa = smem_base + s * Cfg::STAGE_BYTES, sb = sa + Cfg::A_BYTES;
+        const uint64_t adesc = umma_desc_sw128(sa, a_lbo, 1024), bdesc = umma_desc_sw128(sb, b_lbo, 1024);
+#pragma unroll
+        for (int k = 0; k < BK / UMMA_K; k++)
+          umma_f16_ss(tmem, adesc + (uint64_t)(k * a_kstep), bdesc + (uint64_t)(k * b_kstep), idesc, (i > 0 || k > 0) ? 1u : 0u);
+        umma_commit(bar_empty + 8 * s);
+      }
+      if (ok) umma_commit(bar_tfull);
+    }
+  } else if (csum && warp >= 6) {
+    // column sums of this CTA's A tiles, see gemm_kernel
+    const int cw = warp - 6;
+    const int c4 = lane & 3, rsel = ((lane >> 3) & 3) + 4 * ((lane >> 2) & 1), chunk = (cw & 1) * 4 + c4;
+    for (int i = 0; i < nkb; i++) {
+      const int s = i % Cfg::STAGES;
+      if (!mbar_wait(bar_empty + 8 * s, (i / Cfg::STAGES) & 1, abort_flag, 2, p.err)) break;
+      if (tn == 0) {
+        const uint32_t sa = smem_base + s * Cfg::STAGE_BYTES + (uint32_t)(cw >> 1) * (BK * 128);
+#pragma unroll
+        for (int q = 0; q < 8; q++) {
+          const int r = 8 * q + rsel;
+          uint4 v;
+          asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
+                       : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+                       : "r"(sa + (uint32_t)r * 128u + (uint32_t)((chunk ^ (r & 7)) << 4)));
+          const float2 f0 = unpack_bf16(v.x), f1 = unpack_bf16(v.y), f2 = unpack_bf16(v.z), f3 = unpack_bf16(v.w);
+          cs[0] += f0.x; cs[1] += f0.y; cs[2] += f1.x; cs[3] += f1.y;
+          cs[4] += f2.x; cs[5] += f2.y; cs[6] += f3.x; cs[7] += f3.y;
+        }
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar_free + 8 * s);
+    }
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+      cs[j] += __shfl_xor_sync(0xffffffffu, cs[j], 4);
+      cs[j] += __shfl_xor_sync(0xffffffffu, cs[j], 8);
+      cs[j] += __shfl_xor_sync(0xffffffffu, cs[j], 16);
+    }
+  }
+  __syncwarp();
+  if (warp >= 2 && warp < 6) mbar_wait(bar_tfull, 0, abort_flag, 3, p.err);
+  tc_fence_after();
+  __syncthreads();                   // every MMA has retired and the column-sum warps are done: the stages are free
+  const uint32_t tile_smem = smem_base, csum_smem = smem_base + BM * PITCH * 4;
+  if (warp >= 2 && warp < 6) {
+    const int q = warp & 3, row = q * 32 + lane;
+#pragma unroll 1
+    for (int c = 0; c < BN; c += 32) {
+      uint32_t r[32];
+      tmem_ld32(tmem + ((uint32_t)(q * 32) << 16) + c, r);
+      tmem_ld_wait();
+#pragma unroll
+      for (int j = 0; j < 8; j++)
+        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(tile_smem + (uint32_t)(row * PITCH + c + 4 * j) * 4u),
+                     "r"(r[4 * j]), "r"(r[4 * j + 1]), "r"(r[4 * j + 2]), "r"(r[4 * j + 3]) : "memory");
+    }
+  } else if (csum && warp >= 6 && lane < 4) {
+#pragma unroll
+    for (int j = 0; j < 8; j++)
+      asm volatile("st.shared.f32 [%0], %1;" ::"r"(csum_smem + (uint32_t)((warp - 6) * 32 + lane * 8 + j) * 4u), "f"(cs[j]) : "memory");
+  }
+  tc_fence_before();
+  cluster_sync_all();
+  bool all_ok = true;
+  for (int s = 0; s < split; s++) all_ok = all_ok && ld_cluster_u32(mapa_shared(smem_u32((const void*)abort_flag), s)) == 0;
+  if (all_ok) {
+    const int rows = BM / split;
+    for (int i = tid; i < rows * (BN / 4); i += blockDim.x) {
+      const int r = (int)rank * rows + i / (BN / 4), c = (i % (BN / 4)) * 4;
+      if (m0 + r >= p.M || n0 + c >= p.N) continue;
+      const uint32_t at = tile_smem + (uint32_t)(r * PITCH + c) * 4u;
+      float v[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
+      for (int s = 0; s < split; s++) {
+        const float4 f = ld_cluster_v4(mapa_shared(at, s));
+        v[0] += f.x; v[1] += f.y; v[2] += f.z; v[3] += f.w;
+      }
+      epilogue4(p, m0 + r, n0 + c, v);
+    }
+    if (csum && tn == 0 && tid < rows) {
+      const int r = (int)rank * rows + tid;
+      float v = 0.f;
+      for (int s = 0; s < split; s++) v += __uint_as_float(ld_cluster_u32(mapa_shared(csum_smem + (uint32_t)r * 4u, s)));
+      if (m0 + r < p.M) p.colsum[m0 + r] = p.accumulate ? p.colsum[m0 + r] + v : v;
+    }
+  }
+  cluster_sync_all();                // no CTA leaves while another reads its partial tile
+  if (warp == 1) { tc_fence_after(); tmem_dealloc(tmem, BN); }
+}
+
 // ------------------------------------------------------------------------------- launcher
 static int g_num_sms = 0;
 static int num_sms() {
@@ -645,7 +868,7 @@ static int launch_gemm_pair(const CUtensorMap* ta, const CUtensorMap* tb, const 
   attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[1].val.programmaticStreamSerializationAllowed = 1;
-  cfg.blockDim = dim3(p.colsum ? CSUM_THREADS : GEMM_THREADS); cfg.dynamicSmemBytes = Cfg::SMEM; cfg.stream = st; cfg.attrs = attr;
+  cfg.blockDim = dim3(GEMM_THREADS); cfg.dynamicSmemBytes = Cfg::SMEM; cfg.stream = st; cfg.attrs = attr;
   cfg.numAttrs = kh_pdl_enabled() ? 2 : 1;
   if (g_pair_clusters < 0) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM);
@@ -679,14 +902,68 @@ static int launch_gemm(const CUtensorMap* ta, const CUtensorMap* tb, const GemmP
   const int tiles = ((p.M + BM - 1) / BM) * ((p.N + BN - 1) / BN);
   int grid = tiles < num_sms() ? tiles : num_sms();
   if (max_ctas > 0 && grid > max_ctas) grid = max_ctas;
-  cudaError_t e = KH_LAUNCH((gemm_kernel<BN, false>), grid, p.colsum ? CSUM_THREADS : GEMM_THREADS, Cfg::SMEM, st, *ta, *tb, p);
+  cudaError_t e = KH_LAUNCH((gemm_kernel<BN, false>), grid, GEMM_THREADS, Cfg::SMEM, st, *ta, *tb, p);
   if (e != cudaSuccess) { kh_set_error("gemm launch failed: %s", cudaGetErrorString(e)); return -1; }
   return 0;
 }
 
+// Clusters of `split` CTAs that can be resident together (0: not available).
+template <int BN>
+static int splitk_clusters(int split) {
+  static int known[3] = {-1, -1, -1};
+  int& n = known[split == 2 ? 0 : (split == 4 ? 1 : 2)];
+  if (n >= 0) return n;
+  auto kern = gemm_splitk_kernel<BN>;
+  int got = 0;
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, GemmCfg<BN>::SMEM) == cudaSuccess) {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = split; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    cfg.gridDim = dim3(split * (num_sms() / split)); cfg.blockDim = dim3(GEMM_THREADS); cfg.dynamicSmemBytes = GemmCfg<BN>::SMEM;
+    cfg.attrs = attr; cfg.numAttrs = 1;
+    if (cudaOccupancyMaxActiveClusters(&got, kern, &cfg) != cudaSuccess) got = 0;
+  }
+  cudaGetLastError();
+  return n = got;
+}
+template <int BN>
+static int launch_splitk(const CUtensorMap* ta, const CUtensorMap* tb, const GemmParams& p, int split, cudaStream_t st) {
+  if (splitk_clusters<BN>(split) < 1) { kh_set_error("gemm: clusters of %d CTAs are not available", split); return -1; }
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = split; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.gridDim = dim3(((p.M + BM - 1) / BM) * ((p.N + BN - 1) / BN) * split);
+  cfg.blockDim = dim3(GEMM_THREADS); cfg.dynamicSmemBytes = GemmCfg<BN>::SMEM; cfg.stream = st;
+  cfg.attrs = attr; cfg.numAttrs = kh_pdl_enabled() ? 2 : 1;
+  cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_splitk_kernel<BN>, *ta, *tb, p, split);
+  if (e != cudaSuccess) { kh_set_error("gemm split-K launch failed: %s", cudaGetErrorString(e)); return -1; }
+  return 0;
+}
+// Tile width and split for a product that would take `chain` k-blocks one after the other on one CTA (0: no split).
+// A split pays when the shortened chain saves more than the hand-off costs (SPLIT_COST k-blocks: 8 CTAs of 8 k-blocks take as
+// long as one of 16 to 18); only splits whose tiles are all resident at once are taken (a second wave of clusters costs more
+// than it saves: 1024 x 256 x 4096 in 4 x 64 12.2 us, in 8 x 64 25.7).
+static int pick_splitk(int M, int N, int num_kb, int chain, int* bn_out) {
+  constexpr int SPLIT_COST = 8;
+  const int tm = (M + BM - 1) / BM;
+  int best = chain * 4 / 5, pick = 0;
+  for (int bn = 128; bn >= 64; bn >>= 1)
+    for (int split = 2; split <= 8; split <<= 1) {
+      const int per = (num_kb + split - 1) / split, tiles = tm * ((N + bn - 1) / bn);
+      if ((split - 1) * per >= num_kb || tiles * split > num_sms() || per + SPLIT_COST >= best) continue;
+      if (tiles > (bn == 128 ? splitk_clusters<128>(split) : splitk_clusters<64>(split))) continue;
+      best = per + SPLIT_COST; pick = split; *bn_out = bn;
+    }
+  return pick;
+}
+
 // C[M,N] = alpha * op(A) op(B) with a fused epilogue.  lda/ldb/ldc/ldaux are row pitches in
 // elements of the row-major buffers described at the top of this file.  block_n = 0 lets the
-// launcher pick the tile width; max_ctas > 0 caps the grid (used to leave SMs to a
+// launcher pick the tile width (or a split of K over a cluster; 4096 * split + width asks for one); max_ctas > 0 caps the grid (used to leave SMs to a
 // concurrently running communication kernel).  Returns 0 or -1 (see kh_cuda_last_error).
 //
 // kh_gemm_bf16_colsum: same product with `colsum` [M] fp32 receiving colsum[m] (+)= sum_k op(A)[m, k]
@@ -702,7 +979,12 @@ extern "C" int kh_gemm_bf16_colsum(const void* A, int lda, int a_mn, const void*
   if ((ldc % (out_fp32 ? 4 : 8)) != 0 || ((uintptr_t)C & 15)) { kh_set_error("gemm: output pitch/base not 16-byte aligned (ldc %d)", ldc); return -1; }
   if ((epi == EPI_BIAS || epi == EPI_BIAS_GELU || epi == EPI_BIAS_RESID) && (!bias || ((uintptr_t)bias & 15))) { kh_set_error("gemm: bias missing or misaligned"); return -1; }
   if ((epi == EPI_BIAS_GELU || epi == EPI_BIAS_RESID || epi == EPI_DGELU || epi == EPI_RESID) && (!aux || (ldaux % 8) || ((uintptr_t)aux & 15))) { kh_set_error("gemm: aux operand missing or misaligned"); return -1; }
-  int bn = block_n;
+  int bn = block_n & 4095, split = block_n >> 12;
+  if (split && ((split != 2 && split != 4 && split != 8) || (bn != 64 && bn != 128) ||
+                (split - 1) * (((K + BK - 1) / BK + split - 1) / split) >= (K + BK - 1) / BK)) {
+    kh_set_error("gemm: K split %d with tile width %d is not supported for K = %d", split, bn, K);
+    return -1;
+  }
   if (bn == 0) {
     // waves x relative tile time; narrower tiles reuse the A panel less and run at lower efficiency
     const int tm = (M + BM - 1) / BM, sms = num_sms();
@@ -722,8 +1004,13 @@ extern "C" int kh_gemm_bf16_colsum(const void* A, int lda, int a_mn, const void*
       const float cpair = (float)((tiles2 + clusters - 1) / clusters) * 0.93f;
       if (cpair <= best) bn = 512;
     }
+    if (max_ctas == 0) {
+      const int num_kb = (K + BK - 1) / BK, workers = bn == 512 ? sms / 2 : sms;
+      const int tiles = bn == 512 ? ((M + 255) / 256) * ((N + 255) / 256) : tm * ((N + bn - 1) / bn);
+      split = pick_splitk(M, N, num_kb, (tiles + workers - 1) / workers * num_kb, &bn);
+    }
   }
-  const bool pair = (bn == 512);      // 256 x 256 tiles on CTA pairs (cta_group::2)
+  const bool pair = (bn == 512 && !split);      // 256 x 256 tiles on CTA pairs (cta_group::2)
   if (pair) bn = 256;
   if (bn != 64 && bn != 128 && bn != 256) { kh_set_error("gemm: block_n must be 64, 128, 256 or 512 (CTA pairs)"); return -1; }
   const CUtensorMap* ta = a_mn ? kh_tmap_2d_bf16(A, K, M, lda, BK, 64) : kh_tmap_2d_bf16(A, M, K, lda, BM, BK);
@@ -736,6 +1023,7 @@ extern "C" int kh_gemm_bf16_colsum(const void* A, int lda, int a_mn, const void*
   p.colsum = (float*)colsum;
   p.err = kh_error_word_dev();
   cudaStream_t st = (cudaStream_t)stream;
+  if (split) return bn == 128 ? launch_splitk<128>(ta, tb, p, split, st) : launch_splitk<64>(ta, tb, p, split, st);
   if (pair) return launch_gemm_pair(ta, tb, p, max_ctas, st);
   if (bn == 256) return launch_gemm<256>(ta, tb, p, max_ctas, st);
   if (bn == 128) return launch_gemm<128>(ta, tb, p, max_ctas, st);

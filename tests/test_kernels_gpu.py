@@ -94,6 +94,52 @@ def test_gemm_weight_gradient_with_bias_gradient(M, N, K, bn):
     assert torch.equal(db2, db3) and relerr(db2, dy.float().sum(0)) < 1e-5
 
 
+@pytest.mark.parametrize("bn", [64, 128])
+@pytest.mark.parametrize("split", [2, 4, 8])
+@pytest.mark.parametrize("M,N,K", [(128, 64, 512), (200, 72, 1000), (8, 136, 4104), (513, 257, 1032), (256, 512, 9216)])
+def test_gemm_split_over_a_cluster(M, N, K, split, bn):
+    """K split over the CTAs of a cluster: whole and ragged tiles, K remainders, slices of unequal length, with every
+    epilogue.  fp32 sums of K products in another order differ by at most K * 2^-24 of the sum of magnitudes, which for
+    normal operands is about sqrt(K) times the result: 1e-5 and 2e-4 leave a factor of ten; bf16 outputs round at 2^-9."""
+    torch.manual_seed(M + N + K)
+    pad = lambda n: (n + 7) // 8 * 8
+    r = lambda *s: torch.randn(*s, device="cuda").bfloat16()
+    blk = 4096 * split + bn
+    dy, x = r(K, pad(M))[:, :M], r(K, pad(N))[:, :N]
+    want = dy.double().t() @ x.double()
+    dw = torch.ones(M, pad(N), device="cuda")[:, :N]
+    db = torch.ones(M, device="cuda")
+    ops.gemm(dy, x, dw, a_mn=True, b_mn=True, accumulate=True, colsum=db, block_n=blk)
+    assert ((dw - 1 - want).norm() / want.norm()).item() < 1e-5
+    cs = dy.double().sum(0)
+    assert ((db - 1 - cs).norm() / cs.norm()).item() < 2e-4
+    again = torch.ones_like(dw)
+    ops.gemm(dy, x, again, a_mn=True, b_mn=True, accumulate=True, block_n=blk)
+    assert torch.equal(again, dw)
+    a, w = r(M, pad(K))[:, :K], r(N, pad(K))[:, :K]
+    bias, aux = r(pad(N))[:N], r(M, pad(N))[:, :N]
+    acc = a.double() @ w.double().t()
+    for epi in (ops.EPI_NONE, ops.EPI_BIAS, ops.EPI_BIAS_GELU, ops.EPI_BIAS_RESID, ops.EPI_DGELU, ops.EPI_RESID):
+        out = torch.full((M, pad(N)), 7.0, device="cuda").bfloat16()
+        ax = aux.clone() if epi != ops.EPI_BIAS_GELU else torch.empty(M, pad(N), device="cuda", dtype=torch.bfloat16)[:, :N]
+        if epi == ops.EPI_NONE or epi == ops.EPI_BIAS:
+            ax = None
+        elif epi != ops.EPI_BIAS_GELU:
+            ax = torch.zeros(M, pad(N), device="cuda", dtype=torch.bfloat16)[:, :N].copy_(aux)
+        ops.gemm(a, w, out[:, :N], epi=epi, bias=bias if epi in (ops.EPI_BIAS, ops.EPI_BIAS_GELU, ops.EPI_BIAS_RESID) else None,
+                 aux=ax, block_n=blk)
+        one = torch.full((M, pad(N)), 7.0, device="cuda").bfloat16()
+        ax1 = None if ax is None else torch.zeros(M, pad(N), device="cuda", dtype=torch.bfloat16)[:, :N].copy_(aux)
+        ops.gemm(a, w, one[:, :N], epi=epi, bias=bias if epi in (ops.EPI_BIAS, ops.EPI_BIAS_GELU, ops.EPI_BIAS_RESID) else None,
+                 aux=ax1, block_n=bn)
+        err = ((out[:, :N].double() - one[:, :N].double()).norm() / one[:, :N].double().norm()).item()
+        assert err < 2.0 ** -8, (epi, err)
+        assert torch.equal(out[:, N:], one[:, N:])
+        if epi == ops.EPI_NONE:
+            assert ((out[:, :N].double() - acc).norm() / acc.norm()).item() < 2.0 ** -8
+    assert ops.error_word() == 0
+
+
 @pytest.mark.parametrize("ta,tb", [(False, False), (True, False), (False, True), (True, True)])
 def test_gemm_f32_oracle_kernel(ta, tb):
     torch.manual_seed(13)
