@@ -89,19 +89,19 @@ class InferEngine:
             self.skinny = torch.zeros(n, dtype=torch.float32, **z)
         # Decode steps of up to ``persistent_max`` sequences run all layers and the head in one persistent kernel
         # when the shape allows it (ops.decode_layers); KHARON_PERSISTENT_DECODE=0 or persistent_decode=False keeps
-        # the five-kernel chain.  Measured on B200 (L24 d1024): 945 / 6407 / 9614 tok/s against 728 / 4201 / 7301 at
-        # G = 1 / 8 / 16; at G = 32 the chain's 128-row tensor-core tiles win (15.9k against 13.3k), hence 16.
+        # the five-kernel chain.  Measured on B200, us a step (L24 d1024, context 160-200): 507 / 565 / 764 / 1096 / 1217 at
+        # G = 1 / 8 / 16 / 24 / 32 against 1255 / 1776 / 2029 / 1824 / 1851 for the chain.
         if persistent_decode is None:
             persistent_decode = os.environ.get("KHARON_PERSISTENT_DECODE", "1") != "0"
         self.persistent = bool(persistent_decode and self.skinny is not None and self.tp == 1 and self.dt == torch.bfloat16
                                and ops.decode_layers_ok(1, d, cfg.n_head, cfg.head_dim, cfg.seq))
-        self.persistent_max = int(os.environ.get("KHARON_PERSISTENT_MAX_G", "16"))
+        self.persistent_max = int(os.environ.get("KHARON_PERSISTENT_MAX_G", "32"))
         if self.persistent:
             names = ("ln1_w", "ln1_b", "qkv_w", "qkv_b", "proj_w", "proj_b", "ln2_w", "ln2_b", "fc_w", "fc_b",
                      "fcproj_w", "fcproj_b")
             self.layer_table = torch.tensor([[model.L(l, n).data_ptr() for n in names] for l in range(L)],
                                             dtype=torch.int64, device=self.dev)
-            self.grid_bar = torch.zeros(4, dtype=torch.int32, **z)
+            self.decode_work = ops.decode_layers_work(d, self.dev)
         # Contexts beyond 2048 positions: the keys of a token are cut into ranges with a CTA each (split-KV) and merged
         self.attn_splits = int(attn_splits) if attn_splits else (1 if cfg.seq <= 2048 else min(16, (cfg.seq + 2047) // 2048))
         self.attn_scratch = None
@@ -156,7 +156,7 @@ class InferEngine:
         if fused_layers:      # layers and head in one kernel; only the sampler follows
             ops.decode_layers(xs, self.xmid[:ntok], self.qkv[:ntok], self.att[:ntok], self.act[:ntok], self.layer_table,
                               cfg.n_layer, self.Hl, self.hd, self.kc, self.vc, pos, slot, self.d_btab, self.bs, cfg.seq,
-                              self.grid_bar, head_w=m.head_weight(), lnf_w=P["lnf_w"], lnf_b=P["lnf_b"], logits=self.logits,
+                              work=self.decode_work, head_w=m.head_weight(), lnf_w=P["lnf_w"], lnf_b=P["lnf_b"], logits=self.logits,
                               vocab=cfg.vocab, rows=self.d_rows, n_rows=nseq)
             ops.sample(self.logits, cfg.vocab, self.temperature, self.seed, self.step_no, rep, self.d_out, nseq,
                        step_dev=self.d_stepno)

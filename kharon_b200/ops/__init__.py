@@ -195,19 +195,27 @@ def decode_layers_ok(G, d, H, hd, max_ctx):
     return bool(torch.cuda.is_available() and _lib().kh_decode_layers_ok(G, d, H, hd, max_ctx))
 
 
-def decode_layers(x, xmid, qkv, att, act, layers, n_layer, H, hd, kc, vc, pos, slot, btab, bs, max_ctx, bar, *,
-                  head_w=None, lnf_w=None, lnf_b=None, logits=None, vocab=0, rows=None, n_rows=0):
+def decode_layers_work(d, device):
+    """Workspace of ``decode_layers`` for models of width ``d``: the activations travel through it between the kernel's
+    thread blocks.  Zeroed once; its launches must follow one another (one workspace per engine and stream)."""
+    return torch.zeros((int(_lib().kh_decode_layers_work_bytes(d)) + 7) // 8, dtype=torch.int64, device=device)
+
+
+def decode_layers(x, xmid, qkv, att, act, layers, n_layer, H, hd, kc, vc, pos, slot, btab, bs, max_ctx, bar=None, *,
+                  head_w=None, lnf_w=None, lnf_b=None, logits=None, vocab=0, rows=None, n_rows=0, work=None):
     """All transformer layers of one decode step (one new token per sequence) in one persistent kernel:
     ``x [G, d]`` holds the embedded tokens on entry and the last layer's output on return; k and v of the
     new tokens are appended to the paged cache ``kc``, ``vc`` ``[L, blocks, bs, H, hd]``.  ``layers`` is the
-    int64 device table of twelve bf16 pointers per layer, ``bar`` four zeroed int32 words.  With ``head_w``
+    int64 device table of twelve bf16 pointers per layer, ``work`` the kernel's workspace (``decode_layers_work``; a
+    fresh one when absent).  ``xmid``, ``qkv``, ``att``, ``act`` and ``bar`` are not used.  With ``head_w``
     the kernel also writes ``logits[i, :vocab] = LayerNorm_f(x[rows[i]]) @ head_w^T`` for ``i < n_rows``."""
     G, d = x.shape
-    _call(_lib().kh_decode_layers, 1, x.data_ptr(), xmid.data_ptr(), qkv.data_ptr(), att.data_ptr(), act.data_ptr(),
-          layers.data_ptr(), n_layer, G, d, H, hd, kc.data_ptr(), vc.data_ptr(), kc.stride(0), pos.data_ptr(),
-          slot.data_ptr(), btab.data_ptr(), btab.shape[1], bs, max_ctx, 1.0 / float(hd) ** 0.5,
+    if work is None:
+        work = decode_layers_work(d, x.device)
+    _call(_lib().kh_decode_layers, 1, x.data_ptr(), layers.data_ptr(), n_layer, G, d, H, hd, kc.data_ptr(), vc.data_ptr(),
+          kc.stride(0), pos.data_ptr(), slot.data_ptr(), btab.data_ptr(), btab.shape[1], bs, max_ctx, 1.0 / float(hd) ** 0.5,
           _p(head_w), _p(lnf_w), _p(lnf_b), _p(logits), logits.stride(0) if logits is not None else 0, vocab,
-          _p(rows), n_rows, bar.data_ptr(), _stream())
+          _p(rows), n_rows, work.data_ptr(), _stream())
 
 
 def gemm_skinny_scratch_elems(M, N, K):

@@ -222,6 +222,33 @@ def test_persistent_decode_kernel_matches_the_kernel_chain(d, heads, groups):
     assert ops.error_word() == 0
 
 
+@pytest.mark.parametrize("d,heads,G,ctx", [(256, 8, 1, 9), (256, 4, 32, 40), (512, 16, 2, 300), (768, 12, 6, 70), (1024, 8, 16, 150),
+                                           (2048, 16, 31, 33), (4096, 32, 17, 20)])
+def test_persistent_decode_steps_against_the_chain(d, heads, G, ctx):
+    """Single decode steps at the kernel's edges: one warp step per slice (d = 256), head widths 32 / 64 / 128, one to four
+    row groups, several turns of a phase, contexts of more than four keys per lane group, rows that need two launches
+    (d = 2048, 4096).  Same inputs, same rounding points, so the logits differ as two summation orders of bf16 layers do (the
+    bound of the test above); the appended keys and values of layer 0 only pass one product and agree to a bf16 step."""
+    cfg = Config(2, d, heads, 601, 512, 1)
+    m = GPT(cfg, "cuda", torch.bfloat16)
+    m.init_weights_device(5)
+    m.params.w.mul_(3.0); m.sync_bf16()
+    gen = torch.Generator().manual_seed(d + G)
+    prompts = [torch.randint(0, 601, (int(n),), generator=gen).tolist() for n in torch.randint(max(1, ctx // 2), ctx + 1, (G,), generator=gen)]
+    out = {}
+    for flag in (False, True):
+        e = InferEngine(m, block_size=5, max_seqs=G + 1, max_tokens=G * ctx + 64, persistent_decode=flag, use_graphs=False)
+        e.persistent_max = 32
+        assert e.persistent == flag
+        e.generate(prompts, 2)                           # prefill, then one decode step
+        out[flag] = (e.logits[:G, :601].float().clone(), e.kc[0].float().clone(), e.vc[0].float().clone())
+    for i, tol in ((0, 3e-2), (1, 2.0 ** -7), (2, 2.0 ** -7)):
+        x, y = out[False][i], out[True][i]
+        err = ((x - y).norm() / x.norm()).item()
+        assert err < tol, (i, err)
+    assert ops.error_word() == 0
+
+
 def test_fp32_engine_on_gpu_is_token_exact():
     """The fp32 configuration on the GPU (fp32 weights, activations and KV pool; products on the
     CUDA-core fp32 kernel) reproduces the fp32 CPU engine token for token -- staggered continuous
