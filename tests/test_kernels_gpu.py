@@ -96,7 +96,7 @@ def test_gemm_weight_gradient_with_bias_gradient(M, N, K, bn):
 
 @pytest.mark.parametrize("bn", [64, 128])
 @pytest.mark.parametrize("split", [2, 4, 8])
-@pytest.mark.parametrize("M,N,K", [(128, 64, 512), (200, 72, 1000), (8, 136, 4104), (513, 257, 1032), (256, 512, 9216)])
+@pytest.mark.parametrize("M,N,K", [(128, 64, 512), (200, 72, 1000), (8, 136, 4104), (513, 257, 1496), (256, 512, 9216)])
 def test_gemm_split_over_a_cluster(M, N, K, split, bn):
     """K split over the CTAs of a cluster: whole and ragged tiles, K remainders, slices of unequal length, with every
     epilogue.  fp32 sums of K products in another order differ by at most K * 2^-24 of the sum of magnitudes, which for
