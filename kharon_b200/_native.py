@@ -82,6 +82,8 @@ def rt():
         _sig(lib, "kh_eng_seq_len", i32, vp, i32)
         _sig(lib, "kh_eng_seq_tokens", i32, vp, i32, vp, i32)
         _sig(lib, "kh_eng_seq_done", i32, vp, i32)
+        _sig(lib, "kh_eng_push_many", i32, vp, i32, vp, vp)
+        _sig(lib, "kh_eng_collect", i32, vp, i32, vp, vp, i32, vp)
         _sig(lib, "kh_eng_release", None, vp, i32)
         _sig(lib, "kh_eng_stats", None, vp, P(i64))
         _sig(lib, "kh_eng_blocks_in_use", i32, vp)

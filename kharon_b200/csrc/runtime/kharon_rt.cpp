@@ -590,6 +590,26 @@ extern "C" int kh_eng_seq_tokens(const KhEngine* e, int32_t id, int32_t* out, in
   memcpy(out, s.tok.data(), (size_t)n * 4);
   return n;
 }
+extern "C" int kh_eng_push_many(KhEngine* e, int32_t n, const int32_t* ids, const int32_t* tokens) {
+  for (int32_t i = 0; i < n; i++)
+    if (int rc = kh_eng_push(e, ids[i], tokens[i])) return rc;
+  return KH_OK;
+}
+extern "C" int kh_eng_collect(KhEngine* e, int32_t n, const int32_t* ids, int32_t* out, int32_t cap, int32_t* lens) {
+  int64_t total = 0;
+  for (int32_t i = 0; i < n; i++) {
+    if (ids[i] < 0 || ids[i] >= e->max_seqs) return fail(KH_E_ARG, "eng_collect: bad id");
+    total += (int64_t)e->seqs[ids[i]].tok.size();
+  }
+  if (total > cap) return fail(KH_E_ARG, "eng_collect: buffer too small");
+  for (int32_t i = 0; i < n; i++) {
+    lens[i] = kh_eng_seq_tokens(e, ids[i], out, cap);
+    out += lens[i];
+    cap -= lens[i];
+    kh_eng_release(e, ids[i]);
+  }
+  return KH_OK;
+}
 extern "C" int kh_eng_seq_done(const KhEngine* e, int32_t id) { return e->seqs[id].st == S_DONE; }
 extern "C" void kh_eng_release(KhEngine* e, int32_t id) {
   Seq& s = e->seqs[id];

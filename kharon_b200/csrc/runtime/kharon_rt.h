@@ -138,6 +138,10 @@ int       kh_eng_commit(KhEngine* e, const int32_t* sampled, int32_t n_seq);
 int       kh_eng_seq_len(const KhEngine* e, int32_t id);
 int       kh_eng_seq_tokens(const KhEngine* e, int32_t id, int32_t* out, int32_t cap);
 int       kh_eng_seq_done(const KhEngine* e, int32_t id);
+// kh_eng_push for n sequences; stops at the first error.
+int       kh_eng_push_many(KhEngine* e, int32_t n, const int32_t* ids, const int32_t* tokens);
+// Tokens of n sequences one after the other into out (capacity cap), their lengths into lens; releases the sequences.
+int       kh_eng_collect(KhEngine* e, int32_t n, const int32_t* ids, int32_t* out, int32_t cap, int32_t* lens);
 void      kh_eng_release(KhEngine* e, int32_t id);   // drop a finished/parent sequence
 // stats[0..3] = blocks_total, blocks_peak, tokens_decoded, prefix_blocks_saved
 void      kh_eng_stats(const KhEngine* e, int64_t stats[4]);

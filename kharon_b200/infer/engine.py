@@ -64,7 +64,14 @@ class InferEngine:
         self._n_meta = self._o_step + 4                      # {step number, seed low, seed high, unused}
         pin = self.dev.type == "cuda"
         self.h_meta = torch.zeros(self._n_meta, dtype=torch.int32, pin_memory=pin)
+        self.np_meta = self.h_meta.numpy()            # the same memory: element writes without a tensor operation each
         self.h_seq_ids = torch.zeros(ms_, dtype=torch.int32)
+        self._plan_n = (C.c_int32(), C.c_int32(), C.c_int32())
+        base = self.h_meta.data_ptr()
+        at = lambda o: base + 4 * o
+        self._plan_args = (at(self._o_tok), at(self._o_pos), at(self._o_slot), at(self._o_rows), self.h_seq_ids.data_ptr(),
+                           at(self._o_btab), C.byref(self._plan_n[0]), C.byref(self._plan_n[1]), at(self._o_pairs), ms_ * 4,
+                           C.byref(self._plan_n[2]))
         self.d_meta = torch.zeros(self._n_meta, dtype=torch.int32, **z)
         v = lambda t, o, n: t[o:o + n]
         self.d_tok, self.d_pos, self.d_slot = v(self.d_meta, 0, mt), v(self.d_meta, mt, mt), v(self.d_meta, 2 * mt, mt)
@@ -230,9 +237,7 @@ class InferEngine:
         self._fresh = self._fresh_prompts(ntok, nseq)
         sd = self.seed & 0xFFFFFFFFFFFFFFFF
         to_i32 = lambda u: u - (1 << 32) if u >= (1 << 31) else u
-        self.h_meta[self._o_step] = self.step_no & 0x7FFFFFFF
-        self.h_meta[self._o_step + 1] = to_i32(sd & 0xFFFFFFFF)
-        self.h_meta[self._o_step + 2] = to_i32(sd >> 32)
+        self.np_meta[self._o_step:self._o_step + 3] = (self.step_no & 0x7FFFFFFF, to_i32(sd & 0xFFFFFFFF), to_i32(sd >> 32))
         self.d_meta.copy_(self.h_meta, non_blocking=True)
         key = (ntok, nseq, rep, self.temperature)
         if self.use_graphs and ntok == nseq:           # greedy and sampled steps alike: the step number lives in d_meta
@@ -259,15 +264,9 @@ class InferEngine:
 
     # ------------------------------------------------------------------ scheduling
     def _plan(self, max_active):
-        lib, hm = _native.rt(), self.h_meta
-        base = hm.data_ptr()
-        n_tok, n_seq, n_pairs = C.c_int32(), C.c_int32(), C.c_int32()
-        rc = lib.kh_eng_plan(self._h, max_active, self.max_tokens, base + 4 * self._o_tok, base + 4 * self._o_pos,
-                             base + 4 * self._o_slot, base + 4 * self._o_rows, self.h_seq_ids.data_ptr(),
-                             base + 4 * self._o_btab, C.byref(n_tok), C.byref(n_seq), base + 4 * self._o_pairs,
-                             self.max_seqs * 4, C.byref(n_pairs))
+        rc = _native.rt().kh_eng_plan(self._h, max_active, self.max_tokens, *self._plan_args)
         _native.rt_check(rc)
-        return rc, n_tok.value, n_seq.value, n_pairs.value
+        return rc, self._plan_n[0].value, self._plan_n[1].value, self._plan_n[2].value
 
     def _step(self, max_active):
         rc, ntok, nseq, npairs = self._plan(max_active)
@@ -285,12 +284,18 @@ class InferEngine:
         _native.rt().kh_eng_stats(self._h, st)
         return InferStats(blocks_total=st[0], blocks_peak=st[1], tokens_decoded=st[2], prefix_blocks_saved=st[3])
 
-    def _tokens(self, sid):
-        lib = _native.rt()
-        n = lib.kh_eng_seq_len(self._h, sid)
-        buf = torch.empty(n, dtype=torch.int32)
-        lib.kh_eng_seq_tokens(self._h, sid, buf.data_ptr(), n)
-        return buf.tolist()
+    def _collect(self, sids):
+        """Token lists of finished sequences, which are released."""
+        lib, n = _native.rt(), len(sids)
+        ids, lens = (C.c_int32 * n)(*sids), (C.c_int32 * n)()
+        cap = sum(lib.kh_eng_seq_len(self._h, i) for i in sids) if n <= 4 else n * (self.max_lb * self.bs + 1)
+        buf = (C.c_int32 * cap)()
+        _native.rt_check(lib.kh_eng_collect(self._h, n, ids, buf, cap, lens))
+        out, at = [], 0
+        for k in lens:
+            out.append(buf[at:at + k])
+            at += k
+        return out
 
     def _timer(self):
         if self.dev.type == "cuda":
@@ -323,11 +328,10 @@ class InferEngine:
                 sid_of[sid] = i
                 pending.pop(0)
             progressed = self._step(max_active)
-            for sid, i in list(sid_of.items()):
-                if lib.kh_eng_seq_done(self._h, sid):
-                    outs[i] = self._tokens(sid)
-                    lib.kh_eng_release(self._h, sid)
-                    del sid_of[sid]
+            done = [sid for sid in sid_of if lib.kh_eng_seq_done(self._h, sid)]
+            if done:
+                for sid, toks in zip(done, self._collect(done)):
+                    outs[sid_of.pop(sid)] = toks
             if not progressed and not pending and not sid_of:
                 break
             if not progressed and not sid_of and pending:
@@ -351,13 +355,10 @@ class InferEngine:
         kids = torch.zeros(G, dtype=torch.int32)
         _native.rt_check(lib.kh_eng_fork(self._h, parent, G, n_new, kids.data_ptr()))
         lib.kh_eng_release(self._h, parent)
-        for g in range(G):
-            _native.rt_check(lib.kh_eng_push(self._h, int(kids[g]), int(first[g])))
+        _native.rt_check(lib.kh_eng_push_many(self._h, G, kids.data_ptr(), first.data_ptr()))
         while self._step(G):
             pass
-        outs = [self._tokens(int(k)) for k in kids]
-        for k in kids:
-            lib.kh_eng_release(self._h, int(k))
+        outs = self._collect(kids.tolist())
         ms = (self._timer() - t0) * 1e3
         return outs, self._stats(), ms
 
@@ -384,14 +385,11 @@ class InferEngine:
             _native.rt_check(lib.kh_eng_fork(self._h, parent, G, n_new, kids.data_ptr()))
             lib.kh_eng_release(self._h, parent)
             kids_of[parent] = kids.tolist()
-            for g in range(G):
-                _native.rt_check(lib.kh_eng_push(self._h, int(kids[g]), int(first[row * G + g])))
+            _native.rt_check(lib.kh_eng_push_many(self._h, G, kids.data_ptr(), first.data_ptr() + 4 * row * G))
         while self._step(len(prompts) * G):
             pass
-        outs = [[self._tokens(k) for k in kids_of[p]] for p in parents]
-        for p in parents:
-            for k in kids_of[p]:
-                lib.kh_eng_release(self._h, k)
+        flat = self._collect([k for p in parents for k in kids_of[p]])
+        outs = [flat[i * G:(i + 1) * G] for i in range(len(parents))]
         ms = (self._timer() - t0) * 1e3
         return outs, self._stats(), ms
 
