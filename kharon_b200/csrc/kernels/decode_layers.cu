@@ -26,9 +26,9 @@
 // take 106 us at the copy bandwidth).
 //
 // Linear phases.  A work unit is 16 output columns (8 in phases C and E, whose N is only d); S warps share
-// a unit, each multiplying its K / S slice, and a CTA of 16 warps works on 16 / S units at a time.  S is
+// a unit, each multiplying its K / S slice, and a CTA of 16 (8) warps works on 16 / S (8 / S) units at a time.  S is
 // the smallest split whose slice fits a sub-step, and larger where that spreads a narrow product over more
-// CTAs in the same number of turns.  Every lane copies the eight 16-byte pieces of weights that it will use
+// CTAs in the same number of turns.  Every lane copies the eight (sixteen) 16-byte pieces of weights that it will use
 // into its own slots of shared memory with cp.async (no registers are held and no thread waits for another's
 // copy); the first turn's weights of a phase are requested before its activations are polled, a slot is
 // refilled with the next turn's as soon as it has been read, and the units of later phases are prefetched
@@ -36,8 +36,7 @@
 // as the columns: tcgen05's 128-row tiles, TMEM round trip and operand staging are the latency this kernel
 // exists to avoid (the large-M GEMMs of training and prefill use them).  The K order inside a 32-wide block
 // is permuted identically for both operands so that every lane fetches 16 contiguous bytes.  Phases behind a
-// LayerNorm read the normalised rows from shared memory (a warp per row; pitch padded by 64 bytes,
-// conflict-free); the others read their operand fragments straight from the packets.  Partial sums of the S
+// LayerNorm read the normalised rows from shared memory (pitch padded by 64 bytes, conflict-free); the others read their operand fragments straight from the packets.  Partial sums of the S
 // warps meet in shared memory and are added in warp order.
 //
 // Attention.  W warps share a (sequence, head) item; a key is read by HD / 8 lanes in 16-byte pieces and
@@ -51,12 +50,21 @@
 
 namespace {
 
-constexpr int THREADS = 512, WARPS = 16;
-constexpr int NLD = 8;                        // 16-byte weight slots per lane (one sub-step)
+constexpr int MAX_WARPS = 16;
 constexpr int PAD = 32;                       // bf16 elements of padding per activation row (64 bytes)
 constexpr int MAX_ROWS = 32;
 constexpr int ATT_PITCH = 128 + 4;            // floats per warp of the attention hand-off: 128 outputs, maximum, sum
 constexpr int SMEM_LIMIT = 227 * 1024;
+
+// Warps of a CTA (2^LGW) and what follows: 16-byte weight slots per lane (one sub-step; 64 KB a CTA) and the bytes between them.
+// Eight warps for up to eight rows, where index arithmetic that every warp repeats weighs most (L24 d1024 G = 1 / 8: 489 / 538 us
+// against 507 / 565 with sixteen; d2048 G = 4: 1179 against 1248), sixteen beyond, where rows and keys are spread over more
+// warps (G = 16 / 32: 764 / 1217 against 781 / 1320).
+template <int LGW> struct Cfg {
+  static constexpr int WARPS = 1 << LGW, THREADS = 32 * WARPS, NLD = 128 / WARPS;
+  static constexpr uint32_t SLOT = THREADS * 16;
+};
+#define CFG using C_ = Cfg<LGW>; constexpr int WARPS = C_::WARPS, THREADS = C_::THREADS, NLD = C_::NLD; constexpr uint32_t SLOT = C_::SLOT; (void)WARPS; (void)THREADS; (void)NLD; (void)SLOT
 
 // Thread index, read anew in every phase: index arithmetic derived from it would otherwise be kept in registers (and
 // spilled) across the whole layer loop.
@@ -95,8 +103,8 @@ struct DecodeParams {
 
 struct Shared {               // small control block behind the data regions
   LayerW lw[2];               // records of this layer and the next
-  int item_pos[WARPS], item_slot[WARPS];    // position and slot of each warp's first attention item (constant over the layers)
-  int item_row[WARPS][8][4];                // cache rows of its first four keys, per lane group
+  int item_pos[MAX_WARPS], item_slot[MAX_WARPS];    // position and slot of each warp's first attention item (constant over the layers)
+  int item_row[MAX_WARPS][8][4];                // cache rows of its first four keys, per lane group
   volatile int abort_flag;
 };
 
@@ -203,9 +211,9 @@ struct Lin {
 // operand is zero) so that twice as many CTAs have a unit.
 // Copies this lane's 16-byte pieces of weight rows 8 (RG u + i) + lane / 4 from column k0 on: slot RG * j + i holds row group
 // i of the j-th 32-column step.  Steps below `n` are copied; rows that do not exist are left alone.
-constexpr uint32_t SLOT = THREADS * 16;       // bytes between a lane's slots
-template <int RG>
+template <int LGW, int RG>
 __device__ __forceinline__ void copy_w(uint32_t slots, int lane, const Lin& L, int u, int k0, int j, int n) {
+  CFG;
   if (j >= n) return;
 #pragma unroll
   for (int i = 0; i < RG; i++) {
@@ -213,17 +221,20 @@ __device__ __forceinline__ void copy_w(uint32_t slots, int lane, const Lin& L, i
     if (r < L.N) cp_async16(slots + (j * RG + i) * SLOT, L.W + (size_t)r * L.K + k0 + (lane & 3) * 8 + j * 32);
   }
 }
-template <int RG>
+template <int LGW, int RG>
 __device__ __forceinline__ void copy_first(uint32_t wbuf, const Lin& L) {
+  CFG;
   constexpr int KS = NLD / RG;
   const int tid = tid_fresh(), warp = tid >> 5, U = WARPS >> L.lgs, kw = L.K >> L.lgs;
 #pragma unroll
   for (int j = 0; j < KS; j++)
-    copy_w<RG>(wbuf + tid * 16, tid & 31, L, (int)blockIdx.x * U + (warp >> L.lgs), (warp & ((1 << L.lgs) - 1)) * kw, j, kw >> 5);
+    copy_w<LGW, RG>(wbuf + tid * 16, tid & 31, L, (int)blockIdx.x * U + (warp >> L.lgs), (warp & ((1 << L.lgs) - 1)) * kw, j, kw >> 5);
 }
 // ask L2 for the weights of this CTA's units (the first `turns` turns of them); one thread of the last warp, which has the
 // least to do at the start of a phase
+template <int LGW>
 __device__ __forceinline__ void prefetch_units(const bf16* W, int N, int K, int cols, int turns) {
+  CFG;
   if (tid_fresh() != THREADS - 32) return;
 #pragma unroll 1
   for (int r = 0; r < turns; r++) {
@@ -233,7 +244,9 @@ __device__ __forceinline__ void prefetch_units(const bf16* W, int N, int K, int 
   }
 }
 // LayerNorm gain and bias of a later phase -> shared memory (complete at that phase's first barrier)
+template <int LGW>
 __device__ __forceinline__ void fetch_ln(bf16* sln, const bf16* w, const bf16* b, int d) {
+  CFG;
 #pragma unroll 1
   for (int c = tid_fresh(); c < d / 8; c += THREADS) {
     cp_async16(smem_u32(sln + c * 8), w + c * 8);
@@ -243,7 +256,9 @@ __device__ __forceinline__ void fetch_ln(bf16* sln, const bf16* w, const bf16* b
 
 // LayerNorm of rows [0, n) into xs, a warp per row: the row is polled, kept in shared memory as it arrived, and
 // normalised in place (every lane touches only the 16-byte pieces that it wrote).
+template <int LGW>
 __device__ __forceinline__ void stage_ln(bf16* xs, const bf16* sln, const Lin& L, int n, const DecodeParams& p, Shared* sh) {
+  CFG;
   const int tid = tid_fresh(), warp = tid >> 5, lane = tid & 31;
   const int d = L.K, nch = d / 8;
 #pragma unroll 1
@@ -307,9 +322,10 @@ __device__ __forceinline__ void stage_ln(bf16* xs, const bf16* sln, const Lin& L
 // One linear phase over rows [0, n) (n <= 8 MT).  The slots hold this warp's weights of its first unit and sub-step
 // (copy_first).  LN (A, D, head): the rows go through LayerNorm and shared memory; otherwise (C, E) operand fragments come
 // straight from the packets.  One copy of each form serves all layers, which keeps the code small.
-template <int MT, bool LN>
+template <int LGW, int MT, bool LN>
 __device__ __forceinline__ void linear_phase(const DecodeParams& p, const Lin& L, int n, bool last, bf16* xs, const bf16* sln, float* red,
                                              int& flip, Shared* sh, uint32_t wbuf) {
+  CFG;
   constexpr bool RES = !LN;
   constexpr int GP = 8 * MT, LGP = MT == 1 ? 3 : (MT == 2 ? 4 : 5);
   constexpr int RG = LN ? 2 : 1, KS = NLD / RG, CU = 8 * RG, LCP = RG == 2 ? 3 : 2;      // steps per sub-step, columns and log2 column pairs per unit
@@ -342,7 +358,7 @@ __device__ __forceinline__ void linear_phase(const DecodeParams& p, const Lin& L
     uint64_t res2;
     operands(tid, bias2, res2);
     if (LN && !staged) {
-      stage_ln(xs, sln, L, n, p, sh);
+      stage_ln<LGW>(xs, sln, L, n, p, sh);
       __syncthreads();
       staged = true;
     }
@@ -374,7 +390,7 @@ __device__ __forceinline__ void linear_phase(const DecodeParams& p, const Lin& L
               mma_bf16(acc[(2 * j + 1) % NCH][m], w0.z, w1.z, w0.w, w1.w, a.z, a.w);
             }
           }
-          copy_w<RG>(slots, lane, L, nu, nk, j, nn);
+          copy_w<LGW, RG>(slots, lane, L, nu, nk, j, nn);
         }
       } else {
         constexpr int JB = 4 / MT;                                // eight packet pairs in flight per lane
@@ -403,7 +419,7 @@ __device__ __forceinline__ void linear_phase(const DecodeParams& p, const Lin& L
             }
           }
 #pragma unroll
-          for (int j = j0; j < j0 + JB; j++) copy_w<RG>(slots, lane, L, nu, nk, j, nn);
+          for (int j = j0; j < j0 + JB; j++) copy_w<LGW, RG>(slots, lane, L, nu, nk, j, nn);
         }
       }
     }
@@ -459,8 +475,9 @@ __device__ __forceinline__ void linear_phase(const DecodeParams& p, const Lin& L
 // ------------------------------------------------------------------------------------------------
 // Phase B.  Appends the new k, v (from the qkv packets) to the paged cache and attends over positions 0..pos.
 // The W warps of an item hold W * 32 / (HD / 8) lane groups; group i takes keys i, i + ST, i + 2 ST, ...
-template <int HD>
+template <int LGW, int HD>
 __device__ __forceinline__ void attention_phase(const DecodeParams& p, int layer, uint32_t epoch, float* satt, Shared* sh) {
+  CFG;
   constexpr int LPK = HD / 8, KPW = 32 / LPK;     // lanes per key, keys per warp and turn
   const int tid = tid_fresh(), warp = tid >> 5, lane = tid & 31;
   const int W = 1 << p.lgw, slots = WARPS >> p.lgw, ST = W * KPW;
@@ -619,8 +636,12 @@ __device__ __forceinline__ void attention_phase(const DecodeParams& p, int layer
   }
 }
 
+template <int MT> constexpr int lg_warps() { return MT == 1 ? 3 : 4; }
+
 template <int MT, int HD>
-__global__ void __launch_bounds__(THREADS, 1) decode_layers_k(const __grid_constant__ DecodeParams p) {
+__global__ void __launch_bounds__(32 << lg_warps<MT>(), 1) decode_layers_k(const __grid_constant__ DecodeParams p) {
+  constexpr int LGW = lg_warps<MT>();
+  CFG;
   constexpr int GP = 8 * MT;
   extern __shared__ __align__(16) uint8_t smem[];
   const uint32_t wbuf = smem_u32(smem);
@@ -688,10 +709,10 @@ __global__ void __launch_bounds__(THREADS, 1) decode_layers_k(const __grid_const
   };
   const int n_half = 2 * p.L;
   if (p.L > 0) {
-    fetch_ln(sln, sh->lw[0].ln1_w, sh->lw[0].ln1_b, d);
-    prefetch_units(sh->lw[0].proj_w, d, d, (WARPS >> p.lgs_c) * 8, 8);
+    fetch_ln<LGW>(sln, sh->lw[0].ln1_w, sh->lw[0].ln1_b, d);
+    prefetch_units<LGW>(sh->lw[0].proj_w, d, d, (WARPS >> p.lgs_c) * 8, 8);
   } else {
-    fetch_ln(sln, p.lnf_w, p.lnf_b, d);
+    fetch_ln<LGW>(sln, p.lnf_w, p.lnf_b, d);
   }
 #pragma unroll 1
   for (int hl = 0; hl < n_half + (p.head_w ? 1 : 0); hl++) {
@@ -701,9 +722,9 @@ __global__ void __launch_bounds__(THREADS, 1) decode_layers_k(const __grid_const
     const bool even = (hl & 1) == 0, last = l + 1 >= p.L;
     {
       const Lin L = ln_phase(hl);
-      copy_first<2>(wbuf, L);
-      if (even && hl < n_half) prefetch_units(lw->fc_w, 4 * d, d, (WARPS >> p.lgs_d) * 16, 8);
-      linear_phase<MT, true>(p, L, hl == n_half ? p.n_rows : p.G, false, xs, sln, red, flip, sh, wbuf);
+      copy_first<LGW, 2>(wbuf, L);
+      if (even && hl < n_half) prefetch_units<LGW>(lw->fc_w, 4 * d, d, (WARPS >> p.lgs_d) * 16, 8);
+      linear_phase<LGW, MT, true>(p, L, hl == n_half ? p.n_rows : p.G, false, xs, sln, red, flip, sh, wbuf);
     }
     if (hl == n_half) break;
     if (even) {
@@ -712,23 +733,23 @@ __global__ void __launch_bounds__(THREADS, 1) decode_layers_k(const __grid_const
         const int t = tid_fresh();
         if (t < 6) cp_async16(smem_u32(reinterpret_cast<uint4*>(sh->lw + ((l + 1) & 1)) + t), reinterpret_cast<const uint4*>(p.layers + l + 1) + t);
       }
-      attention_phase<HD>(p, l, base + l + 1, satt, sh);
+      attention_phase<LGW, HD>(p, l, base + l + 1, satt, sh);
     }
     const Lin L = res_phase(hl);
-    copy_first<1>(wbuf, L);
+    copy_first<LGW, 1>(wbuf, L);
     const bf16 *lnw = lw->ln2_w, *lnb = lw->ln2_b;
     if (even) {
-      prefetch_units(lw->fcproj_w, d, 4 * d, (WARPS >> p.lgs_e) * 8, 8);
+      prefetch_units<LGW>(lw->fcproj_w, d, 4 * d, (WARPS >> p.lgs_e) * 8, 8);
     } else if (!last) {
       lnw = nw->ln1_w; lnb = nw->ln1_b;
-      prefetch_units(nw->qkv_w, 3 * d, d, (WARPS >> p.lgs_a) * 16, 8);
-      prefetch_units(nw->proj_w, d, d, (WARPS >> p.lgs_c) * 8, 8);
+      prefetch_units<LGW>(nw->qkv_w, 3 * d, d, (WARPS >> p.lgs_a) * 16, 8);
+      prefetch_units<LGW>(nw->proj_w, d, d, (WARPS >> p.lgs_c) * 8, 8);
     } else {
       lnw = p.lnf_w; lnb = p.lnf_b;
-      if (p.head_w) prefetch_units(p.head_w, p.V, d, (WARPS >> p.lgs_h) * 16, 2);
+      if (p.head_w) prefetch_units<LGW>(p.head_w, p.V, d, (WARPS >> p.lgs_h) * 16, 2);
     }
-    if (lnw) fetch_ln(sln, lnw, lnb, d);
-    linear_phase<MT, false>(p, L, p.G, last && !even, xs, sln, red, flip, sh, wbuf);
+    if (lnw) fetch_ln<LGW>(sln, lnw, lnb, d);
+    linear_phase<LGW, MT, false>(p, L, p.G, last && !even, xs, sln, red, flip, sh, wbuf);
   }
   cp_async_wait_all();
   __syncthreads();
@@ -744,35 +765,39 @@ __global__ void __launch_bounds__(THREADS, 1) decode_layers_k(const __grid_const
 }
 
 int smem_bytes(int MT, int d) {
-  return NLD * (int)SLOT + 8 * MT * (d + PAD) * 2 + 4 * d + (MT == 4 ? 1 : 2) * WARPS * 8 * MT * 16 * 4 + WARPS * ATT_PITCH * 4 +
-         (int)sizeof(Shared);
+  const int warps = MT == 1 ? 1 << lg_warps<1>() : 1 << lg_warps<2>();
+  return 65536 + 8 * MT * (d + PAD) * 2 + 4 * d + (MT == 4 ? 1 : 2) * warps * 8 * MT * 16 * 4 + warps * ATT_PITCH * 4 + (int)sizeof(Shared);
 }
 int max_mt(int d) {             // row groups of eight whose normalised rows fit into shared memory
   for (int mt = 4; mt > 1; mt >>= 1)
     if (smem_bytes(mt, d) <= SMEM_LIMIT) return mt;
   return 1;
 }
-// Warps that share a unit of 8 `rg` columns.  Slices are whole 32-column steps and at most one sub-step wide where 16 warps
+// Warps that share a unit of 8 `rg` columns.  Slices are whole 32-column steps and at most one sub-step wide where the warps
 // allow it; beyond that the split grows as long as the units still fit the same number of turns of the grid, so that a narrow
 // product (proj, fcproj) runs on more CTAs with less to fetch per warp.
-int pick_lgs(int N, int K, int rg, int grid) {
-  const int units = (N + 8 * rg - 1) / (8 * rg), sub = NLD / rg * 32;
+int pick_lgs(int N, int K, int rg, int lgw, int grid) {
+  const int units = (N + 8 * rg - 1) / (8 * rg), sub = (128 >> lgw) / rg * 32;
   auto fits = [&](int lg) { return (K / 32) % (1 << lg) == 0; };
-  auto turns = [&](int lg) { const long per = (long)grid * (WARPS >> lg); return (units + per - 1) / per; };
+  auto turns = [&](int lg) { const long per = (long)grid * ((1 << lgw) >> lg); return (units + per - 1) / per; };
   int lg = 0;
-  while (lg < 4 && fits(lg + 1) && (K >> lg) > sub) lg++;
-  while (lg < 4 && fits(lg + 1) && turns(lg + 1) == turns(lg)) lg++;
+  while (lg < lgw && fits(lg + 1) && (K >> lg) > sub) lg++;
+  while (lg < lgw && fits(lg + 1) && turns(lg + 1) == turns(lg)) lg++;
   return lg;
 }
 
 template <int MT, int HD>
 int launch(DecodeParams& p, int grid, cudaStream_t st) {
-  const int smem = smem_bytes(MT, p.d);
+  const int lgw = lg_warps<MT>(), d = p.d, smem = smem_bytes(MT, d);
+  p.lgs_a = pick_lgs(3 * d, d, 2, lgw, grid); p.lgs_c = pick_lgs(d, d, 1, lgw, grid); p.lgs_d = pick_lgs(4 * d, d, 2, lgw, grid);
+  p.lgs_e = pick_lgs(d, 4 * d, 1, lgw, grid); p.lgs_h = p.head_w ? pick_lgs(p.V, d, 2, lgw, grid) : 0;
+  p.lgw = lgw;                                  // as many warps per (sequence, head) as keep all items in one turn
+  while (p.lgw > 0 && (long)p.G * p.H << p.lgw > (long)grid << lgw) p.lgw--;
   cudaError_t e = cudaFuncSetAttribute(decode_layers_k<MT, HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) { kh_set_error("decode_layers: shared memory opt-in failed: %s", cudaGetErrorString(e)); return -1; }
   // cooperative launch: the driver guarantees that all CTAs are resident together (or refuses the launch)
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid); cfg.blockDim = dim3(THREADS); cfg.dynamicSmemBytes = smem; cfg.stream = st;
+  cfg.gridDim = dim3(grid); cfg.blockDim = dim3(32 << lgw); cfg.dynamicSmemBytes = smem; cfg.stream = st;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeCooperative;
   at[0].val.cooperative = 1;
@@ -832,8 +857,6 @@ extern "C" int kh_decode_layers(void* x, const void* layers, int L, int G, int d
   p.ctl = (uint32_t*)work;
   const size_t row2 = (size_t)d / 2 * MAX_ROWS;
   p.xp = (uint64_t*)((uint8_t*)work + 64); p.midp = p.xp + row2; p.attp = p.midp + row2; p.qkvp = p.attp + row2; p.actp = p.qkvp + 3 * row2;
-  p.lgs_a = pick_lgs(3 * d, d, 2, grid); p.lgs_c = pick_lgs(d, d, 1, grid); p.lgs_d = pick_lgs(4 * d, d, 2, grid);
-  p.lgs_e = pick_lgs(d, 4 * d, 1, grid); p.lgs_h = head_w ? pick_lgs(V, d, 2, grid) : 0;
   p.bs_mul = bs > max_ctx ? 0u : (uint32_t)(((1ull << 32) + bs - 1) / bs);
   p.scale = scale;
   p.wait_ns = KH_WAIT_LIMIT_NS;
@@ -850,8 +873,6 @@ extern "C" int kh_decode_layers(void* x, const void* layers, int L, int G, int d
     const int n = G - g0 < cap ? G - g0 : cap;
     p.G = n; p.L = L;
     p.x = (bf16*)x + (size_t)g0 * d; p.pos = (const int*)pos + g0; p.slot = (const int*)slot + g0;
-    p.lgw = 4;                                  // as many warps per (sequence, head) as keep all items in one turn
-    while (p.lgw > 0 && (long)n * H << p.lgw > (long)grid * WARPS) p.lgw--;
     if (head_w && together) set_head(0, n_rows);
     if (launch_any(p, head_w && together && n_rows > n ? n_rows : n, grid, st)) return -1;
   }
