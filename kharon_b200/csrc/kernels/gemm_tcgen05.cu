@@ -9,7 +9,7 @@
 //   input grad     dX = dY * W        A K-major,  B N-major     (reference mm_nn_bf16o, kernels.cu:55-60)
 //   weight grad    dW = dY^T * X      A M-major,  B N-major     (reference mm_tn_bf16[_acc], kernels.cu:41-53)
 //
-// Structure: persistent CTAs (one per SM), 10 warps.  Warp 0 streams operand tiles with TMA
+// Structure: persistent CTAs (one per SM), 6 or 10 warps.  Warp 0 streams operand tiles with TMA
 // into a ring of 128-byte-swizzled shared-memory stages; one lane of warp 1 issues
 // tcgen05.mma (128 x BN x 16 per instruction) into one of two TMEM accumulator buffers and
 // commits stage-release / accumulator-ready mbarriers; warps 2-9 drain the other
@@ -253,7 +253,7 @@ struct GemmParams {
 };
 
 constexpr int BM = 128, BK = 64, UMMA_K = 16;
-constexpr int GEMM_THREADS = 320;          // TMA, MMA and eight epilogue warps (or four and four column-sum warps)
+constexpr int GEMM_THREADS = 320;          // TMA, MMA and eight epilogue warps (or four and four column-sum warps); 192: four epilogue warps
 
 // PAIR: two CTAs of a cluster form one 256 x BN tile (tcgen05 cta_group::2).  Each CTA stages its
 // own 128 rows of A and its own half of B, so a pair moves and re-reads 2/3 of the shared-memory
@@ -288,7 +288,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ C
   const uint32_t bar_free = bar_tempty + 16;         // column-sum warps are done with the stage
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 3 * Cfg::STAGES + 4);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  const bool csum = p.colsum != nullptr;
+  const bool csum = p.colsum != nullptr, wide = !csum && blockDim.x == GEMM_THREADS;      // wide: eight epilogue warps
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int tiles_m = (p.M + TM - 1) / TM, tiles_n = (p.N + BN - 1) / BN;
@@ -300,7 +300,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ C
       mbar_init(bar_full + 8 * s, 1); mbar_init(bar_empty + 8 * s, 1); mbar_init(bar_free + 8 * s, 4);
     }
     // accumulator-free barrier: one arrival per epilogue warp of every CTA that reads the accumulator
-    for (int a = 0; a < 2; a++) { mbar_init(bar_tfull + 8 * a, 1); mbar_init(bar_tempty + 8 * a, (PAIR ? 2 : 1) * (csum ? 4 : 8)); }
+    for (int a = 0; a < 2; a++) { mbar_init(bar_tfull + 8 * a, 1); mbar_init(bar_tempty + 8 * a, (PAIR ? 2 : 1) * (wide ? 8 : 4)); }
     *abort_flag = 0;
     mbar_fence_init();
   }
@@ -463,11 +463,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ C
     }
   } else {
     // ------------------------------------------------------------------ epilogue warps
-    // Eight warps, two per TMEM quadrant, each with half of the tile's columns (four with all columns where the other four
-    // form column sums).  With four warps the epilogue of a 256-wide tile outlasts a main loop of K = 512 and bounds the
-    // products of narrow models.
+    // Four warps with all columns of a tile, or eight, two per TMEM quadrant, with half of the columns each (see epilogue_threads).
     const int q = warp & 3;                    // TMEM lane quadrant this warp may access
-    const int col_lo = (!csum && warp >= 6) ? BN / 2 : 0, col_hi = (!csum && warp < 6) ? BN / 2 : BN;
+    const int col_lo = (wide && warp >= 6) ? BN / 2 : 0, col_hi = (wide && warp < 6) ? BN / 2 : BN;
     int tcount = 0;
     bool ok = true;
     for (int t = worker; ok && t < num_tiles; t += n_workers, tcount++) {
@@ -857,6 +855,11 @@ static int num_sms() {
   return g_num_sms;
 }
 
+// Threads of a gemm_kernel CTA.  Up to K = 1024 the main loop of a tile is shorter than the epilogue of four warps, which then
+// bounds the product: eight warps.  Beyond, the epilogue hides behind the main loop and the second set of warps only takes
+// power and issue slots from it (1.2B training step, K = 2048 and more: 147.3 ms with eight, 144.5 with four).
+static int gemm_threads(const GemmParams& p) { return p.colsum || p.K <= 1024 ? GEMM_THREADS : 192; }
+
 // 256-row tiles on CTA pairs.  Returns the number of clusters that can be resident (0: unsupported).
 static int g_pair_clusters = -1;
 static int launch_gemm_pair(const CUtensorMap* ta, const CUtensorMap* tb, const GemmParams& p, int max_ctas, cudaStream_t st) {
@@ -868,7 +871,7 @@ static int launch_gemm_pair(const CUtensorMap* ta, const CUtensorMap* tb, const 
   attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[1].val.programmaticStreamSerializationAllowed = 1;
-  cfg.blockDim = dim3(GEMM_THREADS); cfg.dynamicSmemBytes = Cfg::SMEM; cfg.stream = st; cfg.attrs = attr;
+  cfg.blockDim = dim3(gemm_threads(p)); cfg.dynamicSmemBytes = Cfg::SMEM; cfg.stream = st; cfg.attrs = attr;
   cfg.numAttrs = kh_pdl_enabled() ? 2 : 1;
   if (g_pair_clusters < 0) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM);
@@ -902,7 +905,7 @@ static int launch_gemm(const CUtensorMap* ta, const CUtensorMap* tb, const GemmP
   const int tiles = ((p.M + BM - 1) / BM) * ((p.N + BN - 1) / BN);
   int grid = tiles < num_sms() ? tiles : num_sms();
   if (max_ctas > 0 && grid > max_ctas) grid = max_ctas;
-  cudaError_t e = KH_LAUNCH((gemm_kernel<BN, false>), grid, GEMM_THREADS, Cfg::SMEM, st, *ta, *tb, p);
+  cudaError_t e = KH_LAUNCH((gemm_kernel<BN, false>), grid, gemm_threads(p), Cfg::SMEM, st, *ta, *tb, p);
   if (e != cudaSuccess) { kh_set_error("gemm launch failed: %s", cudaGetErrorString(e)); return -1; }
   return 0;
 }
