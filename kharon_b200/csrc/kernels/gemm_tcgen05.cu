@@ -255,6 +255,10 @@ struct GemmParams {
 constexpr int BM = 128, BK = 64, UMMA_K = 16;
 constexpr int GEMM_THREADS = 320;          // TMA, MMA and eight epilogue warps (or four and four column-sum warps); 192: four epilogue warps
 
+// Staging buffer of an epilogue warp: 32 rows of 64 bytes (32 bf16 columns), pitch 80 bytes (conflict-free 16-byte accesses both
+// by row and by piece).
+constexpr int EPI_PITCH = 80, EPI_BYTES = 32 * EPI_PITCH;
+
 // PAIR: two CTAs of a cluster form one 256 x BN tile (tcgen05 cta_group::2).  Each CTA stages its
 // own 128 rows of A and its own half of B, so a pair moves and re-reads 2/3 of the shared-memory
 // bytes of two independent 128 x BN tiles.
@@ -265,7 +269,7 @@ template <int BN, bool PAIR = false> struct GemmCfg {
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
   static constexpr int STAGES = PAIR ? 6 : ((BN == 256) ? 4 : (BN == 128 ? 6 : 8));
   static constexpr int TMEM_COLS = 2 * BN < 32 ? 32 : 2 * BN;
-  static constexpr int SMEM = STAGES * STAGE_BYTES + 1024 /*align*/ + 256 /*barriers*/;
+  static constexpr int SMEM = STAGES * STAGE_BYTES + 1024 /*align*/ + 256 /*barriers*/ + 8 * EPI_BYTES;
 };
 
 template <int BN, bool PAIR>
@@ -466,6 +470,33 @@ gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ C
     // Four warps with all columns of a tile, or eight, two per TMEM quadrant, with half of the columns each (see epilogue_threads).
     const int q = warp & 3;                    // TMEM lane quadrant this warp may access
     const int col_lo = (wide && warp >= 6) ? BN / 2 : 0, col_hi = (wide && warp < 6) ? BN / 2 : BN;
+    // A thread owns a row of the accumulator, but global memory is read and written in pieces of 16 bytes, four neighbouring
+    // lanes to a row of the 32-column chunk: the warp turns the chunk around in its staging buffer.  With every lane on its own row an
+    // access touched 32 lines, and the load / store unit bounded the products of narrow models (9216 x 1536 x 512:
+    // 23.6 us plain, 30 with a residual, 38 with GELU and its pre-activation; cuBLAS plain 14.1).
+    const uint32_t stg = smem_base + Cfg::STAGES * Cfg::STAGE_BYTES + 256 + (warp - 2) * EPI_BYTES;
+    const int prow = lane >> 2, pcol = (lane & 3) * 8;          // this lane's piece: row 8 j + prow, columns pcol ..
+    auto put_row = [&](const float (&v)[32]) {                   // own row, bf16 -> staging
+#pragma unroll
+      for (int j = 0; j < 4; j++)
+        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(stg + lane * EPI_PITCH + j * 16), "r"(pack_bf16(v[8 * j], v[8 * j + 1])),
+                     "r"(pack_bf16(v[8 * j + 2], v[8 * j + 3])), "r"(pack_bf16(v[8 * j + 4], v[8 * j + 5])), "r"(pack_bf16(v[8 * j + 6], v[8 * j + 7])) : "memory");
+    };
+    auto lds = [&](uint32_t a) {
+      uint4 u;
+      asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(u.x), "=r"(u.y), "=r"(u.z), "=r"(u.w) : "r"(a) : "memory");
+      return u;
+    };
+    auto store_rows = [&](bf16* base, int ld, int r0, int col, const float (&v)[32]) {      // 32 rows from r0, columns col ..
+      put_row(v);
+      __syncwarp();
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        const uint4 u = lds(stg + (j * 8 + prow) * EPI_PITCH + (lane & 3) * 16);
+        if (r0 + j * 8 + prow < p.M) *reinterpret_cast<uint4*>(base + (size_t)(r0 + j * 8 + prow) * ld + col + pcol) = u;
+      }
+      __syncwarp();
+    };
     int tcount = 0;
     bool ok = true;
     for (int t = worker; ok && t < num_tiles; t += n_workers, tcount++) {
@@ -473,7 +504,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ C
       tile_coord(t, tm, tn);
       const int acc = tcount & 1;
       const uint32_t aph = (tcount >> 1) & 1;
-      const int row = tm * TM + (int)crank * BM + q * 32 + lane;
+      const int row0 = tm * TM + (int)crank * BM + q * 32, row = row0 + lane;
       const bool row_ok = row < p.M;
       const bool use_bias = (p.epi == EPI_BIAS || p.epi == EPI_BIAS_GELU || p.epi == EPI_BIAS_RESID);
       const bool use_aux = (p.epi == EPI_BIAS_RESID || p.epi == EPI_RESID || p.epi == EPI_DGELU);
@@ -488,10 +519,10 @@ gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ C
 #pragma unroll
           for (int j = 0; j < 4; j++) nb[j] = __ldg(bp + j);
         }
-        if (use_aux && row_ok) {
-          const uint4* ap = reinterpret_cast<const uint4*>(p.aux + (size_t)row * p.ldaux + col);
+        if (use_aux) {
 #pragma unroll
-          for (int j = 0; j < 4; j++) nx[j] = ap[j];
+          for (int j = 0; j < 4; j++)
+            if (row0 + j * 8 + prow < p.M) nx[j] = *reinterpret_cast<const uint4*>(p.aux + (size_t)(row0 + j * 8 + prow) * p.ldaux + col + pcol);
         }
       };
       if (use_aux && row_ok) {
@@ -532,75 +563,58 @@ gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ C
             for (int i = 0; i < 32; i++) if (col + i < p.N) v[i] += __bfloat162float(p.bias[col + i]);
           }
         }
-        if (row_ok) {
+        if (full) {                            // uniform over the warp: rows past the end take part without memory accesses
           if (p.epi == EPI_BIAS_GELU) {
-            bf16* ap = p.aux + (size_t)row * p.ldaux + col;
-            if (full) {
-#pragma unroll
-              for (int j = 0; j < 4; j++) {
-                uint4 o;
-                o.x = pack_bf16(v[8 * j], v[8 * j + 1]); o.y = pack_bf16(v[8 * j + 2], v[8 * j + 3]);
-                o.z = pack_bf16(v[8 * j + 4], v[8 * j + 5]); o.w = pack_bf16(v[8 * j + 6], v[8 * j + 7]);
-                reinterpret_cast<uint4*>(ap)[j] = o;
-              }
-            } else {
-              for (int i = 0; i < 32; i++) if (col + i < p.N) ap[i] = __float2bfloat16(v[i]);
-            }
+            store_rows(p.aux, p.ldaux, row0, col, v);
             // the stored pre-activation is bf16; apply GELU to the rounded value so that the
             // backward pass (which only sees the bf16 copy) differentiates the same function
 #pragma unroll
             for (int i = 0; i < 32; i++) v[i] = gelu_tanh(__bfloat162float(__float2bfloat16(v[i])));
           } else if (use_aux) {
-            const bf16* ap = p.aux + (size_t)row * p.ldaux + col;
-            float x[32];
-            if (full) {
 #pragma unroll
-              for (int j = 0; j < 4; j++) {
-                uint4 b = cx[j];
-                float2 f0 = unpack_bf16(b.x), f1 = unpack_bf16(b.y), f2 = unpack_bf16(b.z), f3 = unpack_bf16(b.w);
-                x[8 * j + 0] = f0.x; x[8 * j + 1] = f0.y; x[8 * j + 2] = f1.x; x[8 * j + 3] = f1.y;
-                x[8 * j + 4] = f2.x; x[8 * j + 5] = f2.y; x[8 * j + 6] = f3.x; x[8 * j + 7] = f3.y;
-              }
-            } else {
+            for (int j = 0; j < 4; j++)
+              asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(stg + (j * 8 + prow) * EPI_PITCH + (lane & 3) * 16), "r"(cx[j].x), "r"(cx[j].y),
+                           "r"(cx[j].z), "r"(cx[j].w) : "memory");
+            __syncwarp();
 #pragma unroll
-              for (int i = 0; i < 32; i++) x[i] = (col + i < p.N) ? __bfloat162float(ap[i]) : 0.f;
+            for (int j = 0; j < 4; j++) {
+              const uint4 b = lds(stg + lane * EPI_PITCH + j * 16);
+              const float2 f0 = unpack_bf16(b.x), f1 = unpack_bf16(b.y), f2 = unpack_bf16(b.z), f3 = unpack_bf16(b.w);
+              const float x[8] = {f0.x, f0.y, f1.x, f1.y, f2.x, f2.y, f3.x, f3.y};
+#pragma unroll
+              for (int i = 0; i < 8; i++) v[8 * j + i] = p.epi == EPI_DGELU ? v[8 * j + i] * gelu_tanh_grad(x[i]) : v[8 * j + i] + x[i];
             }
-            if (p.epi == EPI_DGELU) {
+            __syncwarp();
+          }
+          if (!p.out_fp32) store_rows(reinterpret_cast<bf16*>(p.C), p.ldc, row0, col, v);
+          else if (row_ok) {
+            float* cp = reinterpret_cast<float*>(p.C) + (size_t)row * p.ldc + col;
+            if (p.accumulate) {
 #pragma unroll
-              for (int i = 0; i < 32; i++) v[i] *= gelu_tanh_grad(x[i]);
+              for (int j = 0; j < 8; j++) red_add_v4_f32(cp + 4 * j, v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
             } else {
 #pragma unroll
-              for (int i = 0; i < 32; i++) v[i] += x[i];
+              for (int j = 0; j < 8; j++)
+                reinterpret_cast<float4*>(cp)[j] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
             }
           }
-          if (p.out_fp32) {
-            float* cp = reinterpret_cast<float*>(p.C) + (size_t)row * p.ldc + col;
-            if (full) {
-              if (p.accumulate) {
+        } else if (row_ok) {                   // ragged last columns
 #pragma unroll
-                for (int j = 0; j < 8; j++) red_add_v4_f32(cp + 4 * j, v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
-              } else {
-#pragma unroll
-                for (int j = 0; j < 8; j++)
-                  reinterpret_cast<float4*>(cp)[j] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
-              }
-            } else {
-              for (int i = 0; i < 32; i++)
-                if (col + i < p.N) cp[i] = p.accumulate ? cp[i] + v[i] : v[i];
+          for (int i = 0; i < 32; i++) {
+            if (col + i >= p.N) break;
+            float x = v[i];
+            if (p.epi == EPI_BIAS_GELU) {
+              const bf16 pre = __float2bfloat16(x);
+              p.aux[(size_t)row * p.ldaux + col + i] = pre;
+              x = gelu_tanh(__bfloat162float(pre));
+            } else if (use_aux) {
+              const float a = __bfloat162float(p.aux[(size_t)row * p.ldaux + col + i]);
+              x = p.epi == EPI_DGELU ? x * gelu_tanh_grad(a) : x + a;
             }
-          } else {
-            bf16* cp = reinterpret_cast<bf16*>(p.C) + (size_t)row * p.ldc + col;
-            if (full) {
-#pragma unroll
-              for (int j = 0; j < 4; j++) {
-                uint4 o;
-                o.x = pack_bf16(v[8 * j], v[8 * j + 1]); o.y = pack_bf16(v[8 * j + 2], v[8 * j + 3]);
-                o.z = pack_bf16(v[8 * j + 4], v[8 * j + 5]); o.w = pack_bf16(v[8 * j + 6], v[8 * j + 7]);
-                reinterpret_cast<uint4*>(cp)[j] = o;
-              }
-            } else {
-              for (int i = 0; i < 32; i++) if (col + i < p.N) cp[i] = __float2bfloat16(v[i]);
-            }
+            if (p.out_fp32) {
+              float* cp = reinterpret_cast<float*>(p.C) + (size_t)row * p.ldc + col + i;
+              *cp = p.accumulate ? *cp + x : x;
+            } else reinterpret_cast<bf16*>(p.C)[(size_t)row * p.ldc + col + i] = __float2bfloat16(x);
           }
         }
       }
