@@ -24,6 +24,7 @@
 // stores, releases TMEM and returns.
 #include "common.cuh"
 
+
 #define KH_LAUNCH_CHECK(name)                                                     \
   do {                                                                            \
     cudaError_t e_ = cudaGetLastError();                                          \
@@ -95,10 +96,18 @@ struct FwdWs {
   static constexpr int THREADS = 192, TMEM_COLS = 256;     // S: 2 x 64 columns, O: HD columns from 128
 };
 
-template <int HD>
+// NSEG = 1: B sequences of equal length T, one set of tensor maps.  NSEG > 1 (prefill of several prompts in one launch): up to
+// NSEG sequences of their own lengths, each with its own maps, whose row extents keep a sequence's loads and stores within
+// its rows; `seg.pair` lists (sequence, query tile) by falling number of key tiles, an item is a pair and a head.
+constexpr int MAX_SEGS = 16, MAX_PAIRS = 512;
+template <int NSEG> struct FwdMaps { CUtensorMap q[NSEG], kv[NSEG], o[NSEG]; };
+template <int NSEG> struct FwdSegs { int T[NSEG]; uint16_t pair[MAX_PAIRS]; };      // pair = query tile * MAX_SEGS + sequence
+template <> struct FwdSegs<1> {};
+
+template <int HD, int NSEG>
 __global__ void __launch_bounds__(192, 2)
-flash_fwd_ws_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_kv,
-                    const __grid_constant__ CUtensorMap map_o, const AttnParams p, int n_items, int n_qt) {
+flash_fwd_ws_kernel(const __grid_constant__ FwdMaps<NSEG> maps, const __grid_constant__ FwdSegs<NSEG> seg, const AttnParams p,
+                    int n_items, int n_qt) {
   using C = FwdWs<HD>;
   constexpr int BQ = C::BQ, BKV = C::BKV, NS = C::NS;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -126,9 +135,9 @@ flash_fwd_ws_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     *abort_flag = (base & 1023u) ? 6 : 0;       // swizzled tiles need the 1024-byte alignment
     if (base & 1023u) atomicCAS(p.err, 0, 6);
     mbar_fence_init();
-    tma_prefetch_desc(&map_q);
-    tma_prefetch_desc(&map_kv);
-    tma_prefetch_desc(&map_o);
+    tma_prefetch_desc(&maps.q[0]);
+    tma_prefetch_desc(&maps.kv[0]);
+    tma_prefetch_desc(&maps.o[0]);
   }
   if (warp == 5) { tmem_alloc(smem_u32(tmem_slot), C::TMEM_COLS); tmem_relinquish(); }
   tc_fence_before();
@@ -139,11 +148,20 @@ flash_fwd_ws_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
   pdl_launch_dependents();
 
   const int d = p.H * HD, BH = p.B * p.H;
-  // item w -> (query tile, batch, head); the tiles that see the most keys come first
-  auto decode = [&](int w, int& b, int& h, int& q0, int& n) {
-    const int qt = n_qt - 1 - w / BH, bh = w % BH;
-    b = bh / p.H; h = bh % p.H; q0 = qt * BQ;
-    n = (min(q0 + BQ, p.T) + BKV - 1) / BKV;
+  // item w -> (query tile, batch, head) and its number of key tiles; the tiles that see the most keys come first.  Returns
+  // the index of the item's tensor maps; b is 0 there when every sequence has its own.
+  auto decode = [&](int w, int& b, int& h, int& q0, int& n) -> int {
+    if constexpr (NSEG > 1) {
+      const int pr = seg.pair[w / p.H], sg = pr % MAX_SEGS;
+      b = 0; h = w % p.H; q0 = pr / MAX_SEGS * BQ;
+      n = (min(q0 + BQ, seg.T[sg]) + BKV - 1) / BKV;
+      return sg;
+    } else {
+      const int qt = n_qt - 1 - w / BH, bh = w % BH;
+      b = bh / p.H; h = bh % p.H; q0 = qt * BQ;
+      n = (min(q0 + BQ, p.T) + BKV - 1) / BKV;
+      return 0;
+    }
   };
   const bool live = *abort_flag == 0;
 
@@ -154,20 +172,20 @@ flash_fwd_ws_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
       bool ok = true;
       for (int w = blockIdx.x; ok && w < n_items; w += gridDim.x, ic++) {
         int b, h, q0, n;
-        decode(w, b, h, q0, n);
+        const int sg = decode(w, b, h, q0, n);
         if (!mbar_wait(bar_qfree, (ic & 1) ^ 1, abort_flag, 6, p.err)) break;
         mbar_expect_tx(bar_qfull, C::Q_BYTES);
-        load_tile<HD>(sQ, &map_q, bar_qfull, h * HD, b * p.T + q0, BQ);
+        load_tile<HD>(sQ, &maps.q[sg], bar_qfull, h * HD, b * p.T + q0, BQ);
         for (int j = 0; j < n; j++, kvc++) {
           const int s = kvc % NS;
           const uint32_t par = ((kvc / NS) & 1) ^ 1;
           const uint32_t sk = sKV + s * 2 * C::KV_BYTES, sv = sk + C::KV_BYTES;
           if (!mbar_wait(bar_kfree + 8 * s, par, abort_flag, 6, p.err)) { ok = false; break; }
           mbar_expect_tx(bar_kfull + 8 * s, C::KV_BYTES);
-          load_tile<HD>(sk, &map_kv, bar_kfull + 8 * s, d + h * HD, b * p.T + j * BKV, BKV);
+          load_tile<HD>(sk, &maps.kv[sg], bar_kfull + 8 * s, d + h * HD, b * p.T + j * BKV, BKV);
           if (!mbar_wait(bar_vfree + 8 * s, par, abort_flag, 6, p.err)) { ok = false; break; }
           mbar_expect_tx(bar_vfull + 8 * s, C::KV_BYTES);
-          load_tile<HD>(sv, &map_kv, bar_vfull + 8 * s, 2 * d + h * HD, b * p.T + j * BKV, BKV);
+          load_tile<HD>(sv, &maps.kv[sg], bar_vfull + 8 * s, 2 * d + h * HD, b * p.T + j * BKV, BKV);
         }
       }
     }
@@ -229,7 +247,7 @@ flash_fwd_ws_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     bool ok = true;
     for (int w = blockIdx.x; ok && w < n_items; w += gridDim.x) {
       int b, h, q0, n;
-      decode(w, b, h, q0, n);
+      const int sg = decode(w, b, h, q0, n);
       const int qpos = q0 + row;
       float m_ref = -INFINITY, l_run = 0.f;     // reference maximum (scaled to log2 units) and normaliser
       for (int j = 0; j < n; j++) {
@@ -333,7 +351,7 @@ flash_fwd_ws_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         if (!mbar_wait(bar_epi, epc & 1, abort_flag, 6, p.err)) { ok = false; break; }
         epc++;
         if (tid == 0) {
-          tma_store_3d(&map_o, sP, h * HD + hf * 64, q0, b);
+          tma_store_3d(&maps.o[sg], sP, h * HD + hf * 64, q0, b);
           bulk_commit();
           bulk_wait_read_all();           // the buffer may be overwritten (next slab, next item's P)
         }
@@ -869,21 +887,64 @@ static int num_sms_attn() {
   return sms > 0 ? sms : 148;
 }
 
+template <int HD, int NSEG>
+int launch_fwd_items(const FwdMaps<NSEG>& maps, const FwdSegs<NSEG>& seg, const AttnParams& p, int n_items, int n_qt, cudaStream_t st) {
+  using C = FwdWs<HD>;
+  static bool once = false;
+  if (!once) { if (set_smem(flash_fwd_ws_kernel<HD, NSEG>, C::SMEM, "flash_fwd")) return -1; once = true; }
+  const int ctas = 2 * num_sms_attn();                  // two CTAs per SM
+  KH_LAUNCH((flash_fwd_ws_kernel<HD, NSEG>), n_items < ctas ? n_items : ctas, C::THREADS, C::SMEM, st, maps, seg, p, n_items, n_qt);
+  KH_LAUNCH_CHECK("flash_fwd");
+  return 0;
+}
+template <int NSEG>
+int fwd_maps(FwdMaps<NSEG>& maps, int i, const void* qkv, void* out, int B, int T, int H, int hd, int ld) {
+  const size_t rows = (size_t)B * T;
+  const CUtensorMap* mq = kh_tmap_2d_bf16(qkv, rows, 3 * H * hd, ld, 128, 64);
+  const CUtensorMap* mkv = kh_tmap_2d_bf16(qkv, rows, 3 * H * hd, ld, 64, 64);
+  const CUtensorMap* mo = kh_tmap_3d_bf16(out, (uint64_t)H * hd, T, B, (uint64_t)H * hd, (uint64_t)T * H * hd, 128, 64);
+  if (!mq || !mkv || !mo) return -1;
+  maps.q[i] = *mq; maps.kv[i] = *mkv; maps.o[i] = *mo;
+  return 0;
+}
 template <int HD>
 int launch_fwd(const void* qkv, const AttnParams& p, cudaStream_t st) {
-  using C = FwdWs<HD>;
-  const size_t rows = (size_t)p.B * p.T;
-  const CUtensorMap* mq = kh_tmap_2d_bf16(qkv, rows, 3 * p.H * HD, p.ld, C::BQ, 64);
-  const CUtensorMap* mkv = kh_tmap_2d_bf16(qkv, rows, 3 * p.H * HD, p.ld, C::BKV, 64);
-  const CUtensorMap* mo = kh_tmap_3d_bf16(p.out, (uint64_t)p.H * HD, p.T, p.B, (uint64_t)p.H * HD, (uint64_t)p.T * p.H * HD, 128, 64);
-  if (!mq || !mkv || !mo) return -1;
-  static bool once = false;
-  if (!once) { if (set_smem(flash_fwd_ws_kernel<HD>, C::SMEM, "flash_fwd")) return -1; once = true; }
+  FwdMaps<1> maps;
+  if (fwd_maps(maps, 0, qkv, p.out, p.B, p.T, p.H, HD, p.ld)) return -1;
   const int n_qt = (p.T + 127) / 128;
-  const int n_items = p.B * p.H * n_qt;
-  const int ctas = 2 * num_sms_attn();                  // two CTAs per SM
-  KH_LAUNCH((flash_fwd_ws_kernel<HD>), n_items < ctas ? n_items : ctas, C::THREADS, C::SMEM, st, *mq, *mkv, *mo, p, n_items, n_qt);
-  KH_LAUNCH_CHECK("flash_fwd");
+  return launch_fwd_items<HD, 1>(maps, FwdSegs<1>{}, p, p.B * p.H * n_qt, n_qt, st);
+}
+// Sequences of rows [row0[i], row0[i] + len[i]) of qkv and out, as many per launch as the maps and the list of pairs hold.
+template <int HD>
+int launch_fwd_varlen(const bf16* qkv, AttnParams p, const int* row0, const int* len, int n_seg, cudaStream_t st) {
+  bf16* out = p.out;
+  for (int s0 = 0; s0 < n_seg;) {
+    FwdMaps<MAX_SEGS> maps;
+    FwdSegs<MAX_SEGS> seg;
+    int n = 0, pairs = 0, most = 0;
+    while (s0 + n < n_seg && n < MAX_SEGS && pairs + (len[s0 + n] + 127) / 128 <= MAX_PAIRS) {
+      const int i = s0 + n, q = (len[i] + 127) / 128;
+      if (fwd_maps(maps, n, qkv + (size_t)row0[i] * p.ld, out + (size_t)row0[i] * p.H * HD, 1, len[i], p.H, HD, p.ld)) return -1;
+      seg.T[n] = len[i];
+      pairs += q;
+      most = q > most ? q : most;
+      n++;
+    }
+    if (n == 0) {                      // longer than the list: by itself
+      p.B = 1; p.T = len[s0]; p.out = out + (size_t)row0[s0] * p.H * HD;
+      if (launch_fwd<HD>(qkv + (size_t)row0[s0] * p.ld, p, st)) return -1;
+      s0++;
+      continue;
+    }
+    for (int i = n; i < MAX_SEGS; i++) { maps.q[i] = maps.q[0]; maps.kv[i] = maps.kv[0]; maps.o[i] = maps.o[0]; seg.T[i] = 0; }
+    int at = 0;
+    for (int qt = most - 1; qt >= 0; qt--)
+      for (int i = 0; i < n; i++)
+        if (qt < (seg.T[i] + 127) / 128) seg.pair[at++] = (uint16_t)(qt * MAX_SEGS + i);
+    p.B = 1; p.T = 0;
+    if (launch_fwd_items<HD, MAX_SEGS>(maps, seg, p, pairs * p.H, most, st)) return -1;
+    s0 += n;
+  }
   return 0;
 }
 
@@ -922,6 +983,20 @@ extern "C" int kh_flash_fwd(const void* qkv, void* out, void* lse, int B, int T,
   p.B = B; p.T = T; p.H = H; p.ld = ld; p.scale = scale; p.out = (bf16*)out; p.lse = (float*)lse;
   p.err = kh_error_word_dev();
   return hd == 64 ? launch_fwd<64>(qkv, p, (cudaStream_t)stream) : launch_fwd<128>(qkv, p, (cudaStream_t)stream);
+}
+
+// Causal attention of several sequences of different lengths: sequence i occupies rows [row0[i], row0[i] + len[i]) of qkv
+// (pitch ld) and out; row0 and len are host arrays.  No log-sum-exps are written.
+extern "C" int kh_flash_fwd_varlen(const void* qkv, void* out, const void* row0, const void* len, int n_seg, int H, int hd, int ld,
+                                   float scale, void* stream) {
+  if (hd != 64 && hd != 128) { kh_set_error("flash: head dim %d is not supported (64 or 128)", hd); return -1; }
+  for (int i = 0; i < n_seg; i++)
+    if (((const int*)row0)[i] < 0 || ((const int*)len)[i] < 1) { kh_set_error("flash_varlen: sequence %d is empty", i); return -1; }
+  AttnParams p = {};
+  p.H = H; p.ld = ld; p.scale = scale; p.out = (bf16*)out;
+  p.err = kh_error_word_dev();
+  return hd == 64 ? launch_fwd_varlen<64>((const bf16*)qkv, p, (const int*)row0, (const int*)len, n_seg, (cudaStream_t)stream)
+                  : launch_fwd_varlen<128>((const bf16*)qkv, p, (const int*)row0, (const int*)len, n_seg, (cudaStream_t)stream);
 }
 
 extern "C" int kh_flash_bwd(const void* qkv, const void* out, const void* dout, const void* lse, void* dqkv,

@@ -115,11 +115,10 @@ class InferEngine:
         if self.attn_splits > 1 and self.dev.type == "cuda":
             self.attn_scratch = torch.zeros(self.max_tokens * self.Hl * self.attn_splits * (self.hd + 1), dtype=torch.float32, **z)
         # Steps made of whole fresh prompts (every listed token belongs to a sequence that starts at position 0 in this
-        # step) run their attention on the tensor cores with the training forward kernel, one launch per prompt;
+        # step) run their attention on the tensor cores with the training forward kernel, all prompts in one launch;
         # everything else (decode steps, chunked prompts, mixed steps) goes through the paged kernel.
         self.flash_prefill = bool(flash_prefill and self.dev.type == "cuda" and self.dt == torch.bfloat16
                                   and self.hd in (64, 128))
-        self.lse_buf = torch.zeros(self.Hl * self.max_tokens, dtype=torch.float32, **z) if self.flash_prefill else None
         self._fresh = None
         self.temperature, self.seed, self.step_no = 0.0, 0, 0
         # under TP the captured step contains the fused GEMM + all-reduce kernels (their call counter
@@ -175,8 +174,7 @@ class InferEngine:
             if not decode:
                 ops.append_kv(qkv, self.kc[l], self.vc[l], pos, slot, self.d_btab, self.bs, self.Hl, self.hd, ntok)
             if not decode and self._fresh:
-                for r0, T in self._fresh:
-                    ops.flash_fwd(qkv[r0:r0 + T], att[r0:r0 + T], self.lse_buf, 1, T, self.Hl, self.hd)
+                ops.flash_fwd_varlen(qkv, att, self._fresh, self.Hl, self.hd)
             else:
                 ops.paged_attn(qkv, self.kc[l], self.vc[l], att, pos, slot, self.d_btab, self.bs, self.Hl, self.hd, ntok,
                                cfg.seq, append=decode, n_split=self.attn_splits, scratch=self.attn_scratch)

@@ -441,6 +441,20 @@ def _pad_out(src, dst, parts, H, hd, hp):
     dst[:, :parts * H * hd].copy_(src.view(R, parts, H, hp)[:, :, :, :hd].reshape(R, parts * H * hd))
 
 
+def flash_fwd_varlen(qkv, out, segs, H, hd):
+    """``flash_fwd`` of several sequences of their own lengths, ``segs = [(first row, length), ...]``, in one launch (per
+    sixteen); no log-sum-exps.  Head widths 64 and 128."""
+    if _use_reference(qkv):
+        for r, n in segs:
+            ref.flash_fwd(qkv[r:r + n], out[r:r + n], None, 1, n, H, hd)
+        return
+    rows = torch.tensor([r for r, _ in segs] + [n for _, n in segs], dtype=torch.int32)
+    k = len(segs)
+    assert all(0 <= r and r + n <= qkv.shape[0] for r, n in segs)
+    _call(_lib().kh_flash_fwd_varlen, 1, qkv.data_ptr(), out.data_ptr(), rows.data_ptr(), rows.data_ptr() + 4 * k, k, H, hd,
+          qkv.stride(0), 1.0 / math.sqrt(hd), _stream())
+
+
 def flash_fwd(qkv, out, lse, B, T, H, hd):
     """Causal attention over the fused projection ``qkv`` [B*T, 3*H*hd] (q | k | v blocks,
     head-major inside each); writes ``out`` [B*T, H*hd] and ``lse`` [B, H, T] (fp32)."""

@@ -525,3 +525,58 @@ def test_grpo_device_advantages_and_coefficients_match_host():
     ops.grpo_coef(adv_d, p_cur.to(DEV), p_ref.to(DEV), rows, T, 8, T - 2, 0.04, coef_d)
     assert torch.allclose(adv_d.cpu(), adv_h, rtol=1e-5, atol=1e-6)
     assert torch.allclose(coef_d.cpu(), coef_h, rtol=1e-4, atol=1e-7)
+
+
+@pytest.mark.parametrize("hd,H,lens", [(64, 4, [1]), (64, 2, [129, 64, 1, 300, 128, 2]), (128, 3, [65, 511, 127]),
+                                       (64, 1, [40 + 17 * i for i in range(19)]), (64, 1, [1000 * 66, 5])])
+def test_flash_varlen_matches_one_launch_per_sequence(hd, H, lens):
+    """Several sequences in one launch against the single-sequence launch of the same kernel, which does the same arithmetic
+    tile by tile: identical bits.  Rows between the sequences hold NaN and must neither be read into a result nor written;
+    more sequences than one launch holds; a sequence with more query tiles than the list of pairs."""
+    torch.manual_seed(len(lens))
+    rows = sum(lens) + 3 * len(lens)
+    qkv = torch.full((rows, 3 * H * hd), float("nan"), device="cuda").bfloat16()
+    segs, r = [], 2
+    for n in lens:
+        segs.append((r, n))
+        qkv[r:r + n] = torch.randn(n, 3 * H * hd, device="cuda").bfloat16()
+        r += n + 3
+    out = torch.full((rows, H * hd), 7.0, device="cuda").bfloat16()
+    want = out.clone()
+    lse = torch.empty(H * max(lens), device="cuda")
+    for r, n in segs:
+        if n > 64:
+            ops.flash_fwd(qkv[r:r + n], want[r:r + n], lse, 1, n, H, hd)
+        else:                                            # (short sequences by themselves take another kernel)
+            ops.flash_fwd_varlen(qkv[r:r + n], want[r:r + n], [(0, n)], H, hd)
+            ref.flash_fwd(qkv[r:r + n].float(), out[r:r + n], None, 1, n, H, hd)
+            assert relerr(want[r:r + n], out[r:r + n]) < 1e-2
+            out[r:r + n] = 7.0
+    ops.flash_fwd_varlen(qkv, out, segs, H, hd)
+    assert torch.equal(out, want) and not out.isnan().any()
+    assert ops.error_word() == 0
+
+
+@pytest.mark.parametrize("B,T,H,hd", [(1, 1, 1, 64), (3, 5, 2, 64), (40, 18, 8, 64), (2, 16, 3, 128), (5, 33, 2, 128), (4, 48, 4, 64), (2, 64, 3, 64),
+                                      (2, 64, 2, 128)])
+def test_flash_short_sequences(B, T, H, hd):
+    """Attention of up to 64 positions (its own kernels) against fp64: P and dS round to bf16 (2^-9 each), outputs once more;
+    the tile kernels, measured the same way, are off by 2.4e-3."""
+    torch.manual_seed(B + T)
+    d = H * hd
+    qkv, dout = torch.randn(B * T, 3 * d, device="cuda").bfloat16(), torch.randn(B * T, d, device="cuda").bfloat16()
+    out, lse = torch.empty(B * T, d, device="cuda", dtype=torch.bfloat16), torch.empty(B, H, T, device="cuda")
+    dqkv, delta = torch.full_like(qkv, 7.0), torch.empty(B, H, T, device="cuda")
+    ops.flash_fwd(qkv, out, lse, B, T, H, hd)
+    ops.flash_bwd(qkv, out, dout, lse, dqkv, delta, B, T, H, hd)
+    x = qkv.double().requires_grad_()
+    q, k, v = x.view(B, T, 3, H, hd).permute(2, 0, 3, 1, 4)
+    s = (q @ k.transpose(-1, -2)) / hd ** 0.5
+    s = s.masked_fill(~torch.ones(T, T, dtype=torch.bool, device="cuda").tril(), float("-inf"))
+    o = (torch.softmax(s, -1) @ v).permute(0, 2, 1, 3).reshape(B * T, d)
+    o.backward(dout.double())
+    assert relerr(out, o) < 4e-3 and relerr(lse, torch.logsumexp(s, -1)) < 1e-5
+    assert relerr(dqkv, x.grad) < (6e-3 if T > 1 else 1e-2)
+    again = torch.empty_like(dqkv)
+    ops.flash_bwd(qkv, out, dout, lse, again, delta, B, T, H, hd)
+    assert torch.equal(again, dqkv) and ops.error_word() == 0
