@@ -31,7 +31,7 @@ NVCC_FLAGS = [
 # tanh sit in a hot loop: GEMM epilogues (GELU), attention, the decode kernels.  The optimizer
 # (fp32 master weights, Adam moments), LayerNorm statistics, the loss and the ZeRO step are
 # compiled with IEEE division and square root; their softmax exponentials call __expf explicitly.
-FAST_MATH_FILES = {"gemm_tcgen05.cu", "gemm_skinny.cu", "flash_tcgen05.cu", "paged.cu", "fused_tp.cu"}
+FAST_MATH_FILES = {"gemm_tcgen05.cu", "gemm_skinny.cu", "flash_tcgen05.cu", "flash_short.cu", "paged.cu", "fused_tp.cu"}
 
 
 def _newer(srcs, target: Path) -> bool:

@@ -24,6 +24,7 @@
 // stores, releases TMEM and returns.
 #include "common.cuh"
 
+#include "flash_short.h"
 
 #define KH_LAUNCH_CHECK(name)                                                     \
   do {                                                                            \
@@ -979,6 +980,8 @@ int launch_bwd(const void* qkv, const AttnParams& p, cudaStream_t st) {
 extern "C" int kh_flash_fwd(const void* qkv, void* out, void* lse, int B, int T, int H, int hd, int ld, float scale,
                             void* stream) {
   if (hd != 64 && hd != 128) { kh_set_error("flash: head dim %d is not supported (64 or 128)", hd); return -1; }
+  // a tile of 128 rows would be at most half full: see flash_short.cu
+  if (T >= 1 && T <= KH_FLASH_SHORT_T) return kh_flash_short_fwd(qkv, out, lse, B, T, H, hd, ld, scale, stream);
   AttnParams p = {};
   p.B = B; p.T = T; p.H = H; p.ld = ld; p.scale = scale; p.out = (bf16*)out; p.lse = (float*)lse;
   p.err = kh_error_word_dev();
@@ -1002,6 +1005,7 @@ extern "C" int kh_flash_fwd_varlen(const void* qkv, void* out, const void* row0,
 extern "C" int kh_flash_bwd(const void* qkv, const void* out, const void* dout, const void* lse, void* dqkv,
                             void* delta, int B, int T, int H, int hd, int ld, float scale, void* stream) {
   if (hd != 64 && hd != 128) { kh_set_error("flash: head dim %d is not supported (64 or 128)", hd); return -1; }
+  if (T >= 1 && T <= KH_FLASH_SHORT_T) return kh_flash_short_bwd(qkv, out, dout, lse, dqkv, delta, B, T, H, hd, ld, scale, stream);
   AttnParams p = {};
   p.B = B; p.T = T; p.H = H; p.ld = ld; p.scale = scale; p.lse = (float*)lse; p.o = (const bf16*)out;
   p.dout = (const bf16*)dout; p.delta = (float*)delta; p.dqkv = (bf16*)dqkv;
