@@ -292,3 +292,21 @@ def test_index_guards_record_a_status_code_instead_of_reading_out_of_range():
     torch.cuda.synchronize()
     assert ops.error_word() == 8
     assert torch.equal(kc[0, 1].reshape(-1), qkv[0, H * hd:2 * H * hd]) and float(kc[2:].abs().max()) == 0.0
+
+
+@pytest.mark.parametrize("V,ld,off", [(2049, 2056, 0), (50257, 50304, 0), (8193, 8200, 1), (131073, 131080, 0)])
+def test_greedy_rows_of_large_vocabularies(V, ld, off):
+    """Greedy sampling picks the lowest index of the maximum: ties in every position of a 16-byte piece and across threads,
+    NaN ignored, the ragged tail, rows that are not 16-byte aligned, several tokens per row."""
+    g = torch.Generator(device="cuda").manual_seed(V)
+    buf = torch.randn(6 * ld + 8, device="cuda", generator=g).bfloat16()
+    lg = buf[off:off + 6 * ld].view(6, ld)
+    for r, (i, j) in enumerate([(0, 1), (5, V - 1), (V - 1, V - 1), (8 * 1024 + 3 if V > 8200 else 77, 8 * 1024 + 9 if V > 8210 else 78), (1023, 1024)]):
+        lg[r, j] = 100.0
+        lg[r, i] = 100.0
+    lg[5, 3] = float("nan")
+    out = torch.full((6 * 3,), -1, device="cuda", dtype=torch.int32)
+    ops.sample(lg, V, 0.0, 1, 0, 3, out, 6)
+    x = lg[:, :V].float().nan_to_num(nan=float("-inf"))
+    want = (x == x.max(-1, keepdim=True).values).float().argmax(-1).int().repeat_interleave(3)
+    assert torch.equal(out, want)
