@@ -17,7 +17,7 @@
 namespace {
 
 constexpr float LOG2E = 1.4426950408889634f;
-constexpr int MAX_T = KH_FLASH_SHORT_T;
+static_assert(KH_FLASH_SHORT_T == 64, "one to four row tiles of 16");
 
 __device__ __forceinline__ void ldsm4(uint32_t (&r)[4], uint32_t a) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a) : "memory");
@@ -56,10 +56,10 @@ __device__ __forceinline__ void load_rows(uint32_t dst, const bf16* src, size_t 
   }
 }
 // acc[16 x 8 nt] = rows r0.. of X times rows 0.. of Y transposed (nt column tiles of 8, only tiles [lo, hi) are formed)
-template <int HD>
-__device__ __forceinline__ void scores(float (&acc)[MAX_T / 8][4], uint32_t X, uint32_t Y, int lane, int r0, int lo, int hi) {
+template <int HD, int RT>
+__device__ __forceinline__ void scores(float (&acc)[2 * RT][4], uint32_t X, uint32_t Y, int lane, int r0, int lo, int hi) {
 #pragma unroll
-  for (int t = 0; t < MAX_T / 8; t++)
+  for (int t = 0; t < 2 * RT; t++)
 #pragma unroll
     for (int i = 0; i < 4; i++) acc[t][i] = 0.f;
 #pragma unroll
@@ -67,7 +67,7 @@ __device__ __forceinline__ void scores(float (&acc)[MAX_T / 8][4], uint32_t X, u
     uint32_t a[4];
     ldsm4(a, Tile<HD>::a(X, lane, r0, k));
 #pragma unroll
-    for (int t = 0; t < MAX_T / 16; t++)
+    for (int t = 0; t < RT; t++)
       if (2 * t >= lo && 2 * t < hi) {
         uint32_t b[4];
         ldsm4(b, Tile<HD>::b(Y, lane, t * 16, k));
@@ -77,10 +77,10 @@ __device__ __forceinline__ void scores(float (&acc)[MAX_T / 8][4], uint32_t X, u
   }
 }
 // acc[16 x HD] += P[16 x 16 t] times rows of Y (tiles [lo, hi) of P, in bf16)
-template <int HD>
-__device__ __forceinline__ void accumulate(float (&acc)[HD / 8][4], const float (&p)[MAX_T / 8][4], uint32_t Y, int lane, int lo, int hi) {
+template <int HD, int RT>
+__device__ __forceinline__ void accumulate(float (&acc)[HD / 8][4], const float (&p)[2 * RT][4], uint32_t Y, int lane, int lo, int hi) {
 #pragma unroll
-  for (int t = 0; t < MAX_T / 16; t++)
+  for (int t = 0; t < RT; t++)
     if (2 * t >= lo && 2 * t < hi) {
       const uint32_t a[4] = {pack_bf16(p[2 * t][0], p[2 * t][1]), pack_bf16(p[2 * t][2], p[2 * t][3]),
                              pack_bf16(p[2 * t + 1][0], p[2 * t + 1][1]), pack_bf16(p[2 * t + 1][2], p[2 * t + 1][3])};
@@ -103,13 +103,14 @@ __device__ __forceinline__ void store(bf16* dst, size_t ld, const float (&acc)[H
   }
 }
 
-template <int HD>
-__global__ void __launch_bounds__(128)
+template <int HD, int RT>
+__global__ void __launch_bounds__(32 * RT)
 flash_short_fwd_k(const bf16* __restrict__ qkv, int ld, bf16* __restrict__ out, float* __restrict__ lse, int T, int H, float scale) {
   extern __shared__ __align__(16) uint8_t smem[];
   pdl_wait();
   pdl_launch_dependents();
-  const int b = blockIdx.x / H, h = blockIdx.x % H, d = H * HD, rows = blockDim.x / 2;       // 16 rows a warp
+  const int b = blockIdx.x / H, h = blockIdx.x % H, d = H * HD;
+  constexpr int rows = 16 * RT;
   const uint32_t sQ = smem_u32(smem), sK = sQ + rows * Tile<HD>::PITCH, sV = sK + rows * Tile<HD>::PITCH;
   const bf16* src = qkv + (size_t)b * T * ld + h * HD;
   load_rows<HD>(sQ, src, ld, T, rows);
@@ -118,12 +119,12 @@ flash_short_fwd_k(const bf16* __restrict__ qkv, int ld, bf16* __restrict__ out, 
   __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, r0 = warp * 16, g = lane >> 2, c = (lane & 3) * 2;
   const int hi = 2 * (warp + 1);                   // column tiles up to the diagonal
-  float s[MAX_T / 8][4];
-  scores<HD>(s, sQ, sK, lane, r0, 0, hi);
+  float s[2 * RT][4];
+  scores<HD, RT>(s, sQ, sK, lane, r0, 0, hi);
   const float sl2 = scale * LOG2E;
   float mx[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};
 #pragma unroll
-  for (int t = 0; t < MAX_T / 8; t++)
+  for (int t = 0; t < 2 * RT; t++)
     if (t < hi)
 #pragma unroll
       for (int i = 0; i < 4; i++) {
@@ -136,7 +137,7 @@ flash_short_fwd_k(const bf16* __restrict__ qkv, int ld, bf16* __restrict__ out, 
     mx[i] = fmaxf(mx[i], __shfl_xor_sync(0xffffffffu, mx[i], 2)) * sl2;
   }
 #pragma unroll
-  for (int t = 0; t < MAX_T / 8; t++)
+  for (int t = 0; t < 2 * RT; t++)
     if (t < hi)
 #pragma unroll
       for (int i = 0; i < 4; i++) {
@@ -153,7 +154,7 @@ flash_short_fwd_k(const bf16* __restrict__ qkv, int ld, bf16* __restrict__ out, 
   for (int t = 0; t < HD / 8; t++)
 #pragma unroll
     for (int i = 0; i < 4; i++) o[t][i] = 0.f;
-  accumulate<HD>(o, s, sV, lane, 0, hi);
+  accumulate<HD, RT>(o, s, sV, lane, 0, hi);
   store<HD>(out + (size_t)b * T * d + h * HD, d, o, 1.f / l[0], 1.f / l[1], lane, r0, T);
   if (lse && (lane & 3) == 0) {
     float* q = lse + ((size_t)b * H + h) * T;
@@ -162,15 +163,16 @@ flash_short_fwd_k(const bf16* __restrict__ qkv, int ld, bf16* __restrict__ out, 
   }
 }
 
-template <int HD>
-__global__ void __launch_bounds__(256)
+template <int HD, int RT>
+__global__ void __launch_bounds__(64 * RT)
 flash_short_bwd_k(const bf16* __restrict__ qkv, int ld, const bf16* __restrict__ out, const bf16* __restrict__ dout,
                   const float* __restrict__ lse, bf16* __restrict__ dqkv, float* __restrict__ delta, int T, int H, float scale) {
   extern __shared__ __align__(16) uint8_t smem[];
-  __shared__ float s_lse[MAX_T], s_delta[MAX_T];
+  __shared__ float s_lse[16 * RT], s_delta[16 * RT];
   pdl_wait();
   pdl_launch_dependents();
-  const int b = blockIdx.x / H, h = blockIdx.x % H, d = H * HD, RT = blockDim.x / 64, rows = RT * 16;
+  const int b = blockIdx.x / H, h = blockIdx.x % H, d = H * HD;
+  constexpr int rows = 16 * RT;
   const uint32_t sQ = smem_u32(smem), sK = sQ + rows * Tile<HD>::PITCH, sV = sK + rows * Tile<HD>::PITCH, sD = sV + rows * Tile<HD>::PITCH;
   const bf16* src = qkv + (size_t)b * T * ld + h * HD;
   const bf16* dsrc = dout + (size_t)b * T * d + h * HD;
@@ -203,7 +205,7 @@ flash_short_bwd_k(const bf16* __restrict__ qkv, int ld, const bf16* __restrict__
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, c = (lane & 3) * 2;
   const float sl2 = scale * LOG2E;
   bf16* dst = dqkv + (size_t)b * T * ld + h * HD;
-  float s[MAX_T / 8][4], dp[MAX_T / 8][4];
+  float s[2 * RT][4], dp[2 * RT][4];
   float acc[HD / 8][4];
 #pragma unroll
   for (int t = 0; t < HD / 8; t++)
@@ -211,11 +213,11 @@ flash_short_bwd_k(const bf16* __restrict__ qkv, int ld, const bf16* __restrict__
     for (int i = 0; i < 4; i++) acc[t][i] = 0.f;
   if (warp < RT) {                                 // 16 queries, keys up to the diagonal
     const int r0 = warp * 16, hi = 2 * (warp + 1);
-    scores<HD>(s, sQ, sK, lane, r0, 0, hi);
-    scores<HD>(dp, sD, sV, lane, r0, 0, hi);
+    scores<HD, RT>(s, sQ, sK, lane, r0, 0, hi);
+    scores<HD, RT>(dp, sD, sV, lane, r0, 0, hi);
     const float ls[2] = {s_lse[r0 + g], s_lse[r0 + g + 8]}, de[2] = {s_delta[r0 + g], s_delta[r0 + g + 8]};
 #pragma unroll
-    for (int t = 0; t < MAX_T / 8; t++)
+    for (int t = 0; t < 2 * RT; t++)
       if (t < hi)
 #pragma unroll
         for (int i = 0; i < 4; i++) {
@@ -223,13 +225,13 @@ flash_short_bwd_k(const bf16* __restrict__ qkv, int ld, const bf16* __restrict__
           if (t * 8 + c + (i & 1) > r0 + g + (i >> 1) * 8) p = 0.f;
           s[t][i] = p * (dp[t][i] - de[i >> 1]) * scale;
         }
-    accumulate<HD>(acc, s, sK, lane, 0, hi);
+    accumulate<HD, RT>(acc, s, sK, lane, 0, hi);
     store<HD>(dst, ld, acc, 1.f, 1.f, lane, r0, T);
   } else {                                         // 16 keys, queries from the diagonal on
     const int r0 = (warp - RT) * 16, lo = 2 * (warp - RT), hi = 2 * RT;
-    scores<HD>(s, sK, sQ, lane, r0, lo, hi);
+    scores<HD, RT>(s, sK, sQ, lane, r0, lo, hi);
 #pragma unroll
-    for (int t = 0; t < MAX_T / 8; t++)
+    for (int t = 0; t < 2 * RT; t++)
       if (t >= lo && t < hi)
 #pragma unroll
         for (int i = 0; i < 4; i++) {
@@ -238,11 +240,11 @@ flash_short_bwd_k(const bf16* __restrict__ qkv, int ld, const bf16* __restrict__
           if (r0 + g + (i >> 1) * 8 > q) p = 0.f;
           s[t][i] = p;
         }
-    accumulate<HD>(acc, s, sD, lane, lo, hi);
+    accumulate<HD, RT>(acc, s, sD, lane, lo, hi);
     store<HD>(dst + 2 * d, ld, acc, 1.f, 1.f, lane, r0, T);
-    scores<HD>(dp, sV, sD, lane, r0, lo, hi);
+    scores<HD, RT>(dp, sV, sD, lane, r0, lo, hi);
 #pragma unroll
-    for (int t = 0; t < MAX_T / 8; t++)
+    for (int t = 0; t < 2 * RT; t++)
       if (t >= lo && t < hi)
 #pragma unroll
         for (int i = 0; i < 4; i++) s[t][i] = s[t][i] * (dp[t][i] - s_delta[t * 8 + c + (i & 1)]) * scale;
@@ -250,7 +252,7 @@ flash_short_bwd_k(const bf16* __restrict__ qkv, int ld, const bf16* __restrict__
     for (int t = 0; t < HD / 8; t++)
 #pragma unroll
       for (int i = 0; i < 4; i++) acc[t][i] = 0.f;
-    accumulate<HD>(acc, s, sQ, lane, lo, hi);
+    accumulate<HD, RT>(acc, s, sQ, lane, lo, hi);
     store<HD>(dst + d, ld, acc, 1.f, 1.f, lane, r0, T);
   }
 }
@@ -265,34 +267,35 @@ int opt_in(K kernel, int bytes) {
   kh_set_error("flash: cannot opt in to %d bytes of shared memory", bytes);
   return -1;
 }
-template <int HD>
+template <int HD, int RT>
 int fwd(const bf16* qkv, bf16* out, float* lse, int B, int T, int H, int ld, float scale, cudaStream_t st) {
-  const int RT = (T + 15) / 16, smem = 3 * RT * 16 * Tile<HD>::PITCH;
-  if (opt_in(flash_short_fwd_k<HD>, smem)) return -1;
-  if (KH_LAUNCH((flash_short_fwd_k<HD>), B * H, 32 * RT, smem, st, qkv, ld, out, lse, T, H, scale) != cudaSuccess) { kh_set_error("flash_short_fwd: launch failed"); return -1; }
+  const int smem = 3 * RT * 16 * Tile<HD>::PITCH;
+  if (opt_in(flash_short_fwd_k<HD, RT>, smem)) return -1;
+  if (KH_LAUNCH((flash_short_fwd_k<HD, RT>), B * H, 32 * RT, smem, st, qkv, ld, out, lse, T, H, scale) != cudaSuccess) { kh_set_error("flash_short_fwd: launch failed"); return -1; }
   return 0;
 }
-template <int HD>
+template <int HD, int RT>
 int bwd(const bf16* qkv, const bf16* out, const bf16* dout, const float* lse, bf16* dqkv, float* delta, int B, int T, int H, int ld,
         float scale, cudaStream_t st) {
-  const int RT = (T + 15) / 16, smem = 4 * RT * 16 * Tile<HD>::PITCH;
-  if (opt_in(flash_short_bwd_k<HD>, smem)) return -1;
-  if (KH_LAUNCH((flash_short_bwd_k<HD>), B * H, 64 * RT, smem, st, qkv, ld, out, dout, lse, dqkv, delta, T, H, scale) != cudaSuccess) { kh_set_error("flash_short_bwd: launch failed"); return -1; }
+  const int smem = 4 * RT * 16 * Tile<HD>::PITCH;
+  if (opt_in(flash_short_bwd_k<HD, RT>, smem)) return -1;
+  if (KH_LAUNCH((flash_short_bwd_k<HD, RT>), B * H, 64 * RT, smem, st, qkv, ld, out, dout, lse, dqkv, delta, T, H, scale) != cudaSuccess) { kh_set_error("flash_short_bwd: launch failed"); return -1; }
   return 0;
 }
+#define BY_ROWS(FN, HD, ...) (T <= 16 ? FN<HD, 1>(__VA_ARGS__) : T <= 32 ? FN<HD, 2>(__VA_ARGS__) : T <= 48 ? FN<HD, 3>(__VA_ARGS__) : FN<HD, 4>(__VA_ARGS__))
 
 }  // namespace
 
 int kh_flash_short_fwd(const void* qkv, void* out, void* lse, int B, int T, int H, int hd, int ld, float scale, void* stream) {
   if (check(qkv, ld, "qkv") || check(out, 0, "out")) return -1;
   cudaStream_t st = (cudaStream_t)stream;
-  return hd == 64 ? fwd<64>((const bf16*)qkv, (bf16*)out, (float*)lse, B, T, H, ld, scale, st)
-                  : fwd<128>((const bf16*)qkv, (bf16*)out, (float*)lse, B, T, H, ld, scale, st);
+  return hd == 64 ? BY_ROWS(fwd, 64, (const bf16*)qkv, (bf16*)out, (float*)lse, B, T, H, ld, scale, st)
+                  : BY_ROWS(fwd, 128, (const bf16*)qkv, (bf16*)out, (float*)lse, B, T, H, ld, scale, st);
 }
 int kh_flash_short_bwd(const void* qkv, const void* out, const void* dout, const void* lse, void* dqkv, void* delta, int B, int T,
                        int H, int hd, int ld, float scale, void* stream) {
   if (check(qkv, ld, "qkv") || check(out, 0, "out") || check(dout, 0, "dout") || check(dqkv, ld, "dqkv")) return -1;
   cudaStream_t st = (cudaStream_t)stream;
-  return hd == 64 ? bwd<64>((const bf16*)qkv, (const bf16*)out, (const bf16*)dout, (const float*)lse, (bf16*)dqkv, (float*)delta, B, T, H, ld, scale, st)
-                  : bwd<128>((const bf16*)qkv, (const bf16*)out, (const bf16*)dout, (const float*)lse, (bf16*)dqkv, (float*)delta, B, T, H, ld, scale, st);
+  return hd == 64 ? BY_ROWS(bwd, 64, (const bf16*)qkv, (const bf16*)out, (const bf16*)dout, (const float*)lse, (bf16*)dqkv, (float*)delta, B, T, H, ld, scale, st)
+                  : BY_ROWS(bwd, 128, (const bf16*)qkv, (const bf16*)out, (const bf16*)dout, (const float*)lse, (bf16*)dqkv, (float*)delta, B, T, H, ld, scale, st);
 }
