@@ -405,18 +405,24 @@ __global__ void flash_delta_kernel(const bf16* __restrict__ o, const bf16* __res
 }
 
 // ================================================================================ backward, warp-specialised
-// Both backward kernels are persistent (one CTA per SM) with ten warps: eight compute warps (two
+// Both backward kernels are persistent with ten warps: eight compute warps (two
 // threads per row of the CTA's 128-row tile, each taking 32 of a sub-tile's 64 columns), a TMA warp
 // and an MMA warp.  The other sequence dimension is walked in sub-tiles of 64 through a four-stage
 // TMA ring, so S and dP take 64 TMEM columns each and fit twice: the MMA warp issues S(t+1),
 // dP(t+1) while the compute warps turn S(t), dP(t) into P(t), dS(t), and issues the accumulating
 // products of sub-tile t as soon as those are in shared memory.  Gradients stay in TMEM for the
 // whole item.  Work items are handed out longest first.
-template <int HD>
+// TWO (head width 64): S, dP and the gradients take half of the tensor memory when S and dP are held once, and two ring stages
+// half of the shared memory, so two CTAs share an SM and fill each other's gaps in the chain S -> tcgen05.ld -> exponentials ->
+// shared memory -> accumulating products.  B2 H16 T1777: dK/dV 82.5 -> 75 us, dQ 68 -> 58; B32 H8 T256: 26.8 -> 21.5 and 20.6 -> 16.7.
+// Head width 128, or no more items than SMs (B32 H4 T128: 7.6 us with one CTA, 8.3 with this form): one CTA with two S / dP buffers.
+template <int HD, bool TWO>
 struct BwdWs {
-  static constexpr int BT = 128, BS = 64, NS = 4;
+  static constexpr int BT = 128, BS = 64, NS = TWO ? 2 : 4, CTAS = TWO ? 2 : 1;
+  static constexpr int BUFS = TWO ? 1 : 2, ACC = 2 * BUFS * 64;            // S / dP buffers; first TMEM column of the gradients
+  static constexpr int CW = TWO ? 16 : 32;                                 // columns a compute thread takes from TMEM at a time
   static constexpr int TILE = BT * HD * 2, SUB = BS * HD * 2, PS_BYTES = BT * BS * 2;
-  static constexpr int THREADS = 320, TMEM_COLS = 512;
+  static constexpr int THREADS = 320, TMEM_COLS = TWO ? 256 : 512;
   // dK/dV: K, V tiles; ring of (Q, dO) sub-tiles; P^T and dS^T; lse / delta of two sub-tiles
   static constexpr int DATA_KV = 2 * TILE + NS * 2 * SUB + 2 * PS_BYTES + 2 * 128 * 4;
   static constexpr int SMEM_KV = DATA_KV + 256;
@@ -425,14 +431,24 @@ struct BwdWs {
   static constexpr int SMEM_Q = DATA_Q + 256;
 };
 
+// One arrival per warp: the writes of its lanes are ordered before it by the warp barrier (an arrival per thread is 32 updates
+// of the barrier word one after the other).
+__device__ __forceinline__ void warp_arrive(uint32_t bar, int lane) {
+  __syncwarp();
+  if (lane == 0) mbar_arrive(bar);
+}
+template <int W> __device__ __forceinline__ void tmem_cols(uint32_t a, uint32_t* r) {
+  if (W == 32) tmem_ld32(a, r); else tmem_ld16(a, r);
+}
+
 // ---- dK, dV: item = (batch, head, 128 keys); sub-tiles of 64 queries from the diagonal to the end
-template <int HD>
-__global__ void __launch_bounds__(320, 1)
+template <int HD, bool TWO>
+__global__ void __launch_bounds__(320, BwdWs<HD, TWO>::CTAS)
 flash_dkv_ws_kernel(const __grid_constant__ CUtensorMap map_kv, const __grid_constant__ CUtensorMap map_q,
                     const __grid_constant__ CUtensorMap map_do, const __grid_constant__ CUtensorMap map_dqkv, const AttnParams p,
                     int n_items, int n_kt) {
-  using C = BwdWs<HD>;
-  constexpr int BT = C::BT, BS = C::BS, NS = C::NS;
+  using C = BwdWs<HD, TWO>;
+  constexpr int BT = C::BT, BS = C::BS, NS = C::NS, BUFS = C::BUFS, ACC = C::ACC, CW = C::CW;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   const uint32_t base = smem_u32(smem_raw);
   const uint32_t sK = base, sV = sK + C::TILE, sQD = sV + C::TILE, sP = sQD + NS * 2 * C::SUB, sDS = sP + C::PS_BYTES;
@@ -449,7 +465,7 @@ flash_dkv_ws_kernel(const __grid_constant__ CUtensorMap map_kv, const __grid_con
     mbar_init(bar_kvfull, 1); mbar_init(bar_kvfree, 1);
     for (int s = 0; s < NS; s++) { mbar_init(bar_qfull + 8 * s, 1); mbar_init(bar_qfree + 8 * s, 1); }
     mbar_init(bar_sfull, 1); mbar_init(bar_sfull + 8, 1);
-    mbar_init(bar_ready, 8); mbar_init(bar_gdone, 1); mbar_init(bar_accfree, 8); mbar_init(bar_stat, 256);
+    mbar_init(bar_ready, 8); mbar_init(bar_gdone, 1); mbar_init(bar_accfree, 8); mbar_init(bar_stat, 8);
     *abort_flag = (base & 1023u) ? 6 : 0;
     if (base & 1023u) atomicCAS(p.err, 0, 6);
     mbar_fence_init();
@@ -505,34 +521,42 @@ flash_dkv_ws_kernel(const __grid_constant__ CUtensorMap map_kv, const __grid_con
         if (!mbar_wait(bar_kvfull, ic & 1, abort_flag, 6, p.err)) break;
         const int q_base = qc;
         for (int t = 0; t <= n && ok; t++) {
+          // with one S / dP buffer the next products may overwrite it once P and dS of the sub-tile before are in shared memory
+          if (BUFS == 1 && t >= 1) {
+            if (!mbar_wait(bar_ready, rc & 1, abort_flag, 6, p.err)) { ok = false; break; }
+            rc++;
+            tc_fence_after();
+          }
           if (t < n) {
             const int s = qc % NS;
             if (!mbar_wait(bar_qfull + 8 * s, (qc / NS) & 1, abort_flag, 6, p.err)) { ok = false; break; }
             qc++;
             tc_fence_after();
             const uint32_t sq = sQD + s * 2 * C::SUB, sdo = sq + C::SUB;
-            const uint32_t tS = tmem + (t & 1) * 64, tDP = tmem + 128 + (t & 1) * 64;
+            const uint32_t tS = tmem + (t & (BUFS - 1)) * 64, tDP = tmem + BUFS * 64 + (t & (BUFS - 1)) * 64;
             const uint64_t dq0 = dk0(sq), ddo0 = dk0(sdo);
 #pragma unroll
             for (int kk = 0; kk < HD / 16; kk++) {
               umma_f16_ss(tS, DK(dK0, BT, kk), DK(dq0, BS, kk), idesc_s, kk > 0);
               umma_f16_ss(tDP, DK(dV0, BT, kk), DK(ddo0, BS, kk), idesc_s, kk > 0);
             }
-            umma_commit(bar_sfull + 8 * (t & 1));
+            umma_commit(bar_sfull + 8 * (t & (BUFS - 1)));
             if (t == n - 1) umma_commit(bar_kvfree);        // K and V are only read by these products
           }
           if (t >= 1) {
             const int tt = t - 1, s = (q_base + tt) % NS;
             const uint32_t sq = sQD + s * 2 * C::SUB, sdo = sq + C::SUB;
             if (tt == 0 && !mbar_wait(bar_accfree, (ic & 1) ^ 1, abort_flag, 6, p.err)) { ok = false; break; }
-            if (!mbar_wait(bar_ready, rc & 1, abort_flag, 6, p.err)) { ok = false; break; }
-            rc++;
+            if (BUFS == 2) {
+              if (!mbar_wait(bar_ready, rc & 1, abort_flag, 6, p.err)) { ok = false; break; }
+              rc++;
+            }
             tc_fence_after();
             const uint64_t mdo0 = dmn0(sdo, BS), mq0 = dmn0(sq, BS);
 #pragma unroll
             for (int kk = 0; kk < BS / 16; kk++) {
-              umma_f16_ss(tmem + 256, DK(dP0, BT, kk), DMN(mdo0, kk), idesc_g, (tt > 0 || kk > 0));
-              umma_f16_ss(tmem + 256 + HD, DK(dDS0, BT, kk), DMN(mq0, kk), idesc_g, (tt > 0 || kk > 0));
+              umma_f16_ss(tmem + ACC, DK(dP0, BT, kk), DMN(mdo0, kk), idesc_g, (tt > 0 || kk > 0));
+              umma_f16_ss(tmem + ACC + HD, DK(dDS0, BT, kk), DMN(mq0, kk), idesc_g, (tt > 0 || kk > 0));
             }
             umma_commit(bar_gdone);
             umma_commit(bar_qfree + 8 * s);
@@ -560,37 +584,44 @@ flash_dkv_ws_kernel(const __grid_constant__ CUtensorMap map_kv, const __grid_con
         return __ldg((tid < 64 ? p.lse : p.delta) + stat0 + qp);
       };
       if (tid < 128) s_stat[tid] = fetch_stat(0) * stat_mul;
-      mbar_arrive(bar_stat);
+      warp_arrive(bar_stat, lane);
       if (!mbar_wait(bar_stat, stc & 1, abort_flag, 6, p.err)) break;
       stc++;
       for (int t = 0; t < n; t++) {
-        const int buf = t & 1;
+        const int sb = t & 1, buf = t & (BUFS - 1);
         const float next_stat = fetch_stat(t + 1);
-        const float* st = s_stat + buf * 128;
+        const float* st = s_stat + sb * 128;
         if (!mbar_wait(bar_sfull + 8 * buf, sfc[buf] & 1, abort_flag, 6, p.err)) { ok = false; break; }
         sfc[buf]++;
         tc_fence_after();
         const int q0s = k0 + t * BS;
         const bool diag = k0 + BT - 1 > q0s;
         const int c = half * 32;
-        uint32_t rs[32], rd[32];
-        tmem_ld32(tmem + buf * 64 + lane_off + c, rs);
-        tmem_ld32(tmem + 128 + buf * 64 + lane_off + c, rd);
-        tmem_ld_wait();
         uint32_t pp[16], ds[16];
 #pragma unroll
-        for (int e = 0; e < 32; e += 2) {
-          float pv[2], dv[2];
+        for (int w = 0; w < 32; w += CW) {
+          uint32_t rs[CW], rd[CW];
+          tmem_cols<CW>(tmem + buf * 64 + lane_off + c + w, rs);
+          tmem_cols<CW>(tmem + BUFS * 64 + buf * 64 + lane_off + c + w, rd);
+          tmem_ld_wait();
 #pragma unroll
-          for (int u = 0; u < 2; u++) {
-            const int qi = c + e + u;
-            float pr = exp2f(fmaf(__uint_as_float(rs[e + u]), sl2, -st[qi]));
-            if (diag && kpos > q0s + qi) pr = 0.f;
-            pv[u] = pr;
-            dv[u] = pr * (__uint_as_float(rd[e + u]) - st[64 + qi]) * p.scale;
+          for (int e = 0; e < CW; e += 4) {
+            const int q0 = c + w + e;
+            const float4 l4 = *reinterpret_cast<const float4*>(st + q0), d4 = *reinterpret_cast<const float4*>(st + 64 + q0);
+            const float lv[4] = {l4.x, l4.y, l4.z, l4.w}, dl[4] = {d4.x, d4.y, d4.z, d4.w};
+            float pv[4], dv[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+              float pr = exp2f(fmaf(__uint_as_float(rs[e + u]), sl2, -lv[u]));
+              if (diag && kpos > q0s + q0 + u) pr = 0.f;
+              pv[u] = pr;
+              dv[u] = pr * (__uint_as_float(rd[e + u]) - dl[u]) * p.scale;
+            }
+            pp[(w + e) >> 1] = pack_bf16(pv[0], pv[1]);
+            pp[((w + e) >> 1) + 1] = pack_bf16(pv[2], pv[3]);
+            ds[(w + e) >> 1] = pack_bf16(dv[0], dv[1]);
+            ds[((w + e) >> 1) + 1] = pack_bf16(dv[2], dv[3]);
           }
-          pp[e >> 1] = pack_bf16(pv[0], pv[1]);
-          ds[e >> 1] = pack_bf16(dv[0], dv[1]);
         }
         // the products that read P^T / dS^T of the previous sub-tile have retired
         while (obs < uses) {
@@ -608,8 +639,8 @@ flash_dkv_ws_kernel(const __grid_constant__ CUtensorMap map_kv, const __grid_con
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(bar_ready);
-        if (tid < 128) s_stat[(buf ^ 1) * 128 + tid] = next_stat * stat_mul;
-        mbar_arrive(bar_stat);
+        if (tid < 128) s_stat[(sb ^ 1) * 128 + tid] = next_stat * stat_mul;
+        warp_arrive(bar_stat, lane);
         if (!mbar_wait(bar_stat, stc & 1, abort_flag, 6, p.err)) { ok = false; break; }
         stc++;
       }
@@ -624,7 +655,7 @@ flash_dkv_ws_kernel(const __grid_constant__ CUtensorMap map_kv, const __grid_con
       // swizzled layout) -> one TMA store per 64-column slab; rows past the end of the sequence are clipped
 #pragma unroll 1
       for (int which = 0; which < 2; which++) {
-        const uint32_t tacc = tmem + 256 + which * HD + lane_off;
+        const uint32_t tacc = tmem + ACC + which * HD + lane_off;
 #pragma unroll 1
         for (int c = half * (HD / 2); c < (half + 1) * (HD / 2); c += 32) {
           uint32_t r1[32];
@@ -639,7 +670,7 @@ flash_dkv_ws_kernel(const __grid_constant__ CUtensorMap map_kv, const __grid_con
                          pack_bf16(__uint_as_float(r1[8 * g + 6]), __uint_as_float(r1[8 * g + 7])));
         }
         fence_proxy_async_smem();
-        mbar_arrive(bar_stat);
+        warp_arrive(bar_stat, lane);
         if (!mbar_wait(bar_stat, stc & 1, abort_flag, 6, p.err)) { ok = false; break; }
         stc++;
         if (tid == 0) {
@@ -649,7 +680,7 @@ flash_dkv_ws_kernel(const __grid_constant__ CUtensorMap map_kv, const __grid_con
           bulk_commit();
           bulk_wait_read_all();
         }
-        mbar_arrive(bar_stat);
+        warp_arrive(bar_stat, lane);
         if (!mbar_wait(bar_stat, stc & 1, abort_flag, 6, p.err)) { ok = false; break; }
         stc++;
       }
@@ -666,13 +697,13 @@ flash_dkv_ws_kernel(const __grid_constant__ CUtensorMap map_kv, const __grid_con
 }
 
 // ---- dQ: item = (batch, head, 128 queries); sub-tiles of 64 keys up to the diagonal
-template <int HD>
-__global__ void __launch_bounds__(320, 1)
+template <int HD, bool TWO>
+__global__ void __launch_bounds__(320, BwdWs<HD, TWO>::CTAS)
 flash_dq_ws_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_do,
                    const __grid_constant__ CUtensorMap map_kv, const __grid_constant__ CUtensorMap map_dqkv, const AttnParams p,
                    int n_items, int n_qt) {
-  using C = BwdWs<HD>;
-  constexpr int BT = C::BT, BS = C::BS, NS = C::NS;
+  using C = BwdWs<HD, TWO>;
+  constexpr int BT = C::BT, BS = C::BS, NS = C::NS, BUFS = C::BUFS, ACC = C::ACC, CW = C::CW;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   const uint32_t base = smem_u32(smem_raw);
   const uint32_t sQ = base, sDO = sQ + C::TILE, sKV = sDO + C::TILE, sDS = sKV + NS * 2 * C::SUB;
@@ -688,7 +719,7 @@ flash_dq_ws_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
     mbar_init(bar_qfull, 1); mbar_init(bar_qfree, 1);
     for (int s = 0; s < NS; s++) { mbar_init(bar_kvfull + 8 * s, 1); mbar_init(bar_kvfree + 8 * s, 1); }
     mbar_init(bar_sfull, 1); mbar_init(bar_sfull + 8, 1);
-    mbar_init(bar_ready, 8); mbar_init(bar_gdone, 1); mbar_init(bar_accfree, 8); mbar_init(bar_epi, 256);
+    mbar_init(bar_ready, 8); mbar_init(bar_gdone, 1); mbar_init(bar_accfree, 8); mbar_init(bar_epi, 8);
     *abort_flag = (base & 1023u) ? 6 : 0;
     if (base & 1023u) atomicCAS(p.err, 0, 6);
     mbar_fence_init();
@@ -744,33 +775,40 @@ flash_dq_ws_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         if (!mbar_wait(bar_qfull, ic & 1, abort_flag, 6, p.err)) break;
         const int kv_base = kvc;
         for (int j = 0; j <= n && ok; j++) {
+          if (BUFS == 1 && j >= 1) {              // see the dK / dV kernel
+            if (!mbar_wait(bar_ready, rc & 1, abort_flag, 6, p.err)) { ok = false; break; }
+            rc++;
+            tc_fence_after();
+          }
           if (j < n) {
             const int s = kvc % NS;
             if (!mbar_wait(bar_kvfull + 8 * s, (kvc / NS) & 1, abort_flag, 6, p.err)) { ok = false; break; }
             kvc++;
             tc_fence_after();
             const uint32_t sk = sKV + s * 2 * C::SUB, sv = sk + C::SUB;
-            const uint32_t tS = tmem + (j & 1) * 64, tDP = tmem + 128 + (j & 1) * 64;
+            const uint32_t tS = tmem + (j & (BUFS - 1)) * 64, tDP = tmem + BUFS * 64 + (j & (BUFS - 1)) * 64;
             const uint64_t dk_0 = dk0(sk), dv_0 = dk0(sv);
 #pragma unroll
             for (int kk = 0; kk < HD / 16; kk++) {
               umma_f16_ss(tS, DK(dQ0, BT, kk), DK(dk_0, BS, kk), idesc_s, kk > 0);
               umma_f16_ss(tDP, DK(dDO0, BT, kk), DK(dv_0, BS, kk), idesc_s, kk > 0);
             }
-            umma_commit(bar_sfull + 8 * (j & 1));
+            umma_commit(bar_sfull + 8 * (j & (BUFS - 1)));
             if (j == n - 1) umma_commit(bar_qfree);         // Q and dO are only read by these products
           }
           if (j >= 1) {
             const int jj = j - 1, s = (kv_base + jj) % NS;
             const uint32_t sk = sKV + s * 2 * C::SUB;
             if (jj == 0 && !mbar_wait(bar_accfree, (ic & 1) ^ 1, abort_flag, 6, p.err)) { ok = false; break; }
-            if (!mbar_wait(bar_ready, rc & 1, abort_flag, 6, p.err)) { ok = false; break; }
-            rc++;
+            if (BUFS == 2) {
+              if (!mbar_wait(bar_ready, rc & 1, abort_flag, 6, p.err)) { ok = false; break; }
+              rc++;
+            }
             tc_fence_after();
             const uint64_t mk0 = dmn0(sk, BS);
 #pragma unroll
             for (int kk = 0; kk < BS / 16; kk++)
-              umma_f16_ss(tmem + 256, DK(dDS0, BT, kk), DMN(mk0, kk), idesc_g, (jj > 0 || kk > 0));
+              umma_f16_ss(tmem + ACC, DK(dDS0, BT, kk), DMN(mk0, kk), idesc_g, (jj > 0 || kk > 0));
             umma_commit(bar_gdone);
             umma_commit(bar_kvfree + 8 * s);
           }
@@ -792,28 +830,31 @@ flash_dq_ws_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
       const float my_lse = qvalid ? p.lse[sidx] * LOG2E : INFINITY;
       const float my_delta = qvalid ? p.delta[sidx] : 0.f;
       for (int j = 0; j < n; j++) {
-        const int buf = j & 1;
+        const int buf = j & (BUFS - 1);
         if (!mbar_wait(bar_sfull + 8 * buf, sfc[buf] & 1, abort_flag, 6, p.err)) { ok = false; break; }
         sfc[buf]++;
         tc_fence_after();
         const int k0 = j * BS;
         const bool diag = k0 + BS - 1 > q0;
         const int c = half * 32;
-        uint32_t rs[32], rd[32];
-        tmem_ld32(tmem + buf * 64 + lane_off + c, rs);
-        tmem_ld32(tmem + 128 + buf * 64 + lane_off + c, rd);
-        tmem_ld_wait();
         uint32_t ds[16];
 #pragma unroll
-        for (int e = 0; e < 32; e += 2) {
-          float dv[2];
+        for (int w = 0; w < 32; w += CW) {
+          uint32_t rs[CW], rd[CW];
+          tmem_cols<CW>(tmem + buf * 64 + lane_off + c + w, rs);
+          tmem_cols<CW>(tmem + BUFS * 64 + buf * 64 + lane_off + c + w, rd);
+          tmem_ld_wait();
 #pragma unroll
-          for (int u = 0; u < 2; u++) {
-            float pr = exp2f(fmaf(__uint_as_float(rs[e + u]), sl2, -my_lse));
-            if (diag && k0 + c + e + u > qpos) pr = 0.f;
-            dv[u] = pr * (__uint_as_float(rd[e + u]) - my_delta) * p.scale;
+          for (int e = 0; e < CW; e += 2) {
+            float dv[2];
+#pragma unroll
+            for (int u = 0; u < 2; u++) {
+              float pr = exp2f(fmaf(__uint_as_float(rs[e + u]), sl2, -my_lse));
+              if (diag && k0 + c + w + e + u > qpos) pr = 0.f;
+              dv[u] = pr * (__uint_as_float(rd[e + u]) - my_delta) * p.scale;
+            }
+            ds[(w + e) >> 1] = pack_bf16(dv[0], dv[1]);
           }
-          ds[e >> 1] = pack_bf16(dv[0], dv[1]);
         }
         while (obs < uses) {
           if (!mbar_wait(bar_gdone, obs & 1, abort_flag, 6, p.err)) { ok = false; break; }
@@ -840,7 +881,7 @@ flash_dq_ws_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
 #pragma unroll 1
       for (int c = half * (HD / 2); c < (half + 1) * (HD / 2); c += 32) {
         uint32_t r1[32];
-        tmem_ld32(tmem + 256 + lane_off + c, r1);
+        tmem_ld32(tmem + ACC + lane_off + c, r1);
         tmem_ld_wait();
 #pragma unroll
         for (int g = 0; g < 4; g++)
@@ -851,7 +892,7 @@ flash_dq_ws_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
                        pack_bf16(__uint_as_float(r1[8 * g + 6]), __uint_as_float(r1[8 * g + 7])));
       }
       fence_proxy_async_smem();
-      mbar_arrive(bar_epi);
+      warp_arrive(bar_epi, lane);
       if (!mbar_wait(bar_epi, epc & 1, abort_flag, 6, p.err)) { ok = false; break; }
       epc++;
       if (tid == 0) {
@@ -860,7 +901,7 @@ flash_dq_ws_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         bulk_commit();
         bulk_wait_read_all();
       }
-      mbar_arrive(bar_epi);
+      warp_arrive(bar_epi, lane);
       if (!mbar_wait(bar_epi, epc & 1, abort_flag, 6, p.err)) { ok = false; break; }
       epc++;
       tc_fence_before();
@@ -949,9 +990,9 @@ int launch_fwd_varlen(const bf16* qkv, AttnParams p, const int* row0, const int*
   return 0;
 }
 
-template <int HD>
-int launch_bwd(const void* qkv, const AttnParams& p, cudaStream_t st) {
-  using C = BwdWs<HD>;
+template <int HD, bool TWO>
+int launch_bwd_as(const void* qkv, const AttnParams& p, cudaStream_t st) {
+  using C = BwdWs<HD, TWO>;
   const size_t rows = (size_t)p.B * p.T;
   const CUtensorMap* mq = kh_tmap_2d_bf16(qkv, rows, 3 * p.H * HD, p.ld, 128, 64);
   const CUtensorMap* md = kh_tmap_2d_bf16(p.dout, rows, p.H * HD, p.H * HD, 128, 64);
@@ -962,17 +1003,22 @@ int launch_bwd(const void* qkv, const AttnParams& p, cudaStream_t st) {
   KH_LAUNCH((flash_delta_kernel<HD>), (unsigned)((rows * 32 + 255) / 256), 256, 0, st, p.o, p.dout, p.delta, p.B, p.T, p.H);
   static bool once = false;
   if (!once) {
-    if (set_smem(flash_dkv_ws_kernel<HD>, C::SMEM_KV, "flash_dkv") || set_smem(flash_dq_ws_kernel<HD>, C::SMEM_Q, "flash_dq")) return -1;
+    if (set_smem(flash_dkv_ws_kernel<HD, TWO>, C::SMEM_KV, "flash_dkv") || set_smem(flash_dq_ws_kernel<HD, TWO>, C::SMEM_Q, "flash_dq")) return -1;
     once = true;
   }
   const int n_t = (p.T + 127) / 128;
   const int n_items = p.B * p.H * n_t;
-  const int sms = num_sms_attn();
-  const int grid = n_items < sms ? n_items : sms;
-  KH_LAUNCH((flash_dkv_ws_kernel<HD>), grid, C::THREADS, C::SMEM_KV, st, *mq, *mq64, *md64, *mg, p, n_items, n_t);
-  KH_LAUNCH((flash_dq_ws_kernel<HD>), grid, C::THREADS, C::SMEM_Q, st, *mq, *md, *mq64, *mg, p, n_items, n_t);
+  const int ctas = C::CTAS * num_sms_attn();
+  const int grid = n_items < ctas ? n_items : ctas;
+  KH_LAUNCH((flash_dkv_ws_kernel<HD, TWO>), grid, C::THREADS, C::SMEM_KV, st, *mq, *mq64, *md64, *mg, p, n_items, n_t);
+  KH_LAUNCH((flash_dq_ws_kernel<HD, TWO>), grid, C::THREADS, C::SMEM_Q, st, *mq, *md, *mq64, *mg, p, n_items, n_t);
   KH_LAUNCH_CHECK("flash_bwd");
   return 0;
+}
+template <int HD>
+int launch_bwd(const void* qkv, const AttnParams& p, cudaStream_t st) {
+  if (HD == 64 && (long)p.B * p.H * ((p.T + 127) / 128) > num_sms_attn()) return launch_bwd_as<HD, HD == 64>(qkv, p, st);
+  return launch_bwd_as<HD, false>(qkv, p, st);
 }
 
 }  // namespace
