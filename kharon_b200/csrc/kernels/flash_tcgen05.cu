@@ -168,7 +168,7 @@ flash_fwd_ws_kernel(const __grid_constant__ FwdMaps<NSEG> maps, const __grid_con
 
   if (warp == 4) {
     // ------------------------------------------------------------------ TMA producer
-    if (lane == 0 && live) {
+    if (live && elect_one()) {
       int ic = 0, kvc = 0;
       bool ok = true;
       for (int w = blockIdx.x; ok && w < n_items; w += gridDim.x, ic++) {
@@ -192,7 +192,7 @@ flash_fwd_ws_kernel(const __grid_constant__ FwdMaps<NSEG> maps, const __grid_con
     }
   } else if (warp == 5) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0 && live) {
+    if (live && elect_one()) {
       constexpr uint32_t idesc_s = umma_idesc_bf16(128, BKV, 0, 0);
       constexpr uint32_t idesc_o = umma_idesc_bf16(128, HD, 0, 1);
       int ic = 0, pc = 0, kvc = 0;
@@ -488,7 +488,7 @@ flash_dkv_ws_kernel(const __grid_constant__ CUtensorMap map_kv, const __grid_con
   const bool live = *abort_flag == 0;
 
   if (warp == 8) {
-    if (lane == 0 && live) {
+    if (live && elect_one()) {
       int ic = 0, qc = 0;
       bool ok = true;
       for (int w = blockIdx.x; ok && w < n_items; w += gridDim.x, ic++) {
@@ -509,7 +509,7 @@ flash_dkv_ws_kernel(const __grid_constant__ CUtensorMap map_kv, const __grid_con
       }
     }
   } else if (warp == 9) {
-    if (lane == 0 && live) {
+    if (live && elect_one()) {
       constexpr uint32_t idesc_s = umma_idesc_bf16(128, BS, 0, 0);
       constexpr uint32_t idesc_g = umma_idesc_bf16(128, HD, 0, 1);
       int ic = 0, qc = 0, rc = 0;
@@ -742,7 +742,7 @@ flash_dq_ws_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
   const bool live = *abort_flag == 0;
 
   if (warp == 8) {
-    if (lane == 0 && live) {
+    if (live && elect_one()) {
       int ic = 0, kvc = 0;
       bool ok = true;
       for (int w = blockIdx.x; ok && w < n_items; w += gridDim.x, ic++) {
@@ -763,7 +763,7 @@ flash_dq_ws_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
       }
     }
   } else if (warp == 9) {
-    if (lane == 0 && live) {
+    if (live && elect_one()) {
       constexpr uint32_t idesc_s = umma_idesc_bf16(128, BS, 0, 0);
       constexpr uint32_t idesc_g = umma_idesc_bf16(128, HD, 0, 1);
       int ic = 0, kvc = 0, rc = 0;

@@ -334,7 +334,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ C
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    if (elect_one()) {
       int it = 0;
       bool ok = true;
       for (int t = worker; ok && t < num_tiles; t += n_workers) {
@@ -372,7 +372,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ C
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0 && crank == 0) {
+    if (crank == 0 && elect_one()) {
       const uint32_t idesc = umma_idesc_bf16(TM, BN, p.a_mn, p.b_mn);
       // K-major: LBO unused (encoded 16 B), SBO 1024; MN-major: LBO = one 64-wide slab (BK rows x 128 B), SBO 1024
       const uint32_t a_lbo = p.a_mn ? BK * 128 : 16, b_lbo = p.b_mn ? BK * 128 : 16;
@@ -740,7 +740,7 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_const
 #pragma unroll
   for (int j = 0; j < 8; j++) cs[j] = 0.f;
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       for (int i = 0; i < nkb; i++) {
         const int s = i % Cfg::STAGES, kb = kb0 + i;
         const uint32_t ph = (i / Cfg::STAGES) & 1;
@@ -757,7 +757,7 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_const
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc = umma_idesc_bf16(BM, BN, p.a_mn, p.b_mn);
       const uint32_t a_lbo = p.a_mn ? BK * 128 : 16, b_lbo = p.b_mn ? BK * 128 : 16;
       const uint32_t a_kstep = p.a_mn ? (UMMA_K * 128) >> 4 : (UMMA_K * 2) >> 4;
