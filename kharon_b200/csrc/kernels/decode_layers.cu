@@ -40,8 +40,8 @@
 // warps meet in shared memory and are added in warp order.
 //
 // Attention.  W warps share a (sequence, head) item; a key is read by HD / 8 lanes in 16-byte pieces and
-// the running softmax is kept per lane group and merged once.  The first four keys and values of every
-// group are requested before the queries are polled (cached positions do not depend on this step).
+// the running softmax is kept per lane group and merged once.  The first four (eight) keys and values of
+// every group are requested before the queries are polled (cached positions do not depend on this step).
 //
 // Every wait is bounded: status code 9 in the library error word, an abort word for the other CTAs.
 // Numerics follow the five-kernel path: bf16 activations between phases, fp32 accumulation, LayerNorm
@@ -102,9 +102,9 @@ struct DecodeParams {
 };
 
 struct Shared {               // small control block behind the data regions
-  LayerW lw[2];               // records of this layer and the next
+  LayerW lw[4];               // records of this layer and the next two
   int item_pos[MAX_WARPS], item_slot[MAX_WARPS];    // position and slot of each warp's first attention item (constant over the layers)
-  int item_row[MAX_WARPS][8][4];                // cache rows of its first four keys, per lane group
+  int item_row[MAX_WARPS][8][8];                // cache rows of its first keys, per lane group
   volatile int abort_flag;
 };
 
@@ -130,6 +130,8 @@ __device__ __forceinline__ float warp_sum(float v) {
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void cp_async_wait_older() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }     // all but the last group
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 __device__ __forceinline__ void l2_prefetch_bulk(const void* p, uint32_t bytes) {       // 16-byte aligned, multiple of 16
   asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
@@ -229,6 +231,7 @@ __device__ __forceinline__ void copy_first(uint32_t wbuf, const Lin& L) {
 #pragma unroll
   for (int j = 0; j < KS; j++)
     copy_w<LGW, RG>(wbuf + tid * 16, tid & 31, L, (int)blockIdx.x * U + (warp >> L.lgs), (warp & ((1 << L.lgs) - 1)) * kw, j, kw >> 5);
+  cp_async_commit();
 }
 // ask L2 for the weights of this CTA's units (the first `turns` turns of them); one thread of the last warp, which has the
 // least to do at the start of a phase
@@ -252,6 +255,7 @@ __device__ __forceinline__ void fetch_ln(bf16* sln, const bf16* w, const bf16* b
     cp_async16(smem_u32(sln + c * 8), w + c * 8);
     cp_async16(smem_u32(sln + d + c * 8), b + c * 8);
   }
+  cp_async_commit();
 }
 
 // LayerNorm of rows [0, n) into xs, a warp per row: the row is polled, kept in shared memory as it arrived, and
@@ -337,7 +341,7 @@ __device__ __forceinline__ void linear_phase(const DecodeParams& p, const Lin& L
   const int n_units = (N + CU - 1) / CU, stride = (int)gridDim.x * U;
   const int ul = warp >> lgs, ks = warp & (S - 1);
   int unit0 = (int)blockIdx.x * U;
-  if (LN) { cp_async_wait_all(); __syncthreads(); }              // gain, bias and the next layer's record are there; xs is free
+  if (LN) { cp_async_wait_older(); __syncthreads(); }            // gain, bias and layer records are there (the weights need not be); xs is free
   if (unit0 >= n_units) return;                                   // uniform over the CTA
   const int n_out = U * GP * (CU / 2);                            // (unit, row, column pair)
   auto operands = [&](int o, uint32_t& b2, uint64_t& r2) {        // bias and residual packet of output pair o, as they are now
@@ -473,12 +477,16 @@ __device__ __forceinline__ void linear_phase(const DecodeParams& p, const Lin& L
 }
 
 // ------------------------------------------------------------------------------------------------
+// Positions a lane group holds at a time: eight for heads of 64 where registers allow it; four for narrow heads, whose eight groups a warp
+// cover short contexts in one turn anyway (d256: 59 us a step against 64), and for heads of 128 (no difference).
+template <int LGW, int HD> constexpr int keys_ahead() { return LGW == 3 && HD == 64 ? 8 : 4; }
 // Phase B.  Appends the new k, v (from the qkv packets) to the paged cache and attends over positions 0..pos.
 // The W warps of an item hold W * 32 / (HD / 8) lane groups; group i takes keys i, i + ST, i + 2 ST, ...
 template <int LGW, int HD>
 __device__ __forceinline__ void attention_phase(const DecodeParams& p, int layer, uint32_t epoch, float* satt, Shared* sh) {
   CFG;
-  constexpr int LPK = HD / 8, KPW = 32 / LPK;     // lanes per key, keys per warp and turn
+  constexpr int LPK = HD / 8, KPW = 32 / LPK;     // lanes per key, keys of a warp at a time
+  constexpr int NB = keys_ahead<LGW, HD>();        // positions a group holds at a time
   const int tid = tid_fresh(), warp = tid >> 5, lane = tid & 31;
   const int W = 1 << p.lgw, slots = WARPS >> p.lgw, ST = W * KPW;
   const int kg = (warp & (W - 1)) * KPW + lane / LPK, e0 = (lane % LPK) * 8;
@@ -506,24 +514,24 @@ __device__ __forceinline__ void attention_phase(const DecodeParams& p, int layer
         const int jb = p.block_of(j);
         return __ldg(bt + jb) * p.bs + (j - jb * p.bs);
       };
-      int row[4];                     // cache rows of the next four positions of this group
-      uint4 k4[4], v4[4];             // refilled with those positions as soon as they are used
+      int row[NB];                    // cache rows of the next positions of this group
+      uint4 k4[NB], v4[NB];            // refilled with those positions as soon as they are used
       uint2 qkv2[6];
       float q[8];
       const bool owner = pos % ST == kg;
       const int first = (warp & (W - 1)) * KPW;       // uniform over the warp
-      // Turn -1 only requests the first four keys and values and then waits for the query (and the owner of position `pos`
-      // for the new key and value); every other turn uses four positions and requests the next ones in their place.
+      // Turn -1 only requests the first NB keys and values and then waits for the query (and the owner of position `pos`
+      // for the new key and value); every other turn uses NB positions and requests the next ones in their place.
 #pragma unroll 1
-      for (int b0 = -4 * ST; b0 < 0 || first + b0 <= pos; b0 += 4 * ST) {
-        const int j0 = kg + b0, jn = j0 + 4 * ST;
-        float s[4];
+      for (int b0 = -NB * ST; b0 < 0 || first + b0 <= pos; b0 += NB * ST) {
+        const int j0 = kg + b0, jn = j0 + NB * ST;
+        float s[NB];
 #pragma unroll
-        for (int i = 0; i < 4; i++)
+        for (int i = 0; i < NB; i++)
           if (jn + i * ST < pos) row[i] = b0 < 0 && turn0 ? sh->item_row[warp][lane / LPK][i] : row_of(jn + i * ST);
         if (b0 >= 0) {
 #pragma unroll
-          for (int i = 0; i < 4; i++) {
+          for (int i = 0; i < NB; i++) {
             const int j = j0 + i * ST;
             if (j == pos) { k4[i] = make_uint4(qkv2[2].x, qkv2[2].y, qkv2[3].x, qkv2[3].y); v4[i] = make_uint4(qkv2[4].x, qkv2[4].y, qkv2[5].x, qkv2[5].y); }
             if (j > pos) k4[i] = v4[i] = make_uint4(0, 0, 0, 0);
@@ -533,7 +541,7 @@ __device__ __forceinline__ void attention_phase(const DecodeParams& p, int layer
         }
         // cached positions only; the same lines of the next layer are requested into L2
 #pragma unroll
-        for (int i = 0; i < 4; i++)
+        for (int i = 0; i < NB; i++)
           if (jn + i * ST < pos) {
             const bf16* c = kc + (size_t)row[i] * d + h * HD + e0;
             k4[i] = ldg_stream(c);
@@ -543,11 +551,13 @@ __device__ __forceinline__ void attention_phase(const DecodeParams& p, int layer
 #pragma unroll
           for (int x = LPK / 2; x > 0; x >>= 1)
 #pragma unroll
-            for (int i = 0; i < 4; i++) s[i] += __shfl_xor_sync(0xffffffffu, s[i], x);
+            for (int i = 0; i < NB; i++) s[i] += __shfl_xor_sync(0xffffffffu, s[i], x);
 #pragma unroll
-          for (int i = 0; i < 4; i++)
+          for (int i = 0; i < NB; i++)
             if (j0 + i * ST > pos) s[i] = -INFINITY;
-          const float mn = fmaxf(m, fmaxf(fmaxf(s[0], s[1]), fmaxf(s[2], s[3])));
+          float mn = m;
+#pragma unroll
+          for (int i = 0; i < NB; i++) mn = fmaxf(mn, s[i]);
           const float ref = mn == -INFINITY ? 0.f : mn;
           const float sc = __expf(m - ref);
           m = mn;
@@ -555,7 +565,7 @@ __device__ __forceinline__ void attention_phase(const DecodeParams& p, int layer
 #pragma unroll
           for (int k = 0; k < 8; k++) o[k] *= sc;
 #pragma unroll
-          for (int i = 0; i < 4; i++) {
+          for (int i = 0; i < NB; i++) {
             const float pr = __expf(s[i] - ref);
             l += pr;
             const float2 a = unpack_bf16(v4[i].x), b = unpack_bf16(v4[i].y), c = unpack_bf16(v4[i].z), e = unpack_bf16(v4[i].w);
@@ -564,7 +574,7 @@ __device__ __forceinline__ void attention_phase(const DecodeParams& p, int layer
           }
         }
 #pragma unroll
-        for (int i = 0; i < 4; i++)
+        for (int i = 0; i < NB; i++)
           if (jn + i * ST < pos) {
             const bf16* c = vc + (size_t)row[i] * d + h * HD + e0;
             v4[i] = ldg_stream(c);
@@ -651,7 +661,7 @@ __global__ void __launch_bounds__(32 << lg_warps<MT>(), 1) decode_layers_k(const
   float* satt = red + (MT == 4 ? 1 : 2) * WARPS * GP * 16;
   Shared* sh = reinterpret_cast<Shared*>(satt + WARPS * ATT_PITCH);
   if (threadIdx.x == 0) sh->abort_flag = 0;
-  if (threadIdx.x < 2 * 6 && (int)threadIdx.x / 6 < p.L)
+  if (threadIdx.x < 3 * 6 && (int)threadIdx.x / 6 < p.L)
     reinterpret_cast<uint4*>(sh->lw)[threadIdx.x] = __ldg(reinterpret_cast<const uint4*>(p.layers) + threadIdx.x);
   if (p.L > 0) {                  // this warp's first attention item and the cache rows of its first keys
     constexpr int LPK = HD / 8, KPW = 32 / LPK;
@@ -661,7 +671,7 @@ __global__ void __launch_bounds__(32 << lg_warps<MT>(), 1) decode_layers_k(const
       const int pos = p.pos[item / p.H], slot = p.slot[item / p.H];
       if (lane == 0) { sh->item_pos[warp] = pos; sh->item_slot[warp] = slot; }
       if (lane % LPK == 0 && slot >= 0)
-        for (int i = 0; i < 4; i++) {
+        for (int i = 0; i < keys_ahead<LGW, HD>(); i++) {
           const int j = kg + i * ST, jb = p.block_of(j);
           if (j < pos && jb < p.max_lb && j < p.max_ctx)
             sh->item_row[warp][lane / LPK][i] = p.btab[(size_t)slot * p.max_lb + jb] * p.bs + (j - jb * p.bs);
@@ -677,7 +687,7 @@ __global__ void __launch_bounds__(32 << lg_warps<MT>(), 1) decode_layers_k(const
   auto ln_phase = [&](int hl) {
     Lin L;
     const int l = hl >> 1;
-    const LayerW* lw = sh->lw + (l & 1);
+    const LayerW* lw = sh->lw + (l & 3);
     L.K = d; L.res = nullptr; L.e_res = 0;
     if (hl == 2 * p.L) {
       L.W = p.head_w; L.bias = nullptr; L.N = p.V; L.lgs = p.lgs_h; L.kind = PH; L.dst = nullptr;
@@ -695,7 +705,7 @@ __global__ void __launch_bounds__(32 << lg_warps<MT>(), 1) decode_layers_k(const
   auto res_phase = [&](int hl) {
     Lin L;
     const int l = hl >> 1;
-    const LayerW* lw = sh->lw + (l & 1);
+    const LayerW* lw = sh->lw + (l & 3);
     L.N = d;
     L.e_src = L.e_dst = base + l + 1;
     if (hl & 1) {
@@ -708,6 +718,16 @@ __global__ void __launch_bounds__(32 << lg_warps<MT>(), 1) decode_layers_k(const
     return L;
   };
   const int n_half = 2 * p.L;
+  // Weights go into L2 ahead of their phase: the copies into shared memory then take an L2 trip, and the memory streams during
+  // attention and hand-offs too.  `far`: two phases ahead, for layers of up to 40 MB (d1024: 489 -> 470 us a step at G = 1); larger
+  // ones one phase ahead (d2048, 100 MB a layer: 1182 us against 1248).
+  const bool far = d <= 1280;
+  auto prefetch_next = [&](bool last, const LayerW* nw) {
+    if (!last) {
+      prefetch_units<LGW>(nw->qkv_w, 3 * d, d, (WARPS >> p.lgs_a) * 16, 8);
+      prefetch_units<LGW>(nw->proj_w, d, d, (WARPS >> p.lgs_c) * 8, 8);
+    } else if (p.head_w) prefetch_units<LGW>(p.head_w, p.V, d, (WARPS >> p.lgs_h) * 16, 2);
+  };
   if (p.L > 0) {
     fetch_ln<LGW>(sln, sh->lw[0].ln1_w, sh->lw[0].ln1_b, d);
     prefetch_units<LGW>(sh->lw[0].proj_w, d, d, (WARPS >> p.lgs_c) * 8, 8);
@@ -717,36 +737,36 @@ __global__ void __launch_bounds__(32 << lg_warps<MT>(), 1) decode_layers_k(const
 #pragma unroll 1
   for (int hl = 0; hl < n_half + (p.head_w ? 1 : 0); hl++) {
     const int l = hl >> 1;
-    const LayerW* lw = sh->lw + (l & 1);
-    const LayerW* nw = sh->lw + ((l + 1) & 1);
+    const LayerW* lw = sh->lw + (l & 3);
+    const LayerW* nw = sh->lw + ((l + 1) & 3);
     const bool even = (hl & 1) == 0, last = l + 1 >= p.L;
     {
       const Lin L = ln_phase(hl);
       copy_first<LGW, 2>(wbuf, L);
-      if (even && hl < n_half) prefetch_units<LGW>(lw->fc_w, 4 * d, d, (WARPS >> p.lgs_d) * 16, 8);
+      if (hl < n_half) {
+        if (even) prefetch_units<LGW>(lw->fc_w, 4 * d, d, (WARPS >> p.lgs_d) * 16, 8);
+        else if (far) prefetch_next(last, nw);
+      }
       linear_phase<LGW, MT, true>(p, L, hl == n_half ? p.n_rows : p.G, false, xs, sln, red, flip, sh, wbuf);
     }
     if (hl == n_half) break;
     if (even) {
-      // record of the next layer: every warp is past the barrier of this phase, so nobody reads the one it replaces
-      if (!last && l > 0) {
+      // record of the layer after the next, in the place of the last one's: every warp is past the barrier of this phase, so
+      // nobody reads that any more
+      if (l > 0 && l + 2 < p.L) {
         const int t = tid_fresh();
-        if (t < 6) cp_async16(smem_u32(reinterpret_cast<uint4*>(sh->lw + ((l + 1) & 1)) + t), reinterpret_cast<const uint4*>(p.layers + l + 1) + t);
+        if (t < 6) cp_async16(smem_u32(reinterpret_cast<uint4*>(sh->lw + ((l + 2) & 3)) + t), reinterpret_cast<const uint4*>(p.layers + l + 2) + t);
+        cp_async_commit();
       }
+      if (far) prefetch_units<LGW>(lw->fcproj_w, d, 4 * d, (WARPS >> p.lgs_e) * 8, 8);
       attention_phase<LGW, HD>(p, l, base + l + 1, satt, sh);
     }
     const Lin L = res_phase(hl);
     copy_first<LGW, 1>(wbuf, L);
-    const bf16 *lnw = lw->ln2_w, *lnb = lw->ln2_b;
-    if (even) {
-      prefetch_units<LGW>(lw->fcproj_w, d, 4 * d, (WARPS >> p.lgs_e) * 8, 8);
-    } else if (!last) {
-      lnw = nw->ln1_w; lnb = nw->ln1_b;
-      prefetch_units<LGW>(nw->qkv_w, 3 * d, d, (WARPS >> p.lgs_a) * 16, 8);
-      prefetch_units<LGW>(nw->proj_w, d, d, (WARPS >> p.lgs_c) * 8, 8);
-    } else {
-      lnw = p.lnf_w; lnb = p.lnf_b;
-      if (p.head_w) prefetch_units<LGW>(p.head_w, p.V, d, (WARPS >> p.lgs_h) * 16, 2);
+    const bf16 *lnw = even ? lw->ln2_w : last ? p.lnf_w : nw->ln1_w, *lnb = even ? lw->ln2_b : last ? p.lnf_b : nw->ln1_b;
+    if (!far) {
+      if (even) prefetch_units<LGW>(lw->fcproj_w, d, 4 * d, (WARPS >> p.lgs_e) * 8, 8);
+      else prefetch_next(last, nw);
     }
     if (lnw) fetch_ln<LGW>(sln, lnw, lnb, d);
     linear_phase<LGW, MT, false>(p, L, p.G, last && !even, xs, sln, red, flip, sh, wbuf);
