@@ -30,8 +30,8 @@
 // the smallest split whose slice fits a sub-step, and larger where that spreads a narrow product over more
 // CTAs in the same number of turns.  Every lane copies the eight (sixteen) 16-byte pieces of weights that it will use
 // into its own slots of shared memory with cp.async (no registers are held and no thread waits for another's
-// copy); the first turn's weights of a phase are requested before its activations are polled, a slot is
-// refilled with the next turn's as soon as it has been read, and the units of later phases are prefetched
+// copy); the first turn's weights of a phase are requested before its activations are polled, the next turn's
+// are requested under the products of this one (a second set of slots for up to eight rows, else as a slot has been read), and the units of later phases are prefetched
 // into L2 in bulk.  The products are mma.sync m16n8k16 with the weights as the 16-row operand and eight sequences
 // as the columns: tcgen05's 128-row tiles, TMEM round trip and operand staging are the latency this kernel
 // exists to avoid (the large-M GEMMs of training and prefill use them).  The K order inside a 32-wide block
@@ -63,8 +63,11 @@ constexpr int SMEM_LIMIT = 227 * 1024;
 template <int LGW> struct Cfg {
   static constexpr int WARPS = 1 << LGW, THREADS = 32 * WARPS, NLD = 128 / WARPS;
   static constexpr uint32_t SLOT = THREADS * 16;
+  static constexpr bool DB = LGW == 3;        // two sets of slots: shared memory has room for them up to eight rows
 };
 #define CFG using C_ = Cfg<LGW>; constexpr int WARPS = C_::WARPS, THREADS = C_::THREADS, NLD = C_::NLD; constexpr uint32_t SLOT = C_::SLOT; (void)WARPS; (void)THREADS; (void)NLD; (void)SLOT
+
+constexpr uint32_t WBUF = 65536;              // bytes of a set of weight slots
 
 // Thread index, read anew in every phase: index arithmetic derived from it would otherwise be kept in registers (and
 // spilled) across the whole layer loop.
@@ -355,6 +358,8 @@ __device__ __forceinline__ void linear_phase(const DecodeParams& p, const Lin& L
     }
   };
   bool staged = false;
+  constexpr bool DB = C_::DB;
+  int wb = 0;                                                     // set of slots that holds the current weights
 #pragma unroll 1
   for (; unit0 < n_units; unit0 += stride) {
     const int u = unit0 + ul;
@@ -380,13 +385,24 @@ __device__ __forceinline__ void linear_phase(const DecodeParams& p, const Lin& L
       const bool more = s0 + KS < steps, turn = !more && unit0 + stride < n_units;
       const int nu = more ? u : u + stride, nk = more ? k0 + KS * 32 : ks * kw;
       const int nn = more ? min(KS, steps - s0 - KS) : (turn ? min(KS, steps) : 0);
+      // DB: they go into the other set of slots at once, under these products; else into these slots, one by one as they are read
+      const uint32_t cur = slots + (DB && wb ? WBUF : 0), nxt = DB ? slots + (wb ? 0 : WBUF) : cur;
+      wb ^= 1;
+      if (DB && nn > 0) {
+#pragma unroll
+        for (int j = 0; j < KS; j++) copy_w<LGW, RG>(nxt, lane, L, nu, nk, j, nn);
+        cp_async_commit();
+      }
+      auto wait_weights = [&]() {
+        if (DB && nn > 0) cp_async_wait_older(); else cp_async_wait_all();
+      };
       if (LN) {
-        cp_async_wait_all();
+        wait_weights();
         const bf16* xa = xs + (size_t)(lane >> 2) * (K + PAD) + k0 + (lane & 3) * 8;
 #pragma unroll
         for (int j = 0; j < KS; j++) {
           if (j < ns) {
-            const uint4 w0 = lds128(slots + (2 * j) * SLOT), w1 = lds128(slots + (2 * j + 1) * SLOT);
+            const uint4 w0 = lds128(cur + (2 * j) * SLOT), w1 = lds128(cur + (2 * j + 1) * SLOT);
 #pragma unroll
             for (int m = 0; m < MT; m++) {
               const uint4 a = *reinterpret_cast<const uint4*>(xa + (size_t)(m * 8) * (K + PAD) + j * 32);
@@ -394,7 +410,7 @@ __device__ __forceinline__ void linear_phase(const DecodeParams& p, const Lin& L
               mma_bf16(acc[(2 * j + 1) % NCH][m], w0.z, w1.z, w0.w, w1.w, a.z, a.w);
             }
           }
-          copy_w<LGW, RG>(slots, lane, L, nu, nk, j, nn);
+          if (!DB) copy_w<LGW, RG>(nxt, lane, L, nu, nk, j, nn);
         }
       } else {
         constexpr int JB = 4 / MT;                                // eight packet pairs in flight per lane
@@ -406,13 +422,13 @@ __device__ __forceinline__ void linear_phase(const DecodeParams& p, const Lin& L
             read_pairs<8>(t, [&](int i) { return (i >> 1) % MT * 8 + (lane >> 2) < n && j0 + (i >> 1) / MT < ns; },
                           [&](int i) { return q + (size_t)((i >> 1) % MT * 8) * (K / 2) + (j0 + (i >> 1) / MT) * 16 + (i & 1) * 2; },
                           L.e_src, p, sh);
-            if (j0 == 0) cp_async_wait_all();
+            if (j0 == 0) wait_weights();
             __syncwarp();
 #pragma unroll
             for (int jj = 0; jj < JB; jj++) {
               const int j = j0 + jj;
               if (j < ns) {
-                const uint4 w0 = lds128(slots + j * SLOT);
+                const uint4 w0 = lds128(cur + j * SLOT);
 #pragma unroll
                 for (int m = 0; m < MT; m++) {
                   const int i = jj * MT + m;
@@ -423,7 +439,8 @@ __device__ __forceinline__ void linear_phase(const DecodeParams& p, const Lin& L
             }
           }
 #pragma unroll
-          for (int j = j0; j < j0 + JB; j++) copy_w<LGW, RG>(slots, lane, L, nu, nk, j, nn);
+          for (int j = j0; j < j0 + JB; j++)
+            if (!DB) copy_w<LGW, RG>(nxt, lane, L, nu, nk, j, nn);
         }
       }
     }
@@ -655,7 +672,7 @@ __global__ void __launch_bounds__(32 << lg_warps<MT>(), 1) decode_layers_k(const
   constexpr int GP = 8 * MT;
   extern __shared__ __align__(16) uint8_t smem[];
   const uint32_t wbuf = smem_u32(smem);
-  bf16* xs = reinterpret_cast<bf16*>(smem + NLD * SLOT);
+  bf16* xs = reinterpret_cast<bf16*>(smem + (C_::DB ? 2 : 1) * WBUF);
   bf16* sln = xs + (size_t)GP * (p.d + PAD);
   float* red = reinterpret_cast<float*>(sln + 2 * p.d);
   float* satt = red + (MT == 4 ? 1 : 2) * WARPS * GP * 16;
@@ -786,7 +803,7 @@ __global__ void __launch_bounds__(32 << lg_warps<MT>(), 1) decode_layers_k(const
 
 int smem_bytes(int MT, int d) {
   const int warps = MT == 1 ? 1 << lg_warps<1>() : 1 << lg_warps<2>();
-  return 65536 + 8 * MT * (d + PAD) * 2 + 4 * d + (MT == 4 ? 1 : 2) * warps * 8 * MT * 16 * 4 + warps * ATT_PITCH * 4 + (int)sizeof(Shared);
+  return (MT == 1 ? 2 : 1) * (int)WBUF + 8 * MT * (d + PAD) * 2 + 4 * d + (MT == 4 ? 1 : 2) * warps * 8 * MT * 16 * 4 + warps * ATT_PITCH * 4 + (int)sizeof(Shared);
 }
 int max_mt(int d) {             // row groups of eight whose normalised rows fit into shared memory
   for (int mt = 4; mt > 1; mt >>= 1)
@@ -828,7 +845,7 @@ int launch(DecodeParams& p, int grid, cudaStream_t st) {
 }
 template <int HD>
 int launch_rows(DecodeParams& p, int rows, int grid, cudaStream_t st) {
-  if (rows <= 8) return launch<1, HD>(p, grid, st);
+  if (rows <= 8 && smem_bytes(1, p.d) <= SMEM_LIMIT) return launch<1, HD>(p, grid, st);      // (d = 4096 has no room for two sets of slots)
   if (rows <= 16) return launch<2, HD>(p, grid, st);
   return launch<4, HD>(p, grid, st);
 }

@@ -223,7 +223,7 @@ def test_persistent_decode_kernel_matches_the_kernel_chain(d, heads, groups):
 
 
 @pytest.mark.parametrize("d,heads,G,ctx", [(256, 8, 1, 9), (256, 4, 32, 40), (512, 16, 2, 300), (768, 12, 6, 70), (1024, 8, 16, 150),
-                                           (2048, 16, 31, 33), (4096, 32, 17, 20)])
+                                           (2048, 16, 31, 33), (4096, 32, 17, 20), (4096, 32, 3, 12)])
 def test_persistent_decode_steps_against_the_chain(d, heads, G, ctx):
     """Single decode steps at the kernel's edges: one warp step per slice (d = 256), head widths 32 / 64 / 128, one to four
     row groups, several turns of a phase, contexts of more than four keys per lane group, rows that need two launches
