@@ -227,6 +227,208 @@ extern "C" int kh_paged_attn(const void* qkv, int ld, void* kc, void* vc, void* 
   return 0;
 }
 
+// ------------------------------------------------------------------------------- attention of prompt pieces
+// Runs of consecutive positions of one sequence (prompts that join a step beside decoding sequences, short or chunked prompts):
+// CTA = (up to 64 tokens, head), a warp per 16 tokens.  paged_attn_k spends about 14 instructions per token and key (unpacking,
+// fp32 multiplies, shuffles): 6700 prompt tokens x 16 heads took 0.9 ms a layer.  Here the products run on the tensor
+// cores (mma.sync: K and V rows come one by one through the block table), K and V tiles of 64 positions are copied once
+// per CTA with cp.async, two in flight.  Nothing is rounded that was not before: q and k are bf16 in memory and their
+// products accumulate in fp32; the probabilities stay fp32 and enter P V as three bf16 terms, whose 3 x 8 bits hold the 24
+// of an fp32 mantissa.  The K order inside a 32-wide block is permuted identically for q and k so that fragments are whole
+// 16-byte pieces.
+constexpr int PP_ROWS = 64, PP_MAX_TILES = 1024;
+struct PrefillTiles { int row0[PP_MAX_TILES]; uint8_t n[PP_MAX_TILES]; };
+
+__device__ __forceinline__ void pp_mma(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+// x = hi + mid + lo, each bf16 (pairs packed)
+__device__ __forceinline__ void split3(float x, float y, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
+  hi = pack_bf16(x, y);
+  const float2 h = unpack_bf16(hi);
+  mid = pack_bf16(x - h.x, y - h.y);
+  const float2 m = unpack_bf16(mid);
+  lo = pack_bf16(x - h.x - m.x, y - h.y - m.y);
+}
+
+template <int HD>
+__global__ void __launch_bounds__(128)
+paged_prefill_k(const __grid_constant__ PrefillTiles tiles, const bf16* __restrict__ qkv, int ld, const bf16* __restrict__ kc,
+                const bf16* __restrict__ vc, bf16* __restrict__ out, const int* __restrict__ pos, const int* __restrict__ slot,
+                const int* __restrict__ btab, int max_lb, int bs, int H, float scale, int max_ctx, int* err) {
+  constexpr int PITCH = HD * 2 + 16, TILE = PP_ROWS * PITCH, PC = HD / 8;       // bytes per row, per tile; 16-byte pieces per row
+  extern __shared__ __align__(16) uint8_t pp_smem[];                            // [2][K, V][64 rows]
+  pdl_wait();
+  pdl_launch_dependents();
+  const uint32_t base = smem_u32(pp_smem);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, c4 = lane & 3, h = blockIdx.y, d = H * HD;
+  const int r0 = tiles.row0[blockIdx.x], p0 = pos[r0], sl = slot[r0];
+  int n = tiles.n[blockIdx.x];
+  // index guard as in paged_attn_k: tokens beyond the limits are recorded (status code 8) and skipped; they are the last of the run
+  const int ok = sl < 0 || p0 < 0 ? 0 : min(n, min(max_ctx, max_lb * bs) - p0);
+  if (ok < n && tid == 0) atomicCAS(err, 0, 8);
+  if (ok <= 0) return;
+  n = ok;
+  const int ctx = p0 + n;
+  const int* bt = btab + (size_t)sl * max_lb;
+  auto load = [&](int kt) {                                                     // positions 64 kt .. into buffer kt & 1; zeros past the end
+    const uint32_t dst = base + (kt & 1) * 2 * TILE;
+#pragma unroll 4
+    for (int i = tid; i < PP_ROWS * PC; i += 128) {
+      const int r = i / PC, c = i % PC, j = kt * PP_ROWS + r;
+      const int jb = j < ctx ? j / bs : 0;
+      const size_t at = ((size_t)__ldg(bt + jb) * bs + (j < ctx ? j - jb * bs : 0)) * d + h * HD + c * 8;
+      const uint32_t a = dst + r * PITCH + c * 16;
+      const int bytes = j < ctx ? 16 : 0;
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(a), "l"(kc + at), "r"(bytes) : "memory");
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(a + TILE), "l"(vc + at), "r"(bytes) : "memory");
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  load(0);
+  const int w0 = warp * 16;                                                     // this warp's first token of the run
+  uint4 q[HD / 32][2];                                                          // rows g and g + 8, piece c4 of every 32-wide block
+#pragma unroll
+  for (int j = 0; j < HD / 32; j++)
+#pragma unroll
+    for (int i = 0; i < 2; i++) {
+      q[j][i] = make_uint4(0, 0, 0, 0);
+      if (w0 + g + 8 * i < n) q[j][i] = *reinterpret_cast<const uint4*>(qkv + (size_t)(r0 + w0 + g + 8 * i) * ld + h * HD + j * 32 + c4 * 8);
+    }
+  float o[HD / 8][4], m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};
+#pragma unroll
+  for (int t = 0; t < HD / 8; t++)
+#pragma unroll
+    for (int i = 0; i < 4; i++) o[t][i] = 0.f;
+  const int n_kt = (ctx + PP_ROWS - 1) / PP_ROWS;
+#pragma unroll 1
+  for (int kt = 0; kt < n_kt; kt++) {
+    if (kt + 1 < n_kt) {
+      load(kt + 1);
+      asm volatile("cp.async.wait_group 1;" ::: "memory");
+    } else asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    const int k0 = kt * PP_ROWS;
+    if (w0 < n && k0 <= p0 + w0 + 15) {                                         // uniform over the warp
+      const uint32_t sK = base + (kt & 1) * 2 * TILE, sV = sK + TILE;
+      float s[8][4];
+#pragma unroll
+      for (int t = 0; t < 8; t++) {
+#pragma unroll
+        for (int i = 0; i < 4; i++) s[t][i] = 0.f;
+#pragma unroll
+        for (int j = 0; j < HD / 32; j++) {
+          uint4 k;
+          asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(k.x), "=r"(k.y), "=r"(k.z), "=r"(k.w)
+                       : "r"(sK + (t * 8 + g) * PITCH + j * 64 + c4 * 16) : "memory");
+          pp_mma(s[t], q[j][0].x, q[j][1].x, q[j][0].y, q[j][1].y, k.x, k.y);
+          pp_mma(s[t], q[j][0].z, q[j][1].z, q[j][0].w, q[j][1].w, k.z, k.w);
+        }
+      }
+      float mx[2] = {m[0], m[1]};
+#pragma unroll
+      for (int t = 0; t < 8; t++)
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+          s[t][i] *= scale;
+          if (k0 + t * 8 + c4 * 2 + (i & 1) > p0 + w0 + g + 8 * (i >> 1)) s[t][i] = -INFINITY;
+          mx[i >> 1] = fmaxf(mx[i >> 1], s[t][i]);
+        }
+      float ref[2];
+#pragma unroll
+      for (int i = 0; i < 2; i++) {
+        mx[i] = fmaxf(mx[i], __shfl_xor_sync(0xffffffffu, mx[i], 1));
+        mx[i] = fmaxf(mx[i], __shfl_xor_sync(0xffffffffu, mx[i], 2));
+        ref[i] = mx[i] == -INFINITY ? 0.f : mx[i];
+        const float sc = __expf(m[i] - ref[i]);
+        m[i] = mx[i];
+        l[i] *= sc;
+#pragma unroll
+        for (int t = 0; t < HD / 8; t++) { o[t][2 * i] *= sc; o[t][2 * i + 1] *= sc; }
+      }
+#pragma unroll
+      for (int t = 0; t < 8; t++)
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+          s[t][i] = __expf(s[t][i] - ref[i >> 1]);
+          l[i >> 1] += s[t][i];
+        }
+#pragma unroll
+      for (int t = 0; t < 4; t++) {                                             // sixteen keys at a time
+        uint32_t hi[4], mid[4], lo[4];
+        split3(s[2 * t][0], s[2 * t][1], hi[0], mid[0], lo[0]);
+        split3(s[2 * t][2], s[2 * t][3], hi[1], mid[1], lo[1]);
+        split3(s[2 * t + 1][0], s[2 * t + 1][1], hi[2], mid[2], lo[2]);
+        split3(s[2 * t + 1][2], s[2 * t + 1][3], hi[3], mid[3], lo[3]);
+#pragma unroll
+        for (int c = 0; c < HD; c += 16) {
+          uint32_t b[4];
+          asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(b[0]), "=r"(b[1]), "=r"(b[2]), "=r"(b[3])
+                       : "r"(sV + (t * 16 + (lane & 15)) * PITCH + (c + (lane >> 4) * 8) * 2) : "memory");
+          pp_mma(o[c / 8], hi[0], hi[1], hi[2], hi[3], b[0], b[1]);
+          pp_mma(o[c / 8], mid[0], mid[1], mid[2], mid[3], b[0], b[1]);
+          pp_mma(o[c / 8], lo[0], lo[1], lo[2], lo[3], b[0], b[1]);
+          pp_mma(o[c / 8 + 1], hi[0], hi[1], hi[2], hi[3], b[2], b[3]);
+          pp_mma(o[c / 8 + 1], mid[0], mid[1], mid[2], mid[3], b[2], b[3]);
+          pp_mma(o[c / 8 + 1], lo[0], lo[1], lo[2], lo[3], b[2], b[3]);
+        }
+      }
+    }
+    __syncthreads();                                                            // the buffer is refilled in the next turn
+  }
+#pragma unroll
+  for (int i = 0; i < 2; i++) {
+    l[i] += __shfl_xor_sync(0xffffffffu, l[i], 1);
+    l[i] += __shfl_xor_sync(0xffffffffu, l[i], 2);
+    if (w0 + g + 8 * i < n) {
+      const float inv = 1.f / l[i];
+      bf16* dst = out + (size_t)(r0 + w0 + g + 8 * i) * d + h * HD + c4 * 2;
+#pragma unroll
+      for (int t = 0; t < HD / 8; t++) *reinterpret_cast<uint32_t*>(dst + t * 8) = pack_bf16(o[t][2 * i] * inv, o[t][2 * i + 1] * inv);
+    }
+  }
+}
+// Runs of tokens: `row0`, `len` (host arrays) give each run's first row in qkv / pos / slot / out and its length; the positions
+// of a run are consecutive and belong to one sequence, and its K / V are in the cache already.
+extern "C" int kh_paged_prefill(const void* qkv, int ld, const void* kc, const void* vc, void* out, const void* pos, const void* slot,
+                                const void* btab, int max_lb, int bs, int H, int hd, float scale, int max_ctx, const void* row0,
+                                const void* len, int n_runs, void* stream) {
+  if (hd != 32 && hd != 64 && hd != 128) { kh_set_error("paged_prefill: head dim %d is not supported", hd); return -1; }
+  if (((uintptr_t)qkv & 15) || ((uintptr_t)out & 15) || ((uintptr_t)kc & 15) || ((uintptr_t)vc & 15) || ld % 8) { kh_set_error("paged_prefill: misaligned operands"); return -1; }
+  const int smem = 4 * PP_ROWS * (hd * 2 + 16);
+  cudaStream_t st = (cudaStream_t)stream;
+  PrefillTiles tiles;
+  int nt = 0;
+  auto flush = [&]() -> int {
+    if (nt == 0) return 0;
+#define LAUNCH(HD)                                                                                                              \
+  {                                                                                                                             \
+    if (cudaFuncSetAttribute(paged_prefill_k<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) {           \
+      kh_set_error("paged_prefill: shared memory opt-in failed");                                                               \
+      return -1;                                                                                                                \
+    }                                                                                                                           \
+    KH_LAUNCH((paged_prefill_k<HD>), dim3(nt, H), 128, smem, st, tiles, (const bf16*)qkv, ld, (const bf16*)kc, (const bf16*)vc,   \
+              (bf16*)out, (const int*)pos, (const int*)slot, (const int*)btab, max_lb, bs, H, scale, max_ctx, kh_error_word_dev()); \
+  }
+    if (hd == 128) LAUNCH(128) else if (hd == 64) LAUNCH(64) else LAUNCH(32)
+#undef LAUNCH
+    KH_LAUNCH_CHECK("paged_prefill");
+    nt = 0;
+    return 0;
+  };
+  for (int i = 0; i < n_runs; i++) {
+    const int r = ((const int*)row0)[i], n = ((const int*)len)[i];
+    if (r < 0 || n < 1) { kh_set_error("paged_prefill: run %d is empty", i); return -1; }
+    for (int at = (n - 1) / PP_ROWS * PP_ROWS; at >= 0; at -= PP_ROWS) {        // the pieces that see the most keys first
+      tiles.row0[nt] = r + at;
+      tiles.n[nt] = (uint8_t)(n - at < PP_ROWS ? n - at : PP_ROWS);
+      if (++nt == PP_MAX_TILES && flush()) return -1;
+    }
+  }
+  return flush();
+}
+
 // ------------------------------------------------------------------------------- split-KV attention
 // Long contexts: the keys of a token are cut into `n_split` equal ranges, one CTA per (token, head,
 // range) computes the softmax-weighted value sum over its range and its log-sum-exp, and a merge

@@ -23,6 +23,7 @@ import ctypes as C
 import os
 import time
 
+import numpy as np
 import torch
 
 from .. import _native, ops
@@ -96,7 +97,7 @@ class InferEngine:
             self.skinny = torch.zeros(n, dtype=torch.float32, **z)
         # Decode steps of up to ``persistent_max`` sequences run all layers and the head in one persistent kernel
         # when the shape allows it (ops.decode_layers); KHARON_PERSISTENT_DECODE=0 or persistent_decode=False keeps
-        # the five-kernel chain.  Measured on B200, us a step (L24 d1024, context 160-200): 507 / 565 / 764 / 1096 / 1217 at
+        # the five-kernel chain.  Measured on B200, us a step (L24 d1024, context 160-200): 468 / 520 / 741 / 1080 / 1212 at
         # G = 1 / 8 / 16 / 24 / 32 against 1255 / 1776 / 2029 / 1824 / 1851 for the chain.
         if persistent_decode is None:
             persistent_decode = os.environ.get("KHARON_PERSISTENT_DECODE", "1") != "0"
@@ -116,10 +117,11 @@ class InferEngine:
             self.attn_scratch = torch.zeros(self.max_tokens * self.Hl * self.attn_splits * (self.hd + 1), dtype=torch.float32, **z)
         # Steps made of whole fresh prompts (every listed token belongs to a sequence that starts at position 0 in this
         # step) run their attention on the tensor cores with the training forward kernel, all prompts in one launch;
-        # everything else (decode steps, chunked prompts, mixed steps) goes through the paged kernel.
+        # prompts beside decoding sequences, short and chunked ones go through the paged tile kernel (fp32 probabilities),
+        # everything else through the paged kernel.
         self.flash_prefill = bool(flash_prefill and self.dev.type == "cuda" and self.dt == torch.bfloat16
                                   and self.hd in (64, 128))
-        self._fresh = None
+        self._fresh = self._runs = None
         self.temperature, self.seed, self.step_no = 0.0, 0, 0
         # under TP the captured step contains the fused GEMM + all-reduce kernels (their call counter
         # is a device word); the NCCL seam is left to eager launches
@@ -175,6 +177,12 @@ class InferEngine:
                 ops.append_kv(qkv, self.kc[l], self.vc[l], pos, slot, self.d_btab, self.bs, self.Hl, self.hd, ntok)
             if not decode and self._fresh:
                 ops.flash_fwd_varlen(qkv, att, self._fresh, self.Hl, self.hd)
+            elif not decode and self._runs:
+                runs, rest = self._runs
+                ops.paged_prefill(qkv, self.kc[l], self.vc[l], att, pos, slot, self.d_btab, self.bs, self.Hl, self.hd, runs, cfg.seq)
+                for a, b in rest:
+                    ops.paged_attn(qkv[a:b], self.kc[l], self.vc[l], att[a:b], pos[a:b], slot[a:b], self.d_btab, self.bs, self.Hl,
+                                   self.hd, b - a, cfg.seq)
             else:
                 ops.paged_attn(qkv, self.kc[l], self.vc[l], att, pos, slot, self.d_btab, self.bs, self.Hl, self.hd, ntok,
                                cfg.seq, append=decode, n_split=self.attn_splits, scratch=self.attn_scratch)
@@ -230,9 +238,34 @@ class InferEngine:
             out.append((a, b - a))
         return out if len(out) == nseq else None
 
+    def _prompt_runs(self, ntok, nseq):
+        """(runs, rest) of a step that lists several tokens of a sequence: runs = [(first row, length)] of at least sixteen
+        consecutive positions of one sequence (shorter ones are faster a warp per token: nine-token prompts 1177 us a
+        completion against 1224), rest = [(a, b)] the row ranges between them; None when there are no runs or the tile
+        kernel does not take the configuration."""
+        if (ntok < nseq + 15 or self.dev.type != "cuda" or self.dt != torch.bfloat16 or self.attn_splits > 1
+                or self.hd not in (32, 64, 128)):
+            return None
+        pos = self.np_meta[self._o_pos:self._o_pos + ntok]
+        slot = self.np_meta[self._o_slot:self._o_slot + ntok]
+        cuts = np.flatnonzero((slot[1:] != slot[:-1]) | (pos[1:] != pos[:-1] + 1)) + 1
+        lo = np.concatenate(([0], cuts)).tolist()
+        hi = lo[1:] + [ntok]
+        runs, rest, at = [], [], 0
+        for a, b in zip(lo, hi):
+            if b - a >= 16:
+                if at < a:
+                    rest.append((at, a))
+                runs.append((a, b - a))
+                at = b
+        if at < ntok:
+            rest.append((at, ntok))
+        return (runs, rest) if runs else None
+
     def _run(self, ntok, nseq, rep=1):
         """Metadata is already in ``h_meta``; runs one step and returns the sampled ids (host)."""
         self._fresh = self._fresh_prompts(ntok, nseq)
+        self._runs = None if self._fresh else self._prompt_runs(ntok, nseq)
         sd = self.seed & 0xFFFFFFFFFFFFFFFF
         to_i32 = lambda u: u - (1 << 32) if u >= (1 << 31) else u
         self.np_meta[self._o_step:self._o_step + 3] = (self.step_no & 0x7FFFFFFF, to_i32(sd & 0xFFFFFFFF), to_i32(sd >> 32))

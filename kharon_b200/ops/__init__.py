@@ -557,6 +557,21 @@ def paged_attn(qkv, kc, vc, out, pos, slot, btab, bs, H, hd, ntok, max_ctx, appe
                               1.0 / math.sqrt(hd), ntok, max_ctx, int(append), _stream())
 
 
+def paged_prefill(qkv, kc, vc, out, pos, slot, btab, bs, H, hd, runs, max_ctx):
+    """``paged_attn`` for runs of consecutive positions of one sequence each, ``runs = [(first row, length), ...]``, whose K/V
+    are in the cache already (``append_kv``); on the tensor cores, with fp32 probabilities.  Head widths 32, 64 and 128."""
+    if _use_reference(qkv):
+        for r, n in runs:
+            ref.paged_attn(qkv[r:r + n], kc, vc, out[r:r + n], pos[r:r + n], slot[r:r + n], btab, bs, H, hd, n)
+        return
+    k = len(runs)
+    rows = torch.tensor([r for r, _ in runs] + [n for _, n in runs], dtype=torch.int32)
+    assert all(0 <= r and r + n <= qkv.shape[0] for r, n in runs)
+    _call(_lib().kh_paged_prefill, 1, qkv.data_ptr(), qkv.stride(0), kc.data_ptr(), vc.data_ptr(), out.data_ptr(), pos.data_ptr(),
+          slot.data_ptr(), btab.data_ptr(), btab.stride(0), bs, H, hd, 1.0 / math.sqrt(hd), max_ctx, rows.data_ptr(),
+          rows.data_ptr() + 4 * k, k, _stream())
+
+
 def gather_rows(x, rows, out, nseq):
     if _use_reference(x):
         out[:nseq].copy_(x[rows[:nseq].long()])

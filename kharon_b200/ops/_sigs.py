@@ -64,6 +64,7 @@ _OPTIONAL = {
     "kh_decode_layers_work_bytes": (long_, i32),
     "kh_paged_attn_split": (i32, vp, i32, vp, vp, vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, f32, i32, i32, i32, i32, vp),
     "kh_paged_attn": (i32, vp, i32, vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, f32, i32, i32, i32, vp),
+    "kh_paged_prefill": (i32, vp, i32, vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, f32, i32, vp, vp, i32, vp),
     "kh_gather_rows": (i32, vp, vp, vp, i32, i32, vp),
     "kh_copy_blocks": (i32, vp, vp, vp, i32, i32, long_, long_, vp),
     "kh_sample2": (i32, vp, i32, i32, f32, C.c_uint64, i32, vp, i32, vp, i32, vp),
