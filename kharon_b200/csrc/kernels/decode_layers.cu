@@ -21,8 +21,8 @@
 // the fetch of a barrier; a CTA without work in a phase does not take part in it.  Packets double the
 // bytes of an activation, which are a few KB per row.  A buffer is overwritten one layer later; by then every
 // reader is done, because each phase's output depends on all rows and columns of the one before it.
-// Measured, L24 d1024 with the head, context 160, a captured step with embedding and sampler: 507 us for one
-// sequence and 565 for eight (grid barriers and weights held in registers: 1000 and 1090; the weights alone
+// Measured, L24 d1024 with the head, context 160, a captured step with embedding and sampler: 468 us for one
+// sequence and 520 for eight (grid barriers and weights held in registers: 1000 and 1090; the weights alone
 // take 106 us at the copy bandwidth).
 //
 // Linear phases.  A work unit is 16 output columns (8 in phases C and E, whose N is only d); S warps share

@@ -87,7 +87,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
   // still running.  Weights that the previous kernel cannot have written (decode steps: the engine says
   // so) are requested right away, so the weight stream of this product overlaps the tail of the previous
   // one; everything an earlier kernel produces (the token rows) is touched after the wait.
-  if (tid == 0) {
+  if (warp == 0 && elect_one()) {
     for (int i = 0; i < nkb; i++) {
       mbar_expect_tx(bar_full + 8 * i, fuse_ln ? W_BYTES : STAGE);
       if (p.w_static) tma_load_2d(base + i * STAGE, &map_w, bar_full + 8 * i, (kb0 + i) * BK, nt * TN);
@@ -95,7 +95,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
   }
   pdl_wait();
   pdl_launch_dependents();
-  if (tid == 0) {
+  if (warp == 0 && elect_one()) {
     for (int i = 0; i < nkb; i++) {
       const uint32_t sw = base + i * STAGE, sx = sw + W_BYTES;
       if (!p.w_static) tma_load_2d(sw, &map_w, bar_full + 8 * i, (kb0 + i) * BK, nt * TN);
@@ -148,7 +148,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     fence_proxy_async_smem();        // generic-proxy writes -> visible to the tensor core's async proxy
   }
   __syncthreads();
-  if (tid == 0) {
+  if (warp == 0 && elect_one()) {
     constexpr uint32_t idesc = umma_idesc_bf16(TN, MP, 0, 0);
     for (int i = 0; i < nkb && ok; i++) {
       if (!mbar_wait(bar_full + 8 * i, 0, abort_flag, 1, p.err)) { ok = false; break; }
