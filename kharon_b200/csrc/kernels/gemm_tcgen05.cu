@@ -1006,7 +1006,9 @@ extern "C" int kh_gemm_bf16_colsum(const void* A, int lda, int a_mn, const void*
     // waves x relative tile time; narrower tiles reuse the A panel less and run at lower efficiency
     const int tm = (M + BM - 1) / BM, sms = num_sms();
     auto waves = [&](int w) { return (tm * ((N + w - 1) / w) + sms - 1) / sms; };
-    const float c256 = waves(256) * 1.0f, c128 = waves(128) * 0.7f, c64 = waves(64) * 0.5f;
+    // (up to K = 512 the epilogue weighs more and a 128-wide wave costs less: 8192 x 768 x 256 9.2 us in three waves of 128,
+    // 10.0 in two of 256; 4096 x 1536 x 512 11.7 and 11.9)
+    const float c256 = waves(256) * 1.0f, c128 = waves(128) * (K <= 512 ? 0.62f : 0.7f), c64 = waves(64) * 0.5f;
     bn = 256;
     float best = c256;
     if (c128 < best) { best = c128; bn = 128; }
@@ -1014,8 +1016,10 @@ extern "C" int kh_gemm_bf16_colsum(const void* A, int lda, int a_mn, const void*
     if (N <= 64) bn = 64;
     else if (N <= 128 && bn == 256) bn = 128;
     // 256 x 256 tiles on CTA pairs: a wave of pairs takes about 0.93 of a wave of single tiles
-    // (measured 6-19 % faster on large shapes), so prefer it unless wave quantisation eats the gain
-    if (bn == 256 && M >= 512 && g_pair_clusters != 0) {
+    // (measured 6-19 % faster on large shapes), so prefer it unless wave quantisation eats the gain.  A pair also pays about
+    // 1 us for its cluster, which short main loops do not earn back: single tiles in up to four waves at K = 512
+    // (9216 x 1536 16.5 us against 18.3; 8192 x 50257 in 86 waves 450 against 416), and up to K = 4096 where one wave does (4200 x 1024 x 1024 12.8 against 13.8; 2048 x 2048 x 8192 56.3 against 51.5)
+    if (bn == 256 && M >= 512 && g_pair_clusters != 0 && (waves(256) > (K <= 512 ? 4 : 1) || K > 4096)) {
       const int clusters = g_pair_clusters > 0 ? g_pair_clusters : sms / 2;
       const int tiles2 = ((M + 255) / 256) * ((N + 255) / 256);
       const float cpair = (float)((tiles2 + clusters - 1) / clusters) * 0.93f;
