@@ -93,15 +93,24 @@ __global__ void embed_bwd_wte_k(const int* __restrict__ tok, const bf16* __restr
     // warp 0 collects the later rows with the same id, in row order (ballot + prefix popcount)
     if (threadIdx.x < 32) {
       int n = 0;
-      for (int base = r + 1; base < rows && n < dup - 1; base += 32) {
-        const int i = base + threadIdx.x;
-        const bool hit = i < rows && tok[i] == t;
-        const unsigned mask = __ballot_sync(0xffffffffu, hit);
-        if (hit) {
-          const int at = n + __popc(mask & ((1u << threadIdx.x) - 1));
-          if (at < 64) s_list[at] = i;
+      // 256 ids per turn, eight loads in flight a lane: the scan is a chain of memory latencies (9216 rows, 256 ids: 73 us with one)
+      for (int base = r + 1; base < rows && n < dup - 1; base += 256) {
+        int id[8];
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+          const int i = base + k * 32 + threadIdx.x;
+          id[k] = i < rows ? __ldg(tok + i) : -1;
         }
-        n += __popc(mask);
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+          const bool hit = id[k] == t;
+          const unsigned mask = __ballot_sync(0xffffffffu, hit);
+          if (hit) {
+            const int at = n + __popc(mask & ((1u << threadIdx.x) - 1));
+            if (at < 64) s_list[at] = base + k * 32 + threadIdx.x;
+          }
+          n += __popc(mask);
+        }
       }
       if (threadIdx.x == 0) s_n = n;
     }
@@ -111,9 +120,17 @@ __global__ void embed_bwd_wte_k(const int* __restrict__ tok, const bf16* __restr
   for (int e = threadIdx.x * 2; e < d; e += blockDim.x * 2) {
     float2 acc = unpack_bf16(*reinterpret_cast<const uint32_t*>(dx + (size_t)r * d + e));
     if (n_list <= 64) {
-      for (int k = 0; k < n_list; k++) {
-        float2 v = unpack_bf16(*reinterpret_cast<const uint32_t*>(dx + (size_t)s_list[k] * d + e));
-        acc.x += v.x; acc.y += v.y;
+      for (int k0 = 0; k0 < n_list; k0 += 8) {       // eight rows fetched together, added in row order
+        uint32_t u[8];
+#pragma unroll
+        for (int k = 0; k < 8; k++)
+          if (k0 + k < n_list) u[k] = *reinterpret_cast<const uint32_t*>(dx + (size_t)s_list[k0 + k] * d + e);
+#pragma unroll
+        for (int k = 0; k < 8; k++)
+          if (k0 + k < n_list) {
+            const float2 v = unpack_bf16(u[k]);
+            acc.x += v.x; acc.y += v.y;
+          }
       }
     } else {   // very frequent id: plain ordered scan
       for (int i = r + 1; i < rows; i++)

@@ -580,3 +580,19 @@ def test_flash_short_sequences(B, T, H, hd):
     again = torch.empty_like(dqkv)
     ops.flash_bwd(qkv, out, dout, lse, again, delta, B, T, H, hd)
     assert torch.equal(again, dqkv) and ops.error_word() == 0
+
+
+@pytest.mark.parametrize("rows,V,d", [(1, 3, 64), (257, 2, 64), (1000, 9, 130), (2049, 700, 256)])
+def test_embedding_gradient_with_repeated_ids(rows, V, d):
+    """Ids that occur 1 to 500 times (the list of later rows holds 64), rows around the scan's turns of 256: fp32 sums in row order,
+    the order of the reference loop, so the bits agree."""
+    g = torch.Generator().manual_seed(rows)
+    tok = torch.randint(0, V, (rows,), generator=g)
+    tok[: min(rows, 66)] = 0
+    dx = torch.randn(rows, d, generator=g).bfloat16()
+    want = torch.zeros(V, d)
+    for i in range(rows):
+        want[tok[i]] += dx[i].float()
+    dwte = torch.zeros(V, d, device="cuda")
+    ops.embed_bwd(tok.int().cuda(), dx.cuda(), dwte, None, 1, rows)
+    assert torch.equal(dwte.cpu(), want)
