@@ -252,6 +252,54 @@ __device__ __forceinline__ void split3(float x, float y, uint32_t& hi, uint32_t&
   lo = pack_bf16(x - h.x - m.x, y - h.y - m.y);
 }
 
+// One token and head by one warp: positions 0..p of a cache at kc / vc (head offset included), output to dst.  The arithmetic of
+// paged_attn_k, a key per lane group at a time.
+template <int HD>
+__device__ __noinline__ void attend_row(const bf16* q, const bf16* kc, const bf16* vc, const int* bt, int bs, int d, int p, float scale, bf16* dst) {
+  constexpr int LPK = HD / 8, KPW = 32 / LPK;
+  const int lane = threadIdx.x & 31, e0 = (lane % LPK) * 8;
+  auto unpack8 = [](const uint4& u, float (&f)[8]) {
+    const float2 a = unpack_bf16(u.x), b = unpack_bf16(u.y), c = unpack_bf16(u.z), e = unpack_bf16(u.w);
+    f[0] = a.x; f[1] = a.y; f[2] = b.x; f[3] = b.y; f[4] = c.x; f[5] = c.y; f[6] = e.x; f[7] = e.y;
+  };
+  float x[8], k8[8], v8[8], o[8], m = -INFINITY, l = 0.f;
+  unpack8(*reinterpret_cast<const uint4*>(q + e0), x);
+#pragma unroll
+  for (int i = 0; i < 8; i++) { x[i] *= scale; o[i] = 0.f; }
+#pragma unroll 1
+  for (int j0 = 0; j0 <= p; j0 += KPW) {
+    const int j = j0 + lane / LPK, jj = min(j, p);
+    const size_t at = ((size_t)__ldg(bt + jj / bs) * bs + jj % bs) * d + e0;
+    unpack8(*reinterpret_cast<const uint4*>(kc + at), k8);
+    unpack8(*reinterpret_cast<const uint4*>(vc + at), v8);
+    float s = 0.f;
+#pragma unroll
+    for (int i = 0; i < 8; i++) s += k8[i] * x[i];
+#pragma unroll
+    for (int i = LPK / 2; i > 0; i >>= 1) s += __shfl_xor_sync(0xffffffffu, s, i);
+    if (j <= p) {
+      const float mn = fmaxf(m, s), ref = mn == -INFINITY ? 0.f : mn, sc = __expf(m - ref), pr = __expf(s - ref);
+      m = mn;
+      l = l * sc + pr;
+#pragma unroll
+      for (int i = 0; i < 8; i++) o[i] = o[i] * sc + pr * v8[i];
+    }
+  }
+#pragma unroll
+  for (int x2 = LPK; x2 < 32; x2 <<= 1) {
+    const float m2 = __shfl_xor_sync(0xffffffffu, m, x2), l2 = __shfl_xor_sync(0xffffffffu, l, x2);
+    const float mn = fmaxf(m, m2), ref = mn == -INFINITY ? 0.f : mn, c1 = __expf(m - ref), c2 = __expf(m2 - ref);
+    m = mn;
+    l = l * c1 + l2 * c2;
+#pragma unroll
+    for (int i = 0; i < 8; i++) o[i] = o[i] * c1 + __shfl_xor_sync(0xffffffffu, o[i], x2) * c2;
+  }
+  const float inv = 1.f / l;
+  if (lane < LPK)
+    *reinterpret_cast<uint4*>(dst + e0) = make_uint4(pack_bf16(o[0] * inv, o[1] * inv), pack_bf16(o[2] * inv, o[3] * inv),
+                                                     pack_bf16(o[4] * inv, o[5] * inv), pack_bf16(o[6] * inv, o[7] * inv));
+}
+
 template <int HD>
 __global__ void __launch_bounds__(128)
 paged_prefill_k(const __grid_constant__ PrefillTiles tiles, const bf16* __restrict__ qkv, int ld, const bf16* __restrict__ kc,
@@ -376,6 +424,20 @@ paged_prefill_k(const __grid_constant__ PrefillTiles tiles, const bf16* __restri
       }
     }
     __syncthreads();                                                            // the buffer is refilled in the next turn
+  }
+  // An infinity or NaN in V reaches the rows that see its position and no others.  The products above multiply it with the zeros of
+  // masked positions and of the lower terms of P too, which leaves a NaN in every row of the warp: such a warp does its rows anew.
+  uint32_t top = 0;
+#pragma unroll
+  for (int t = 0; t < HD / 8; t++)
+#pragma unroll
+    for (int i = 0; i < 4; i++) top = max(top, __float_as_uint(o[t][i]) & 0x7fffffffu);
+  if (__any_sync(0xffffffffu, top >= 0x7f800000u)) {
+#pragma unroll 1
+    for (int r = w0; r < min(n, w0 + 16); r++)
+      attend_row<HD>(qkv + (size_t)(r0 + r) * ld + h * HD, kc + h * HD, vc + h * HD, bt, bs, d, p0 + r, scale,
+                     out + (size_t)(r0 + r) * d + h * HD);
+    return;
   }
 #pragma unroll
   for (int i = 0; i < 2; i++) {

@@ -355,3 +355,34 @@ def test_paged_prefill_tiles(hd, H, bs):
     late = P >= 100
     assert ops.error_word(reset=True) == 8
     assert (out[late] == 7.0).all() and not (out[~late] == 7.0).all(-1).any()
+
+
+@pytest.mark.parametrize("hd,H,bs", [(32, 2, 5), (64, 3, 16), (128, 1, 8)])
+@pytest.mark.parametrize("bad", [float("inf"), float("-inf"), float("nan")])
+def test_paged_prefill_keeps_non_finite_values_behind_the_causal_edge(hd, H, bs, bad):
+    """An infinity or NaN in V of a later prompt position (first tile, a tile in the middle, last position) changes no earlier row
+    by a bit beyond the order of its sums (bf16 outputs: 2^-8 of the row's largest value), and the rows that see it get what the
+    kernel for single tokens gives them: the same infinities and NaNs."""
+    torch.manual_seed(hd)
+    d, n, max_lb = H * hd, 150, (150 + bs - 1) // bs
+    qkv = torch.randn(n, 3 * d, device="cuda").bfloat16()
+    pos = torch.arange(n, device="cuda", dtype=torch.int32); slot = torch.zeros_like(pos)
+    btab = torch.randperm(max_lb, device="cuda").int().view(1, max_lb)
+    def attend(x):
+        kc = torch.zeros(max_lb, bs, H, hd, device="cuda").bfloat16(); vc = kc.clone()
+        ops.append_kv(x, kc, vc, pos, slot, btab, bs, H, hd, n)
+        tile, one = torch.empty(n, d, device="cuda", dtype=torch.bfloat16), torch.empty(n, d, device="cuda", dtype=torch.bfloat16)
+        ops.paged_prefill(x, kc, vc, tile, pos, slot, btab, bs, H, hd, [(0, n)], n)
+        ops.paged_attn(x, kc, vc, one, pos, slot, btab, bs, H, hd, n, n)
+        return tile.float(), one.float()
+    clean, _ = attend(qkv)
+    for at, col in ((9, 3), (63, 0), (64, hd - 1), (100, 5), (n - 1, 7)):
+        x = qkv.clone()
+        x[at, 2 * d + col] = bad
+        tile, one = attend(x)
+        assert ((tile[:at] - clean[:at]).abs().amax(1) <= 2.0 ** -8 * clean[:at].abs().amax(1)).all(), at
+        assert torch.equal(tile.isnan(), one.isnan()) and torch.equal(tile.isinf(), one.isinf()), at
+        assert not tile[at:, col].isfinite().any()
+        fin = one.isfinite()
+        assert torch.equal(fin, tile.isfinite()) and ((tile - one)[fin].abs() <= 2.0 ** -7 * one[fin].abs().max()).all()
+    assert ops.error_word() == 0
