@@ -626,7 +626,7 @@ __device__ __forceinline__ void attention_phase(const DecodeParams& p, int layer
           o[k] = o[k] * c1 + o2 * c2;
         }
       }
-    }
+    } else { m = 0.f; l = 1.f; }       // an item with a bad index writes zeros: its row must not stall
     float* mine = satt + warp * ATT_PITCH;
     if (lane < LPK) {
 #pragma unroll
@@ -644,7 +644,7 @@ __device__ __forceinline__ void attention_phase(const DecodeParams& p, int layer
       float c = k16 < W ? part[k16 * ATT_PITCH + 128] : -INFINITY, den = k16 < W ? part[k16 * ATT_PITCH + 129] : 0.f, mx = c;
 #pragma unroll
       for (int x = 8; x > 0; x >>= 1) mx = fmaxf(mx, __shfl_xor_sync(mask, mx, x));
-      c = mx == -INFINITY ? 0.f : __expf(c - mx);
+      c = __expf(c - mx);              // (NaN when every score is -inf, as in the kernel chain)
       den *= c;
 #pragma unroll
       for (int x = 8; x > 0; x >>= 1) den += __shfl_xor_sync(mask, den, x);
@@ -655,7 +655,7 @@ __device__ __forceinline__ void attention_phase(const DecodeParams& p, int layer
         const float2 f = *reinterpret_cast<const float2*>(part + k * ATT_PITCH + e);
         v0 += ck * f.x; v1 += ck * f.y;
       }
-      const float inv = mx == -INFINITY ? 0.f : 1.f / den;       // (an item with a bad index writes zeros: its row must not stall)
+      const float inv = 1.f / den;
       const int tt = it / p.H;
       if (it < items) st_packet(p.attp + ((size_t)tt * d + (it - tt * p.H) * HD + e) / 2, pack_bf16(v0 * inv, v1 * inv), epoch);
     }

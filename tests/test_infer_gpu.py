@@ -386,3 +386,20 @@ def test_paged_prefill_keeps_non_finite_values_behind_the_causal_edge(hd, H, bs,
         fin = one.isfinite()
         assert torch.equal(fin, tile.isfinite()) and ((tile - one)[fin].abs() <= 2.0 ** -7 * one[fin].abs().max()).all()
     assert ops.error_word() == 0
+
+
+@pytest.mark.parametrize("G", [1, 20])
+def test_persistent_decode_does_not_hide_scores_that_overflow(G):
+    """Scores that are all -inf (q and k of one head so large that their product overflows) have no softmax: the persistent kernel
+    hands on the NaN that the kernel chain gives, not zeros that look like an answer."""
+    cfg = Config(2, 512, 8, 300, 32, 1)
+    m = GPT(cfg, "cuda", torch.bfloat16); m.init_weights_device(3)
+    b = m.params.p["l0.qkv_b"]
+    b[:64] = 3e38
+    b[512:576] = -3e38
+    m.sync_bf16()
+    for flag in (False, True):
+        e = InferEngine(m, block_size=4, max_seqs=G + 1, persistent_decode=flag, use_graphs=False)
+        e.generate([[5 + g] for g in range(G)], 1)          # one-token prompts: a decode step at position 0
+        assert e.persistent == flag and e.logits[:G, :300].isnan().all(), flag
+    assert ops.error_word() == 0
