@@ -44,10 +44,11 @@ def _chk(rc, n=1):
     launch_count += n
 
 
-def _call(fn, n, *args):
-    """Invoke a native entry point; remember the exact call when a plan is being recorded."""
+def _call(fn, n, *args, keep=None):
+    """Invoke a native entry point; remember the exact call when a plan is being recorded.  ``keep``: objects made for this call
+    alone whose memory it points to; a recorded call holds them for its replays."""
     if _recording is not None:
-        _recording.append((fn, args, n))
+        _recording.append((fn, args, n, keep))
     _chk(fn(*args), n)
 
 
@@ -85,7 +86,7 @@ class LaunchPlan:
     def replay(self):
         global launch_count
         err = 0
-        for fn, args, n in self.calls:
+        for fn, args, n, _ in self.calls:
             if n < 0:
                 fn(*args)            # host callable
             else:
@@ -98,7 +99,7 @@ class LaunchPlan:
 def plan_call(fn, *args):
     """Run a host-side callable (a collective, a copy) and make it part of the plan being recorded."""
     if _recording is not None:
-        _recording.append((fn, args, -1))
+        _recording.append((fn, args, -1, None))
     fn(*args)
 
 
@@ -109,7 +110,7 @@ def plan_call_host(fn, *args):
     global _recording
     rec = _recording
     if rec is not None:
-        rec.append((fn, args, -1))
+        rec.append((fn, args, -1, None))
     _recording = None
     try:
         fn(*args)
@@ -215,7 +216,7 @@ def decode_layers(x, xmid, qkv, att, act, layers, n_layer, H, hd, kc, vc, pos, s
     _call(_lib().kh_decode_layers, 1, x.data_ptr(), layers.data_ptr(), n_layer, G, d, H, hd, kc.data_ptr(), vc.data_ptr(),
           kc.stride(0), pos.data_ptr(), slot.data_ptr(), btab.data_ptr(), btab.shape[1], bs, max_ctx, 1.0 / float(hd) ** 0.5,
           _p(head_w), _p(lnf_w), _p(lnf_b), _p(logits), logits.stride(0) if logits is not None else 0, vocab,
-          _p(rows), n_rows, work.data_ptr(), _stream())
+          _p(rows), n_rows, work.data_ptr(), _stream(), keep=work)
 
 
 def gemm_skinny_scratch_elems(M, N, K):
@@ -452,7 +453,7 @@ def flash_fwd_varlen(qkv, out, segs, H, hd):
     k = len(segs)
     assert all(0 <= r and r + n <= qkv.shape[0] for r, n in segs)
     _call(_lib().kh_flash_fwd_varlen, 1, qkv.data_ptr(), out.data_ptr(), rows.data_ptr(), rows.data_ptr() + 4 * k, k, H, hd,
-          qkv.stride(0), 1.0 / math.sqrt(hd), _stream())
+          qkv.stride(0), 1.0 / math.sqrt(hd), _stream(), keep=rows)
 
 
 def flash_fwd(qkv, out, lse, B, T, H, hd):
@@ -569,7 +570,7 @@ def paged_prefill(qkv, kc, vc, out, pos, slot, btab, bs, H, hd, runs, max_ctx):
     assert all(0 <= r and r + n <= qkv.shape[0] for r, n in runs)
     _call(_lib().kh_paged_prefill, 1, qkv.data_ptr(), qkv.stride(0), kc.data_ptr(), vc.data_ptr(), out.data_ptr(), pos.data_ptr(),
           slot.data_ptr(), btab.data_ptr(), btab.stride(0), bs, H, hd, 1.0 / math.sqrt(hd), max_ctx, rows.data_ptr(),
-          rows.data_ptr() + 4 * k, k, _stream())
+          rows.data_ptr() + 4 * k, k, _stream(), keep=rows)
 
 
 def gather_rows(x, rows, out, nseq):

@@ -140,3 +140,51 @@ def test_fresh_prompt_detection_reads_the_step_metadata():
     assert e._fresh_prompts(*fill([(0, 64), (5, 100)])) is None          # a chunk that continues a prompt
     assert e._fresh_prompts(*fill([(0, 64), (0, 10)])) is None           # a short prompt
     assert e._fresh_prompts(*fill([(7, 1), (9, 1)])) is None             # decode step
+
+
+def _fake_lib(monkeypatch, seen):
+    """Native calls on CPU tensors: every entry point is noted in ``seen`` as (name, arguments) and succeeds."""
+    from kharon_b200 import ops
+
+    class Lib:
+        def __getattr__(self, name):
+            if name == "kh_decode_layers_work_bytes":
+                return lambda d: 64 + 32 * 10 * (d // 2) * 8
+            return lambda *a: (seen.append((name, a)), 0)[1]
+    monkeypatch.setattr(ops, "_lib", lambda: Lib())
+    monkeypatch.setattr(ops, "_stream", lambda: 0)
+    monkeypatch.setattr(ops, "_use_reference", lambda t: False)
+
+
+def test_recorded_calls_keep_the_memory_they_point_to(monkeypatch):
+    """Row lists and workspaces that an operator makes for one call still hold their values when a recorded plan replays it,
+    whatever was allocated in between."""
+    import ctypes as C
+    import gc
+    import weakref
+    from kharon_b200 import ops
+    seen = []
+    _fake_lib(monkeypatch, seen)
+    runs = [(0, 3), (3, 5), (8, 17)]
+    qkv, out = torch.zeros(25, 96), torch.zeros(25, 32)
+    z = torch.zeros(4, dtype=torch.int32)
+    made = []
+    real = ops.decode_layers_work
+    monkeypatch.setattr(ops, "decode_layers_work", lambda d, dev: (made.append(real(d, dev)), made[-1])[1])
+    plan = ops.LaunchPlan()
+    with plan.record():
+        ops.flash_fwd_varlen(qkv, out, runs, 1, 32)
+        ops.paged_prefill(qkv, out, out, out, z, z, z.view(2, 2), 2, 1, 32, runs, 64)
+        x = torch.zeros(2, 256)
+        ops.decode_layers(x, x, x, x, x, z, 1, 4, 64, x, x, z, z, z.view(2, 2), 2, 64)
+    work = weakref.ref(made.pop())
+    gc.collect()
+    junk = [torch.full((6,), 7, dtype=torch.int32) for _ in range(200)]
+    seen.clear()
+    plan.replay()
+    assert work() is not None
+    read = lambda p: list((C.c_int32 * 3).from_address(p))
+    for name, rows, lens in (("kh_flash_fwd_varlen", 2, 3), ("kh_paged_prefill", 14, 15)):
+        args = dict(seen)[name]
+        assert read(args[rows]) == [0, 3, 8] and read(args[lens]) == [3, 5, 17], name
+    assert len(junk) == 200
