@@ -213,6 +213,9 @@ def decode_layers(x, xmid, qkv, att, act, layers, n_layer, H, hd, kc, vc, pos, s
     G, d = x.shape
     if work is None:
         work = decode_layers_work(d, x.device)
+    elif (work.device != x.device or not work.is_contiguous()
+          or work.numel() * work.element_size() < int(_lib().kh_decode_layers_work_bytes(d))):
+        raise ValueError("decode_layers: the workspace must be contiguous, on %s and made for width %d" % (x.device, d))
     _call(_lib().kh_decode_layers, 1, x.data_ptr(), layers.data_ptr(), n_layer, G, d, H, hd, kc.data_ptr(), vc.data_ptr(),
           kc.stride(0), pos.data_ptr(), slot.data_ptr(), btab.data_ptr(), btab.shape[1], bs, max_ctx, 1.0 / float(hd) ** 0.5,
           _p(head_w), _p(lnf_w), _p(lnf_b), _p(logits), logits.stride(0) if logits is not None else 0, vocab,

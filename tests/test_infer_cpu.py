@@ -188,3 +188,23 @@ def test_recorded_calls_keep_the_memory_they_point_to(monkeypatch):
         args = dict(seen)[name]
         assert read(args[rows]) == [0, 3, 8] and read(args[lens]) == [3, 5, 17], name
     assert len(junk) == 200
+
+
+def test_decode_layers_refuses_a_workspace_that_is_too_small(monkeypatch):
+    """The workspace of a narrower model, a strided view and a buffer of another device are refused before anything is launched;
+    the exact size is taken."""
+    from kharon_b200 import ops
+    seen = []
+    _fake_lib(monkeypatch, seen)
+    z = torch.zeros(4, dtype=torch.int32)
+    x = torch.zeros(2, 512)
+    call = lambda w: ops.decode_layers(x, x, x, x, x, z, 1, 8, 64, x, x, z, z, z.view(2, 2), 2, 64, work=w)
+    good = ops.decode_layers_work(512, "cpu")
+    for bad in (ops.decode_layers_work(256, "cpu"), good[:-1], torch.zeros(2 * good.numel(), dtype=torch.int64)[::2],
+                torch.zeros(good.numel(), dtype=torch.int64, device="meta")):
+        with pytest.raises(ValueError):
+            call(bad)
+    assert not seen
+    call(good)
+    call(torch.zeros(2 * good.numel(), dtype=torch.int64))
+    assert [n for n, _ in seen] == ["kh_decode_layers"] * 2
