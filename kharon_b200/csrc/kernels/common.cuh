@@ -346,15 +346,19 @@ int kh_pdl_enabled();
 // Launch `kernel` on `stream` with the library's launch attributes; arguments are converted to the
 // kernel's parameter types.
 template <typename... P, typename... A>
-inline cudaError_t kh_launch_ex(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A... args) {
+inline cudaError_t kh_launch_ex(bool pdl, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = stream;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = kh_pdl_enabled() ? 1 : 0;
+  cfg.numAttrs = pdl && kh_pdl_enabled() ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
 }
 #define KH_LAUNCH(kernel, grid, block, smem, stream, ...) \
-  kh_launch_ex(kernel, dim3(grid), dim3(block), (size_t)(smem), (cudaStream_t)(stream), __VA_ARGS__)
+  kh_launch_ex(true, kernel, dim3(grid), dim3(block), (size_t)(smem), (cudaStream_t)(stream), __VA_ARGS__)
+// Without the attribute: the kernel's blocks are placed when the stream's earlier kernels are done.  A kernel with several long
+// blocks per SM needs that: blocks that come while the previous kernel still holds the shared memory of some SMs all go to the others.
+#define KH_LAUNCH_AFTER(kernel, grid, block, smem, stream, ...) \
+  kh_launch_ex(false, kernel, dim3(grid), dim3(block), (size_t)(smem), (cudaStream_t)(stream), __VA_ARGS__)

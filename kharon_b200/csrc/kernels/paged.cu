@@ -497,6 +497,8 @@ extern "C" int kh_paged_prefill(const void* qkv, int ld, const void* kc, const v
 // kernel combines the ranges (weights exp(lse_s - max lse)).  More CTAs per token than heads when a
 // decode step has few sequences, and a score buffer of one range instead of the whole context.
 // The range that holds position `pos` appends the token's k, v first (decode steps).
+// Launched without programmatic dependence (KH_LAUNCH_AFTER): blocks that came while the GEMM before them still held the shared
+// memory of part of the SMs all went to the others (4 layers of d2048, 32 sequences at 16300 positions: 5477 us a step, 3883 so).
 template <int HD>
 __global__ void __launch_bounds__(128)
 paged_attn_split_k(const bf16* __restrict__ qkv, int ld, bf16* __restrict__ kc, bf16* __restrict__ vc,
@@ -624,7 +626,7 @@ extern "C" int kh_paged_attn_split(const void* qkv, int ld, void* kc, void* vc, 
   {                                                                                                                       \
     static size_t attr = 48 * 1024;                                                                                       \
     if (smem > attr) { cudaFuncSetAttribute(paged_attn_split_k<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); attr = smem; } \
-    KH_LAUNCH((paged_attn_split_k<HD>), grid, 128, smem, st, (const bf16*)qkv, ld, (bf16*)kc, (bf16*)vc, (float*)o_part,  \
+    KH_LAUNCH_AFTER((paged_attn_split_k<HD>), grid, 128, smem, st, (const bf16*)qkv, ld, (bf16*)kc, (bf16*)vc, (float*)o_part,  \
               (float*)lse_part, (const int*)pos, (const int*)slot, (const int*)btab, max_lb, bs, H, scale, max_ctx, chunk, \
               append, kh_error_word_dev());                                                                               \
   }
