@@ -863,6 +863,9 @@ extern "C" int kh_decode_layers_ok(int G, int d, int H, int hd, int max_ctx) {
          max_ctx >= 1 && max_ctx <= 32768;
 }
 
+// Sequences of width d that one launch holds (more run in groups, and every group reads all weights again).
+extern "C" int kh_decode_layers_rows(int d) { return 8 * max_mt(d); }
+
 // Bytes of the packet workspace (zero-initialised once, then only used by launches that follow one another).
 extern "C" long kh_decode_layers_work_bytes(int d) { return 64 + (long)MAX_ROWS * 10 * (d / 2) * 8; }
 

@@ -97,14 +97,21 @@ class InferEngine:
             self.skinny = torch.zeros(n, dtype=torch.float32, **z)
         # Decode steps of up to ``persistent_max`` sequences run all layers and the head in one persistent kernel
         # when the shape allows it (ops.decode_layers); KHARON_PERSISTENT_DECODE=0 or persistent_decode=False keeps
-        # the five-kernel chain.  Measured on B200, us a step (L24 d1024, context 160-200): 468 / 520 / 741 / 1080 / 1212 at
-        # G = 1 / 8 / 16 / 24 / 32 against 1255 / 1776 / 2029 / 1824 / 1851 for the chain.
+        # the five-kernel chain.  The limit by width is measured (us a step, persistent / chain):
+        #   L24 d1024, context 200: G = 8 524 / 1654, 16 737 / 1887, 17 938 / 1127, 24 1082 / 1155, 32 1208 / 1206;
+        #   L24 d1280: G = 16 1349 / 2115, 17 1994 / 1298, 32 3025 / 1495 (the chain's tensor-core GEMM starts at 17 rows);
+        #   L24 d2048, context 300: G = 16 2062 / 3486, 17 3156 / 1815 (two launches), 32 4122 / 1983.
         if persistent_decode is None:
             persistent_decode = os.environ.get("KHARON_PERSISTENT_DECODE", "1") != "0"
         self.persistent = bool(persistent_decode and self.skinny is not None and self.tp == 1 and self.dt == torch.bfloat16
                                and ops.decode_layers_ok(1, d, cfg.n_head, cfg.head_dim, cfg.seq))
-        self.persistent_max = int(os.environ.get("KHARON_PERSISTENT_MAX_G", "32"))
+        self.persistent_max, self.skinny_rows = 0, ops.SKINNY_BEST_ROWS
         if self.persistent:
+            rows = ops.decode_layers_rows(d)
+            self.persistent_max = int(os.environ.get("KHARON_PERSISTENT_MAX_G", rows if d <= 1024 else min(16, rows)))
+            # Widths of which one launch holds eight (3584 and more): steps of 9 to 16 rows take the chain with the tensor-core GEMM
+            # (d4096, 16 rows, qkv / proj / fc / fcproj / head: 22 / 10 / 30 / 29 / 79 us; skinny 48 / 28 / 59 / 132 / 113).
+            self.skinny_rows = min(self.skinny_rows, rows)
             names = ("ln1_w", "ln1_b", "qkv_w", "qkv_b", "proj_w", "proj_b", "ln2_w", "ln2_b", "fc_w", "fc_b",
                      "fcproj_w", "fcproj_b")
             self.layer_table = torch.tensor([[model.L(l, n).data_ptr() for n in names] for l in range(L)],
@@ -122,6 +129,7 @@ class InferEngine:
         self.flash_prefill = bool(flash_prefill and self.dev.type == "cuda" and self.dt == torch.bfloat16
                                   and self.hd in (64, 128))
         self._fresh = self._runs = None
+        self._fused = False
         self.temperature, self.seed, self.step_no = 0.0, 0, 0
         # under TP the captured step contains the fused GEMM + all-reduce kernels (their call counter
         # is a device word); the NCCL seam is left to eager launches
@@ -159,9 +167,7 @@ class InferEngine:
         tok, pos, slot = self.d_tok[:ntok], self.d_pos[:ntok], self.d_slot[:ntok]
         xs = x[:ntok]
         ops.embed_fwd(tok, pos, P["wte"], P["wpe"], xs, cfg.seq)
-        fused_layers = (self.persistent and ntok == nseq and ntok <= self.persistent_max
-                        and ops.decode_layers_ok(ntok, cfg.d_model, cfg.n_head, cfg.head_dim, cfg.seq))
-        if fused_layers:      # layers and head in one kernel; only the sampler follows
+        if self._fused:       # layers and head in one kernel; only the sampler follows
             ops.decode_layers(xs, self.xmid[:ntok], self.qkv[:ntok], self.att[:ntok], self.act[:ntok], self.layer_table,
                               cfg.n_layer, self.Hl, self.hd, self.kc, self.vc, pos, slot, self.d_btab, self.bs, cfg.seq,
                               work=self.decode_work, head_w=m.head_weight(), lnf_w=P["lnf_w"], lnf_b=P["lnf_b"], logits=self.logits,
@@ -202,7 +208,7 @@ class InferEngine:
 
     def _lin(self, x, w, out, epi=ops.EPI_NONE, bias=None, aux=None):
         """Column-parallel / replicated linear layer: skinny kernel for decode-sized inputs."""
-        if self.skinny is not None and x.shape[0] <= ops.SKINNY_BEST_ROWS:
+        if self.skinny is not None and x.shape[0] <= self.skinny_rows:
             ops.gemm_skinny(x, w, out, self.skinny, epi=epi, bias=bias, aux=aux, weights_static=True)
         else:
             ops.gemm(x, w, out, epi=epi, bias=bias, aux=aux)
@@ -210,7 +216,7 @@ class InferEngine:
     def _ln_lin(self, x, ln_w, ln_b, ln_out, w, out, epi=ops.EPI_NONE, bias=None, aux=None):
         """LayerNorm followed by a linear layer: for decode-sized inputs the skinny kernel normalises
         the rows itself (no LayerNorm launch, ``ln_out`` stays unused)."""
-        if self.skinny is not None and x.shape[0] <= ops.SKINNY_BEST_ROWS and x.shape[1] % 8 == 0:
+        if self.skinny is not None and x.shape[0] <= self.skinny_rows and x.shape[1] % 8 == 0:
             ops.gemm_skinny(x, w, out, self.skinny, epi=epi, bias=bias, aux=aux, ln_w=ln_w, ln_b=ln_b, weights_static=True)
         else:
             ops.layernorm_fwd(x, ln_w, ln_b, ln_out)
@@ -262,15 +268,25 @@ class InferEngine:
             rest.append((at, ntok))
         return (runs, rest) if runs else None
 
+    def _one_kernel(self, ntok, nseq):
+        """Whether this step runs in the persistent kernel.  Beyond 4096 positions its W warps per (sequence, head) lose to the
+        chain's split-KV attention once the sequences fill the SMs (L4 d1024, us a step, persistent / chain: context 4000 of 4096
+        G = 17 568 / 597, 32 942 / 737; 8100 G = 17 944 / 791, 24 1426 / 973; 16300 G = 17 1714 / 1395, 32 3134 / 2169; 200 of
+        4096 G = 17 198 / 252, 32 245 / 258; eight heads, context 8000, G = 17 437 / 524, 32 739 / 672)."""
+        if not (self.persistent and ntok == nseq and ntok <= self.persistent_max and ntok <= 32):
+            return False
+        return ntok <= 16 or ntok * self.Hl <= 148 or int(self.np_meta[self._o_pos:self._o_pos + ntok].max()) < 4096
+
     def _run(self, ntok, nseq, rep=1):
         """Metadata is already in ``h_meta``; runs one step and returns the sampled ids (host)."""
+        self._fused = self._one_kernel(ntok, nseq)
         self._fresh = self._fresh_prompts(ntok, nseq)
         self._runs = None if self._fresh else self._prompt_runs(ntok, nseq)
         sd = self.seed & 0xFFFFFFFFFFFFFFFF
         to_i32 = lambda u: u - (1 << 32) if u >= (1 << 31) else u
         self.np_meta[self._o_step:self._o_step + 3] = (self.step_no & 0x7FFFFFFF, to_i32(sd & 0xFFFFFFFF), to_i32(sd >> 32))
         self.d_meta.copy_(self.h_meta, non_blocking=True)
-        key = (ntok, nseq, rep, self.temperature)
+        key = (ntok, nseq, rep, self.temperature, self._fused)
         if self.use_graphs and ntok == nseq:           # greedy and sampled steps alike: the step number lives in d_meta
             g = self.graphs.get(key)
             if g is None and key in self._warm:

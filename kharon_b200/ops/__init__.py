@@ -196,6 +196,12 @@ def decode_layers_ok(G, d, H, hd, max_ctx):
     return bool(torch.cuda.is_available() and _lib().kh_decode_layers_ok(G, d, H, hd, max_ctx))
 
 
+def decode_layers_rows(d):
+    """Sequences of width ``d`` that one launch of ``decode_layers`` holds: 32, 16 or 8.  More of them run in groups, and every
+    group reads all weights again."""
+    return int(_lib().kh_decode_layers_rows(d))
+
+
 def decode_layers_work(d, device):
     """Workspace of ``decode_layers`` for models of width ``d``: the activations travel through it between the kernel's
     thread blocks.  Zeroed once; its launches must follow one another (one workspace per engine and stream)."""

@@ -403,3 +403,33 @@ def test_persistent_decode_does_not_hide_scores_that_overflow(G):
         e.generate([[5 + g] for g in range(G)], 1)          # one-token prompts: a decode step at position 0
         assert e.persistent == flag and e.logits[:G, :300].isnan().all(), flag
     assert ops.error_word() == 0
+
+
+@pytest.mark.parametrize("d,heads,most", [(256, 8, 32), (1024, 16, 32), (1280, 20, 16), (2048, 16, 16), (3072, 24, 16), (4096, 32, 8)])
+def test_decode_steps_that_need_two_launches_take_the_chain(d, heads, most):
+    """The persistent kernel takes the step sizes at which one launch holds all sequences and beats the chain; the steps beyond them
+    (the chain, from eight rows on with the tensor-core GEMM at the largest widths) give the same logits."""
+    cfg = Config(2, d, heads, 601, 64, 1)
+    m = GPT(cfg, "cuda", torch.bfloat16); m.init_weights_device(5); m.params.w.mul_(3.0); m.sync_bf16()
+    e = InferEngine(m, block_size=5, max_seqs=34, max_tokens=256, use_graphs=False)
+    assert e.persistent and e.persistent_max == most <= ops.decode_layers_rows(d)
+    prompts = [[(7 * g + i) % 601 for i in range(1 + g % 7)] for g in range(33)]
+    for G in (most, most + 1):
+        rows = {}
+        for limit in (most, 32):
+            e.persistent_max = limit
+            e.generate(prompts[:G], 2)
+            assert e._fused == (G <= min(limit, 32))
+            rows[limit] = e.logits[:G, :601].float().clone()
+        assert ((rows[32] - rows[most]).norm() / rows[32].norm()).item() < 3e-2
+    assert ops.error_word() == 0
+
+
+def test_long_contexts_of_many_sequences_take_split_attention():
+    cfg = Config(1, 512, 16, 300, 4200, 1)
+    m = GPT(cfg, "cuda", torch.bfloat16); m.init_weights_device(5)
+    e = InferEngine(m, block_size=64, n_blocks=200, max_seqs=18, max_tokens=4400, use_graphs=False)
+    for first, G, fused in ((4090, 17, False), (4090, 16, True), (4090 - 20, 17, True)):
+        e.generate([[3] * first] + [[5 + g] for g in range(G - 1)], 8)      # the last steps stand at first + 6
+        assert e._fused == fused, (first, G)
+    assert ops.error_word() == 0
