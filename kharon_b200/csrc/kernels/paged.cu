@@ -753,35 +753,39 @@ sample_k(const bf16* __restrict__ logits, int ld, int V, float temperature, unsi
     }
   }
 }
-// Greedy rows: the same argmax (lowest index wins ties, NaN never wins) with 1024 threads and 16-byte loads, eight in flight a
-// thread.  sample_k's contiguous chunks per thread, which the draw needs, read 2 bytes at a time: 15 us for 50257 logits.
-__global__ void __launch_bounds__(1024)
+// Greedy rows: the same argmax (lowest index wins ties, NaN never wins) with 16-byte loads, eight in flight a thread, and 1024 or
+// 256 threads.  sample_k's contiguous chunks per thread, which the draw needs, read 2 bytes at a time.  us for 1 / 512 rows, sample_k /
+// 1024 / 256 threads: V = 2049 2.6 / 2.2 / 2.0 and 3.3 / 7.3 / 2.6, V = 8000 4.2 / 2.1 / 1.9 and 10.8 / 7.2 / 3.4,
+// V = 50257 13.2 / 3.4 / 4.4 and 46.8 / 12.6 / 9.8.
+template <int THREADS>
+__global__ void __launch_bounds__(THREADS)
 argmax_k(const bf16* __restrict__ logits, int ld, int V, int rep, int* __restrict__ out) {
   pdl_wait();
   pdl_launch_dependents();
-  __shared__ float s_v[32];
-  __shared__ int s_i[32];
+  constexpr int WARPS = THREADS / 32;
+  __shared__ float s_v[WARPS];
+  __shared__ int s_i[WARPS];
   const int row = blockIdx.x, tid = threadIdx.x, lane = tid & 31;
   const bf16* lg = logits + (size_t)row * ld;
   float best = -INFINITY;
   int bi = V;
   auto take = [&](float x, int i) { if (x > best) { best = x; bi = i; } };       // indices rise within a thread
   const int nv = ((uintptr_t)lg & 15) == 0 ? V / 8 : 0;                           // whole 16-byte pieces
-  for (int c0 = tid; c0 < nv; c0 += 8 * 1024) {
+  for (int c0 = tid; c0 < nv; c0 += 8 * THREADS) {
     uint4 u[8];
 #pragma unroll
     for (int k = 0; k < 8; k++)
-      if (c0 + k * 1024 < nv) u[k] = __ldg(reinterpret_cast<const uint4*>(lg) + c0 + k * 1024);
+      if (c0 + k * THREADS < nv) u[k] = __ldg(reinterpret_cast<const uint4*>(lg) + c0 + k * THREADS);
 #pragma unroll
     for (int k = 0; k < 8; k++)
-      if (c0 + k * 1024 < nv) {
-        const int i = (c0 + k * 1024) * 8;
+      if (c0 + k * THREADS < nv) {
+        const int i = (c0 + k * THREADS) * 8;
         const float2 a = unpack_bf16(u[k].x), b = unpack_bf16(u[k].y), c = unpack_bf16(u[k].z), e = unpack_bf16(u[k].w);
         take(a.x, i); take(a.y, i + 1); take(b.x, i + 2); take(b.y, i + 3);
         take(c.x, i + 4); take(c.y, i + 5); take(e.x, i + 6); take(e.y, i + 7);
       }
   }
-  for (int i = nv * 8 + tid; i < V; i += 1024) take(__bfloat162float(lg[i]), i);
+  for (int i = nv * 8 + tid; i < V; i += THREADS) take(__bfloat162float(lg[i]), i);
   auto reduce = [&]() {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -794,7 +798,8 @@ argmax_k(const bf16* __restrict__ logits, int ld, int V, int rep, int* __restric
   if (lane == 0) { s_v[tid >> 5] = best; s_i[tid >> 5] = bi; }
   __syncthreads();
   if (tid >= 32) return;
-  best = s_v[lane]; bi = s_i[lane];
+  best = lane < WARPS ? s_v[lane] : -INFINITY;
+  bi = lane < WARPS ? s_i[lane] : V;
   reduce();
   for (int r = lane; r < rep; r += 32) out[row * rep + r] = bi;
 }
@@ -804,7 +809,10 @@ extern "C" int kh_sample2(const void* logits, int ld, int V, float temperature, 
                           const void* step_dev, int rep, void* out, int nseq, void* stream) {
   if (rep < 1 || rep > 256) { kh_set_error("sample: rep must be in [1, 256]"); return -1; }
   if (temperature <= 0.f && V > 2048) {
-    KH_LAUNCH(argmax_k, nseq, 1024, 0, (cudaStream_t)stream, (const bf16*)logits, ld, V, rep, (int*)out);
+    // one turn of loads takes up to 16384 logits with 256 threads; more rows than SMs share an SM, where a CTA of 1024 threads
+    // costs more than it loads
+    if (V > 16384 && nseq <= 148) KH_LAUNCH(argmax_k<1024>, nseq, 1024, 0, (cudaStream_t)stream, (const bf16*)logits, ld, V, rep, (int*)out);
+    else KH_LAUNCH(argmax_k<256>, nseq, 256, 0, (cudaStream_t)stream, (const bf16*)logits, ld, V, rep, (int*)out);
     KH_LAUNCH_CHECK("sample");
     return 0;
   }

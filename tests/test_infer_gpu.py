@@ -433,3 +433,19 @@ def test_long_contexts_of_many_sequences_take_split_attention():
         e.generate([[3] * first] + [[5 + g] for g in range(G - 1)], 8)      # the last steps stand at first + 6
         assert e._fused == fused, (first, G)
     assert ops.error_word() == 0
+
+
+@pytest.mark.parametrize("V", [2049, 16384, 16385, 50257])
+@pytest.mark.parametrize("n", [1, 148, 149, 700])
+def test_greedy_rows_on_both_sides_of_the_thread_count_rule(V, n):
+    """Few and many rows, up to and beyond one turn of loads: 256 and 1024 threads a row pick the lowest index of the maximum.
+    Logits of 8 bits tie often."""
+    g = torch.Generator(device="cuda").manual_seed(V + n)
+    lg = torch.randint(-60, 60, (n, (V + 7) // 8 * 8), device="cuda", generator=g).bfloat16()
+    lg[:, V:] = 100.0
+    lg[0, V - 1] = 99.0
+    out = torch.full((n,), -1, device="cuda", dtype=torch.int32)
+    ops.sample(lg, V, 0.0, 1, 0, 1, out, n)
+    x = lg[:, :V].float()
+    want = torch.where(x == x.max(-1, keepdim=True).values, torch.arange(V, device="cuda"), V).min(-1).values.int()
+    assert torch.equal(out, want)
