@@ -1021,13 +1021,23 @@ int launch_bwd(const void* qkv, const AttnParams& p, cudaStream_t st) {
   return launch_bwd_as<HD, false>(qkv, p, st);
 }
 
+// Whether flash_short.cu takes sequences of T <= 64 positions.  Its cost is the arithmetic of mma.sync on the rows that are there,
+// that of the kernels here the latency of an item per resident CTA.  Head width 64: always (B 32-1000 H8 T 33-64: 0.4 to 0.93 of the
+// time forward, 0.3 to 0.91 backward).  Head width 128, forward, us (short / tcgen05): T 64, 592 items 9.3 / 10.7, 1536 31.8 / 23.5;
+// T 48, 1536 21.1 / 22.2, 2048 30.8 / 26.9; T 40, 2048 24.4 / 26.1, 3200 47.5 / 38.1; T 32, 4096 39.7 / 46.1.  Backward: T 64,
+// 384 items 29.1 / 31.0, 768 71.6 / 56.6; T 48, 4800 218 / 277.
+static bool use_short(bool backward, int T, int hd, long items) {
+  if (T < 1 || T > KH_FLASH_SHORT_T) return false;
+  if (hd == 64 || T <= 32 || (backward && T <= 48)) return true;
+  return items <= (backward ? 3L : T <= 40 ? 14L : T <= 48 ? 10L : 4L) * num_sms_attn();
+}
+
 }  // namespace
 
 extern "C" int kh_flash_fwd(const void* qkv, void* out, void* lse, int B, int T, int H, int hd, int ld, float scale,
                             void* stream) {
   if (hd != 64 && hd != 128) { kh_set_error("flash: head dim %d is not supported (64 or 128)", hd); return -1; }
-  // a tile of 128 rows would be at most half full: see flash_short.cu
-  if (T >= 1 && T <= KH_FLASH_SHORT_T) return kh_flash_short_fwd(qkv, out, lse, B, T, H, hd, ld, scale, stream);
+  if (use_short(false, T, hd, (long)B * H)) return kh_flash_short_fwd(qkv, out, lse, B, T, H, hd, ld, scale, stream);
   AttnParams p = {};
   p.B = B; p.T = T; p.H = H; p.ld = ld; p.scale = scale; p.out = (bf16*)out; p.lse = (float*)lse;
   p.err = kh_error_word_dev();
@@ -1051,7 +1061,7 @@ extern "C" int kh_flash_fwd_varlen(const void* qkv, void* out, const void* row0,
 extern "C" int kh_flash_bwd(const void* qkv, const void* out, const void* dout, const void* lse, void* dqkv,
                             void* delta, int B, int T, int H, int hd, int ld, float scale, void* stream) {
   if (hd != 64 && hd != 128) { kh_set_error("flash: head dim %d is not supported (64 or 128)", hd); return -1; }
-  if (T >= 1 && T <= KH_FLASH_SHORT_T) return kh_flash_short_bwd(qkv, out, dout, lse, dqkv, delta, B, T, H, hd, ld, scale, stream);
+  if (use_short(true, T, hd, (long)B * H)) return kh_flash_short_bwd(qkv, out, dout, lse, dqkv, delta, B, T, H, hd, ld, scale, stream);
   AttnParams p = {};
   p.B = B; p.T = T; p.H = H; p.ld = ld; p.scale = scale; p.lse = (float*)lse; p.o = (const bf16*)out;
   p.dout = (const bf16*)dout; p.delta = (float*)delta; p.dqkv = (bf16*)dqkv;

@@ -341,6 +341,14 @@ def test_flash_fwd_bwd(B, T, H, hd):
     assert torch.equal(out, out3) and torch.equal(lse, lse3) and torch.equal(dqkv, dqkv3)
 
 
+@pytest.mark.parametrize("B,T,H,hd", [(74, 64, 8, 128), (75, 64, 8, 128), (55, 49, 8, 128), (56, 49, 8, 128), (185, 48, 8, 128),
+                                      (186, 48, 8, 128), (259, 40, 8, 128), (260, 33, 8, 128)])
+def test_flash_short_sequences_of_many_items(B, T, H, hd):
+    """Up to 64 positions at head width 128, on both sides of the item counts at which the kernel for short sequences hands over
+    to the 128-row tiles, forward and backward independently."""
+    test_flash_fwd_bwd(B, T, H, hd)
+
+
 def test_flash_large_scores_rescale():
     """Scores that keep growing along the keys force the in-place rescaling of the output accumulator."""
     torch.manual_seed(21)
