@@ -105,7 +105,10 @@ template <int NSEG> struct FwdMaps { CUtensorMap q[NSEG], kv[NSEG], o[NSEG]; };
 template <int NSEG> struct FwdSegs { int T[NSEG]; uint16_t pair[MAX_PAIRS]; };      // pair = query tile * MAX_SEGS + sequence
 template <> struct FwdSegs<1> {};
 
-template <int HD, int NSEG>
+// ONE_TILE (head width 128, one sequence length of up to 128 positions, more than four items per SM): the MMA role is entered by
+// lane 0, as in the dK / dV kernel below (T 40, 4800 items: 53.9 us, 56.8 with the elected lane; T 66, 32 items: 6.4 and 6.2;
+// T 512, 256 items: 40.0 and 39.4).
+template <int HD, int NSEG, bool ONE_TILE>
 __global__ void __launch_bounds__(192, 2)
 flash_fwd_ws_kernel(const __grid_constant__ FwdMaps<NSEG> maps, const __grid_constant__ FwdSegs<NSEG> seg, const AttnParams p,
                     int n_items, int n_qt) {
@@ -192,7 +195,7 @@ flash_fwd_ws_kernel(const __grid_constant__ FwdMaps<NSEG> maps, const __grid_con
     }
   } else if (warp == 5) {
     // ------------------------------------------------------------------ MMA issuer
-    if (live && elect_one()) {
+    if (live && (ONE_TILE ? lane == 0 : elect_one())) {
       constexpr uint32_t idesc_s = umma_idesc_bf16(128, BKV, 0, 0);
       constexpr uint32_t idesc_o = umma_idesc_bf16(128, HD, 0, 1);
       int ic = 0, pc = 0, kvc = 0;
@@ -442,7 +445,10 @@ template <int W> __device__ __forceinline__ void tmem_cols(uint32_t a, uint32_t*
 }
 
 // ---- dK, dV: item = (batch, head, 128 keys); sub-tiles of 64 queries from the diagonal to the end
-template <int HD, bool TWO>
+// ONE_TILE (head width 128, up to 128 positions, one key tile per item, more than four items per SM): the MMA role is entered by
+// lane 0.  With the elected lane the kernel is faster on longer sequences and few items (whole backward B 32 H8 T1777: 1357 -> 1130 us;
+// T 66, 32 items: 16.4 -> 15.8) and slower there (T 100, 4800 items: 386 -> 419).
+template <int HD, bool TWO, bool ONE_TILE>
 __global__ void __launch_bounds__(320, BwdWs<HD, TWO>::CTAS)
 flash_dkv_ws_kernel(const __grid_constant__ CUtensorMap map_kv, const __grid_constant__ CUtensorMap map_q,
                     const __grid_constant__ CUtensorMap map_do, const __grid_constant__ CUtensorMap map_dqkv, const AttnParams p,
@@ -509,7 +515,7 @@ flash_dkv_ws_kernel(const __grid_constant__ CUtensorMap map_kv, const __grid_con
       }
     }
   } else if (warp == 9) {
-    if (live && elect_one()) {
+    if (live && (ONE_TILE ? lane == 0 : elect_one())) {
       constexpr uint32_t idesc_s = umma_idesc_bf16(128, BS, 0, 0);
       constexpr uint32_t idesc_g = umma_idesc_bf16(128, HD, 0, 1);
       int ic = 0, qc = 0, rc = 0;
@@ -929,13 +935,13 @@ static int num_sms_attn() {
   return sms > 0 ? sms : 148;
 }
 
-template <int HD, int NSEG>
+template <int HD, int NSEG, bool ONE_TILE>
 int launch_fwd_items(const FwdMaps<NSEG>& maps, const FwdSegs<NSEG>& seg, const AttnParams& p, int n_items, int n_qt, cudaStream_t st) {
   using C = FwdWs<HD>;
   static bool once = false;
-  if (!once) { if (set_smem(flash_fwd_ws_kernel<HD, NSEG>, C::SMEM, "flash_fwd")) return -1; once = true; }
+  if (!once) { if (set_smem(flash_fwd_ws_kernel<HD, NSEG, ONE_TILE>, C::SMEM, "flash_fwd")) return -1; once = true; }
   const int ctas = 2 * num_sms_attn();                  // two CTAs per SM
-  KH_LAUNCH((flash_fwd_ws_kernel<HD, NSEG>), n_items < ctas ? n_items : ctas, C::THREADS, C::SMEM, st, maps, seg, p, n_items, n_qt);
+  KH_LAUNCH((flash_fwd_ws_kernel<HD, NSEG, ONE_TILE>), n_items < ctas ? n_items : ctas, C::THREADS, C::SMEM, st, maps, seg, p, n_items, n_qt);
   KH_LAUNCH_CHECK("flash_fwd");
   return 0;
 }
@@ -954,7 +960,8 @@ int launch_fwd(const void* qkv, const AttnParams& p, cudaStream_t st) {
   FwdMaps<1> maps;
   if (fwd_maps(maps, 0, qkv, p.out, p.B, p.T, p.H, HD, p.ld)) return -1;
   const int n_qt = (p.T + 127) / 128;
-  return launch_fwd_items<HD, 1>(maps, FwdSegs<1>{}, p, p.B * p.H * n_qt, n_qt, st);
+  if (HD == 128 && n_qt == 1 && p.B * p.H > 4 * num_sms_attn()) return launch_fwd_items<HD, 1, HD == 128>(maps, FwdSegs<1>{}, p, p.B * p.H, n_qt, st);
+  return launch_fwd_items<HD, 1, false>(maps, FwdSegs<1>{}, p, p.B * p.H * n_qt, n_qt, st);
 }
 // Sequences of rows [row0[i], row0[i] + len[i]) of qkv and out, as many per launch as the maps and the list of pairs hold.
 template <int HD>
@@ -984,7 +991,7 @@ int launch_fwd_varlen(const bf16* qkv, AttnParams p, const int* row0, const int*
       for (int i = 0; i < n; i++)
         if (qt < (seg.T[i] + 127) / 128) seg.pair[at++] = (uint16_t)(qt * MAX_SEGS + i);
     p.B = 1; p.T = 0;
-    if (launch_fwd_items<HD, MAX_SEGS>(maps, seg, p, pairs * p.H, most, st)) return -1;
+    if (launch_fwd_items<HD, MAX_SEGS, false>(maps, seg, p, pairs * p.H, most, st)) return -1;
     s0 += n;
   }
   return 0;
@@ -1001,16 +1008,18 @@ int launch_bwd_as(const void* qkv, const AttnParams& p, cudaStream_t st) {
   const CUtensorMap* mg = kh_tmap_3d_bf16(p.dqkv, (uint64_t)3 * p.H * HD, p.T, p.B, (uint64_t)p.ld, (uint64_t)p.T * p.ld, 128, 64);
   if (!mq || !md || !mq64 || !md64 || !mg) return -1;
   KH_LAUNCH((flash_delta_kernel<HD>), (unsigned)((rows * 32 + 255) / 256), 256, 0, st, p.o, p.dout, p.delta, p.B, p.T, p.H);
+  const int n_t = (p.T + 127) / 128;
+  auto dkv = HD == 128 && n_t == 1 && p.B * p.H > 4 * num_sms_attn() ? flash_dkv_ws_kernel<HD, TWO, HD == 128> : flash_dkv_ws_kernel<HD, TWO, false>;
   static bool once = false;
   if (!once) {
-    if (set_smem(flash_dkv_ws_kernel<HD, TWO>, C::SMEM_KV, "flash_dkv") || set_smem(flash_dq_ws_kernel<HD, TWO>, C::SMEM_Q, "flash_dq")) return -1;
+    if (set_smem(flash_dkv_ws_kernel<HD, TWO, HD == 128>, C::SMEM_KV, "flash_dkv") ||
+        set_smem(flash_dkv_ws_kernel<HD, TWO, false>, C::SMEM_KV, "flash_dkv") || set_smem(flash_dq_ws_kernel<HD, TWO>, C::SMEM_Q, "flash_dq")) return -1;
     once = true;
   }
-  const int n_t = (p.T + 127) / 128;
   const int n_items = p.B * p.H * n_t;
   const int ctas = C::CTAS * num_sms_attn();
   const int grid = n_items < ctas ? n_items : ctas;
-  KH_LAUNCH((flash_dkv_ws_kernel<HD, TWO>), grid, C::THREADS, C::SMEM_KV, st, *mq, *mq64, *md64, *mg, p, n_items, n_t);
+  KH_LAUNCH(dkv, grid, C::THREADS, C::SMEM_KV, st, *mq, *mq64, *md64, *mg, p, n_items, n_t);
   KH_LAUNCH((flash_dq_ws_kernel<HD, TWO>), grid, C::THREADS, C::SMEM_Q, st, *mq, *md, *mq64, *mg, p, n_items, n_t);
   KH_LAUNCH_CHECK("flash_bwd");
   return 0;

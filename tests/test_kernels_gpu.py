@@ -342,10 +342,11 @@ def test_flash_fwd_bwd(B, T, H, hd):
 
 
 @pytest.mark.parametrize("B,T,H,hd", [(74, 64, 8, 128), (75, 64, 8, 128), (55, 49, 8, 128), (56, 49, 8, 128), (185, 48, 8, 128),
-                                      (186, 48, 8, 128), (259, 40, 8, 128), (260, 33, 8, 128)])
+                                      (186, 48, 8, 128), (259, 40, 8, 128), (260, 33, 8, 128), (74, 128, 8, 128), (75, 128, 8, 128),
+                                      (80, 65, 16, 128)])
 def test_flash_short_sequences_of_many_items(B, T, H, hd):
-    """Up to 64 positions at head width 128, on both sides of the item counts at which the kernel for short sequences hands over
-    to the 128-row tiles, forward and backward independently."""
+    """Up to 128 positions at head width 128, on both sides of the item counts at which the kernel for short sequences hands over
+    to the 128-row tiles, forward and backward independently, and the kernels for one tile per item come in."""
     test_flash_fwd_bwd(B, T, H, hd)
 
 
