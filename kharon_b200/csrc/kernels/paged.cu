@@ -56,7 +56,8 @@ extern "C" int kh_append_kv(const void* qkv, int ld, void* kc, void* vc, const v
 // shared memory in warp order across warps).  K and V of a position are fetched together, and the next four positions replace
 // the current ones in their registers as soon as those are used: one trip to memory per four keys and no CTA barrier in the
 // loop.  Neighbouring items are tokens of the same head, which read mostly the same rows (L1).
-// W = 1 when the items fill the chip by themselves (prefill, large batches), else 4.
+// W = 1 when the items fill the chip by themselves (prefill, large batches), else 4, and 2 between for narrow heads (8 heads of 32,
+// 128 tokens, us with W = 1 / 2 / 4: context 20 3.7 / 4.1 / 6.3, context 200 10.1 / 8.8 / 10.7, context 1000 41.7 / 31.1 / 32.6).
 // A CTA of 128 threads per item with barriers between scores, maximum, sum and value passes took 25.6 us for 512 tokens x 8
 // heads at contexts of 9 to 18.
 // Context = positions 0..pos of the token's own sequence.  With `append` != 0 (decode steps: one new token per sequence) the
@@ -170,7 +171,7 @@ paged_attn_k(const bf16* __restrict__ qkv, int ld, bf16* kc, bf16* vc, bf16* __r
       for (int k = 0; k < 8; k++) o[k] = o[k] * c1 + __shfl_xor_sync(0xffffffffu, o[k], x) * c2;
     }
   }
-  if (W > 1) {                                      // merge the warps in order; the first one writes
+  if (W > 1) {                                      // merge an item's warps in order; the first one writes
     float* part = s_part + warp * (HD + 2);
     if (lane < LPK) {
 #pragma unroll
@@ -178,19 +179,20 @@ paged_attn_k(const bf16* __restrict__ qkv, int ld, bf16* kc, bf16* vc, bf16* __r
       if (lane == 0) { part[HD] = m; part[HD + 1] = l; }
     }
     __syncthreads();
-    if (warp != 0 || !valid) return;
+    if (wi != 0 || !valid) return;
+    const float* parts = s_part + warp * (HD + 2);
     float mx = -INFINITY;
 #pragma unroll
-    for (int w = 0; w < W; w++) mx = fmaxf(mx, s_part[w * (HD + 2) + HD]);
+    for (int w = 0; w < W; w++) mx = fmaxf(mx, parts[w * (HD + 2) + HD]);
     l = 0.f;
 #pragma unroll
     for (int k = 0; k < 8; k++) o[k] = 0.f;
 #pragma unroll
     for (int w = 0; w < W; w++) {
-      const float c = __expf(s_part[w * (HD + 2) + HD] - mx);      // (position 0 is always there: mx is finite or NaN)
-      l += c * s_part[w * (HD + 2) + HD + 1];
+      const float c = __expf(parts[w * (HD + 2) + HD] - mx);      // (position 0 is always there: mx is finite or NaN)
+      l += c * parts[w * (HD + 2) + HD + 1];
 #pragma unroll
-      for (int k = 0; k < 8; k++) o[k] += c * s_part[w * (HD + 2) + e0 + k];
+      for (int k = 0; k < 8; k++) o[k] += c * parts[w * (HD + 2) + e0 + k];
     }
   }
   if (valid && lane < LPK) {
@@ -207,20 +209,25 @@ extern "C" int kh_paged_attn(const void* qkv, int ld, void* kc, void* vc, void* 
                              const void* slot, const void* btab, int max_lb, int bs, int H, int hd, float scale,
                              int ntok, int max_ctx, int append, void* stream) {
   cudaStream_t st = (cudaStream_t)stream;
+  // one range per token ends at some 50000 positions; longer contexts belong to kh_paged_attn_split
   if ((size_t)(hd + max_ctx + 1024 + 8) * sizeof(float) > 200 * 1024) { kh_set_error("paged_attn: context %d is too long for one range", max_ctx); return -1; }
   const int vec = ((uintptr_t)qkv & 15) == 0 && ((uintptr_t)out & 15) == 0 && ld % 8 == 0;
-  // one warp per item once the items alone give every SM some sixteen warps
-  const bool one = (long)ntok * H >= 148 * 16;
+  // one warp per item once the items alone give every SM some sixteen warps, else four; two for narrow heads, whose warp covers 32
+  // (64) positions a turn, once four would not fit the chip together
+  const long items = (long)ntok * H;
+  const int W = items >= 148 * 16 ? 1 : hd <= 32 && items > 148 * 4 ? 2 : 4;
 #define LAUNCH_W(HD, W)                                                                                                     \
   KH_LAUNCH((paged_attn_k<HD, W>), dim3(cdiv((long)ntok * W, 4), H), 128, 0, st, (const bf16*)qkv, ld, (bf16*)kc, (bf16*)vc, \
             (bf16*)out, (const int*)pos, (const int*)slot, (const int*)btab, max_lb, bs, H, ntok, scale, max_ctx, append, vec, \
             kh_error_word_dev())
-#define LAUNCH(HD) { if (one) LAUNCH_W(HD, 1); else LAUNCH_W(HD, 4); }
+#define LAUNCH(HD) { if (W == 1) LAUNCH_W(HD, 1); else LAUNCH_W(HD, 4); }
+#define LAUNCH_NARROW(HD) { if (W == 2) LAUNCH_W(HD, 2); else LAUNCH(HD) }
   if (hd == 128) LAUNCH(128)
   else if (hd == 64) LAUNCH(64)
-  else if (hd == 32) LAUNCH(32)
-  else if (hd == 16) LAUNCH(16)
+  else if (hd == 32) LAUNCH_NARROW(32)
+  else if (hd == 16) LAUNCH_NARROW(16)
   else { kh_set_error("paged_attn: head dim %d is not supported", hd); return -1; }
+#undef LAUNCH_NARROW
 #undef LAUNCH
 #undef LAUNCH_W
   KH_LAUNCH_CHECK("paged_attn");

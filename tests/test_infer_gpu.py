@@ -449,3 +449,40 @@ def test_greedy_rows_on_both_sides_of_the_thread_count_rule(V, n):
     x = lg[:, :V].float()
     want = torch.where(x == x.max(-1, keepdim=True).values, torch.arange(V, device="cuda"), V).min(-1).values.int()
     assert torch.equal(out, want)
+
+
+@pytest.mark.parametrize("hd,ntok", [(16, 74), (16, 75), (32, 75), (32, 296), (32, 295), (64, 75)])
+@pytest.mark.parametrize("append", [False, True])
+def test_paged_attention_warps_per_item(hd, ntok, append):
+    """Eight heads at the token counts where four warps an item become two (narrow heads) and two become one: contexts of 1 to 300
+    positions side by side in a CTA, one token with a bad position (status 8, its row left alone).  fp32 sums, bf16 outputs."""
+    torch.manual_seed(ntok + hd)
+    H, bs, max_lb = 8, 16, 20
+    d, nb = H * hd, ntok * max_lb
+    kc = torch.randn(nb, bs, H, hd, device="cuda").bfloat16(); vc = torch.randn_like(kc)
+    btab = torch.randperm(nb, device="cuda").int().view(ntok, max_lb)
+    pos = torch.tensor([(i * 37) % 300 for i in range(ntok)], device="cuda", dtype=torch.int32)
+    pos[7] = 999
+    slot = torch.arange(ntok, device="cuda", dtype=torch.int32)
+    qkv = torch.randn(ntok, 3 * d, device="cuda").bfloat16()
+    out = torch.full((ntok, d), 7.0, device="cuda").bfloat16()
+    k2, v2 = kc.clone(), vc.clone()
+    ops.paged_attn(qkv, kc, vc, out, pos, slot, btab, bs, H, hd, ntok, 320, append=append)
+    assert ops.error_word(reset=True) == 8 and (out[7] == 7.0).all()
+    good = [i for i in range(ntok) if i != 7]
+    x = qkv.float().view(ntok, 3, H, hd)
+    for i in good:
+        n = int(pos[i]) + 1
+        b = btab[i].long()
+        k, v = k2[b].reshape(-1, H, hd)[:n].float(), v2[b].reshape(-1, H, hd)[:n].float()
+        if append:
+            k[-1], v[-1] = x[i, 1], x[i, 2]
+        p = (torch.einsum("hd,khd->hk", x[i, 0], k) / hd ** 0.5).softmax(-1)
+        want = torch.einsum("hk,khd->hd", p, v).reshape(d)
+        assert ((out[i].float() - want).norm() / want.norm()).item() < 4e-3, i
+    if append:
+        i = good[-1]
+        b, p = int(btab[i, int(pos[i]) // bs]), int(pos[i]) % bs
+        assert torch.equal(kc[b, p], qkv[i, d:2 * d].view(H, hd)) and torch.equal(vc[b, p], qkv[i, 2 * d:].view(H, hd))
+    else:
+        assert torch.equal(kc, k2) and torch.equal(vc, v2)
