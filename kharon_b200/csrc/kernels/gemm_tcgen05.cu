@@ -1007,8 +1007,9 @@ extern "C" int kh_gemm_bf16_colsum(const void* A, int lda, int a_mn, const void*
     const int tm = (M + BM - 1) / BM, sms = num_sms();
     auto waves = [&](int w) { return (tm * ((N + w - 1) / w) + sms - 1) / sms; };
     // (up to K = 512 the epilogue weighs more and a 128-wide wave costs less: 8192 x 768 x 256 9.2 us in three waves of 128,
-    // 10.0 in two of 256; 4096 x 1536 x 512 11.7 and 11.9)
-    const float c256 = waves(256) * 1.0f, c128 = waves(128) * (K <= 512 ? 0.62f : 0.7f), c64 = waves(64) * 0.5f;
+    // 10.0 in two of 256; 4096 x 1536 x 512 11.7 and 11.9; but with up to 64 rows half of the epilogue warps have nothing to do, and
+    // at K = 512 the main loop counts again: 16 x 50257 x 512 13.5 us in two waves of 256, 15.4 in three of 128; K = 256 10.2, 10.1)
+    const float c256 = waves(256) * 1.0f, c128 = waves(128) * (K <= (M > 64 ? 512 : 256) ? 0.62f : 0.7f), c64 = waves(64) * 0.5f;
     bn = 256;
     float best = c256;
     if (c128 < best) { best = c128; bn = 128; }
