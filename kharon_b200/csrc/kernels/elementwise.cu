@@ -10,6 +10,8 @@
 
 #include "common.cuh"
 
+#include <type_traits>
+
 static inline int cdiv(long a, long b) { return (int)((a + b - 1) / b); }
 #define KH_LAUNCH_CHECK(name)                                                     \
   do {                                                                            \
@@ -78,67 +80,98 @@ __global__ void embed_bwd_index_k(const int* __restrict__ tok, int* __restrict__
   atomicMin(first + t, r);
   atomicAdd(cnt + t, 1);
 }
+constexpr int EMB_LIST = 64;
+// Warp 0 lists the next rows from `base` on with id t, in row order (ballot + prefix popcount), until it has `most` of them:
+// the first EMB_LIST go to `list`, n = their number, next (MORE: there may be more of them) = the row to go on from.
+template <bool MORE>
+__device__ __forceinline__ void embed_collect(const int* __restrict__ tok, int rows, int t, int base, int most, int* list, int* n_out, int* next) {
+  int n = 0;
+  // 256 ids per turn, eight loads in flight a lane: the scan is a chain of memory latencies (9216 rows, 256 ids: 73 us with one)
+  for (; base < rows && n < most; base += 256) {
+    int id[8];
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+      const int i = base + k * 32 + threadIdx.x;
+      id[k] = i < rows ? __ldg(tok + i) : -1;
+    }
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+      const bool hit = id[k] == t;
+      const unsigned mask = __ballot_sync(0xffffffffu, hit);
+      if (hit) {
+        const int at = n + __popc(mask & ((1u << threadIdx.x) - 1));
+        if (at < EMB_LIST) list[at] = base + k * 32 + threadIdx.x;
+        if (MORE && at == EMB_LIST) *next = base + k * 32 + threadIdx.x;
+      }
+      n += __popc(mask);
+    }
+  }
+  if (threadIdx.x == 0) {
+    *n_out = min(n, EMB_LIST);
+    if (MORE && n <= EMB_LIST) *next = base;
+  }
+}
+// acc += columns e, e + 1 of the n listed rows, in order: eight rows fetched together, then four, two and one
+__device__ __forceinline__ void embed_add(float2& acc, const bf16* __restrict__ dx, const int* list, int n, int d, int e) {
+  auto add = [&](int k0, auto c) {
+    uint32_t u[decltype(c)::value];
+#pragma unroll
+    for (int k = 0; k < decltype(c)::value; k++) u[k] = *reinterpret_cast<const uint32_t*>(dx + (size_t)list[k0 + k] * d + e);
+#pragma unroll
+    for (int k = 0; k < decltype(c)::value; k++) {
+      const float2 v = unpack_bf16(u[k]);
+      acc.x += v.x; acc.y += v.y;
+    }
+  };
+  int k = 0;
+  for (; k + 8 <= n; k += 8) add(k, std::integral_constant<int, 8>());
+  if (n & 4) { add(k, std::integral_constant<int, 4>()); k += 4; }
+  if (n & 2) { add(k, std::integral_constant<int, 2>()); k += 2; }
+  if (n & 1) add(k, std::integral_constant<int, 1>());
+}
+// An id with more later rows than a list holds: list by list, anew for every 256 columns (16384 rows, 256 ids, d256: 489 us when
+// every thread scanned the ids itself, 56 so).  Called by the whole CTA.
+__device__ __noinline__ void embed_bwd_frequent(const int* tok, const bf16* dx, float* dwte, int rows, int d, int r, int t, int left, int* list, int* n, int* next) {
+  for (int e0 = 0; e0 < d; e0 += blockDim.x * 2) {
+    const int e = e0 + threadIdx.x * 2;
+    float2 acc = make_float2(0.f, 0.f);
+    if (e < d) acc = unpack_bf16(*reinterpret_cast<const uint32_t*>(dx + (size_t)r * d + e));
+    int at = r + 1;
+    for (int done = 0; done < left; done += *n, at = *next) {
+      __syncthreads();                              // everybody has read the last list
+      if (threadIdx.x < 32) embed_collect<true>(tok, rows, t, at, min(left - done, EMB_LIST + 1), list, n, next);
+      __syncthreads();
+      if (*n == 0) break;
+      if (e < d) embed_add(acc, dx, list, *n, d, e);
+    }
+    if (e < d) {
+      float2* o = reinterpret_cast<float2*>(dwte + (size_t)t * d + e);
+      float2 old = *o;
+      old.x += acc.x; old.y += acc.y;
+      *o = old;
+    }
+  }
+}
 __global__ void embed_bwd_wte_k(const int* __restrict__ tok, const bf16* __restrict__ dx, float* __restrict__ dwte,
                                 const int* __restrict__ first, const int* __restrict__ cnt, int rows, int d, int V) {
   pdl_wait();
   pdl_launch_dependents();
-  __shared__ int s_list[64];
-  __shared__ int s_n;
+  __shared__ int s_list[EMB_LIST];
+  __shared__ int s_n, s_next;
   const int r = blockIdx.x;
   const int t = tok[r];
   if (t < 0 || t >= V || first[t] != r) return;
-  const int dup = cnt[t];
+  const int left = cnt[t] - 1;                      // later rows with this id
+  if (left > EMB_LIST) { embed_bwd_frequent(tok, dx, dwte, rows, d, r, t, left, s_list, &s_n, &s_next); return; }
   int n_list = 0;
-  if (dup > 1) {
-    // warp 0 collects the later rows with the same id, in row order (ballot + prefix popcount)
-    if (threadIdx.x < 32) {
-      int n = 0;
-      // 256 ids per turn, eight loads in flight a lane: the scan is a chain of memory latencies (9216 rows, 256 ids: 73 us with one)
-      for (int base = r + 1; base < rows && n < dup - 1; base += 256) {
-        int id[8];
-#pragma unroll
-        for (int k = 0; k < 8; k++) {
-          const int i = base + k * 32 + threadIdx.x;
-          id[k] = i < rows ? __ldg(tok + i) : -1;
-        }
-#pragma unroll
-        for (int k = 0; k < 8; k++) {
-          const bool hit = id[k] == t;
-          const unsigned mask = __ballot_sync(0xffffffffu, hit);
-          if (hit) {
-            const int at = n + __popc(mask & ((1u << threadIdx.x) - 1));
-            if (at < 64) s_list[at] = base + k * 32 + threadIdx.x;
-          }
-          n += __popc(mask);
-        }
-      }
-      if (threadIdx.x == 0) s_n = n;
-    }
+  if (left > 0) {
+    if (threadIdx.x < 32) embed_collect<false>(tok, rows, t, r + 1, left, s_list, &s_n, nullptr);
     __syncthreads();
     n_list = s_n;
   }
   for (int e = threadIdx.x * 2; e < d; e += blockDim.x * 2) {
     float2 acc = unpack_bf16(*reinterpret_cast<const uint32_t*>(dx + (size_t)r * d + e));
-    if (n_list <= 64) {
-      for (int k0 = 0; k0 < n_list; k0 += 8) {       // eight rows fetched together, added in row order
-        uint32_t u[8];
-#pragma unroll
-        for (int k = 0; k < 8; k++)
-          if (k0 + k < n_list) u[k] = *reinterpret_cast<const uint32_t*>(dx + (size_t)s_list[k0 + k] * d + e);
-#pragma unroll
-        for (int k = 0; k < 8; k++)
-          if (k0 + k < n_list) {
-            const float2 v = unpack_bf16(u[k]);
-            acc.x += v.x; acc.y += v.y;
-          }
-      }
-    } else {   // very frequent id: plain ordered scan
-      for (int i = r + 1; i < rows; i++)
-        if (tok[i] == t) {
-          float2 v = unpack_bf16(*reinterpret_cast<const uint32_t*>(dx + (size_t)i * d + e));
-          acc.x += v.x; acc.y += v.y;
-        }
-    }
+    embed_add(acc, dx, s_list, n_list, d, e);
     float2* o = reinterpret_cast<float2*>(dwte + (size_t)t * d + e);
     float2 old = *o;
     old.x += acc.x; old.y += acc.y;

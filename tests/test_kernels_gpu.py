@@ -605,3 +605,22 @@ def test_embedding_gradient_with_repeated_ids(rows, V, d):
     dwte = torch.zeros(V, d, device="cuda")
     ops.embed_bwd(tok.int().cuda(), dx.cuda(), dwte, None, 1, rows)
     assert torch.equal(dwte.cpu(), want)
+
+
+@pytest.mark.parametrize("later", [1, 7, 63, 64, 65, 127, 128, 129, 300, 1000])
+def test_embedding_gradient_of_an_id_with_many_later_rows(later):
+    """One id with exactly so many later rows (a list holds 64), close together and far apart, over three column chunks: the order of
+    the reference loop, so the bits agree."""
+    g = torch.Generator().manual_seed(later)
+    for rows in (later + 1, later + 300, 3 * later + 700):
+        tok = torch.full((rows,), 1)
+        at = torch.randperm(rows, generator=g)[:later + 1]
+        tok[at] = 0
+        tok[(tok == 1).nonzero().flatten()[::2]] = 2
+        dx = torch.randn(rows, 514, generator=g).bfloat16()
+        want = torch.zeros(3, 514)
+        for i in range(rows):
+            want[tok[i]] += dx[i].float()
+        dwte = torch.zeros(3, 514, device="cuda")
+        ops.embed_bwd(tok.int().cuda(), dx.cuda(), dwte, None, 1, rows)
+        assert torch.equal(dwte.cpu(), want), rows
