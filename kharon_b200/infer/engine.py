@@ -247,8 +247,10 @@ class InferEngine:
     def _prompt_runs(self, ntok, nseq):
         """(runs, rest) of a step that lists several tokens of a sequence: runs = [(first row, length)] of at least sixteen
         consecutive positions of one sequence (shorter ones are faster a warp per token: nine-token prompts 1177 us a
-        completion against 1224), rest = [(a, b)] the row ranges between them; None when there are no runs or the tile
-        kernel does not take the configuration."""
+        completion against 1224), rest = [(a, b)] the row ranges between them; None when there are no runs, when the tile
+        kernel does not take the configuration, or when it would not earn its launch beside the one for the rest (us, one launch /
+        two, 8 decoding sequences at 200 positions: H16 hd64 and a prompt of 16 8.2 / 9.6, 64 10.5 / 10.1, 128 17.5 / 11.8; H8 hd32,
+        128 7.6 / 8.8, 4 x 64 9.9 / 7.8; by itself H16 hd128, 16 3.4 / 5.1, 48 7.5 / 5.9)."""
         if (ntok < nseq + 15 or self.dev.type != "cuda" or self.dt != torch.bfloat16 or self.attn_splits > 1
                 or self.hd not in (32, 64, 128)):
             return None
@@ -266,7 +268,9 @@ class InferEngine:
                 at = b
         if at < ntok:
             rest.append((at, ntok))
-        return (runs, rest) if runs else None
+        items = sum(n for _, n in runs) * self.Hl
+        least = (1280 if self.hd == 32 else 1024) if rest else 600 if self.hd == 128 else 1
+        return (runs, rest) if items >= least else None
 
     def _one_kernel(self, ntok, nseq):
         """Whether this step runs in the persistent kernel.  Beyond 4096 positions its W warps per (sequence, head) lose to the

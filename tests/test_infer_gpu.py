@@ -486,3 +486,25 @@ def test_paged_attention_warps_per_item(hd, ntok, append):
         assert torch.equal(kc[b, p], qkv[i, d:2 * d].view(H, hd)) and torch.equal(vc[b, p], qkv[i, 2 * d:].view(H, hd))
     else:
         assert torch.equal(kc, k2) and torch.equal(vc, v2)
+
+
+@pytest.mark.parametrize("H,hd,decoding,lens,tiles", [(16, 64, 8, [16], False), (16, 64, 8, [63], False), (16, 64, 8, [64], True),
+                                                      (16, 64, 1, [9, 40, 24], True), (16, 64, 0, [16], True), (8, 32, 3, [128], False),
+                                                      (8, 32, 3, [160], True), (8, 32, 0, [15, 15], False), (4, 128, 0, [128], False),
+                                                      (4, 128, 0, [150], True), (4, 16, 0, [200], False)])
+def test_prompt_pieces_take_the_tile_kernel_where_it_earns_its_launch(H, hd, decoding, lens, tiles):
+    """The row ranges that a step hands to the tile kernel and to the kernel for single tokens cover every row once, and the step's
+    attention is the same either way."""
+    cfg = Config(1, H * hd, H, 300, 512, 1)
+    m = GPT(cfg, "cuda", torch.bfloat16); m.init_weights_device(5)
+    e = InferEngine(m, block_size=16, max_seqs=20, max_tokens=1024, use_graphs=False, flash_prefill=False)
+    pos = [200 + i for i in range(decoding)] + [p for n in lens for p in range(n)]
+    slot = list(range(decoding)) + [decoding + i for i, n in enumerate(lens) for _ in range(n)]
+    e.np_meta[e._o_pos:e._o_pos + len(pos)] = pos
+    e.np_meta[e._o_slot:e._o_slot + len(slot)] = slot
+    got = e._prompt_runs(len(pos), decoding + len(lens))
+    assert (got is not None) == tiles
+    if tiles:
+        runs, rest = got
+        rows = sorted([i for r, n in runs for i in range(r, r + n)] + [i for a, b in rest for i in range(a, b)])
+        assert rows == list(range(len(pos))) and all(n >= 16 for _, n in runs)
