@@ -736,8 +736,9 @@ __global__ void __launch_bounds__(32 << lg_warps<MT>(), 1) decode_layers_k(const
   };
   const int n_half = 2 * p.L;
   // Weights go into L2 ahead of their phase: the copies into shared memory then take an L2 trip, and the memory streams during
-  // attention and hand-offs too.  `far`: two phases ahead, for layers of up to 40 MB (d1024: 489 -> 470 us a step at G = 1); larger
-  // ones one phase ahead (d2048, 100 MB a layer: 1182 us against 1248).
+  // attention and hand-offs too.  `far`: two phases ahead, for layers of up to 40 MB (L24 d1024: 489 -> 470 us a step at G = 1); larger
+  // ones one phase ahead (L12, G = 1 / 8, one against two phases: d1280 359 / 452 and 360 / 446, d1536 390 / 502 and 397 / 518,
+  // d2048 522 / 618 and 551 / 660).
   const bool far = d <= 1280;
   auto prefetch_next = [&](bool last, const LayerW* nw) {
     if (!last) {
@@ -801,10 +802,11 @@ __global__ void __launch_bounds__(32 << lg_warps<MT>(), 1) decode_layers_k(const
   }
 }
 
-int smem_bytes(int MT, int d) {
+constexpr int smem_bytes(int MT, int d) {
   const int warps = MT == 1 ? 1 << lg_warps<1>() : 1 << lg_warps<2>();
   return (MT == 1 ? 2 : 1) * (int)WBUF + 8 * MT * (d + PAD) * 2 + 4 * d + (MT == 4 ? 1 : 2) * warps * 8 * MT * 16 * 4 + warps * ATT_PITCH * 4 + (int)sizeof(Shared);
 }
+static_assert(smem_bytes(1, 4096) <= SMEM_LIMIT, "eight rows of every accepted width fit");
 int max_mt(int d) {             // row groups of eight whose normalised rows fit into shared memory
   for (int mt = 4; mt > 1; mt >>= 1)
     if (smem_bytes(mt, d) <= SMEM_LIMIT) return mt;
@@ -845,7 +847,7 @@ int launch(DecodeParams& p, int grid, cudaStream_t st) {
 }
 template <int HD>
 int launch_rows(DecodeParams& p, int rows, int grid, cudaStream_t st) {
-  if (rows <= 8 && smem_bytes(1, p.d) <= SMEM_LIMIT) return launch<1, HD>(p, grid, st);      // (d = 4096 has no room for two sets of slots)
+  if (rows <= 8) return launch<1, HD>(p, grid, st);
   if (rows <= 16) return launch<2, HD>(p, grid, st);
   return launch<4, HD>(p, grid, st);
 }

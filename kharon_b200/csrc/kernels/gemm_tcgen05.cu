@@ -12,8 +12,8 @@
 // Structure: persistent CTAs (one per SM), 6 or 10 warps.  Warp 0 streams operand tiles with TMA
 // into a ring of 128-byte-swizzled shared-memory stages; one lane of warp 1 issues
 // tcgen05.mma (128 x BN x 16 per instruction) into one of two TMEM accumulator buffers and
-// commits stage-release / accumulator-ready mbarriers; warps 2-9 drain the other
-// accumulator with tcgen05.ld and run the fused epilogue, so the epilogue of tile i
+// commits stage-release / accumulator-ready mbarriers; warps 2-9 (2-5 beyond K = 1024 and with
+// column sums) drain the other accumulator with tcgen05.ld and run the fused epilogue, so the epilogue of tile i
 // overlaps the main loop of tile i+1.
 //
 // Fused epilogues replace the reference's separate elementwise kernels
@@ -1019,7 +1019,8 @@ extern "C" int kh_gemm_bf16_colsum(const void* A, int lda, int a_mn, const void*
     // 256 x 256 tiles on CTA pairs: a wave of pairs takes about 0.93 of a wave of single tiles
     // (measured 6-19 % faster on large shapes), so prefer it unless wave quantisation eats the gain.  A pair also pays about
     // 1 us for its cluster, which short main loops do not earn back: single tiles in up to four waves at K = 512
-    // (9216 x 1536 16.5 us against 18.3; 8192 x 50257 in 86 waves 450 against 416), and up to K = 4096 where one wave does (4200 x 1024 x 1024 12.8 against 13.8; 2048 x 2048 x 8192 56.3 against 51.5)
+    // (9216 x 1536 16.5 us against 18.3; 8192 x 50257 in 86 waves 450 against 416), and up to K = 4096 where one wave does
+    // (4200 x 1024, single tiles / pairs: K = 1024 11.0 / 11.9, 2048 17.2 / 17.9, 4096 26.9 / 27.5, 6144 40.9 / 38.1)
     if (bn == 256 && M >= 512 && g_pair_clusters != 0 && (waves(256) > (K <= 512 ? 4 : 1) || K > 4096)) {
       const int clusters = g_pair_clusters > 0 ? g_pair_clusters : sms / 2;
       const int tiles2 = ((M + 255) / 256) * ((N + 255) / 256);

@@ -168,7 +168,7 @@ class InferEngine:
         xs = x[:ntok]
         ops.embed_fwd(tok, pos, P["wte"], P["wpe"], xs, cfg.seq)
         if self._fused:       # layers and head in one kernel; only the sampler follows
-            ops.decode_layers(xs, self.xmid[:ntok], self.qkv[:ntok], self.att[:ntok], self.act[:ntok], self.layer_table,
+            ops.decode_layers(xs, None, None, None, None, self.layer_table,
                               cfg.n_layer, self.Hl, self.hd, self.kc, self.vc, pos, slot, self.d_btab, self.bs, cfg.seq,
                               work=self.decode_work, head_w=m.head_weight(), lnf_w=P["lnf_w"], lnf_b=P["lnf_b"], logits=self.logits,
                               vocab=cfg.vocab, rows=self.d_rows, n_rows=nseq)
