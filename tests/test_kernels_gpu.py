@@ -140,6 +140,51 @@ def test_gemm_split_over_a_cluster(M, N, K, split, bn):
     assert ops.error_word() == 0
 
 
+@pytest.mark.parametrize("M,N,K,blk", [(200, 72, 1000, 4096 * 2 + 64), (513, 257, 1496, 4096 * 4 + 128), (130, 136, 4104, 4096 * 8 + 64),
+                                       (200, 328, 1032, 256), (520, 264, 2048, 512), (200, 72, 1032, 64)])
+def test_gemm_gelu_stores_the_pre_activation(M, N, K, blk):
+    """The second output of the GELU epilogue (read by the backward pass) from split, wide and paired tiles, whole and ragged columns:
+    the bf16 of acc + bias, nothing outside the M x N block, and the output is the GELU of exactly that bf16 value."""
+    torch.manual_seed(M + K)
+    pad = (N + 7) // 8 * 8 + 8
+    a, w = _rand(M, K, scale=0.3), _rand(N, K, scale=0.1)
+    bias = _rand(pad)[:N]
+    out, aux = torch.full((M + 3, pad), 7.0, device=DEV).bfloat16(), torch.full((M + 3, pad), 5.0, device=DEV).bfloat16()
+    ops.gemm(a, w, out[:M, :N], epi=ops.EPI_BIAS_GELU, bias=bias, aux=aux[:M, :N], block_n=blk)
+    pre = (a.double() @ w.double().t() + bias.double())
+    assert ((aux[:M, :N].double() - pre).abs() <= 2.0 ** -8 * pre.abs() + 1e-4).all()       # one rounding; fp32 sums of K products
+    x = aux[:M, :N].float()
+    want = 0.5 * x * (1 + torch.tanh(0.7978845608 * (x + 0.044715 * x ** 3)))
+    assert ((out[:M, :N].float() - want).abs() <= 2.0 ** -8 * want.abs() + 2e-3).all()      # and the kernel's approximate tanh
+    for t, v in ((out, 7.0), (aux, 5.0)):
+        assert (t[M:] == v).all() and (t[:M, N:] == v).all()
+    assert ops.error_word() == 0
+
+
+@pytest.mark.parametrize("M,N,bn", [(7680, 2048, 256), (7700, 2000, 512)])
+@pytest.mark.parametrize("K", [1032, 2048])
+def test_gemm_long_k_tiles(M, N, K, bn):
+    """K beyond 1024 without column sums: four epilogue warps with all columns of a tile (single tiles and CTA pairs), at least three
+    tiles a worker so that both accumulator buffers come round, every epilogue of the training step and fp32 accumulation."""
+    torch.manual_seed(K)
+    a, w, bias = _rand(M, K, scale=0.3), _rand(N, K, scale=0.1), _rand(N)
+    aux = _rand(M, N)
+    acc = a.float() @ w.float().t()
+    out = torch.empty(M, N, device=DEV, dtype=torch.bfloat16)
+    for epi in (ops.EPI_NONE, ops.EPI_BIAS, ops.EPI_BIAS_GELU, ops.EPI_BIAS_RESID, ops.EPI_DGELU, ops.EPI_RESID):
+        ax, ax_ref = aux.clone(), aux.clone()
+        want = torch.empty_like(out)
+        ops.gemm(a, w, out, epi=epi, bias=bias, aux=ax, block_n=bn)
+        ref.gemm(a, w, want, False, False, False, epi, bias, ax_ref, 1.0)
+        assert relerr(out, want) < 8e-3, epi
+        assert relerr(ax, ax_ref) < 8e-3, epi
+    base = torch.randn(M, N, device=DEV)
+    c = base.clone()
+    ops.gemm(a, w, c, accumulate=True, alpha=0.5, block_n=bn)
+    assert relerr(c - base, 0.5 * acc) < 1e-4          # fp32 sums of K products and one addition to values of size one
+    assert ops.error_word() == 0
+
+
 @pytest.mark.parametrize("ta,tb", [(False, False), (True, False), (False, True), (True, True)])
 def test_gemm_f32_oracle_kernel(ta, tb):
     torch.manual_seed(13)
@@ -347,6 +392,13 @@ def test_flash_fwd_bwd(B, T, H, hd):
 def test_flash_short_sequences_of_many_items(B, T, H, hd):
     """Up to 128 positions at head width 128, on both sides of the item counts at which the kernel for short sequences hands over
     to the 128-row tiles, forward and backward independently, and the kernels for one tile per item come in."""
+    test_flash_fwd_bwd(B, T, H, hd)
+
+
+@pytest.mark.parametrize("B,T,H,hd", [(32, 256, 8, 64), (40, 130, 8, 64), (3, 1777, 4, 64), (75, 72, 2, 64), (74, 72, 2, 64)])
+def test_flash_backward_with_two_ctas_per_sm(B, T, H, hd):
+    """Head width 64 with more (batch, head, tile) items than SMs: two CTAs share an SM, with one S / dP buffer and a two-stage ring
+    each.  Up to several items a CTA (the barrier phases carry over), ragged lengths; the last shape is one item below the line."""
     test_flash_fwd_bwd(B, T, H, hd)
 
 
