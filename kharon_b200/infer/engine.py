@@ -248,9 +248,10 @@ class InferEngine:
         """(runs, rest) of a step that lists several tokens of a sequence: runs = [(first row, length)] of at least sixteen
         consecutive positions of one sequence (shorter ones are faster a warp per token: nine-token prompts 1177 us a
         completion against 1224), rest = [(a, b)] the row ranges between them; None when there are no runs, when the tile
-        kernel does not take the configuration, or when it would not earn its launch beside the one for the rest (us, one launch /
-        two, 8 decoding sequences at 200 positions: H16 hd64 and a prompt of 16 8.2 / 9.6, 64 10.5 / 10.1, 128 17.5 / 11.8; H8 hd32,
-        128 7.6 / 8.8, 4 x 64 9.9 / 7.8; by itself H16 hd128, 16 3.4 / 5.1, 48 7.5 / 5.9)."""
+        kernel does not take the configuration, or when it would not earn its launch: beside the one for the rest while the
+        step's (token, head) items are few (us, one launch / two, decoding sequences at 200 positions + prompt: H16 hd64, 8 + 16
+        8.2 / 9.6, 8 + 48 10.1 / 9.9, 8 + 128 17.5 / 11.8, 31 + 24 12.4 / 12.3; H16 hd128, 31 + 32 18.3 / 19.5, 31 + 48 21.5 / 19.9;
+        H8 hd32, 31 + 128 8.5 / 9.2, 31 + 4 x 64 10.7 / 8.2), and at head width 128 by itself (H16, 16 3.4 / 5.1, 48 7.5 / 5.9)."""
         if (ntok < nseq + 15 or self.dev.type != "cuda" or self.dt != torch.bfloat16 or self.attn_splits > 1
                 or self.hd not in (32, 64, 128)):
             return None
@@ -268,9 +269,8 @@ class InferEngine:
                 at = b
         if at < ntok:
             rest.append((at, ntok))
-        items = sum(n for _, n in runs) * self.Hl
-        least = (1280 if self.hd == 32 else 1024) if rest else 600 if self.hd == 128 else 1
-        return (runs, rest) if items >= least else None
+        least = {32: 1280, 64: 896, 128: 1100}[self.hd] if rest else 600 if self.hd == 128 else 1
+        return (runs, rest) if runs and ntok * self.Hl >= least else None
 
     def _one_kernel(self, ntok, nseq):
         """Whether this step runs in the persistent kernel.  Beyond 4096 positions its W warps per (sequence, head) lose to the

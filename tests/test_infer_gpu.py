@@ -488,7 +488,8 @@ def test_paged_attention_warps_per_item(hd, ntok, append):
         assert torch.equal(kc, k2) and torch.equal(vc, v2)
 
 
-@pytest.mark.parametrize("H,hd,decoding,lens,tiles", [(16, 64, 8, [16], False), (16, 64, 8, [63], False), (16, 64, 8, [64], True),
+@pytest.mark.parametrize("H,hd,decoding,lens,tiles", [(16, 64, 8, [16], False), (16, 64, 8, [47], False), (16, 64, 8, [48], True),
+                                                      (16, 128, 8, [60], False), (16, 128, 8, [61], True),
                                                       (16, 64, 1, [9, 40, 24], True), (16, 64, 0, [16], True), (8, 32, 3, [128], False),
                                                       (8, 32, 3, [160], True), (8, 32, 0, [15, 15], False), (4, 128, 0, [128], False),
                                                       (4, 128, 0, [150], True), (4, 16, 0, [200], False)])
