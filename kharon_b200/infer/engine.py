@@ -230,8 +230,10 @@ class InferEngine:
             self.model._row_parallel(x, w, out, bias, resid)
 
     def _fresh_prompts(self, ntok, nseq):
-        """[(first row, length)] when every token of the step belongs to a prompt that starts at position 0 and is
-        listed whole and contiguously; None otherwise (read from the host copy of the step's metadata)."""
+        """[(first row, length)] when every token of the step belongs to a prompt of at least 64 tokens that starts at position
+        0 and is listed whole and contiguously; None otherwise (read from the host copy of the step's metadata).  A batch with
+        a shorter prompt keeps the fp32 probabilities of the paged kernels: short prompts gain nothing from the 128-row tiles
+        (16 heads of 64, 64 tokens: 3.9 us in the tile kernel, 4.4 here), longer ones beside them would (6 x 1000: 131 and 38)."""
         if not self.flash_prefill or ntok == nseq:
             return None
         pos = self.h_meta[self._o_pos:self._o_pos + ntok]
@@ -239,7 +241,7 @@ class InferEngine:
         cuts = [0] + (torch.nonzero(slot[1:] != slot[:-1]).flatten() + 1).tolist() + [ntok]
         out = []
         for a, b in zip(cuts[:-1], cuts[1:]):
-            if int(pos[a]) != 0 or int(pos[b - 1]) != b - a - 1 or b - a < 64:     # (short prompts: not worth a launch each)
+            if int(pos[a]) != 0 or int(pos[b - 1]) != b - a - 1 or b - a < 64:
                 return None
             out.append((a, b - a))
         return out if len(out) == nseq else None
