@@ -263,6 +263,7 @@ int check(const void* p, long ld, const char* what) {
 }
 template <typename K>
 int opt_in(K kernel, int bytes) {
+  if (bytes <= 48 * 1024) return 0;
   if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess) return 0;
   kh_set_error("flash: cannot opt in to %d bytes of shared memory", bytes);
   return -1;

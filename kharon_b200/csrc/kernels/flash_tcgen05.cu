@@ -979,7 +979,7 @@ int launch_fwd_varlen(const bf16* qkv, AttnParams p, const int* row0, const int*
       most = q > most ? q : most;
       n++;
     }
-    if (n == 0) {                      // longer than the list: by itself
+    if (n == 0 || (n == 1 && s0 + 1 == n_seg)) {      // longer than the list, or one alone: by itself, without the sixteen sets of maps
       p.B = 1; p.T = len[s0]; p.out = out + (size_t)row0[s0] * p.H * HD;
       if (launch_fwd<HD>(qkv + (size_t)row0[s0] * p.ld, p, st)) return -1;
       s0++;

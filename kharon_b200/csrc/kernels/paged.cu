@@ -473,7 +473,8 @@ extern "C" int kh_paged_prefill(const void* qkv, int ld, const void* kc, const v
     if (nt == 0) return 0;
 #define LAUNCH(HD)                                                                                                              \
   {                                                                                                                             \
-    if (cudaFuncSetAttribute(paged_prefill_k<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) {           \
+    if (smem > 48 * 1024 &&                                                                                                     \
+        cudaFuncSetAttribute(paged_prefill_k<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) {           \
       kh_set_error("paged_prefill: shared memory opt-in failed");                                                               \
       return -1;                                                                                                                \
     }                                                                                                                           \

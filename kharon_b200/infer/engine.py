@@ -175,20 +175,21 @@ class InferEngine:
             ops.sample(self.logits, cfg.vocab, self.temperature, self.seed, self.step_no, rep, self.d_out, nseq,
                        step_dev=self.d_stepno)
             return
+        ln, qkv, att, xmid = self.ln[:ntok], self.qkv[:ntok], self.att[:ntok], self.xmid[:ntok]
+        decode = ntok == nseq            # one new token per sequence: the attention kernel appends k, v itself
+        if self._runs:
+            runs = self._runs[0]
+            rest = [(qkv[a:b], att[a:b], pos[a:b], slot[a:b]) for a, b in self._runs[1]]
         for l in range(cfg.n_layer):
-            ln, qkv, att, xmid = self.ln[:ntok], self.qkv[:ntok], self.att[:ntok], self.xmid[:ntok]
             self._ln_lin(xs, m.L(l, "ln1_w"), m.L(l, "ln1_b"), ln, m.L(l, "qkv_w"), qkv, ops.EPI_BIAS, m.L(l, "qkv_b"))
-            decode = ntok == nseq        # one new token per sequence: the attention kernel appends k, v itself
             if not decode:
                 ops.append_kv(qkv, self.kc[l], self.vc[l], pos, slot, self.d_btab, self.bs, self.Hl, self.hd, ntok)
             if not decode and self._fresh:
                 ops.flash_fwd_varlen(qkv, att, self._fresh, self.Hl, self.hd)
             elif not decode and self._runs:
-                runs, rest = self._runs
                 ops.paged_prefill(qkv, self.kc[l], self.vc[l], att, pos, slot, self.d_btab, self.bs, self.Hl, self.hd, runs, cfg.seq)
-                for a, b in rest:
-                    ops.paged_attn(qkv[a:b], self.kc[l], self.vc[l], att[a:b], pos[a:b], slot[a:b], self.d_btab, self.bs, self.Hl,
-                                   self.hd, b - a, cfg.seq)
+                for q, o, p, s in rest:
+                    ops.paged_attn(q, self.kc[l], self.vc[l], o, p, s, self.d_btab, self.bs, self.Hl, self.hd, q.shape[0], cfg.seq)
             else:
                 ops.paged_attn(qkv, self.kc[l], self.vc[l], att, pos, slot, self.d_btab, self.bs, self.Hl, self.hd, ntok,
                                cfg.seq, append=decode, n_split=self.attn_splits, scratch=self.attn_scratch)

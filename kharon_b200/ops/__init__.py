@@ -8,6 +8,7 @@ numerical oracle of the GPU tests and what the CPU test tier exercises.
 """
 from __future__ import annotations
 
+import ctypes as C
 import math
 
 import torch
@@ -451,6 +452,16 @@ def _pad_out(src, dst, parts, H, hd, hp):
     dst[:, :parts * H * hd].copy_(src.view(R, parts, H, hp)[:, :, :, :hd].reshape(R, parts * H * hd))
 
 
+def _row_lists(runs, limit):
+    """``[(first row, length), ...]`` as two host int32 arrays for a native call; every run lies within ``limit`` rows."""
+    k = len(runs)
+    rows, lens = (C.c_int32 * k)(), (C.c_int32 * k)()
+    for i, (r, n) in enumerate(runs):
+        assert 0 <= r and r + n <= limit
+        rows[i], lens[i] = r, n
+    return rows, lens
+
+
 def flash_fwd_varlen(qkv, out, segs, H, hd):
     """``flash_fwd`` of several sequences of their own lengths, ``segs = [(first row, length), ...]``, in one launch (per
     sixteen); no log-sum-exps.  Head widths 64 and 128."""
@@ -458,11 +469,9 @@ def flash_fwd_varlen(qkv, out, segs, H, hd):
         for r, n in segs:
             ref.flash_fwd(qkv[r:r + n], out[r:r + n], None, 1, n, H, hd)
         return
-    rows = torch.tensor([r for r, _ in segs] + [n for _, n in segs], dtype=torch.int32)
-    k = len(segs)
-    assert all(0 <= r and r + n <= qkv.shape[0] for r, n in segs)
-    _call(_lib().kh_flash_fwd_varlen, 1, qkv.data_ptr(), out.data_ptr(), rows.data_ptr(), rows.data_ptr() + 4 * k, k, H, hd,
-          qkv.stride(0), 1.0 / math.sqrt(hd), _stream(), keep=rows)
+    rows, lens = _row_lists(segs, qkv.shape[0])
+    _call(_lib().kh_flash_fwd_varlen, 1, qkv.data_ptr(), out.data_ptr(), C.addressof(rows), C.addressof(lens), len(segs), H, hd,
+          qkv.stride(0), 1.0 / math.sqrt(hd), _stream(), keep=(rows, lens))
 
 
 def flash_fwd(qkv, out, lse, B, T, H, hd):
@@ -574,12 +583,10 @@ def paged_prefill(qkv, kc, vc, out, pos, slot, btab, bs, H, hd, runs, max_ctx):
         for r, n in runs:
             ref.paged_attn(qkv[r:r + n], kc, vc, out[r:r + n], pos[r:r + n], slot[r:r + n], btab, bs, H, hd, n)
         return
-    k = len(runs)
-    rows = torch.tensor([r for r, _ in runs] + [n for _, n in runs], dtype=torch.int32)
-    assert all(0 <= r and r + n <= qkv.shape[0] for r, n in runs)
+    rows, lens = _row_lists(runs, qkv.shape[0])
     _call(_lib().kh_paged_prefill, 1, qkv.data_ptr(), qkv.stride(0), kc.data_ptr(), vc.data_ptr(), out.data_ptr(), pos.data_ptr(),
-          slot.data_ptr(), btab.data_ptr(), btab.stride(0), bs, H, hd, 1.0 / math.sqrt(hd), max_ctx, rows.data_ptr(),
-          rows.data_ptr() + 4 * k, k, _stream(), keep=rows)
+          slot.data_ptr(), btab.data_ptr(), btab.stride(0), bs, H, hd, 1.0 / math.sqrt(hd), max_ctx, C.addressof(rows),
+          C.addressof(lens), len(runs), _stream(), keep=(rows, lens))
 
 
 def gather_rows(x, rows, out, nseq):
