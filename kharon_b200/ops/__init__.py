@@ -45,9 +45,15 @@ def _chk(rc, n=1):
     launch_count += n
 
 
-def _call(fn, n, *args, keep=None):
-    """Invoke a native entry point; remember the exact call when a plan is being recorded.  ``keep``: objects made for this call
-    alone whose memory it points to; a recorded call holds them for its replays."""
+def _call(fn, n, *args):
+    """Invoke a native entry point; remember the exact call when a plan is being recorded."""
+    if _recording is not None:
+        _recording.append((fn, args, n, None))
+    _chk(fn(*args), n)
+
+
+def _call_keeping(keep, fn, n, *args):
+    """``_call`` with objects made for this call alone whose memory it points to; a recorded call holds them for its replays."""
     if _recording is not None:
         _recording.append((fn, args, n, keep))
     _chk(fn(*args), n)
@@ -223,10 +229,10 @@ def decode_layers(x, xmid, qkv, att, act, layers, n_layer, H, hd, kc, vc, pos, s
     elif (work.device != x.device or not work.is_contiguous()
           or work.numel() * work.element_size() < int(_lib().kh_decode_layers_work_bytes(d))):
         raise ValueError("decode_layers: the workspace must be contiguous, on %s and made for width %d" % (x.device, d))
-    _call(_lib().kh_decode_layers, 1, x.data_ptr(), layers.data_ptr(), n_layer, G, d, H, hd, kc.data_ptr(), vc.data_ptr(),
+    _call_keeping(work, _lib().kh_decode_layers, 1, x.data_ptr(), layers.data_ptr(), n_layer, G, d, H, hd, kc.data_ptr(), vc.data_ptr(),
           kc.stride(0), pos.data_ptr(), slot.data_ptr(), btab.data_ptr(), btab.shape[1], bs, max_ctx, 1.0 / float(hd) ** 0.5,
           _p(head_w), _p(lnf_w), _p(lnf_b), _p(logits), logits.stride(0) if logits is not None else 0, vocab,
-          _p(rows), n_rows, work.data_ptr(), _stream(), keep=work)
+          _p(rows), n_rows, work.data_ptr(), _stream())
 
 
 def gemm_skinny_scratch_elems(M, N, K):
@@ -470,8 +476,8 @@ def flash_fwd_varlen(qkv, out, segs, H, hd):
             ref.flash_fwd(qkv[r:r + n], out[r:r + n], None, 1, n, H, hd)
         return
     rows, lens = _row_lists(segs, qkv.shape[0])
-    _call(_lib().kh_flash_fwd_varlen, 1, qkv.data_ptr(), out.data_ptr(), C.addressof(rows), C.addressof(lens), len(segs), H, hd,
-          qkv.stride(0), 1.0 / math.sqrt(hd), _stream(), keep=(rows, lens))
+    _call_keeping((rows, lens), _lib().kh_flash_fwd_varlen, 1, qkv.data_ptr(), out.data_ptr(), C.addressof(rows),
+                  C.addressof(lens), len(segs), H, hd, qkv.stride(0), 1.0 / math.sqrt(hd), _stream())
 
 
 def flash_fwd(qkv, out, lse, B, T, H, hd):
@@ -584,9 +590,9 @@ def paged_prefill(qkv, kc, vc, out, pos, slot, btab, bs, H, hd, runs, max_ctx):
             ref.paged_attn(qkv[r:r + n], kc, vc, out[r:r + n], pos[r:r + n], slot[r:r + n], btab, bs, H, hd, n)
         return
     rows, lens = _row_lists(runs, qkv.shape[0])
-    _call(_lib().kh_paged_prefill, 1, qkv.data_ptr(), qkv.stride(0), kc.data_ptr(), vc.data_ptr(), out.data_ptr(), pos.data_ptr(),
-          slot.data_ptr(), btab.data_ptr(), btab.stride(0), bs, H, hd, 1.0 / math.sqrt(hd), max_ctx, C.addressof(rows),
-          C.addressof(lens), len(runs), _stream(), keep=(rows, lens))
+    _call_keeping((rows, lens), _lib().kh_paged_prefill, 1, qkv.data_ptr(), qkv.stride(0), kc.data_ptr(), vc.data_ptr(),
+                  out.data_ptr(), pos.data_ptr(), slot.data_ptr(), btab.data_ptr(), btab.stride(0), bs, H, hd, 1.0 / math.sqrt(hd),
+                  max_ctx, C.addressof(rows), C.addressof(lens), len(runs), _stream())
 
 
 def gather_rows(x, rows, out, nseq):
