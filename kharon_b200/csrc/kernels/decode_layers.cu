@@ -13,68 +13,74 @@
 //   phase E                         x    = act Wfcproj^T + b + xmid             (N = d,  K = 4d)
 //   head     xs = LNf(x[rows])      logits = xs Whead^T                         (N = V,  K = d)
 //
-// Links.  What bounds the step is the trip from the CTAs that write an activation to those that read
-// it.  There is no grid barrier: an activation travels as 8-byte packets {two bf16 columns, epoch},
-// written with one 64-bit store and polled by its readers until the epoch of this launch and layer
-// shows (a 64-bit access is single-copy atomic, so a packet with the right epoch holds the right
-// data).  One trip through L2 replaces the release fence, the arrival atomic, the polled counter and
-// the fetch of a barrier; a CTA without work in a phase does not take part in it.  Packets double the
-// bytes of an activation, which are a few KB per row.  A buffer is overwritten one layer later; by then every
-// reader is done, because each phase's output depends on all rows and columns of the one before it.
-// Measured, L24 d1024 with the head, context 160, a captured step with embedding and sampler: 468 us for one
-// sequence and 520 for eight (grid barriers and weights held in registers: 1000 and 1090; the weights alone
-// take 106 us at the copy bandwidth).
+// Links.  What bounds the step is the trip from the CTAs that write an activation to those that read it (about 850 cycles
+// from store to successful poll) and the instructions between two trips.  There is no grid barrier: activations are 32-bit words
+// of two bf16 columns in a workspace whose empty words are zero, and a reader polls the words that it needs until none of
+// them is zero (a result of two +0.0 is written as {-0.0, +0.0}).  A word is a single-copy atomic unit, so a word that is not zero
+// is the result; there are no flags, no extra bytes and no fences on the way.  The words are laid out so that a 128-byte line has
+// one writer (word_at).  Every activation has three slots that the
+// layers use in turn: when a CTA is done with a phase of layer l - 1, a helper warp empties the words that it will write in
+// that phase of layer l + 1 (last used at l - 2; whoever has seen all inputs of the phase at l - 1 knows that their readers are
+// done, since every output of a phase depends on all outputs of the one before), and its fence precedes the CTA's outputs of
+// layer l, so the words are empty before anybody can come to poll them.
+// Launches alternate between two halves of the workspace and empty the other half for the next launch, which also
+// repairs what a launch that gave up has left.
 //
-// Linear phases.  A work unit is 16 output columns (8 in phases C and E, whose N is only d); S warps share
-// a unit, each multiplying its K / S slice, and a CTA of 16 (8) warps works on 16 / S (8 / S) units at a time.  S is
-// the smallest split whose slice fits a sub-step, and larger where that spreads a narrow product over more
-// CTAs in the same number of turns.  Every lane copies the eight (sixteen) 16-byte pieces of weights that it will use
-// into its own slots of shared memory with cp.async (no registers are held and no thread waits for another's
-// copy); the first turn's weights of a phase are requested before its activations are polled, the next turn's
-// are requested under the products of this one (a second set of slots for up to eight rows, else as a slot has been read), and the units of later phases are prefetched
-// into L2 in bulk.  The products are mma.sync m16n8k16 with the weights as the 16-row operand and eight sequences
-// as the columns: tcgen05's 128-row tiles, TMEM round trip and operand staging are the latency this kernel
-// exists to avoid (the large-M GEMMs of training and prefill use them).  The K order inside a 32-wide block
-// is permuted identically for both operands so that every lane fetches 16 contiguous bytes.  Phases behind a
-// LayerNorm read the normalised rows from shared memory (pitch padded by 64 bytes, conflict-free); the others read their operand fragments straight from the packets.  Partial sums of the S
-// warps meet in shared memory and are added in warp order.
+// Weights.  Rows of a weight matrix come in groups of eight; a CTA owns a contiguous share of the groups of every product.  A
+// producer warp streams them in the order of use, chunks of eight rows x 1024 columns, with bulk copies through a ring
+// that fills the shared memory (12 chunks at d = 1024: about a layer ahead), so neither HBM latency nor copy instructions
+// are in the chain (cp.async by the computing warps cost them 900-1500 cycles a phase, ahead of the first poll).
 //
-// Attention.  W warps share a (sequence, head) item; a key is read by HD / 8 lanes in 16-byte pieces and
-// the running softmax is kept per lane group and merged once.  The first four (eight) keys and values of
-// every group are requested before the queries are polled (cached positions do not depend on this step).
+// Products.  Eight warps split K: warp w takes columns 32 (8 s + w) ... + 31 for s = 0, 1, ..., and multiplies all rows of a chunk.
+// Each lane polls exactly the 16 bytes (row lane / 4, eight columns) that are its operand fragment of mma.sync m16n8k16: for
+// proj and fcproj an activation goes from L2 to the tensor cores through registers, in front of a LayerNorm it passes through
+// shared memory, where a warp normalises a row.  The K order inside a 32-wide step is permuted identically for both operands.  The
+// weight fragments of the first chunks are in registers before the input arrives.  Up to eight sequences: weights as the
+// 16-row operand (two groups), else sequences.  tcgen05's 128-row tiles, TMEM round trip and operand staging are the latency
+// that this kernel exists to avoid.  Partial sums of the warps meet in shared memory and are added in warp order.
 //
-// Every wait is bounded: status code 9 in the library error word, an abort word for the other CTAs.
-// Numerics follow the five-kernel path: bf16 activations between phases, fp32 accumulation, LayerNorm
-// statistics in two passes, GELU applied to the bf16-rounded pre-activation.
+// Attention.  W warps share a (sequence, head) item; the four lanes of a group hold the keys and values of a position in
+// 16-byte pieces that are operand fragments of the score product (mma.sync, the query as all eight columns); probabilities and
+// outputs stay fp32 on the CUDA cores, a running softmax per lane group merged once.  The first keys and values of every
+// group are requested before the query is polled (cached positions do not depend on this step), those of the next layer
+// are prefetched into L2.
+//
+// Every wait is bounded: status code 9 in the library error word.
+//
+// Measured (L24 d1024 V50257, a captured step with embedding and sampler, this form / epoch-tagged 8-byte packets, cp.async weights and rows
+// of activations before): context 160, G = 1 / 8 / 16 366 / 402 / 557 us (468 / 518 / 737), context 200, G = 32 926 (1206); L24 d2048 G = 4 935
+// (1143); L8 d4096 G = 8 1068 (1606); L4 d256 G = 1 51 (58).  Of the 28 000 cycles of a layer at G = 1, 1000 each are the trips, 2000 a
+// LayerNorm, 900 the products of qkv and fc, 1500 those of fcproj, 6000 the attention, 600 each the sums and epilogues.
+// Numerics follow the five-kernel path: bf16 activations between phases, fp32 accumulation, GELU applied to the bf16-rounded
+// pre-activation.
 #include "common.cuh"
 
 namespace {
 
-constexpr int MAX_WARPS = 16;
-constexpr int PAD = 32;                       // bf16 elements of padding per activation row (64 bytes)
+// Eight computing warps, and a warpgroup of helpers: a producer of weights, a warp that empties activation words, two that empty the
+// other half of the workspace.  With setmaxnreg the computing warps get the registers that the helpers do not need (256 x 232 + 128 x 40
+// = 384 x 168).
+constexpr int NW = 8, CT = NW * 32, THREADS = CT + 128;
+constexpr int KC = 1024;                      // columns of a chunk: four 32-column steps of every warp
+constexpr int PITCH = KC * 2 + 64;            // bytes between its rows (conflict-free fragments)
+constexpr int SLOT = 8 * PITCH;
+constexpr int MAX_SLOTS = 13;
 constexpr int MAX_ROWS = 32;
 constexpr int ATT_PITCH = 128 + 4;            // floats per warp of the attention hand-off: 128 outputs, maximum, sum
 constexpr int SMEM_LIMIT = 227 * 1024;
+constexpr uint32_t POLL_LIMIT = 1u << 23;     // rounds of at least 290 cycles: 1.3 s and more
 
-// Warps of a CTA (2^LGW) and what follows: 16-byte weight slots per lane (one sub-step; 64 KB a CTA) and the bytes between them.
-// Eight warps for up to eight rows, where index arithmetic that every warp repeats weighs most (L24 d1024 G = 1 / 8: 489 / 538 us
-// against 507 / 565 with sixteen; d2048 G = 4: 1179 against 1248), sixteen beyond, where rows and keys are spread over more
-// warps (G = 16 / 32: 764 / 1217 against 781 / 1320).
-template <int LGW> struct Cfg {
-  static constexpr int WARPS = 1 << LGW, THREADS = 32 * WARPS, NLD = 128 / WARPS;
-  static constexpr uint32_t SLOT = THREADS * 16;
-  static constexpr bool DB = LGW == 3;        // two sets of slots: shared memory has room for them up to eight rows
-};
-#define CFG using C_ = Cfg<LGW>; constexpr int WARPS = C_::WARPS, THREADS = C_::THREADS, NLD = C_::NLD; constexpr uint32_t SLOT = C_::SLOT; (void)WARPS; (void)THREADS; (void)NLD; (void)SLOT
-
-constexpr uint32_t WBUF = 65536;              // bytes of a set of weight slots
-
-// Thread index, read anew in every phase: index arithmetic derived from it would otherwise be kept in registers (and
-// spilled) across the whole layer loop.
+// Thread index, read anew in every phase: index arithmetic derived from it would otherwise be kept in registers across the layer loop.
 __device__ __forceinline__ int tid_fresh() {
   int t;
   asm volatile("mov.u32 %0, %%tid.x;" : "=r"(t));
   return t;
+}
+
+// A value that the compiler must not carry (with all that follows from it) across the phases.
+__device__ __forceinline__ int fresh(int v) {
+  asm volatile("" : "+r"(v));
+  return v;
 }
 
 struct LayerW {               // bf16 pointers of one layer (device array, one entry per layer)
@@ -82,11 +88,12 @@ struct LayerW {               // bf16 pointers of one layer (device array, one e
 };
 
 struct DecodeParams {
-  int G, d, H, hd, L, bs, max_lb, max_ctx;
-  int lgs_a, lgs_c, lgs_d, lgs_e, lgs_h, lgw;    // log2 of the warps per unit of each product and per attention item
+  int G, d, H, L, bs, max_lb, max_ctx;
+  int lgw;                                // log2 of the warps per attention item
+  int slots;                              // chunks in the ring
   const LayerW* layers;
   bf16* x;                                // [G, d] in: embedded tokens, out: last layer's output
-  uint64_t *xp, *midp, *qkvp, *attp, *actp;   // packets: [32, d/2], [32, d/2], [32, 3d/2], [32, d/2], [32, 4d/2]
+  uint32_t* words;                        // activations: [2 halves][3 slots][x d/2 | mid d/2 | att d/2 | qkv 3d/2 | act 4d/2][32 rows]
   bf16 *kc, *vc;                          // [L, blocks, bs, H, hd]
   size_t layer_elems;
   const int *pos, *slot, *btab;
@@ -95,20 +102,25 @@ struct DecodeParams {
   bf16* logits;
   int ld_logits, V, n_rows;
   const int* rows;
-  uint32_t* ctl;                          // [0] epochs used by earlier launches, [1] abort, [2] CTAs that left
-  float scale;
+  uint32_t* ctl;                          // [0] launches so far, [2] CTAs that left, [3 + half] rows that the half was last used for, [16..] zeros
+  float scale, inv_d;
   uint64_t wait_ns;
   int* err;
+  uint32_t h_mul;                         // ceil(2^32 / H)
   uint32_t bs_mul;                        // ceil(2^32 / bs); 0 when one block holds every position
+  __device__ __forceinline__ int seq_of(int item) const { return H == 1 ? item : (int)__umulhi((uint32_t)item, h_mul); }     // item / H
   // j / bs by multiplication: exact for j < max_ctx, since max_ctx * bs stays below 2^32
   __device__ __forceinline__ int block_of(int j) const { return bs == 1 ? j : (int)__umulhi((uint32_t)j, bs_mul); }
 };
+constexpr int CTL_BYTES = 512;                // 64 bytes of counters, and zeros that stand in for cache rows that do not exist
 
 struct Shared {               // small control block behind the data regions
-  LayerW lw[4];               // records of this layer and the next two
-  int item_pos[MAX_WARPS], item_slot[MAX_WARPS];    // position and slot of each warp's first attention item (constant over the layers)
-  int item_row[MAX_WARPS][8][8];                // cache rows of its first keys, per lane group
+  uint64_t full[MAX_SLOTS], empty[MAX_SLOTS], ln_full[2], ln_empty[2];
+  int item_pos[NW], item_slot[NW], pos_row[NW];     // position, slot and cache row of each warp's first attention item (constant over the layers)
+  int share[4][2];                                  // this CTA's groups of eight weight rows of 3d, d, 4d and V rows
+  int item_row[NW][8][4];                           // cache rows of its first keys, per lane group
   volatile int abort_flag;
+  volatile int phase, cleared;                      // phases that the computing warps have entered / whose words of the next layer are empty
 };
 
 __device__ __forceinline__ uint4 ldg_stream(const void* p) {      // read-once data: do not keep it in L1
@@ -121,740 +133,969 @@ __device__ __forceinline__ uint4 lds128(uint32_t a) {
   asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a) : "memory");
   return v;
 }
+__device__ __forceinline__ void sts128(uint32_t a, uint4 v) {
+  asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(a), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+}
 __device__ __forceinline__ void mma_bf16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
   asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
                : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
-__device__ __forceinline__ float warp_sum(float v) {
+// rows 0..7 of the product from `a`, rows 8..15 from `b`, 32 permuted columns
+__device__ __forceinline__ void mma_rows(float (&c)[4], const uint4& a, const uint4& b, const uint4& x) {
+  mma_bf16(c, a.x, b.x, a.y, b.y, x.x, x.y);
+  mma_bf16(c, a.z, b.z, a.w, b.w, x.z, x.w);
+}
+__device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {     // 16-byte aligned, multiple of 16
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+               ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
+}
+__device__ __forceinline__ void compute_sync() { asm volatile("bar.sync 1, %0;" ::"n"(CT) : "memory"); }
+
+// ---- pairs of fp32 values in one instruction (same rounding as the scalar ones)
+typedef unsigned long long f2;
+__device__ __forceinline__ f2 mk2(float a, float b) {
+  f2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ float lo2(f2 v) { return __uint_as_float((uint32_t)v); }
+__device__ __forceinline__ float hi2(f2 v) { return __uint_as_float((uint32_t)(v >> 32)); }
+__device__ __forceinline__ f2 add2(f2 a, f2 b) { f2 r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+__device__ __forceinline__ f2 mul2(f2 a, f2 b) { f2 r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) { f2 r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c)); return r; }
+__device__ __forceinline__ f2 un2(uint32_t w) { return mk2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u)); }
+__device__ __forceinline__ void un8(f2* f, const uint4& v) { f[0] = un2(v.x); f[1] = un2(v.y); f[2] = un2(v.z); f[3] = un2(v.w); }
+__device__ __forceinline__ f2 sum8(const uint4& v) {
+  f2 f[4];
+  un8(f, v);
+  return add2(add2(f[0], f[1]), add2(f[2], f[3]));
+}
+__device__ __forceinline__ f2 dev8(const uint4& v, f2 nmean, f2 acc) {       // acc + squared deviations
+  f2 f[4];
+  un8(f, v);
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
+  for (int i = 0; i < 4; i++) { const f2 t = add2(f[i], nmean); acc = fma2(t, t, acc); }
+  return acc;
 }
-__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait_older() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }     // all but the last group
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
-__device__ __forceinline__ void l2_prefetch_bulk(const void* p, uint32_t bytes) {       // 16-byte aligned, multiple of 16
-  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
+__device__ __forceinline__ uint4 norm8(const uint4& v, const uint4& gw, const uint4& gb, f2 nmean, f2 rstd) {
+  auto n2 = [&](uint32_t x2, uint32_t w2, uint32_t b2) {
+    const f2 y = fma2(mul2(add2(un2(x2), nmean), rstd), un2(w2), un2(b2));
+    return pack_bf16(lo2(y), hi2(y));
+  };
+  return make_uint4(n2(v.x, gw.x, gb.x), n2(v.y, gw.y, gb.y), n2(v.z, gw.z, gb.z), n2(v.w, gw.w, gb.w));
 }
 
-// ---- packets
-__device__ __forceinline__ void ld_packets(uint64_t& a, uint64_t& b, const uint64_t* p) {     // two packets, 16-byte aligned
-  asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "l"(p) : "memory");
+// ---- bounded waits.  One that runs out sets the CTA's abort flag, which ends all others of the CTA at once; the CTAs that depend on
+// this one run out by themselves.  Kept short on purpose: what a layer executes has to fit into the instruction cache.
+__device__ __forceinline__ void wait_bar(uint32_t bar, uint32_t parity, Shared* sh, uint64_t limit_ns) {
+  if (mbar_try(bar, parity)) return;
+  const uint64_t t0 = kh_globaltimer();
+#pragma unroll 1
+  while (!mbar_try(bar, parity))
+    if (sh->abort_flag || kh_globaltimer() - t0 > limit_ns) { sh->abort_flag = 1; return; }
 }
-__device__ __forceinline__ uint64_t ld_packet(const uint64_t* p) {
-  uint64_t a;
-  asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(a) : "l"(p) : "memory");
+// after an unsuccessful round of a poll: true when the wait is over
+__device__ __forceinline__ bool expired(uint32_t& it, Shared* sh) {
+  if (++it > POLL_LIMIT) sh->abort_flag = 1;
+  return sh->abort_flag != 0;
+}
+
+// ---- activations
+__device__ __forceinline__ uint32_t ld_word(const uint32_t* p) {
+  uint32_t a;
+  asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(a) : "l"(p) : "memory");
   return a;
 }
-__device__ __forceinline__ void st_packet(uint64_t* p, uint32_t data, uint32_t epoch) {
-  asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(((uint64_t)epoch << 32) | data) : "memory");
+__device__ __forceinline__ void st_word(uint32_t* p, uint32_t v) { asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory"); }
+__device__ __forceinline__ uint32_t full_word(uint32_t v) { return v == 0u ? 0x80000000u : v; }
+__device__ __forceinline__ void ld_words(uint4& v, const uint32_t* p) {       // four words, 16-byte aligned
+  asm volatile("ld.relaxed.gpu.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
 }
-// After an unsuccessful poll: true when the wait is over (limit reached, or another thread or CTA gave up).  Inline on
-// purpose: a call would make the compiler keep the values in flight in local memory.
-__device__ __forceinline__ bool poll_expired(uint32_t& it, uint64_t& t0, Shared* sh, const DecodeParams& p) {
-  if ((++it & 127) != 0) return false;
-  if (sh->abort_flag) return true;
-  uint32_t a;
-  asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(a) : "l"(p.ctl + 1) : "memory");
-  const uint64_t now = kh_globaltimer();
-  if (t0 == 0) t0 = now;
-  if (a == 0 && now - t0 <= p.wait_ns) return false;
-  if (a == 0) {
-    atomicCAS(p.err, 0, 9);
-    atomicExch(p.ctl + 1, 1u);
-  }
-  sh->abort_flag = 1;
-  return true;
+__device__ __forceinline__ uint32_t least(const uint4& v) { return min(min(v.x, v.y), min(v.z, v.w)); }
+constexpr int STEP_BYTES = NW * 64;             // bytes of a row between a warp's steps
+constexpr int GROUP = 32;
+// Position of (row, column) in the words of an activation of width N: tiles of eight rows, in which the eight rows of eight columns are
+// one 128-byte line.  Such a group belongs to one CTA: a line with several writers that others poll takes 2 us to settle (L24 d1024, from
+// the last store of a residual to the first successful poll: 1.5-2.5 us in rows, 0.3-1.2 us in groups; a step of G = 8 511 us and 436).
+__device__ __forceinline__ uint32_t word_at(int N, int row, int col, int pitch = GROUP) {
+  return (row >> 3) * (4 * N) + (col >> 3) * pitch + (row & 7) * 4 + ((col & 7) >> 1);
 }
-// Reads N pairs of packets (pair i from addr(i), when use(i)) once all of them carry `epoch`; out[i] = four columns.
-template <int N, class Use, class Addr>
-__device__ __forceinline__ void read_pairs(uint2 (&out)[N], Use use, Addr addr, uint32_t epoch, const DecodeParams& p, Shared* sh) {
+// Words between the groups of fc's output: a CTA writes three or four neighbours of them, so that for few sequences two rows (G <= 2) or
+// four (G <= 4) are enough; every reader then touches a quarter or half of the lines.
+__device__ __forceinline__ int act_pitch(int G) { return G <= 2 ? 8 : G <= 4 ? 16 : GROUP; }
+// Where a lane's operand fragments lie: the words of its row and eight columns in step 0 of tile 0, and the distance of steps.
+struct Frags {
+  const uint32_t* at;
+  int step, tile;
+};
+// `group`: words between the groups, 0: rows [n, K] of an ordinary tensor or of the attention outputs (a head of a sequence is one CTA's)
+__device__ __forceinline__ Frags frags(const uint32_t* src, int group, int K, int row, int warp, int lane) {
+  Frags f;
+  const int pitch = group ? group : 4;
+  f.at = src + row * (group ? 4 : K / 2) + (warp * 4 + (lane & 3)) * pitch;
+  f.step = NW * 4 * pitch;
+  f.tile = 4 * K;
+  return f;
+}
+// A lane's fragments of four steps; of a partial last quad (`left` < 4) the last step that exists stands in for the others.
+__device__ __forceinline__ void ld_quad(uint4* v, int stride, const uint32_t* p, int step, int left) {
+  const uint32_t* p1 = p + (left > 1 ? step : 0);
+  const uint32_t* p2 = p1 + (left > 2 ? step : 0);
+  ld_words(v[0], p); ld_words(v[stride], p1); ld_words(v[2 * stride], p2); ld_words(v[3 * stride], p2 + (left > 3 ? step : 0));
+}
+// Until none of the words of a quad is empty (its loads have been issued).  Lanes of rows that do not exist read the last row that does, and
+// nothing is loaded conditionally: a register that one path leaves unset counts as live all the way back through the layer
+// loop, and the spills that follow cost an L2 trip each (shared memory leaves no L1; L24 d1024 G = 1 708 us a step with
+// them, 461 without).
+__device__ __forceinline__ void poll_quad(uint4* v, int stride, const uint32_t* p, int step, int left, Shared* sh) {
   uint32_t it = 0;
-  uint64_t t0 = 0;
 #pragma unroll 1
-  while (true) {
-    uint64_t a[N], b[N];
-    bool ok = true;
-#pragma unroll
-    for (int i = 0; i < N; i++) {
-      a[i] = b[i] = (uint64_t)epoch << 32;
-      if (use(i)) ld_packets(a[i], b[i], addr(i));
-    }
-#pragma unroll
-    for (int i = 0; i < N; i++) {
-      ok = ok && (uint32_t)(a[i] >> 32) == epoch && (uint32_t)(b[i] >> 32) == epoch;
-      out[i] = make_uint2((uint32_t)a[i], (uint32_t)b[i]);
-    }
-    if (ok || poll_expired(it, t0, sh, p)) return;
-  }
-}
-__device__ __forceinline__ uint32_t read_one(const uint64_t* q, uint32_t epoch, const DecodeParams& p, Shared* sh) {
-  uint32_t it = 0;
-  uint64_t t0 = 0;
-#pragma unroll 1
-  while (true) {
-    const uint64_t a = ld_packet(q);
-    if ((uint32_t)(a >> 32) == epoch || poll_expired(it, t0, sh, p)) return (uint32_t)a;
+  while (min(min(least(v[0]), least(v[stride])), min(least(v[2 * stride]), least(v[3 * stride]))) == 0u) {
+    if (expired(it, sh)) break;
+    ld_quad(v, stride, p, step, left);
   }
 }
 
-// One of the five products.
+// ---- the five products
 enum Phase { PA, PC, PD, PE, PH };
 struct Lin {
-  const bf16 *W, *bias;     // [N, K] row-major, [N] (null for the head)
-  int N, K, lgs;
-  int kind;                 // PA ... PH
-  const uint64_t* src;      // packets [32, K / 2] of the input, of epoch e_src (null: plain rows of p.x)
-  const uint64_t* res;      // C, E: packets [32, N / 2] of the residual, of epoch e_res (null: plain rows of p.x)
-  uint64_t* dst;            // packets [32, N / 2] of the output, epoch e_dst (null for the head)
-  uint32_t e_src, e_res, e_dst;
+  const bf16* bias;         // [N] (null for the head)
+  int N, K, kind, seq;      // kind PA ... PE, PH; seq: number of the phase
+  const uint32_t* src;      // words [32, K / 2] of the input (null: plain rows of p.x)
+  const uint32_t* res;      // C, E: words [32, N / 2] of the residual (null: plain rows of p.x)
+  uint32_t* dst;            // words [32, N / 2] of the output (null for the head)
 };
-// Row groups of eight columns per unit: two fill the 16 rows of an mma (A, D, head); C and E take one (the other half of the
-// operand is zero) so that twice as many CTAs have a unit.
-// Copies this lane's 16-byte pieces of weight rows 8 (RG u + i) + lane / 4 from column k0 on: slot RG * j + i holds row group
-// i of the j-th 32-column step.  Steps below `n` are copied; rows that do not exist are left alone.
-template <int LGW, int RG>
-__device__ __forceinline__ void copy_w(uint32_t slots, int lane, const Lin& L, int u, int k0, int j, int n) {
-  CFG;
-  if (j >= n) return;
-#pragma unroll
-  for (int i = 0; i < RG; i++) {
-    const int r = (u * RG + i) * 8 + (lane >> 2);
-    if (r < L.N) cp_async16(slots + (j * RG + i) * SLOT, L.W + (size_t)r * L.K + k0 + (lane & 3) * 8 + j * 32);
-  }
-}
-template <int LGW, int RG>
-__device__ __forceinline__ void copy_first(uint32_t wbuf, const Lin& L) {
-  CFG;
-  constexpr int KS = NLD / RG;
-  const int tid = tid_fresh(), warp = tid >> 5, U = WARPS >> L.lgs, kw = L.K >> L.lgs;
-#pragma unroll
-  for (int j = 0; j < KS; j++)
-    copy_w<LGW, RG>(wbuf + tid * 16, tid & 31, L, (int)blockIdx.x * U + (warp >> L.lgs), (warp & ((1 << L.lgs) - 1)) * kw, j, kw >> 5);
-  cp_async_commit();
-}
-// ask L2 for the weights of this CTA's units (the first `turns` turns of them); one thread of the last warp, which has the
-// least to do at the start of a phase
-template <int LGW>
-__device__ __forceinline__ void prefetch_units(const bf16* W, int N, int K, int cols, int turns) {
-  CFG;
-  if (tid_fresh() != THREADS - 32) return;
-#pragma unroll 1
-  for (int r = 0; r < turns; r++) {
-    const int c0 = (r * (int)gridDim.x + (int)blockIdx.x) * cols;
-    if (c0 >= N) return;
-    l2_prefetch_bulk(W + (size_t)c0 * K, (uint32_t)min(cols, N - c0) * (uint32_t)K * 2u);
-  }
-}
-// LayerNorm gain and bias of a later phase -> shared memory (complete at that phase's first barrier)
-template <int LGW>
-__device__ __forceinline__ void fetch_ln(bf16* sln, const bf16* w, const bf16* b, int d) {
-  CFG;
-#pragma unroll 1
-  for (int c = tid_fresh(); c < d / 8; c += THREADS) {
-    cp_async16(smem_u32(sln + c * 8), w + c * 8);
-    cp_async16(smem_u32(sln + d + c * 8), b + c * 8);
-  }
-  cp_async_commit();
-}
+constexpr int LN_GROUPS = 4;                  // groups that a turn takes behind a LayerNorm (proj and fcproj: one)
+constexpr int PAD = 32;                       // bf16 elements behind a normalised row (64 bytes: conflict-free fragments)
 
-// LayerNorm of rows [0, n) into xs, a warp per row: the row is polled, kept in shared memory as it arrived, and
-// normalised in place (every lane touches only the 16-byte pieces that it wrote).
-template <int LGW>
-__device__ __forceinline__ void stage_ln(bf16* xs, const bf16* sln, const Lin& L, int n, const DecodeParams& p, Shared* sh) {
-  CFG;
-  const int tid = tid_fresh(), warp = tid >> 5, lane = tid & 31;
-  const int d = L.K, nch = d / 8;
+// The ring as a warp sees it: the next chunk's slot and the parity of its barrier.
+struct Ring {
+  uint32_t base, full, empty, ln_full, ln_empty;
+  int n, slot;
+  uint32_t par;
+  uint8_t* ln;              // buffers of LayerNorm gain and bias (4 d bytes each), how many, the next one and its parity
+  int n_ln, ln_slot;
+  uint32_t ln_par;
+  __device__ __forceinline__ void ln_step() {
+    if (++ln_slot == n_ln) { ln_slot = 0; ln_par ^= 1u; }
+  }
+  __device__ __forceinline__ void step() {
+    if (++slot == n) { slot = 0; par ^= 1u; }
+  }
+};
+// hands the last `n` chunks that were taken back to the producer
+__device__ __forceinline__ void release(const Ring& r, int n, int lane) {
+  __syncwarp();
+  if (lane < n) {
+    int s = r.slot - 1 - lane;
+    if (s < 0) s += r.n;
+    mbar_arrive(r.empty + 8 * s);
+  }
+}
+constexpr int lg_rows(int MT) { return MT == 1 ? 3 : (MT == 2 ? 4 : 5); }
+// Output pair o of a turn: group, row (sequence) and first column inside the group.
+template <int MT>
+__device__ __forceinline__ void out_pair(int o, int& g, int& row, int& c) {
+  c = (o & 3) * 2;
+  row = (o >> 2) & (8 * MT - 1);
+  g = o >> (2 + lg_rows(MT));
+}
+constexpr int n_red(int MT) { return MT == 4 ? 1 : 2; }        // buffers of partial sums (shared memory for a second one lacks at 32 rows)
+
+// Steps of a quad that exist, known at compile time for widths 256 and 512 (LEFT = 1, 2: a LayerNorm's only quad) and multiples of 1024 (LEFT = 4,
+// every quad): without the branches of the general form (LEFT = 0) the pieces of a row are worked on together.
+template <int LEFT> __device__ __forceinline__ int steps_left(int st, int first) { return LEFT ? LEFT : st - first; }
+
+// LayerNorm of rows [0, n) -> xs [8 MT][K + PAD]: the warps fetch the fragments that they will multiply, then a warp takes a row, pieces
+// lane, lane + 32, ... of 16 bytes in blocks of four.
+template <int MT, int LEFT>
+__device__ __forceinline__ void normalise(const DecodeParams& p, const Lin& L, int n, bf16* xs, Ring& ring, Shared* sh) {
+  const int tid = tid_fresh(), warp = tid >> 5, lane = tid & 31, d = L.K, st = LEFT == 1 || LEFT == 2 ? LEFT : d >> 8;
+  const uint32_t pitch = (d + PAD) * 2, ln = smem_u32(ring.ln) + ring.ln_slot * (4 * d) + lane * 16;
+  {
+    const uint32_t to = smem_u32(xs) + (lane >> 2) * pitch + warp * 64 + (lane & 3) * 16;
+    Frags f[MT];
+#pragma unroll
+    for (int t = 0; t < MT; t++) {
+      int r = min(t * 8 + (lane >> 2), n - 1);
+      if (L.kind == PH) r = __ldg(p.rows + r);
+      f[t] = frags(L.src ? L.src : reinterpret_cast<const uint32_t*>(p.x), L.src ? GROUP : 0, d, L.src ? r & 7 : r, warp, lane);
+      if (L.src) f[t].at += (r >> 3) * f[t].tile;
+    }
 #pragma unroll 1
-  for (int r = warp; r < n; r += WARPS) {
-    const int sr = L.kind == PH ? p.rows[r] : r;
-    uint4* row = reinterpret_cast<uint4*>(xs + (size_t)r * (d + PAD));
-    float sum = 0.f;
-#pragma unroll 1
-    for (int c0 = lane; c0 < nch; c0 += 128) {
-      uint4 v[4];
-      if (L.src) {
-        const uint64_t* q = L.src + (size_t)sr * (d / 2) + c0 * 4;
-        uint2 t[8];
-        read_pairs<8>(t, [&](int i) { return c0 + (i >> 1) * 32 < nch; }, [&](int i) { return q + (i >> 1) * 128 + (i & 1) * 2; },
-                      L.e_src, p, sh);
+    for (int b = 0; b < st; b += 4) {                    // all rows of a block are requested together
+      uint4 v[4 * MT];
 #pragma unroll
-        for (int i = 0; i < 4; i++) v[i] = make_uint4(t[2 * i].x, t[2 * i].y, t[2 * i + 1].x, t[2 * i + 1].y);
-      } else {
-        const uint4* q = reinterpret_cast<const uint4*>(p.x + (size_t)sr * d) + c0;
+      for (int t = 0; t < MT; t++) ld_quad(v + 4 * t, 1, f[t].at, f[t].step, steps_left<LEFT>(st, b));
 #pragma unroll
-        for (int i = 0; i < 4; i++) v[i] = c0 + i * 32 < nch ? __ldcg(q + i * 32) : make_uint4(0, 0, 0, 0);
-      }
+      for (int t = 0; t < MT; t++) {
+        if (L.src) poll_quad(v + 4 * t, 1, f[t].at, f[t].step, steps_left<LEFT>(st, b), sh);
+        f[t].at += 4 * f[t].step;
 #pragma unroll
-      for (int i = 0; i < 4; i++) {
-        if (c0 + i * 32 >= nch) break;
-        row[c0 + i * 32] = v[i];
-        const float2 a = unpack_bf16(v[i].x), b = unpack_bf16(v[i].y), cc = unpack_bf16(v[i].z), e = unpack_bf16(v[i].w);
-        sum += (a.x + a.y) + (b.x + b.y) + (cc.x + cc.y) + (e.x + e.y);
+        for (int i = 0; i < 4; i++)
+          if (i < steps_left<LEFT>(st, b)) sts128(to + t * 8 * pitch + (b + i) * STEP_BYTES, v[4 * t + i]);
       }
     }
-    const float mean = warp_sum(sum) / (float)d;
-    float sq = 0.f;
+  }
+  wait_bar(ring.ln_full + 8 * ring.ln_slot, ring.ln_par, sh, p.wait_ns);
+  compute_sync();
+  uint32_t row = smem_u32(xs) + warp * pitch + lane * 16;
 #pragma unroll 1
-    for (int c0 = lane; c0 < nch; c0 += 128)
+  for (int r = warp; r < n; r += NW, row += NW * pitch) {
+    f2 s = 0, v = 0;
+    uint4 x[4];
+    auto load = [&](int b) {
 #pragma unroll
-      for (int i = 0; i < 4; i++) {
-        if (c0 + i * 32 >= nch) break;
-        const uint4 v = row[c0 + i * 32];
-        const float2 a = unpack_bf16(v.x), b = unpack_bf16(v.y), cc = unpack_bf16(v.z), e = unpack_bf16(v.w);
-        const float d0 = a.x - mean, d1 = a.y - mean, d2 = b.x - mean, d3 = b.y - mean, d4 = cc.x - mean, d5 = cc.y - mean,
-                    d6 = e.x - mean, d7 = e.y - mean;
-        sq += d0 * d0 + d1 * d1 + d2 * d2 + d3 * d3 + d4 * d4 + d5 * d5 + d6 * d6 + d7 * d7;
-      }
-    const float rstd = rsqrtf(warp_sum(sq) / (float)d + 1e-5f);
-    auto n2 = [&](uint32_t x2, uint32_t w2, uint32_t b2) {
-      const float2 xv = unpack_bf16(x2), wv = unpack_bf16(w2), bv = unpack_bf16(b2);
-      return pack_bf16((xv.x - mean) * rstd * wv.x + bv.x, (xv.y - mean) * rstd * wv.y + bv.y);
+      for (int i = 0; i < 4; i++) x[i] = lds128(row + (b + (i < steps_left<LEFT>(st, b) ? i : 0)) * 512);
     };
-#pragma unroll 1
-    for (int c0 = lane; c0 < nch; c0 += 64)
+    auto warp_sum = [&](float a) {
 #pragma unroll
-      for (int i = 0; i < 2; i++) {
-        const int c = c0 + i * 32;
-        if (c >= nch) break;
-        const uint4 v = row[c], gw = reinterpret_cast<const uint4*>(sln)[c], gb = reinterpret_cast<const uint4*>(sln + d)[c];
-        row[c] = make_uint4(n2(v.x, gw.x, gb.x), n2(v.y, gw.y, gb.y), n2(v.z, gw.z, gb.z), n2(v.w, gw.w, gb.w));
-      }
+      for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+      return a;
+    };
+    const bool one = (LEFT == 1 || LEFT == 2) || st <= 4;       // one block: it stays in registers
+    load(0);
+    int b = 0;
+#pragma unroll 1
+    do {
+      if (!one) load(b);
+#pragma unroll
+      for (int i = 0; i < 4; i++) if (i < steps_left<LEFT>(st, b)) s = add2(s, sum8(x[i]));
+    } while ((b += 4) < st);
+    const float mean = warp_sum(lo2(s) + hi2(s)) * p.inv_d;
+    const f2 nm = mk2(-mean, -mean);
+    b = 0;
+#pragma unroll 1
+    do {
+      if (!one) load(b);
+#pragma unroll
+      for (int i = 0; i < 4; i++) if (i < steps_left<LEFT>(st, b)) v = dev8(x[i], nm, v);
+    } while ((b += 4) < st);
+    const float rstd = rsqrtf(warp_sum(lo2(v) + hi2(v)) * p.inv_d + 1e-5f);
+    const f2 rs = mk2(rstd, rstd);
+    b = 0;
+#pragma unroll 1
+    do {
+      if (!one) load(b);
+#pragma unroll
+      for (int i = 0; i < 4; i++)
+        if (i < steps_left<LEFT>(st, b)) sts128(row + (b + i) * 512, norm8(x[i], lds128(ln + (b + i) * 512), lds128(ln + 2 * d + (b + i) * 512), nm, rs));
+    } while ((b += 4) < st);
   }
+  __syncwarp();
+  if (lane == 0) mbar_arrive(ring.ln_empty + 8 * ring.ln_slot);
+  ring.ln_step();
 }
 
-// One linear phase over rows [0, n) (n <= 8 MT).  The slots hold this warp's weights of its first unit and sub-step
-// (copy_first).  LN (A, D, head): the rows go through LayerNorm and shared memory; otherwise (C, E) operand fragments come
-// straight from the packets.  One copy of each form serves all layers, which keeps the code small.
-template <int LGW, int MT, bool LN>
-__device__ __forceinline__ void linear_phase(const DecodeParams& p, const Lin& L, int n, bool last, bf16* xs, const bf16* sln, float* red,
-                                             int& flip, Shared* sh, uint32_t wbuf) {
-  CFG;
-  constexpr bool RES = !LN;
-  constexpr int GP = 8 * MT, LGP = MT == 1 ? 3 : (MT == 2 ? 4 : 5);
-  constexpr int RG = LN ? 2 : 1, KS = NLD / RG, CU = 8 * RG, LCP = RG == 2 ? 3 : 2;      // steps per sub-step, columns and log2 column pairs per unit
-  constexpr int NCH = MT == 1 ? 4 : (MT == 2 ? 2 : 1);          // independent accumulator chains
+// A product over rows [0, n), n <= 8 MT: behind a LayerNorm (A, D, head; turns of four groups) or with a residual (C, E; turns of one group).
+// One copy of the code serves all phases: a layer's instructions should fit into the instruction cache (measured: straight-line
+// code of up to 32 KB runs at full speed; beyond, every jump to a line that is not there costs 50 cycles, beyond 128 KB 190).
+template <int MT, int LEFT>
+__device__ __forceinline__ void product(const DecodeParams& p, const Lin& L, bool ln, int n, bool last, bf16* xs, float* red0, int& flip,
+                                        Ring& ring, Shared* sh) {
+  constexpr int MH = MT == 1 ? 1 : MT / 2;               // accumulators of a group
+  constexpr int QB = 4 / MT;                             // C, E: chunks whose weights and activations are in flight together
+  constexpr int NA = LN_GROUPS * MH;
   const int tid = tid_fresh(), warp = tid >> 5, lane = tid & 31;
-  const uint32_t slots = wbuf + tid * 16;
-  const int N = L.N, K = L.K, lgs = L.lgs;
-  const int S = 1 << lgs, U = WARPS >> lgs, kw = K >> lgs, steps = kw >> 5;
-  const int n_units = (N + CU - 1) / CU, stride = (int)gridDim.x * U;
-  const int ul = warp >> lgs, ks = warp & (S - 1);
-  int unit0 = (int)blockIdx.x * U;
-  if (LN) { cp_async_wait_older(); __syncthreads(); }            // gain, bias and layer records are there (the weights need not be); xs is free
-  if (unit0 >= n_units) return;                                   // uniform over the CTA
-  const int n_out = U * GP * (CU / 2);                            // (unit, row, column pair)
-  auto operands = [&](int o, uint32_t& b2, uint64_t& r2) {        // bias and residual packet of output pair o, as they are now
-    b2 = 0; r2 = (uint64_t)L.e_res << 32;
-    const int g = (o >> LCP) & (GP - 1), col = (unit0 + (o >> (LCP + LGP))) * CU + (o & (CU / 2 - 1)) * 2;
-    if (o >= n_out || g >= n || col >= N) return;
-    if (L.bias) b2 = __ldg(reinterpret_cast<const unsigned int*>(L.bias + col));
-    if (RES) {
-      if (!L.res) r2 |= __ldcg(reinterpret_cast<const unsigned int*>(p.x + (size_t)g * N + col));
-      else r2 = ld_packet(L.res + ((size_t)g * N + col) / 2);
-    }
-  };
-  bool staged = false;
-  constexpr bool DB = C_::DB;
-  int wb = 0;                                                     // set of slots that holds the current weights
+  if (tid == 0) sh->phase = L.seq + 1;
+  const int sx = L.kind == PA ? 0 : L.kind == PD ? 2 : L.kind == PH ? 3 : 1;
+  const int g0 = sh->share[sx][0], g1 = sh->share[sx][1];
+  if (g0 >= g1) return;                                  // uniform over the CTA
+  const int st = L.K >> 8, nq = (st + 3) >> 2;           // steps of a warp and chunks of a row
+  const uint32_t lane_off = ring.base + (lane >> 2) * PITCH + warp * 64 + (lane & 3) * 16;
+  bool first = true;
 #pragma unroll 1
-  for (; unit0 < n_units; unit0 += stride) {
-    const int u = unit0 + ul;
-    uint32_t bias2;
-    uint64_t res2;
-    operands(tid, bias2, res2);
-    if (LN && !staged) {
-      stage_ln<LGW>(xs, sln, L, n, p, sh);
-      __syncthreads();
-      staged = true;
-    }
-    float acc[NCH][MT][4];
-#pragma unroll
-    for (int c = 0; c < NCH; c++)
-#pragma unroll
-      for (int m = 0; m < MT; m++)
-#pragma unroll
-        for (int i = 0; i < 4; i++) acc[c][m][i] = 0.f;
-#pragma unroll 1
-    for (int s0 = 0; s0 < steps; s0 += KS) {
-      const int k0 = ks * kw + s0 * 32, ns = min(KS, steps - s0);
-      // the weights that follow these in the same slots: next sub-step, or first sub-step of the next turn
-      const bool more = s0 + KS < steps, turn = !more && unit0 + stride < n_units;
-      const int nu = more ? u : u + stride, nk = more ? k0 + KS * 32 : ks * kw;
-      const int nn = more ? min(KS, steps - s0 - KS) : (turn ? min(KS, steps) : 0);
-      // DB: they go into the other set of slots at once, under these products; else into these slots, one by one as they are read
-      const uint32_t cur = slots + (DB && wb ? WBUF : 0), nxt = DB ? slots + (wb ? 0 : WBUF) : cur;
-      wb ^= 1;
-      if (DB && nn > 0) {
-#pragma unroll
-        for (int j = 0; j < KS; j++) copy_w<LGW, RG>(nxt, lane, L, nu, nk, j, nn);
-        cp_async_commit();
+  for (int t0 = g0; t0 < g1; t0 += ln ? LN_GROUPS : 1) {
+    const int ng = ln ? min(LN_GROUPS, g1 - t0) : 1;
+    uint32_t bias2 = 0, res2 = 0;                        // of output pair tid, as they are now
+    auto operands = [&](int g, int row, int col) {
+      if (L.bias) bias2 = __ldg(reinterpret_cast<const unsigned int*>(L.bias + col));
+      if (!ln) {
+        res2 = L.res ? ld_word(L.res + word_at(L.N, row, col)) : __ldcg(reinterpret_cast<const unsigned int*>(p.x) + (uint32_t)(row * L.N + col) / 2);
       }
-      auto wait_weights = [&]() {
-        if (DB && nn > 0) cp_async_wait_older(); else cp_async_wait_all();
-      };
-      if (LN) {
-        wait_weights();
-        const bf16* xa = xs + (size_t)(lane >> 2) * (K + PAD) + k0 + (lane & 3) * 8;
+    };
+    {
+      int g, row, c;
+      out_pair<MT>(tid, g, row, c);
+      if (g < ng && row < n && (t0 + g) * 8 + c < L.N) operands(g, row, (t0 + g) * 8 + c);
+    }
+    float acc[NA][4];
 #pragma unroll
-        for (int j = 0; j < KS; j++) {
-          if (j < ns) {
-            const uint4 w0 = lds128(cur + (2 * j) * SLOT), w1 = lds128(cur + (2 * j + 1) * SLOT);
+    for (int a = 0; a < NA; a++)
 #pragma unroll
-            for (int m = 0; m < MT; m++) {
-              const uint4 a = *reinterpret_cast<const uint4*>(xa + (size_t)(m * 8) * (K + PAD) + j * 32);
-              mma_bf16(acc[(2 * j) % NCH][m], w0.x, w1.x, w0.y, w1.y, a.x, a.y);
-              mma_bf16(acc[(2 * j + 1) % NCH][m], w0.z, w1.z, w0.w, w1.w, a.z, a.w);
+      for (int i = 0; i < 4; i++) acc[a][i] = 0.f;
+#pragma unroll 1
+    for (int q0 = 0; q0 < nq; q0 += ln ? 1 : QB) {
+      const int nc = ln ? ng : min(QB, nq - q0), left = ln ? steps_left<LEFT>(st, 4 * q0) : steps_left<LEFT == 4 ? 4 : 0>(st, 4 * q0);
+      uint4 x[16], w[16];                                // LN: [step][tile]; C, E: [chunk][step][tile] of QB chunks.  [chunk][step]
+#pragma unroll
+      for (int c = 0; c < 4; c++) {
+        const uint32_t a = lane_off + ring.slot * SLOT;
+        if (c < nc) {                                    // (else: whatever is there, for rows that nobody reads)
+          wait_bar(ring.full + 8 * ring.slot, ring.par, sh, p.wait_ns);
+          ring.step();
+        }
+#pragma unroll
+        for (int i = 0; i < 4; i++) w[4 * c + i] = lds128(a + i * STEP_BYTES);
+      }
+      if (ln) {
+        if (first) {
+          first = false;
+          normalise<MT, LEFT>(p, L, n, xs, ring, sh);
+          compute_sync();
+        }
+        {
+          const uint32_t xa = smem_u32(xs) + (lane >> 2) * ((L.K + PAD) * 2) + warp * 64 + (lane & 3) * 16 + q0 * (4 * STEP_BYTES);
+#pragma unroll
+          for (int i = 0; i < 4 * MT; i++) x[i] = lds128(xa + i % MT * 16 * (L.K + PAD) + (i / MT < left ? i / MT * STEP_BYTES : 0));
+        }
+#pragma unroll
+        for (int s = 0; s < 4; s++)
+          if (s < left) {
+            if constexpr (MT == 1) {      // weights of two groups are the 16 rows; two chains per pair
+#pragma unroll
+              for (int g = 0; g < LN_GROUPS; g += 2) {
+                const uint4 w0 = w[g * 4 + s], w1 = w[g * 4 + 4 + s];
+                mma_bf16(acc[g], w0.x, w1.x, w0.y, w1.y, x[s].x, x[s].y);
+                mma_bf16(acc[g + 1], w0.z, w1.z, w0.w, w1.w, x[s].z, x[s].w);
+              }
+            } else {                      // sequences are the 16 rows
+#pragma unroll
+              for (int g = 0; g < LN_GROUPS; g++)
+#pragma unroll
+                for (int m = 0; m < MH; m++) mma_rows(acc[g * MH + m], x[s * MT + 2 * m], x[s * MT + 2 * m + 1], w[g * 4 + s]);
             }
           }
-          if (!DB) copy_w<LGW, RG>(nxt, lane, L, nu, nk, j, nn);
-        }
       } else {
-        constexpr int JB = 4 / MT;                                // eight packet pairs in flight per lane
-        const uint64_t* q = L.src + (size_t)(lane >> 2) * (K / 2) + (k0 + (lane & 3) * 8) / 2;
+        // ---- proj, fcproj: the fragments come straight from the words
+        const int group = L.kind == PE ? act_pitch(n) : 0;
+        const uint32_t* rows[MT];
+        int step = 0;
 #pragma unroll
-        for (int j0 = 0; j0 < KS; j0 += JB) {
-          if (j0 < ns) {
-            uint2 t[8];
-            read_pairs<8>(t, [&](int i) { return (i >> 1) % MT * 8 + (lane >> 2) < n && j0 + (i >> 1) / MT < ns; },
-                          [&](int i) { return q + (size_t)((i >> 1) % MT * 8) * (K / 2) + (j0 + (i >> 1) / MT) * 16 + (i & 1) * 2; },
-                          L.e_src, p, sh);
-            if (j0 == 0) wait_weights();
+        for (int t = 0; t < MT; t++) {
+          const int r = min(t * 8 + (lane >> 2), n - 1);
+          const Frags f = frags(L.src, group, L.K, group ? r & 7 : r, warp, lane);
+          step = f.step;
+          rows[t] = f.at + (group ? (r >> 3) * f.tile : 0) + q0 * 4 * step;
+        }
+#pragma unroll
+        for (int c = 0; c < QB; c++)
+#pragma unroll
+          for (int t = 0; t < MT; t++)
+            if (c < nc) ld_quad(x + c * 4 * MT + t, MT, rows[t] + c * 4 * step, step, steps_left<LEFT == 4 ? 4 : 0>(left, 4 * c));
+            else
+#pragma unroll
+              for (int i = 0; i < 4; i++) x[(c * 4 + i) * MT + t] = make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+        for (int c = 0; c < QB; c++)
+          if (c < nc) {
+#pragma unroll
+            for (int t = 0; t < MT; t++) poll_quad(x + c * 4 * MT + t, MT, rows[t] + c * 4 * step, step, steps_left<LEFT == 4 ? 4 : 0>(left, 4 * c), sh);
             __syncwarp();
 #pragma unroll
-            for (int jj = 0; jj < JB; jj++) {
-              const int j = j0 + jj;
-              if (j < ns) {
-                const uint4 w0 = lds128(cur + j * SLOT);
+            for (int s = 0; s < 4; s++)
+              if (s < steps_left<LEFT == 4 ? 4 : 0>(left, 4 * c)) {
+                const uint4 w0 = w[c * 4 + s];
+                const uint4* xv = x + (c * 4 + s) * MT;
+                if constexpr (MT == 1) {
+                  mma_bf16(acc[(2 * s) & 3], w0.x, 0u, w0.y, 0u, xv[0].x, xv[0].y);
+                  mma_bf16(acc[(2 * s + 1) & 3], w0.z, 0u, w0.w, 0u, xv[0].z, xv[0].w);
+                } else {
 #pragma unroll
-                for (int m = 0; m < MT; m++) {
-                  const int i = jj * MT + m;
-                  mma_bf16(acc[(2 * j) % NCH][m], w0.x, 0u, w0.y, 0u, t[2 * i].x, t[2 * i].y);
-                  mma_bf16(acc[(2 * j + 1) % NCH][m], w0.z, 0u, w0.w, 0u, t[2 * i + 1].x, t[2 * i + 1].y);
+                  for (int m = 0; m < MH; m++) {      // two chains per pair of tiles
+                    mma_bf16(acc[m], xv[2 * m].x, xv[2 * m + 1].x, xv[2 * m].y, xv[2 * m + 1].y, w0.x, w0.y);
+                    mma_bf16(acc[MH + m], xv[2 * m].z, xv[2 * m + 1].z, xv[2 * m].w, xv[2 * m + 1].w, w0.z, w0.w);
+                  }
                 }
               }
-            }
           }
+      }
+      release(ring, nc, lane);
+    }
+    // ---- partial sums -> red[warp][group][sequence][weight row]
+    float* red = red0;
+    if (n_red(MT) == 1) compute_sync();                   // everybody has read the previous turn's
+    else { flip ^= 1; red += flip * (NW * LN_GROUPS * 64 * MT); }
+    {
+      float* mine = red + warp * (LN_GROUPS * 64 * MT);
+      if constexpr (MT == 1) {
+        mine += (lane & 3) * 16 + (lane >> 2);
+        if (!ln)
 #pragma unroll
-          for (int j = j0; j < j0 + JB; j++)
-            if (!DB) copy_w<LGW, RG>(nxt, lane, L, nu, nk, j, nn);
-        }
+          for (int i = 0; i < 2; i++) { acc[0][i] += acc[2][i]; acc[1][i] += acc[3][i]; }
+#pragma unroll
+        for (int g = 0; g < LN_GROUPS; g++)
+          if (g < ng)
+#pragma unroll
+            for (int i = 0; i < 2; i++) mine[g * 64 + i * 8] = acc[g & ~1][(g & 1) * 2 + i] + acc[g | 1][(g & 1) * 2 + i];
+      } else {
+        mine += lane * 2;
+        if (!ln)
+#pragma unroll
+          for (int m = 0; m < MH; m++)
+#pragma unroll
+            for (int i = 0; i < 4; i++) acc[m][i] += acc[MH + m][i];
+#pragma unroll
+        for (int g = 0; g < LN_GROUPS; g++)
+          if (g < ng)
+#pragma unroll
+            for (int m = 0; m < MH; m++) {
+              const float* c = acc[g * MH + m];
+              *reinterpret_cast<float2*>(mine + g * (64 * MT) + m * 128) = make_float2(c[0], c[1]);
+              *reinterpret_cast<float2*>(mine + g * (64 * MT) + m * 128 + 64) = make_float2(c[2], c[3]);
+            }
       }
     }
-    // partial sums -> shared memory; thread (unit, row, column pair) adds the S slices in order
-    float* rb = red + (MT == 4 ? 0 : flip * (WARPS * GP * 16));
-    flip ^= 1;
-    if (MT == 4) __syncthreads();             // one buffer only: everybody has read the previous turn's
-#pragma unroll
-    for (int m = 0; m < MT; m++)
-#pragma unroll
-      for (int i = 0; i < 2 * RG; i++) {
-        float v = acc[0][m][i];
-#pragma unroll
-        for (int c = 1; c < NCH; c++) v += acc[c][m][i];
-        rb[((size_t)warp * GP + m * 8 + (lane & 3) * 2 + (i & 1)) * CU + (i >> 1) * 8 + (lane >> 2)] = v;
-      }
-    __syncthreads();
+    compute_sync();
+    // ---- sum over the warps in order, epilogue, and on their way
 #pragma unroll 1
-    for (int o = tid; o < n_out; o += THREADS) {
-      const int g = (o >> LCP) & (GP - 1), cp = (o & (CU / 2 - 1)) * 2, uu = o >> (LCP + LGP), col = (unit0 + uu) * CU + cp;
-      if (g >= n || col >= N) continue;
-      if (o != tid) operands(o, bias2, res2);
-      if (RES && (uint32_t)(res2 >> 32) != L.e_res) res2 = read_one(L.res + ((size_t)g * N + col) / 2, L.e_res, p, sh);
-      const float* t = rb + ((size_t)(uu << lgs) * GP + g) * CU + cp;
-      float v0 = 0.f, v1 = 0.f;
-#pragma unroll 4
-      for (int s = 0; s < S; s++) {
-        const float2 f = *reinterpret_cast<const float2*>(t + (size_t)s * (GP * CU));
-        v0 += f.x; v1 += f.y;
-      }
-      const float2 b = unpack_bf16(bias2), rr = unpack_bf16((uint32_t)res2);
-      v0 += b.x; v1 += b.y;
-      if (RES) { v0 += rr.x; v1 += rr.y; }
-      if (LN && L.kind == PD) {
+    for (int o = tid; o < ng * 32 * MT; o += CT) {
+      int g, row, c;
+      out_pair<MT>(o, g, row, c);
+      const int col = (t0 + g) * 8 + c;
+      if (row >= n || col >= L.N) continue;
+      if (MT > 2 && o != tid) operands(g, row, col);
+      const float* t = red + g * (64 * MT) + row * 8 + c;
+      const uint32_t at = word_at(L.N, row, col, L.kind == PD ? act_pitch(n) : GROUP);
+      float2 f[NW];
+#pragma unroll
+      for (int i = 0; i < NW; i++) f[i] = *reinterpret_cast<const float2*>(t + i * (LN_GROUPS * 64 * MT));
+      uint32_t it = 0;
+#pragma unroll 1
+      while (!ln && L.res && res2 == 0 && !expired(it, sh)) res2 = ld_word(L.res + at);
+      f2 v = 0;
+#pragma unroll
+      for (int i = 0; i < NW; i++) v = add2(v, mk2(f[i].x, f[i].y));
+      v = add2(v, un2(bias2));
+      if (!ln) v = add2(v, un2(res2));
+      float v0 = lo2(v), v1 = hi2(v);
+      if (L.kind == PD) {
         v0 = gelu_tanh(__bfloat162float(__float2bfloat16(v0)));
         v1 = gelu_tanh(__bfloat162float(__float2bfloat16(v1)));
       }
       const uint32_t pk = pack_bf16(v0, v1);
-      if (!LN || L.kind != PH) st_packet(L.dst + ((size_t)g * N + col) / 2, pk, L.e_dst);
-      if (!LN && last) *reinterpret_cast<uint32_t*>(p.x + (size_t)g * N + col) = pk;
-      if (LN && L.kind == PH) {
-        bf16* q = p.logits + (size_t)g * p.ld_logits + col;
-        if (col + 1 < N && ((uintptr_t)q & 3) == 0) *reinterpret_cast<uint32_t*>(q) = pk;
+      if (L.dst) {
+        it = 0;
+#pragma unroll 1
+        while (sh->cleared <= L.seq && !expired(it, sh)) {}       // the next layer's words are empty before these are there
+        st_word(L.dst + at, full_word(pk));
+        if (last) reinterpret_cast<uint32_t*>(p.x)[(uint32_t)(row * L.N + col) / 2] = pk;
+      } else {
+        bf16* q = p.logits + (size_t)row * p.ld_logits + col;
+        if (col + 1 < L.N && ((uintptr_t)q & 3) == 0) *reinterpret_cast<uint32_t*>(q) = pk;
         else {
           q[0] = __float2bfloat16(v0);
-          if (col + 1 < N) q[1] = __float2bfloat16(v1);
+          if (col + 1 < L.N) q[1] = __float2bfloat16(v1);
         }
       }
     }
   }
 }
 
-// ------------------------------------------------------------------------------------------------
-// Positions a lane group holds at a time: eight for heads of 64 where registers allow it; four for narrow heads, whose eight groups a warp
-// cover short contexts in one turn anyway (d256: 59 us a step against 64), and for heads of 128 (no difference).
-template <int LGW, int HD> constexpr int keys_ahead() { return LGW == 3 && HD == 64 ? 8 : 4; }
-// Phase B.  Appends the new k, v (from the qkv packets) to the paged cache and attends over positions 0..pos.
-// The W warps of an item hold W * 32 / (HD / 8) lane groups; group i takes keys i, i + ST, i + 2 ST, ...
-template <int LGW, int HD>
-__device__ __forceinline__ void attention_phase(const DecodeParams& p, int layer, uint32_t epoch, float* satt, Shared* sh) {
-  CFG;
-  constexpr int LPK = HD / 8, KPW = 32 / LPK;     // lanes per key, keys of a warp at a time
-  constexpr int NB = keys_ahead<LGW, HD>();        // positions a group holds at a time
-  const int tid = tid_fresh(), warp = tid >> 5, lane = tid & 31;
-  const int W = 1 << p.lgw, slots = WARPS >> p.lgw, ST = W * KPW;
-  const int kg = (warp & (W - 1)) * KPW + lane / LPK, e0 = (lane % LPK) * 8;
-  const int d = p.d, items = p.G * p.H;
-  const bf16* kc = p.kc + (size_t)layer * p.layer_elems;
-  const bf16* vc = p.vc + (size_t)layer * p.layer_elems;
+// ---- helpers
+// Producer: the chunks of this CTA's share of W [N, K] in the order in which the computing warps take them.
+__device__ __forceinline__ bool stream(const bf16* W, int N, int K, int per_turn, const int* range, Ring& r, Shared* sh, const DecodeParams& p) {
+  const int lane = threadIdx.x & 31, g1 = range[1];
 #pragma unroll 1
-  for (int it0 = (int)blockIdx.x * slots; it0 < items; it0 += (int)gridDim.x * slots) {
-    const int item = it0 + (warp >> p.lgw);
-    const int t = item / p.H, h = item - t * p.H;
+  for (int t0 = range[0]; t0 < g1; t0 += per_turn)
+#pragma unroll 1
+    for (int k0 = 0; k0 < K; k0 += KC)
+#pragma unroll 1
+      for (int g = t0; g < min(t0 + per_turn, g1); g++) {
+        wait_bar(r.empty + 8 * r.slot, r.par ^ 1u, sh, 2 * p.wait_ns);
+        if (sh->abort_flag) return false;
+        const int rows = min(8, N - g * 8), bytes = min(KC, K - k0) * 2;
+        if (lane == 0) mbar_expect_tx(r.full + 8 * r.slot, rows * bytes);
+        __syncwarp();
+        if (lane < rows) bulk_load(r.base + r.slot * SLOT + lane * PITCH, W + (size_t)(g * 8 + lane) * K + k0, bytes, r.full + 8 * r.slot);
+        r.step();
+      }
+  return true;
+}
+__device__ __forceinline__ void produce(const DecodeParams& p, Ring ring, Shared* sh) {
+  const int d = p.d;
+  bool ok = true;
+#pragma unroll 1
+  for (int k = 0; ok && k < 4 * p.L + (p.head_w ? 1 : 0); k++) {
+    const int j = k & 3;
+    const bool head = k == 4 * p.L;
+    const bf16* const* lw = reinterpret_cast<const bf16* const*>(p.layers + (k >> 2));
+    const bf16* W = head ? p.head_w : lw[j == 0 ? 2 : j == 1 ? 4 : j == 2 ? 8 : 10];
+    const int* range = sh->share[head ? 3 : j == 3 ? 1 : j];
+    if (!(j & 1) && range[0] < range[1]) {               // gain and bias of the LayerNorm in front
+      wait_bar(ring.ln_empty + 8 * ring.ln_slot, ring.ln_par ^ 1u, sh, 2 * p.wait_ns);
+      if (sh->abort_flag) { ok = false; break; }
+      if ((threadIdx.x & 31) == 0) {
+        const uint32_t bar = ring.ln_full + 8 * ring.ln_slot, dst = smem_u32(ring.ln + ring.ln_slot * (4 * d));
+        mbar_expect_tx(bar, 4 * d);
+        bulk_load(dst, head ? p.lnf_w : lw[j ? 6 : 0], 2 * d, bar);
+        bulk_load(dst + 2 * d, head ? p.lnf_b : lw[j ? 7 : 1], 2 * d, bar);
+      }
+      ring.ln_step();
+    }
+    ok = stream(W, head ? p.V : j == 0 ? 3 * d : j == 2 ? 4 * d : d, j == 3 ? 4 * d : d, j & 1 ? 1 : LN_GROUPS, range, ring, sh, p);
+  }
+  if (!ok) {                     // given up: no copy may be in flight when the CTA leaves
+#pragma unroll 1
+    for (int k = 0; k < ring.n_ln; k++) {
+      if (ring.ln_slot == 0) { ring.ln_slot = ring.n_ln; ring.ln_par ^= 1u; }
+      ring.ln_slot--;
+      const uint64_t t0 = kh_globaltimer();
+      while (!mbar_try(ring.ln_full + 8 * ring.ln_slot, ring.ln_par) && kh_globaltimer() - t0 < 100000000ull) {}
+    }
+#pragma unroll 1
+    for (int k = 0; k < ring.n; k++) {
+      if (ring.slot == 0) { ring.slot = ring.n; ring.par ^= 1u; }
+      ring.slot--;               // backwards over the ring (a slot that was never filled passes at once)
+      const uint64_t t0 = kh_globaltimer();
+      while (!mbar_try(ring.full + 8 * ring.slot, ring.par) && kh_globaltimer() - t0 < 100000000ull) {}
+    }
+  }
+}
+// Empties this CTA's words of the slot that the next layer writes, as soon as the CTA is done with the same phase of the last layer; the
+// fence and the `cleared` count order that before the phase's own outputs.
+template <int HD>
+__device__ __forceinline__ void empty_words(const DecodeParams& p, uint32_t* words, size_t block, Shared* sh) {
+  const int d = p.d, lane = threadIdx.x & 31, per = NW >> p.lgw, items = p.G * p.H;
+  const size_t row = (size_t)MAX_ROWS * (d / 2);
+  const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll 1
+  for (int k = 0; k < 5 * p.L; k++) {
+    const int l = k / 5, j = k - 5 * l;
+    uint32_t* nxt = words + (size_t)((l + 1) % 3) * block;
+    const uint64_t t0 = kh_globaltimer();
+    while (sh->phase <= k - 4) {       // until this CTA is done with the same phase of the layer before
+      if (sh->abort_flag || kh_globaltimer() - t0 > 2 * p.wait_ns) { sh->abort_flag = 1; return; }
+      __nanosleep(50);
+    }
+    if (j == 1) {
+      uint32_t* a = nxt + 2 * row;
+#pragma unroll 1
+      for (int it0 = (int)blockIdx.x * per; it0 < items; it0 += (int)gridDim.x * per)
+#pragma unroll 1
+        for (int i = lane; i < per * (HD / 8); i += 32) {
+          const int it = it0 + i / (HD / 8), t = p.seq_of(it);
+          if (it < items) *reinterpret_cast<uint4*>(a + ((size_t)t * d + (it - t * p.H) * HD) / 2 + (i % (HD / 8)) * 4) = zero;
+        }
+    } else {
+      const int N = j == 0 ? 3 * d : j == 3 ? 4 * d : d;
+      uint32_t* a = nxt + (j == 0 ? 3 : j == 2 ? 1 : j == 3 ? 6 : 0) * row;
+      const int* range = sh->share[j == 0 ? 0 : j == 3 ? 2 : 1];
+      const int pitch = j == 3 ? act_pitch(p.G) : GROUP;
+#pragma unroll 1
+      for (int r = 0; r < p.G; r += 8)
+#pragma unroll 1
+        for (int i = range[0] * pitch + lane * 4; i < range[1] * pitch; i += 128) *reinterpret_cast<uint4*>(a + r / 8 * (4 * N) + i) = zero;
+    }
+    __threadfence();
+    __syncwarp();
+    if (lane == 0) sh->cleared = k + 1;
+  }
+}
+// The other half of the workspace is emptied for the next launch.
+__device__ __forceinline__ void empty_half(const DecodeParams& p, uint32_t half, size_t block) {
+  const int used = min((int)*reinterpret_cast<volatile uint32_t*>(p.ctl + 3 + (half ^ 1u)) + 7 & ~7, MAX_ROWS), d = p.d;
+  const int me = (int)blockIdx.x * 64 + (int)threadIdx.x % 64, all = (int)gridDim.x * 64;
+  uint32_t* w = p.words + (half ^ 1u) * 3 * block;
+#pragma unroll 1
+  for (int s = 0; s < 3; s++)
+#pragma unroll 1
+    for (int f = 0; f < 5; f++) {
+      const int width = (f < 3 ? d : (f == 3 ? 3 * d : 4 * d)) / 2, from = f < 4 ? f * d / 2 : 3 * d;
+      uint4* q = reinterpret_cast<uint4*>(w + s * block + (size_t)MAX_ROWS * from);
+#pragma unroll 1
+      for (int i = me; i < used * width / 4; i += all) q[i] = make_uint4(0u, 0u, 0u, 0u);
+    }
+}
+
+// ------------------------------------------------------------------------------------------------
+// Positions that a lane group (four lanes) holds at a time: the 16 rows of a score product; twice as many for many sequences with narrow heads,
+// whose rows are short (L4 d512 H16 G = 32, contexts of 20 / 200 / 900: 116 / 131 / 194 us a step, 105 / 125 / 216 with two; d256 H8 100 / 108 /
+// 135 and 93 / 103 / 142), but not elsewhere (head width 64, L12 d1024 G = 8, 160: 205 us with two, 222 with four).
+template <int MT, int HD> constexpr int keys_ahead() { return HD == 32 && MT == 4 ? 4 : 2; }
+// Bytes of a layer's keys and values up to which the next layer's are prefetched into L2; beyond, they are gone before they are used and
+// come from memory twice (G = 32, 900 positions, 118 MB: L12 d1024 977 us with, 889 without; 59 MB, G = 16: 492 and 500; 65 MB, L4 d2048 G = 8: 252 and 240).
+constexpr float FETCH_LIMIT = 60e6f;
+// Phase B.  Appends the new k, v to the paged cache and attends over positions 0..pos.
+// The W warps of an item hold 8 W lane groups; group i takes positions i, i + 8 W, i + 16 W, ...; the group that would take `pos` starts with
+// the new key and value.
+template <int MT, int HD>
+__device__ __forceinline__ void attention_phase(const DecodeParams& p, int layer, int seq, const uint32_t* qkvw, uint32_t* attw, float* satt, Shared* sh) {
+  constexpr int NB = keys_ahead<MT, HD>(), NC = HD / 32;      // 16-byte pieces of a row per lane
+  const int tid = tid_fresh(), warp = tid >> 5, lane = tid & 31, lgw = fresh(p.lgw), H = fresh(p.H), bid = fresh(blockIdx.x);
+  if (tid == 0) sh->phase = seq + 1;
+  const int W = 1 << lgw, slots = NW >> lgw, ST = W * 8;
+  const int first = (warp & (W - 1)) * 8, kg = first + (lane >> 2), e0 = (lane & 3) * 8;       // (first: uniform over the warp)
+  const int d = fresh(p.d), items = p.G * H;
+#pragma unroll 1
+  for (int it0 = bid * slots; it0 < items; it0 += (int)gridDim.x * slots) {
+    const int item = it0 + (warp >> lgw);
+    const int t = p.seq_of(item), h = item - t * H;
     int pos = -1, slot = -1;
-    const bool turn0 = it0 == (int)blockIdx.x * slots;
+    const bool turn0 = it0 == bid * slots;
     if (item < items) {
       pos = turn0 ? sh->item_pos[warp] : __ldg(p.pos + t);
       slot = turn0 ? sh->item_slot[warp] : __ldg(p.slot + t);
     }
     const bool valid = pos >= 0 && pos < p.max_ctx && p.block_of(pos) < p.max_lb && slot >= 0;       // uniform over the item's warps
     if (item < items && !valid && lane == 0) atomicCAS(p.err, 0, 8);
-    float m = -INFINITY, l = 0.f, o[8];
+    float m = -INFINITY, l = 0.f;
+    f2 o[4 * NC];
 #pragma unroll
-    for (int k = 0; k < 8; k++) o[k] = 0.f;
+    for (int k = 0; k < 4 * NC; k++) o[k] = 0;
     if (valid) {
       const int* bt = p.btab + (size_t)slot * p.max_lb;
       auto row_of = [&](int j) {
         const int jb = p.block_of(j);
         return __ldg(bt + jb) * p.bs + (j - jb * p.bs);
       };
-      int row[NB];                    // cache rows of the next positions of this group
-      uint4 k4[NB], v4[NB];            // refilled with those positions as soon as they are used
-      uint2 qkv2[6];
-      float q[8];
-      const bool owner = pos % ST == kg;
-      const int first = (warp & (W - 1)) * KPW;       // uniform over the warp
-      // Turn -1 only requests the first NB keys and values and then waits for the query (and the owner of position `pos`
-      // for the new key and value); every other turn uses NB positions and requests the next ones in their place.
-#pragma unroll 1
-      for (int b0 = -NB * ST; b0 < 0 || first + b0 <= pos; b0 += NB * ST) {
-        const int j0 = kg + b0, jn = j0 + NB * ST;
-        float s[NB];
+      const int at = h * HD + e0;
+      // this lane asks L2 for a line of the next layer, while a layer's keys and values (as many for all sequences as for this one) stay there until then
+      const bool fetch = (lane & 3) < (HD == 128 ? 2 : 1) && layer + 1 < p.L && (float)pos * (float)(p.G * d) < FETCH_LIMIT / 4.f;
+      const bf16 *kc = p.kc + (size_t)layer * p.layer_elems + at, *vc = p.vc + (size_t)layer * p.layer_elems + at;
+      const bf16* none = reinterpret_cast<const bf16*>(p.ctl + 16) + e0;       // zeros, for positions that do not exist
+      const bf16* vp[NB];              // this group's next values
+      int row[NB];                     // cache rows of its next positions; the block table is read a turn ahead
 #pragma unroll
-        for (int i = 0; i < NB; i++)
-          if (jn + i * ST < pos) row[i] = b0 < 0 && turn0 ? sh->item_row[warp][lane / LPK][i] : row_of(jn + i * ST);
+      for (int i = 0; i < NB; i++) {
+        row[i] = 0;
+        if (kg + i * ST < pos) row[i] = turn0 ? sh->item_row[warp][lane >> 2][i] : row_of(kg + i * ST);
+      }
+      uint4 k4[NB][NC], v4[NB][NC];    // refilled with the next positions as soon as they are used
+      uint4 q[NC];
+#pragma unroll
+      for (int k = 0; k < NC; k++) {
+        q[k] = make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+        for (int i = 0; i < NB; i++) k4[i][k] = v4[i][k] = make_uint4(0u, 0u, 0u, 0u);
+      }
+      // Turn -1 only requests the first NB keys and values and then waits for the query; every other turn uses NB positions
+      // and requests the next ones in their place.
+#pragma unroll 1
+      for (int b0 = -NB * ST; b0 < 0 || first + b0 < pos; b0 += NB * ST) {
+        const int jn = kg + b0 + NB * ST;
+        float s[NB];
+        int e[NB];
+#pragma unroll
+        for (int i = 0; i < NB; i++) {
+          s[i] = 0.f;
+          e[i] = 0;
+          if (jn + (NB + i) * ST < pos) e[i] = __ldg(bt + p.block_of(jn + (NB + i) * ST));
+        }
         if (b0 >= 0) {
 #pragma unroll
-          for (int i = 0; i < NB; i++) {
-            const int j = j0 + i * ST;
-            if (j == pos) { k4[i] = make_uint4(qkv2[2].x, qkv2[2].y, qkv2[3].x, qkv2[3].y); v4[i] = make_uint4(qkv2[4].x, qkv2[4].y, qkv2[5].x, qkv2[5].y); }
-            if (j > pos) k4[i] = v4[i] = make_uint4(0, 0, 0, 0);
-            const float2 a = unpack_bf16(k4[i].x), b = unpack_bf16(k4[i].y), c = unpack_bf16(k4[i].z), e = unpack_bf16(k4[i].w);
-            s[i] = a.x * q[0] + a.y * q[1] + b.x * q[2] + b.y * q[3] + c.x * q[4] + c.y * q[5] + e.x * q[6] + e.y * q[7];
+          for (int i = 0; i < NB; i += 2) {
+            float c[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+            for (int k = 0; k < NC; k++) mma_rows(c, k4[i][k], k4[i + 1][k], q[k]);
+            s[i] = c[0]; s[i + 1] = c[2];
           }
         }
         // cached positions only; the same lines of the next layer are requested into L2
 #pragma unroll
-        for (int i = 0; i < NB; i++)
-          if (jn + i * ST < pos) {
-            const bf16* c = kc + (size_t)row[i] * d + h * HD + e0;
-            k4[i] = ldg_stream(c);
-            if (e0 % 64 == 0 && layer + 1 < p.L) prefetch_l2(c + p.layer_elems);
+        for (int i = 0; i < NB; i++) {
+          const bool in = jn + i * ST < pos;
+          const bf16* kp = none;
+          vp[i] = none;
+          if (in) {
+            const size_t r = (size_t)(uint32_t)row[i] * (uint32_t)d;
+            kp = kc + r;
+            vp[i] = vc + r;
+            if (fetch) { prefetch_l2(kp + p.layer_elems + e0 * 7); prefetch_l2(vp[i] + p.layer_elems + e0 * 7); }
           }
+#pragma unroll
+          for (int k = 0; k < NC; k++) k4[i][k] = ldg_stream(kp + k * 32);
+        }
         if (b0 >= 0) {
-#pragma unroll
-          for (int x = LPK / 2; x > 0; x >>= 1)
-#pragma unroll
-            for (int i = 0; i < NB; i++) s[i] += __shfl_xor_sync(0xffffffffu, s[i], x);
-#pragma unroll
-          for (int i = 0; i < NB; i++)
-            if (j0 + i * ST > pos) s[i] = -INFINITY;
           float mn = m;
 #pragma unroll
-          for (int i = 0; i < NB; i++) mn = fmaxf(mn, s[i]);
-          const float ref = mn == -INFINITY ? 0.f : mn;
-          const float sc = __expf(m - ref);
+          for (int i = 0; i < NB; i++) {
+            s[i] = kg + b0 + i * ST < pos ? s[i] * p.scale : -INFINITY;
+            mn = fmaxf(mn, s[i]);
+          }
+          const float ref = mn == -INFINITY ? 0.f : mn, sc = __expf(m - ref);
           m = mn;
           l *= sc;
 #pragma unroll
-          for (int k = 0; k < 8; k++) o[k] *= sc;
+          for (int k = 0; k < 4 * NC; k++) o[k] = mul2(o[k], mk2(sc, sc));
 #pragma unroll
           for (int i = 0; i < NB; i++) {
             const float pr = __expf(s[i] - ref);
             l += pr;
-            const float2 a = unpack_bf16(v4[i].x), b = unpack_bf16(v4[i].y), c = unpack_bf16(v4[i].z), e = unpack_bf16(v4[i].w);
-            o[0] += pr * a.x; o[1] += pr * a.y; o[2] += pr * b.x; o[3] += pr * b.y;
-            o[4] += pr * c.x; o[5] += pr * c.y; o[6] += pr * e.x; o[7] += pr * e.y;
+#pragma unroll
+            for (int k = 0; k < NC; k++) {
+              f2 f[4];
+              un8(f, v4[i][k]);
+#pragma unroll
+              for (int e = 0; e < 4; e++) o[4 * k + e] = fma2(mk2(pr, pr), f[e], o[4 * k + e]);
+            }
           }
         }
 #pragma unroll
         for (int i = 0; i < NB; i++)
-          if (jn + i * ST < pos) {
-            const bf16* c = vc + (size_t)row[i] * d + h * HD + e0;
-            v4[i] = ldg_stream(c);
-            if (e0 % 64 == 0 && layer + 1 < p.L) prefetch_l2(c + p.layer_elems);
-          }
+#pragma unroll
+          for (int k = 0; k < NC; k++) v4[i][k] = ldg_stream(vp[i] + k * 32);
         if (b0 < 0) {
-          const uint64_t* qp = p.qkvp + ((size_t)t * 3 * d + h * HD + e0) / 2;
-          read_pairs<6>(qkv2, [&](int i) { return i < 2 || owner; }, [&](int i) { return qp + (size_t)(i >> 1) * (d / 2) + (i & 1) * 2; },
-                        epoch, p, sh);
+          const uint32_t* qp = qkvw + word_at(3 * d, t, at);        // (32 columns are 128 words on)
+          const bool owner = (pos & (ST - 1)) == kg;
+          uint4 kn[NC], vn[NC];
+#pragma unroll
+          for (int k = 0; k < NC; k++) kn[k] = vn[k] = make_uint4(0u, 0u, 0u, 0u);
+          uint32_t it = 0;
+#pragma unroll 1
+          while (true) {
+            uint32_t e = 0xffffffffu;
+#pragma unroll
+            for (int k = 0; k < NC; k++) ld_words(q[k], qp + 128 * k);
+            if (owner) {
+#pragma unroll
+              for (int k = 0; k < NC; k++) { ld_words(kn[k], qp + 4 * d + 128 * k); ld_words(vn[k], qp + 8 * d + 128 * k); }
+#pragma unroll
+              for (int k = 0; k < NC; k++) e = min(e, min(least(kn[k]), least(vn[k])));
+            }
+#pragma unroll
+            for (int k = 0; k < NC; k++) e = min(e, least(q[k]));
+            if (e != 0u || expired(it, sh)) break;
+          }
           __syncwarp();
-          const float2 a = unpack_bf16(qkv2[0].x), b = unpack_bf16(qkv2[0].y), c = unpack_bf16(qkv2[1].x), e = unpack_bf16(qkv2[1].y);
-          q[0] = a.x * p.scale; q[1] = a.y * p.scale; q[2] = b.x * p.scale; q[3] = b.y * p.scale;
-          q[4] = c.x * p.scale; q[5] = c.y * p.scale; q[6] = e.x * p.scale; q[7] = e.y * p.scale;
+          float c[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+          for (int k = 0; k < NC; k++) mma_rows(c, kn[k], make_uint4(0u, 0u, 0u, 0u), q[k]);
+          if (owner) {
+            m = c[0] * p.scale;
+            l = __expf(m - (m == -INFINITY ? 0.f : m));
+            const size_t dst = (size_t)(uint32_t)(turn0 ? sh->pos_row[warp] : row_of(pos)) * (uint32_t)d;
+#pragma unroll
+            for (int k = 0; k < NC; k++) {
+              f2 f[4];
+              un8(f, vn[k]);
+#pragma unroll
+              for (int e = 0; e < 4; e++) o[4 * k + e] = mul2(mk2(l, l), f[e]);
+              *reinterpret_cast<uint4*>(const_cast<bf16*>(kc) + dst + k * 32) = kn[k];
+              *reinterpret_cast<uint4*>(const_cast<bf16*>(vc) + dst + k * 32) = vn[k];
+            }
+          }
+        }
+#pragma unroll
+        for (int i = 0; i < NB; i++) {
+          const int j = jn + (NB + i) * ST;
+          row[i] = e[i] * p.bs + (j - p.block_of(j) * p.bs);
         }
       }
-      if (owner) {
-        const size_t at = (size_t)layer * p.layer_elems + (size_t)row_of(pos) * d + h * HD + e0;
-        *reinterpret_cast<uint4*>(p.kc + at) = make_uint4(qkv2[2].x, qkv2[2].y, qkv2[3].x, qkv2[3].y);
-        *reinterpret_cast<uint4*>(p.vc + at) = make_uint4(qkv2[4].x, qkv2[4].y, qkv2[5].x, qkv2[5].y);
-      }
-      // merge the lane groups of the warp
-#pragma unroll 1
-      for (int x = LPK; x < 32; x <<= 1) {
-        const float m2 = __shfl_xor_sync(0xffffffffu, m, x), l2 = __shfl_xor_sync(0xffffffffu, l, x);
-        const float mn = fmaxf(m, m2), ref = mn == -INFINITY ? 0.f : mn;
-        const float c1 = __expf(m - ref), c2 = __expf(m2 - ref);
-        m = mn;
-        l = l * c1 + l2 * c2;
+      __syncwarp();
+    } else { m = 0.f; l = 0.125f; }    // an item with a bad index writes zeros: its row must not stall
+    // merge the lane groups of the warp: every round adds half of the values of the partner and gives it the other half
+    float mx = m;
 #pragma unroll
-        for (int k = 0; k < 8; k++) {
-          const float o2 = __shfl_xor_sync(0xffffffffu, o[k], x);
-          o[k] = o[k] * c1 + o2 * c2;
-        }
-      }
-    } else { m = 0.f; l = 1.f; }       // an item with a bad index writes zeros: its row must not stall
-    float* mine = satt + warp * ATT_PITCH;
-    if (lane < LPK) {
+    for (int x = 4; x < 32; x <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, x));
+    const float c = __expf(m - (mx == -INFINITY ? 0.f : mx));
+    l *= c;
 #pragma unroll
-      for (int k = 0; k < 8; k += 4) *reinterpret_cast<float4*>(mine + e0 + k) = make_float4(o[k], o[k + 1], o[k + 2], o[k + 3]);
-      if (lane == 0) { mine[128] = m; mine[129] = l; }
+    for (int x = 4; x < 32; x <<= 1) l += __shfl_xor_sync(0xffffffffu, l, x);
+    float v[8 * NC];
+#pragma unroll
+    for (int k = 0; k < 4 * NC; k++) { v[2 * k] = lo2(o[k]) * c; v[2 * k + 1] = hi2(o[k]) * c; }
+    int f0 = 0;
+#pragma unroll
+    for (int r = 0; r < 3; r++) {
+      const int x = 16 >> r, half = (4 * NC) >> r;
+      const bool up = (lane & x) != 0;
+      if (up) f0 += half;
+#pragma unroll
+      for (int i = 0; i < half; i++) {
+        const float give = up ? v[i] : v[i + half], keep = up ? v[i + half] : v[i];
+        v[i] = keep + __shfl_xor_sync(0xffffffffu, give, x);
+      }
     }
-    __syncthreads();
-    // Merge the W warps of each item: lane k (of 16) weighs the k-th partial result of its item.
+    float* mine = satt + warp * ATT_PITCH;
+#pragma unroll
+    for (int i = 0; i < NC; i++) mine[((f0 + i) >> 3) * 32 + e0 + ((f0 + i) & 7)] = v[i];
+    if (lane == 0) *reinterpret_cast<float2*>(mine + 128) = make_float2(mx, l);
+    compute_sync();
+    // merge the W warps of each item
 #pragma unroll 1
-    for (int i = tid; i < slots * (HD / 2); i += THREADS) {
+    for (int i = tid; i < slots * (HD / 2); i += CT) {
       const int sl = i / (HD / 2), e = (i % (HD / 2)) * 2, it = it0 + sl;
-      const unsigned mask = HD == 32 ? 0xffffu << (lane & 16) : 0xffffffffu;       // the lanes of this item
-      const float* part = satt + (size_t)(sl << p.lgw) * ATT_PITCH;
-      const int k16 = lane & 15;
-      float c = k16 < W ? part[k16 * ATT_PITCH + 128] : -INFINITY, den = k16 < W ? part[k16 * ATT_PITCH + 129] : 0.f, mx = c;
-#pragma unroll
-      for (int x = 8; x > 0; x >>= 1) mx = fmaxf(mx, __shfl_xor_sync(mask, mx, x));
-      c = __expf(c - mx);              // (NaN when every score is -inf, as in the kernel chain)
-      den *= c;
-#pragma unroll
-      for (int x = 8; x > 0; x >>= 1) den += __shfl_xor_sync(mask, den, x);
-      float v0 = 0.f, v1 = 0.f;
+      const float* part = satt + (size_t)(sl << lgw) * ATT_PITCH;
+      float top = -INFINITY;
+#pragma unroll 4
+      for (int k = 0; k < W; k++) top = fmaxf(top, part[k * ATT_PITCH + 128]);
+      float den = 0.f, v0 = 0.f, v1 = 0.f;
 #pragma unroll 4
       for (int k = 0; k < W; k++) {
-        const float ck = __shfl_sync(mask, c, (lane & 16) + k);
-        const float2 f = *reinterpret_cast<const float2*>(part + k * ATT_PITCH + e);
+        const float2 ml = *reinterpret_cast<const float2*>(part + k * ATT_PITCH + 128), f = *reinterpret_cast<const float2*>(part + k * ATT_PITCH + e);
+        const float ck = __expf(ml.x - top);           // (NaN when every score is -inf, as in the kernel chain)
+        den += ck * ml.y;
         v0 += ck * f.x; v1 += ck * f.y;
       }
       const float inv = 1.f / den;
-      const int tt = it / p.H;
-      if (it < items) st_packet(p.attp + ((size_t)tt * d + (it - tt * p.H) * HD + e) / 2, pack_bf16(v0 * inv, v1 * inv), epoch);
+      const int tt = p.seq_of(it);
+      uint32_t wt = 0;
+#pragma unroll 1
+      while (sh->cleared <= seq && !expired(wt, sh)) {}
+      if (it < items) st_word(attw + ((size_t)tt * d + (it - tt * H) * HD + e) / 2, full_word(pack_bf16(v0 * inv, v1 * inv)));
     }
-    __syncthreads();               // satt is reused by the next turn or layer
+    compute_sync();                // satt is reused by the next turn or layer
   }
 }
 
-template <int MT> constexpr int lg_warps() { return MT == 1 ? 3 : 4; }
+__host__ __device__ constexpr int n_ln(int d) { return d <= 1536 ? 2 : 1; }     // buffers of LayerNorm gain and bias (wide models: the ring is no deeper than a phase)
 
-template <int MT, int HD>
-__global__ void __launch_bounds__(32 << lg_warps<MT>(), 1) decode_layers_k(const __grid_constant__ DecodeParams p) {
-  constexpr int LGW = lg_warps<MT>();
-  CFG;
-  constexpr int GP = 8 * MT;
-  extern __shared__ __align__(16) uint8_t smem[];
-  const uint32_t wbuf = smem_u32(smem);
-  bf16* xs = reinterpret_cast<bf16*>(smem + (C_::DB ? 2 : 1) * WBUF);
-  bf16* sln = xs + (size_t)GP * (p.d + PAD);
-  float* red = reinterpret_cast<float*>(sln + 2 * p.d);
-  float* satt = red + (MT == 4 ? 1 : 2) * WARPS * GP * 16;
-  Shared* sh = reinterpret_cast<Shared*>(satt + WARPS * ATT_PITCH);
-  if (threadIdx.x == 0) sh->abort_flag = 0;
-  if (threadIdx.x < 3 * 6 && (int)threadIdx.x / 6 < p.L)
-    reinterpret_cast<uint4*>(sh->lw)[threadIdx.x] = __ldg(reinterpret_cast<const uint4*>(p.layers) + threadIdx.x);
-  if (p.L > 0) {                  // this warp's first attention item and the cache rows of its first keys
-    constexpr int LPK = HD / 8, KPW = 32 / LPK;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, W = 1 << p.lgw, ST = W * KPW;
-    const int item = (int)blockIdx.x * (WARPS >> p.lgw) + (warp >> p.lgw), kg = (warp & (W - 1)) * KPW + lane / LPK;
-    if (item < p.G * p.H) {
-      const int pos = p.pos[item / p.H], slot = p.slot[item / p.H];
-      if (lane == 0) { sh->item_pos[warp] = pos; sh->item_slot[warp] = slot; }
-      if (lane % LPK == 0 && slot >= 0)
-        for (int i = 0; i < keys_ahead<LGW, HD>(); i++) {
-          const int j = kg + i * ST, jb = p.block_of(j);
-          if (j < pos && jb < p.max_lb && j < p.max_ctx)
-            sh->item_row[warp][lane / LPK][i] = p.btab[(size_t)slot * p.max_lb + jb] * p.bs + (j - jb * p.bs);
-        }
-    }
+template <int MT, int HD, int LEFT>
+__global__ void __launch_bounds__(THREADS, 1) decode_layers_k(const __grid_constant__ DecodeParams p) {
+  extern __shared__ __align__(128) uint8_t smem[];
+  const int d = p.d;
+  uint8_t* at = smem + p.slots * SLOT;
+  bf16* xs = reinterpret_cast<bf16*>(at);
+  at += 16 * MT * (d + PAD);
+  uint8_t* sln = at;
+  at += n_ln(d) * 4 * d;
+  float* red = reinterpret_cast<float*>(at);
+  at += n_red(MT) * NW * LN_GROUPS * 64 * MT * 4;
+  float* satt = reinterpret_cast<float*>(at);
+  at += NW * ATT_PITCH * 4;
+  Shared* sh = reinterpret_cast<Shared*>(at);
+
+  const int warp = threadIdx.x >> 5;
+  Ring ring = {smem_u32(smem), smem_u32(sh->full), smem_u32(sh->empty), smem_u32(sh->ln_full), smem_u32(sh->ln_empty), p.slots, 0, 0u, sln, n_ln(d), 0, 0u};
+  if (threadIdx.x == 0) {
+    sh->abort_flag = 0;
+    sh->phase = sh->cleared = 0;
+    for (int s = 0; s < p.slots; s++) { mbar_init(ring.full + 8 * s, 1); mbar_init(ring.empty + 8 * s, NW); }
+    for (int s = 0; s < 2; s++) { mbar_init(ring.ln_full + 8 * s, 1); mbar_init(ring.ln_empty + 8 * s, NW); }
+    mbar_fence_init();
+  }
+  if (threadIdx.x < 8) {
+    const int k = (int)threadIdx.x >> 1, e = (int)threadIdx.x & 1;
+    const unsigned groups = (unsigned)(k == 0 ? 3 * d : k == 1 ? d : k == 2 ? 4 * d : p.V + 7) / 8;
+    sh->share[k][e] = (int)(groups * (blockIdx.x + e) / gridDim.x);
   }
   __syncthreads();
-  // epochs used before this launch: constant while it runs (only its last CTA to leave advances the word)
-  const uint32_t base = *reinterpret_cast<volatile uint32_t*>(p.ctl);
-  const int d = p.d;
-  int flip = 0;
-  // the product behind a LayerNorm of half layer hl: qkv (even), fc (odd), after the last one the head
-  auto ln_phase = [&](int hl) {
-    Lin L;
-    const int l = hl >> 1;
-    const LayerW* lw = sh->lw + (l & 3);
-    L.K = d; L.res = nullptr; L.e_res = 0;
-    if (hl == 2 * p.L) {
-      L.W = p.head_w; L.bias = nullptr; L.N = p.V; L.lgs = p.lgs_h; L.kind = PH; L.dst = nullptr;
-    } else if (hl & 1) {
-      L.W = lw->fc_w; L.bias = lw->fc_b; L.N = 4 * d; L.lgs = p.lgs_d; L.kind = PD; L.dst = p.actp;
-    } else {
-      L.W = lw->qkv_w; L.bias = lw->qkv_b; L.N = 3 * d; L.lgs = p.lgs_a; L.kind = PA; L.dst = p.qkvp;
+  // launches before this one: constant while it runs (only its last CTA to leave advances the word)
+  const uint32_t launch = *reinterpret_cast<volatile uint32_t*>(p.ctl), half = launch & 1u;
+  const size_t block = (size_t)MAX_ROWS * 5 * d;         // words of a slot
+  uint32_t* const words = p.words + half * 3 * block;
+
+  if (warp >= NW) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
+    if (warp == NW) produce(p, ring, sh);
+    else if (warp == NW + 1) empty_words<HD>(p, words, block, sh);
+    else {
+      empty_half(p, half, block);
+      if (blockIdx.x == 0 && threadIdx.x == CT + 64) p.ctl[3 + half] = (uint32_t)p.G;
     }
-    L.src = L.kind == PD ? p.midp : (hl == 0 ? nullptr : p.xp);
-    L.e_dst = base + l + 1;
-    L.e_src = L.kind == PD ? L.e_dst : base + l;
-    return L;
-  };
-  // the product that writes the residual stream in half layer hl: proj (even), fcproj (odd)
-  auto res_phase = [&](int hl) {
-    Lin L;
-    const int l = hl >> 1;
-    const LayerW* lw = sh->lw + (l & 3);
-    L.N = d;
-    L.e_src = L.e_dst = base + l + 1;
-    if (hl & 1) {
-      L.W = lw->fcproj_w; L.bias = lw->fcproj_b; L.K = 4 * d; L.lgs = p.lgs_e; L.kind = PE;
-      L.src = p.actp; L.res = p.midp; L.e_res = L.e_dst; L.dst = p.xp;
-    } else {
-      L.W = lw->proj_w; L.bias = lw->proj_b; L.K = d; L.lgs = p.lgs_c; L.kind = PC;
-      L.src = p.attp; L.res = l == 0 ? nullptr : p.xp; L.e_res = base + l; L.dst = p.midp;
-    }
-    return L;
-  };
-  const int n_half = 2 * p.L;
-  // Weights go into L2 ahead of their phase: the copies into shared memory then take an L2 trip, and the memory streams during
-  // attention and hand-offs too.  `far`: two phases ahead, for layers of up to 40 MB (L24 d1024: 489 -> 470 us a step at G = 1); larger
-  // ones one phase ahead (L12, G = 1 / 8, one against two phases: d1280 359 / 452 and 360 / 446, d1536 390 / 502 and 397 / 518,
-  // d2048 522 / 618 and 551 / 660).
-  const bool far = d <= 1280;
-  auto prefetch_next = [&](bool last, const LayerW* nw) {
-    if (!last) {
-      prefetch_units<LGW>(nw->qkv_w, 3 * d, d, (WARPS >> p.lgs_a) * 16, 8);
-      prefetch_units<LGW>(nw->proj_w, d, d, (WARPS >> p.lgs_c) * 8, 8);
-    } else if (p.head_w) prefetch_units<LGW>(p.head_w, p.V, d, (WARPS >> p.lgs_h) * 16, 2);
-  };
-  if (p.L > 0) {
-    fetch_ln<LGW>(sln, sh->lw[0].ln1_w, sh->lw[0].ln1_b, d);
-    prefetch_units<LGW>(sh->lw[0].proj_w, d, d, (WARPS >> p.lgs_c) * 8, 8);
   } else {
-    fetch_ln<LGW>(sln, p.lnf_w, p.lnf_b, d);
-  }
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 232;");
+    const int lane = threadIdx.x & 31;
+    if (p.L > 0) {                  // this warp's first attention item and the cache rows of its first keys
+      const int W = 1 << p.lgw, ST = W * 8;
+      const int item = (int)blockIdx.x * (NW >> p.lgw) + (warp >> p.lgw), kg = (warp & (W - 1)) * 8 + (lane >> 2);
+      if (item < p.G * p.H) {
+        const int pos = p.pos[item / p.H], slot = p.slot[item / p.H];
+        auto row_at = [&](int j) {
+          const int jb = p.block_of(j);
+          return p.btab[(size_t)slot * p.max_lb + jb] * p.bs + (j - jb * p.bs);
+        };
+        const bool good = pos >= 0 && slot >= 0 && pos < p.max_ctx && p.block_of(pos) < p.max_lb;
+        if (lane == 0) { sh->item_pos[warp] = pos; sh->item_slot[warp] = slot; sh->pos_row[warp] = good ? row_at(pos) : 0; }
+        const int i = lane & 3;
+        if (good && i < keys_ahead<MT, HD>() && kg + i * ST < pos) sh->item_row[warp][lane >> 2][i] = row_at(kg + i * ST);
+      }
+      __syncwarp();
+    }
+    // lane i < 12 holds the i-th pointer of this layer's record and of the next one's
+    auto record = [&](int l) { return lane < 12 && l < p.L ? __ldg(reinterpret_cast<const unsigned long long*>(p.layers + l) + lane) : 0ull; };
+    unsigned long long rec = record(0), nrec = record(1);
+    auto ptr = [&](unsigned long long r, int i) { return reinterpret_cast<const bf16*>(__shfl_sync(0xffffffffu, r, i)); };
+    int flip = 0;
+    uint32_t *cur = words, *nxt = words + block, *prv = words + 2 * block;      // slots of this layer, the next and the last
 #pragma unroll 1
-  for (int hl = 0; hl < n_half + (p.head_w ? 1 : 0); hl++) {
-    const int l = hl >> 1;
-    const LayerW* lw = sh->lw + (l & 3);
-    const LayerW* nw = sh->lw + ((l + 1) & 3);
-    const bool even = (hl & 1) == 0, last = l + 1 >= p.L;
-    {
-      const Lin L = ln_phase(hl);
-      copy_first<LGW, 2>(wbuf, L);
-      if (hl < n_half) {
-        if (even) prefetch_units<LGW>(lw->fc_w, 4 * d, d, (WARPS >> p.lgs_d) * 16, 8);
-        else if (far) prefetch_next(last, nw);
+    for (int k = 0; k < 4 * p.L + (p.head_w ? 1 : 0); k++) {
+      const int l = k >> 2, j = k & 3, d = fresh(p.d);
+      const uint32_t row = (uint32_t)MAX_ROWS * (d / 2);    // words: x at 0, mid at row, att at 2 row, qkv at 3 row, act at 6 row
+      const bool head = k == 4 * p.L, ln = (j & 1) == 0;
+      if (j == 1) attention_phase<MT, HD>(p, l, 5 * l + 1, cur + 3 * row, cur + 2 * row, satt, sh);
+      Lin L;
+      L.bias = ptr(rec, j == 0 ? 3 : j == 1 ? 5 : j == 2 ? 9 : 11);
+      L.K = j == 3 ? 4 * d : d;
+      L.N = j == 0 ? 3 * d : j == 2 ? 4 * d : d;
+      L.kind = j == 0 ? PA : j == 1 ? PC : j == 2 ? PD : PE;
+      L.seq = 5 * l + (j == 0 ? 0 : j + 1);
+      L.src = j == 0 ? (l ? prv : nullptr) : cur + (j == 1 ? 2 : j == 2 ? 1 : 6) * row;
+      L.res = j == 1 ? (l ? prv : nullptr) : j == 3 ? cur + row : nullptr;
+      L.dst = cur + (j == 0 ? 3 : j == 1 ? 1 : j == 2 ? 6 : 0) * row;
+      if (head) { L.bias = nullptr; L.N = p.V; L.kind = PH; L.dst = nullptr; }
+      product<MT, LEFT>(p, L, ln, head ? p.n_rows : p.G, j == 3 && l + 1 == p.L, xs, red, flip, ring, sh);
+      if (j == 3) {
+        uint32_t* t = prv;
+        prv = cur; cur = nxt; nxt = t;
+        rec = nrec;                    // (layer l + 2 is requested two layers ahead of its first use)
+        nrec = record(l + 2);
       }
-      linear_phase<LGW, MT, true>(p, L, hl == n_half ? p.n_rows : p.G, false, xs, sln, red, flip, sh, wbuf);
     }
-    if (hl == n_half) break;
-    if (even) {
-      // record of the layer after the next, in the place of the last one's: every warp is past the barrier of this phase, so
-      // nobody reads that any more
-      if (l > 0 && l + 2 < p.L) {
-        const int t = tid_fresh();
-        if (t < 6) cp_async16(smem_u32(reinterpret_cast<uint4*>(sh->lw + ((l + 2) & 3)) + t), reinterpret_cast<const uint4*>(p.layers + l + 2) + t);
-        cp_async_commit();
-      }
-      if (far) prefetch_units<LGW>(lw->fcproj_w, d, 4 * d, (WARPS >> p.lgs_e) * 8, 8);
-      attention_phase<LGW, HD>(p, l, base + l + 1, satt, sh);
-    }
-    const Lin L = res_phase(hl);
-    copy_first<LGW, 1>(wbuf, L);
-    const bf16 *lnw = even ? lw->ln2_w : last ? p.lnf_w : nw->ln1_w, *lnb = even ? lw->ln2_b : last ? p.lnf_b : nw->ln1_b;
-    if (!far) {
-      if (even) prefetch_units<LGW>(lw->fcproj_w, d, 4 * d, (WARPS >> p.lgs_e) * 8, 8);
-      else prefetch_next(last, nw);
-    }
-    if (lnw) fetch_ln<LGW>(sln, lnw, lnb, d);
-    linear_phase<LGW, MT, false>(p, L, p.G, last && !even, xs, sln, red, flip, sh, wbuf);
   }
-  cp_async_wait_all();
   __syncthreads();
   if (threadIdx.x == 0) {
+    if (sh->abort_flag) atomicCAS(p.err, 0, 9);
     __threadfence();
     if (atomicAdd(p.ctl + 2, 1u) == gridDim.x - 1) {
-      p.ctl[1] = 0;
       p.ctl[2] = 0;
       __threadfence();
-      *reinterpret_cast<volatile uint32_t*>(p.ctl) = base + (uint32_t)p.L + 1u;
+      *reinterpret_cast<volatile uint32_t*>(p.ctl) = launch + 1u;
     }
   }
 }
 
-constexpr int smem_bytes(int MT, int d) {
-  const int warps = MT == 1 ? 1 << lg_warps<1>() : 1 << lg_warps<2>();
-  return (MT == 1 ? 2 : 1) * (int)WBUF + 8 * MT * (d + PAD) * 2 + 4 * d + (MT == 4 ? 1 : 2) * warps * 8 * MT * 16 * 4 + warps * ATT_PITCH * 4 + (int)sizeof(Shared);
+constexpr int fixed_bytes(int MT, int d) {         // shared memory beside the ring
+  return 16 * MT * (d + PAD) + n_ln(d) * 4 * d + n_red(MT) * NW * LN_GROUPS * 64 * MT * 4 + NW * ATT_PITCH * 4 + (int)sizeof(Shared);
 }
-static_assert(smem_bytes(1, 4096) <= SMEM_LIMIT, "eight rows of every accepted width fit");
-int max_mt(int d) {             // row groups of eight whose normalised rows fit into shared memory
-  for (int mt = 4; mt > 1; mt >>= 1)
-    if (smem_bytes(mt, d) <= SMEM_LIMIT) return mt;
-  return 1;
+constexpr int ring_slots(int MT, int d) {
+  const int n = (SMEM_LIMIT - fixed_bytes(MT, d)) / SLOT;
+  return n < MAX_SLOTS ? n : MAX_SLOTS;
 }
-// Warps that share a unit of 8 `rg` columns.  Slices are whole 32-column steps and at most one sub-step wide where the warps
-// allow it; beyond that the split grows as long as the units still fit the same number of turns of the grid, so that a narrow
-// product (proj, fcproj) runs on more CTAs with less to fetch per warp.
-int pick_lgs(int N, int K, int rg, int lgw, int grid) {
-  const int units = (N + 8 * rg - 1) / (8 * rg), sub = (128 >> lgw) / rg * 32;
-  auto fits = [&](int lg) { return (K / 32) % (1 << lg) == 0; };
-  auto turns = [&](int lg) { const long per = (long)grid * ((1 << lgw) >> lg); return (units + per - 1) / per; };
-  int lg = 0;
-  while (lg < lgw && fits(lg + 1) && (K >> lg) > sub) lg++;
-  while (lg < lgw && fits(lg + 1) && turns(lg + 1) == turns(lg)) lg++;
-  return lg;
-}
+// Row groups of eight that one launch takes: by the shared memory that the normalised rows of wide models need beside a ring of at least the
+// four chunks of a turn.
+constexpr int max_mt(int d) { return d <= 1536 ? 4 : (d <= 3328 ? 2 : 1); }
+static_assert(ring_slots(4, 1024) >= 4 && ring_slots(4, 1536) >= 4 && ring_slots(2, 3328) >= 4 && ring_slots(1, 4096) >= 4, "a turn's chunks fit");
 
-template <int MT, int HD>
+template <int MT, int HD, int LEFT>
 int launch(DecodeParams& p, int grid, cudaStream_t st) {
-  const int lgw = lg_warps<MT>(), d = p.d, smem = smem_bytes(MT, d);
-  p.lgs_a = pick_lgs(3 * d, d, 2, lgw, grid); p.lgs_c = pick_lgs(d, d, 1, lgw, grid); p.lgs_d = pick_lgs(4 * d, d, 2, lgw, grid);
-  p.lgs_e = pick_lgs(d, 4 * d, 1, lgw, grid); p.lgs_h = p.head_w ? pick_lgs(p.V, d, 2, lgw, grid) : 0;
-  p.lgw = lgw;                                  // as many warps per (sequence, head) as keep all items in one turn
-  while (p.lgw > 0 && (long)p.G * p.H << p.lgw > (long)grid << lgw) p.lgw--;
-  cudaError_t e = cudaFuncSetAttribute(decode_layers_k<MT, HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  p.slots = ring_slots(MT, p.d);
+  const int smem = p.slots * SLOT + fixed_bytes(MT, p.d);
+  p.lgw = 3;                                    // as many warps per (sequence, head) as keep all items in one turn
+  while (p.lgw > 0 && (long)p.G * p.H << p.lgw > (long)grid * NW) p.lgw--;
+  cudaError_t e = cudaFuncSetAttribute(decode_layers_k<MT, HD, LEFT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) { kh_set_error("decode_layers: shared memory opt-in failed: %s", cudaGetErrorString(e)); return -1; }
   // cooperative launch: the driver guarantees that all CTAs are resident together (or refuses the launch)
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid); cfg.blockDim = dim3(32 << lgw); cfg.dynamicSmemBytes = smem; cfg.stream = st;
+  cfg.gridDim = dim3(grid); cfg.blockDim = dim3(THREADS); cfg.dynamicSmemBytes = smem; cfg.stream = st;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeCooperative;
   at[0].val.cooperative = 1;
   cfg.attrs = at; cfg.numAttrs = 1;
-  e = cudaLaunchKernelEx(&cfg, decode_layers_k<MT, HD>, p);
+  e = cudaLaunchKernelEx(&cfg, decode_layers_k<MT, HD, LEFT>, p);
   if (e != cudaSuccess) { kh_set_error("decode_layers launch failed: %s", cudaGetErrorString(e)); return -1; }
   return 0;
 }
-template <int HD>
+template <int HD, int LEFT>
 int launch_rows(DecodeParams& p, int rows, int grid, cudaStream_t st) {
-  if (rows <= 8) return launch<1, HD>(p, grid, st);
-  if (rows <= 16) return launch<2, HD>(p, grid, st);
-  return launch<4, HD>(p, grid, st);
+  if (rows <= 8) return launch<1, HD, LEFT>(p, grid, st);
+  if (rows <= 16) return launch<2, HD, LEFT>(p, grid, st);
+  return launch<4, HD, LEFT>(p, grid, st);
 }
-int launch_any(DecodeParams& p, int rows, int grid, cudaStream_t st) {
-  if (p.hd == 128) return launch_rows<128>(p, rows, grid, st);
-  if (p.hd == 64) return launch_rows<64>(p, rows, grid, st);
-  return launch_rows<32>(p, rows, grid, st);
+template <int HD>
+int launch_width(DecodeParams& p, int rows, int grid, cudaStream_t st) {
+  if (p.d % 1024 == 0) return launch_rows<HD, 4>(p, rows, grid, st);
+  if constexpr (HD < 128) {
+    if (p.d == 256) return launch_rows<HD, 1>(p, rows, grid, st);
+    if (p.d == 512) return launch_rows<HD, 2>(p, rows, grid, st);
+  }
+  return launch_rows<HD, 0>(p, rows, grid, st);
+}
+int launch_any(DecodeParams& p, int hd, int rows, int grid, cudaStream_t st) {
+  if (hd == 128) return launch_width<128>(p, rows, grid, st);
+  if (hd == 64) return launch_width<64>(p, rows, grid, st);
+  return launch_width<32>(p, rows, grid, st);
 }
 
 }  // namespace
@@ -868,13 +1109,13 @@ extern "C" int kh_decode_layers_ok(int G, int d, int H, int hd, int max_ctx) {
 // Sequences of width d that one launch holds (more run in groups, and every group reads all weights again).
 extern "C" int kh_decode_layers_rows(int d) { return 8 * max_mt(d); }
 
-// Bytes of the packet workspace (zero-initialised once, then only used by launches that follow one another).
-extern "C" long kh_decode_layers_work_bytes(int d) { return 64 + (long)MAX_ROWS * 10 * (d / 2) * 8; }
+// Bytes of the workspace of activations (zero-initialised once, then only used by launches that follow one another).
+extern "C" long kh_decode_layers_work_bytes(int d) { return CTL_BYTES + 2l * 3 * MAX_ROWS * 5 * d * 4; }
 
 // x [G, d] holds the embedded tokens on entry and the last layer's output on return.  `layers`: device
 // array of L records of twelve bf16 pointers (ln1_w, ln1_b, qkv_w, qkv_b, proj_w, proj_b, ln2_w, ln2_b,
 // fc_w, fc_b, fcproj_w, fcproj_b).  With `head_w` ([V, d]) the kernel also writes
-// logits[i, :V] = LNf(x[rows[i]]) head_w^T for i < n_rows (row pitch ld_logits).  `work`: the packet workspace,
+// logits[i, :V] = LNf(x[rows[i]]) head_w^T for i < n_rows (row pitch ld_logits).  `work`: the workspace,
 // not used by anything else in flight.  Rows whose normalised copies do not fit into shared memory together
 // run in groups, one launch after the other.  Returns 0 or -1.
 extern "C" int kh_decode_layers(void* x, const void* layers, int L, int G, int d, int H, int hd, void* kc, void* vc,
@@ -892,13 +1133,14 @@ extern "C" int kh_decode_layers(void* x, const void* layers, int L, int G, int d
   cudaDeviceGetAttribute(&grid, cudaDevAttrMultiProcessorCount, dev);      // one CTA per SM
   if (grid < 1) { kh_set_error("decode_layers: no device"); return -1; }
   DecodeParams p = {};
-  p.d = d; p.H = H; p.hd = hd; p.bs = bs; p.max_lb = max_lb; p.max_ctx = max_ctx;
+  p.d = d; p.H = H; p.bs = bs; p.max_lb = max_lb; p.max_ctx = max_ctx;
   p.layers = (const LayerW*)layers;
   p.kc = (bf16*)kc; p.vc = (bf16*)vc; p.layer_elems = (size_t)layer_elems;
   p.btab = (const int*)btab;
   p.ctl = (uint32_t*)work;
-  const size_t row2 = (size_t)d / 2 * MAX_ROWS;
-  p.xp = (uint64_t*)((uint8_t*)work + 64); p.midp = p.xp + row2; p.attp = p.midp + row2; p.qkvp = p.attp + row2; p.actp = p.qkvp + 3 * row2;
+  p.words = (uint32_t*)((uint8_t*)work + CTL_BYTES);
+  p.inv_d = 1.f / (float)d;
+  p.h_mul = (uint32_t)(((1ull << 32) + H - 1) / H);
   p.bs_mul = bs > max_ctx ? 0u : (uint32_t)(((1ull << 32) + bs - 1) / bs);
   p.scale = scale;
   p.wait_ns = KH_WAIT_LIMIT_NS;
@@ -916,14 +1158,14 @@ extern "C" int kh_decode_layers(void* x, const void* layers, int L, int G, int d
     p.G = n; p.L = L;
     p.x = (bf16*)x + (size_t)g0 * d; p.pos = (const int*)pos + g0; p.slot = (const int*)slot + g0;
     if (head_w && together) set_head(0, n_rows);
-    if (launch_any(p, head_w && together && n_rows > n ? n_rows : n, grid, st)) return -1;
+    if (launch_any(p, hd, head_w && together && n_rows > n ? n_rows : n, grid, st)) return -1;
   }
   if (head_w && !together) {
     for (int r0 = 0; r0 < n_rows; r0 += cap) {
       const int n = n_rows - r0 < cap ? n_rows - r0 : cap;
       p.G = n; p.L = 0; p.x = (bf16*)x;
       set_head(r0, n);
-      if (launch_any(p, n, grid, st)) return -1;
+      if (launch_any(p, hd, n, grid, st)) return -1;
     }
   }
   return 0;

@@ -98,9 +98,10 @@ class InferEngine:
         # Decode steps of up to ``persistent_max`` sequences run all layers and the head in one persistent kernel
         # when the shape allows it (ops.decode_layers); KHARON_PERSISTENT_DECODE=0 or persistent_decode=False keeps
         # the five-kernel chain.  The limit by width is measured (us a step, persistent / chain):
-        #   L24 d1024, context 200: G = 8 524 / 1654, 16 737 / 1887, 17 938 / 1127, 24 1082 / 1155, 32 1208 / 1206;
-        #   L24 d1280: G = 16 1349 / 2115, 17 1994 / 1298, 32 3025 / 1495 (the chain's tensor-core GEMM starts at 17 rows);
-        #   L24 d2048, context 300: G = 16 2062 / 3486, 17 3156 / 1815 (two launches), 32 4122 / 1983.
+        #   L24 d1024, context 200: G = 8 415 / 1633, 16 561 / 1886, 17 772 / 1133, 24 850 / 1155, 32 902 / 1205; context 900: G = 17 1214 /
+        #   1502, 32 1769 / 1779;
+        #   L24 d1280: G = 16 1138 / 2126, 17 1671 / 1285, 32 2068 / 1474 (the chain's tensor-core GEMM starts at 17 rows);
+        #   L24 d2048, context 300: G = 16 1532 / 3471, 17 2454 / 1760 (two launches), 32 3062 / 1981.
         if persistent_decode is None:
             persistent_decode = os.environ.get("KHARON_PERSISTENT_DECODE", "1") != "0"
         self.persistent = bool(persistent_decode and self.skinny is not None and self.tp == 1 and self.dt == torch.bfloat16
@@ -278,8 +279,8 @@ class InferEngine:
     def _one_kernel(self, ntok, nseq):
         """Whether this step runs in the persistent kernel.  Beyond 4096 positions its W warps per (sequence, head) lose to the
         chain's split-KV attention once the sequences fill the SMs (L4 d1024, us a step, persistent / chain: context 4000 of 4096
-        G = 17 568 / 597, 32 942 / 737; 8100 G = 17 944 / 791, 24 1426 / 973; 16300 G = 17 1714 / 1395, 32 3134 / 2169; 200 of
-        4096 G = 17 198 / 252, 32 245 / 258; eight heads, context 8000, G = 17 437 / 524, 32 739 / 672)."""
+        G = 17 503 / 562, 32 879 / 713; 8100 G = 16 837 / 957, 17 880 / 819, 24 1586 / 1011; 16300 G = 17 1650 / 1389, 32 3164 / 2179; 200 of
+        4096 G = 17 144 / 223, 32 170 / 234; eight heads, context 8000, G = 17 845 / 988, 32 1549 / 1388)."""
         if not (self.persistent and ntok == nseq and ntok <= self.persistent_max and ntok <= 32):
             return False
         return ntok <= 16 or ntok * self.Hl <= 148 or int(self.np_meta[self._o_pos:self._o_pos + ntok].max()) < 4096

@@ -509,3 +509,40 @@ def test_prompt_pieces_take_the_tile_kernel_where_it_earns_its_launch(H, hd, dec
         runs, rest = got
         rows = sorted([i for r, n in runs for i in range(r, r + n)] + [i for a, b in rest for i in range(a, b)])
         assert rows == list(range(len(pos))) and all(n >= 16 for _, n in runs)
+
+
+@pytest.mark.parametrize("d,heads", [(256, 8), (512, 8), (768, 6), (1024, 16), (1280, 20)])
+def test_persistent_decode_workspace_between_steps_of_other_sizes(d, heads):
+    """The activation words of a launch are emptied by the next one: steps of one engine with rising and falling numbers of sequences
+    (one to four row tiles, both halves of the workspace, the three line pitches of fc's output) give the logits of the kernel chain (bound
+    of the tests above)."""
+    cfg = Config(4, d, heads, 601, 64, 1)
+    m = GPT(cfg, "cuda", torch.bfloat16); m.init_weights_device(5); m.params.w.mul_(3.0); m.sync_bf16()
+    e = InferEngine(m, block_size=5, max_seqs=33, max_tokens=320, use_graphs=False)
+    c = InferEngine(m, block_size=5, max_seqs=33, max_tokens=320, persistent_decode=False, use_graphs=False)
+    e.persistent_max = 32
+    prompts = [[(7 * g + i) % 601 for i in range(2 + g % 7)] for g in range(32)]
+    for G in (9, 1, 32, 2, 8, 4, 17, 3):
+        got = []
+        for eng in (c, e):
+            eng.generate(prompts[:G], 2)                     # one decode step: a later one would follow the token chosen here
+            got.append(eng.logits[:G, :601].float().clone())
+        assert e._fused
+        assert ((got[0] - got[1]).norm() / got[0].norm()).item() < 3e-2, G
+    assert ops.error_word() == 0
+
+
+@pytest.mark.parametrize("G", [1, 8, 20])
+def test_persistent_decode_hands_zeros_on(G):
+    """An empty activation word is zero, so results that are zero travel as {-0.0, +0.0}: a model whose every product is zero neither
+    stalls nor differs from the kernel chain."""
+    cfg = Config(2, 512, 8, 300, 32, 1)
+    m = GPT(cfg, "cuda", torch.bfloat16); m.params.w.zero_(); m.sync_bf16()
+    for flag in (False, True):
+        e = InferEngine(m, block_size=4, max_seqs=G + 1, persistent_decode=flag, use_graphs=False)
+        e.persistent_max = 32
+        e.logits.fill_(7.0)
+        outs, _, _ = e.generate([[5 + g, 9] for g in range(G)], 3)
+        assert e._fused == flag and (e.logits[:G, :300] == 0).all() and all(o[2:] == [0, 0, 0] for o in outs)
+        assert (e.kc.float() == 0).all() and (e.vc.float() == 0).all()
+    assert ops.error_word() == 0
