@@ -619,7 +619,8 @@ def copy_blocks(kc, vc, pairs, npairs):
 def sample(logits, V, temperature, seed, step, rep, out, nseq, step_dev=None):
     """Greedy argmax (temperature <= 0) or a categorical draw from softmax(logits / T), on device.  With
     ``step_dev`` (three int32 words on the device: step number, low and high half of the seed) both are read
-    from device memory at launch time, so a captured step can be replayed with fresh random numbers."""
+    from device memory at launch time, so a captured step can be replayed with fresh random numbers.  ``out``
+    may be pinned host memory, which holds the ids once the stream has been waited for."""
     if _use_reference(logits):
         return ref.sample(logits, V, temperature, seed, step, rep, out, nseq)
     _call(_lib().kh_sample2, 1, logits.data_ptr(), logits.stride(0), V, float(temperature), int(seed), int(step),
