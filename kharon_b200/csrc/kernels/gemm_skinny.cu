@@ -30,7 +30,7 @@
 namespace {
 constexpr int TN = 128, BK = 64, UMMA_K = 16, MAX_KB = 4;      // <= 4 k-blocks per CTA: two to three CTAs fit on an SM
 constexpr int COUNTER_SLOTS = 1024;
-enum { EPI_NONE = 0, EPI_BIAS = 1, EPI_BIAS_GELU = 2, EPI_BIAS_RESID = 3 };
+enum { EPI_NONE = 0, EPI_BIAS = 1, EPI_BIAS_GELU = 2, EPI_BIAS_RESID = 3, EPI_GELU = 6 };
 
 struct SkinnyParams {
   int M, N, K;
@@ -213,9 +213,9 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     for (int m = 0; m < MP; m++) {
       if (m >= p.M) break;
       float x = v[m] + b;
-      if (p.epi == EPI_BIAS_GELU) {
+      if (p.epi == EPI_BIAS_GELU || p.epi == EPI_GELU) {
         const bf16 pre = __float2bfloat16(x);
-        p.aux[(size_t)m * p.ldaux + n] = pre;
+        if (p.epi == EPI_BIAS_GELU) p.aux[(size_t)m * p.ldaux + n] = pre;
         x = gelu_tanh(__bfloat162float(pre));
       } else if (p.epi == EPI_BIAS_RESID) {
         x += __bfloat162float(p.aux[(size_t)m * p.ldaux + n]);

@@ -83,7 +83,7 @@ class InferEngine:
         e = lambda *s: torch.empty(*s, dtype=self.dt, **z)
         self.x = [e(mt, d), e(mt, d)]
         self.xmid, self.ln, self.qkv, self.att = e(mt, d), e(mt, d), e(mt, 3 * dl), e(mt, dl)
-        self.pre, self.act = e(mt, fo), e(mt, fo)
+        self.act = e(mt, fo)
         self.last = e(ms_, d)
         self.lnf = e(ms_, d)
         self.logits = torch.zeros(ms_, model.Vp, dtype=self.dt, **z)
@@ -200,8 +200,7 @@ class InferEngine:
                                cfg.seq, append=decode, n_split=self.attn_splits, scratch=self.attn_scratch)
             # row-parallel products: one GEMM, or under TP the fused GEMM + all-reduce kernel / NCCL seam
             self._row(att, m.L(l, "proj_w"), xmid, m.L(l, "proj_b"), xs)
-            self._ln_lin(xmid, m.L(l, "ln2_w"), m.L(l, "ln2_b"), ln, m.L(l, "fc_w"), self.act[:ntok], ops.EPI_BIAS_GELU,
-                         m.L(l, "fc_b"), self.pre[:ntok])
+            self._ln_lin(xmid, m.L(l, "ln2_w"), m.L(l, "ln2_b"), ln, m.L(l, "fc_w"), self.act[:ntok], ops.EPI_GELU, m.L(l, "fc_b"))
             ys = nxt[:ntok]
             self._row(self.act[:ntok], m.L(l, "fcproj_w"), ys, m.L(l, "fcproj_b"), xmid)
             x, nxt = nxt, x

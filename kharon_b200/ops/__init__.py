@@ -16,7 +16,7 @@ import torch
 from .. import _native
 from . import reference as ref
 
-EPI_NONE, EPI_BIAS, EPI_BIAS_GELU, EPI_BIAS_RESID, EPI_DGELU, EPI_RESID = range(6)
+EPI_NONE, EPI_BIAS, EPI_BIAS_GELU, EPI_BIAS_RESID, EPI_DGELU, EPI_RESID, EPI_GELU = range(7)
 
 #: number of native kernel launches issued through this module (bench.py reports it)
 launch_count = 0
@@ -167,7 +167,8 @@ def gemm(a, b, out, *, a_mn=False, b_mn=False, accumulate=False, epi=EPI_NONE, b
 
     ``a`` is [M,K] (or [K,M] when ``a_mn``), ``b`` is [N,K] (or [K,N] when ``b_mn``); both
     bf16, row-major, last dim contiguous.  ``out`` is bf16 or fp32 (``accumulate`` only fp32).
-    Epilogues: bias add; bias+GELU (``aux`` receives the pre-activation); bias+residual and
+    Epilogues: bias add; bias+GELU (``aux`` receives the pre-activation; ``EPI_GELU`` is the same without
+    it, for passes that have no backward); bias+residual and
     residual (``aux`` is the residual); dGELU (``out = acc * gelu'(aux)``).
     ``colsum`` (fp32 [M], needs ``a_mn``): also receives the column sums of ``a`` -- the bias gradient
     of a weight-gradient product dW = dY^T X -- added to its content when ``accumulate``, formed from
@@ -242,7 +243,7 @@ def gemm_skinny_scratch_elems(M, N, K):
 def gemm_skinny(x, w, out, scratch, *, epi=EPI_NONE, bias=None, aux=None, ln_w=None, ln_b=None, weights_static=False):
     """out[M,N] = x[M,K] @ w[N,K]^T (+ epilogue) for M <= 64: the weight-streaming split-K kernel used
     by decode steps.  ``scratch`` (gemm_skinny_scratch_elems fp32, zeroed once) holds ticket counters
-    and split-K partials.  Epilogues: EPI_NONE, EPI_BIAS, EPI_BIAS_GELU (aux = pre-activation out),
+    and split-K partials.  Epilogues: EPI_NONE, EPI_BIAS, EPI_BIAS_GELU (aux = pre-activation out), EPI_GELU,
     EPI_BIAS_RESID (aux = residual in).  With ``ln_w``/``ln_b`` (M <= SKINNY_BEST_ROWS) the product is
     taken of LayerNorm(x) * ln_w + ln_b, normalised inside the kernel.  ``weights_static``: the kernel
     launched just before this one on the stream does not write ``w`` (always true inside a decode step);

@@ -11,7 +11,7 @@ import math
 import torch
 import torch.nn.functional as F
 
-EPI_NONE, EPI_BIAS, EPI_BIAS_GELU, EPI_BIAS_RESID, EPI_DGELU, EPI_RESID = range(6)
+EPI_NONE, EPI_BIAS, EPI_BIAS_GELU, EPI_BIAS_RESID, EPI_DGELU, EPI_RESID, EPI_GELU = range(7)
 
 _K = 0.79788456
 _C = 0.044715
@@ -42,11 +42,13 @@ def gemm(a, b, out, a_mn, b_mn, accumulate, epi, bias, aux, alpha):
     A = a.float().t() if a_mn else a.float()
     Bm = b.float() if b_mn else b.float().t()
     acc = _mm(A, Bm) * alpha
-    if epi in (EPI_BIAS, EPI_BIAS_GELU, EPI_BIAS_RESID):
+    if epi in (EPI_BIAS, EPI_BIAS_GELU, EPI_BIAS_RESID, EPI_GELU):
         acc = acc + bias.float()
     if epi == EPI_BIAS_GELU:
         aux.copy_(acc)
         acc = gelu(aux.float())
+    elif epi == EPI_GELU:
+        acc = gelu(acc.to(out.dtype).float())
     elif epi in (EPI_BIAS_RESID, EPI_RESID):
         acc = acc + aux.float()
     elif epi == EPI_DGELU:

@@ -676,3 +676,21 @@ def test_embedding_gradient_of_an_id_with_many_later_rows(later):
         dwte = torch.zeros(3, 514, device="cuda")
         ops.embed_bwd(tok.int().cuda(), dx.cuda(), dwte, None, 1, rows)
         assert torch.equal(dwte.cpu(), want), rows
+
+
+@pytest.mark.parametrize("M,N,K,blk", [(1, 328, 64, 0), (9, 4096, 1024, 0), (130, 1000, 72, 64), (300, 520, 2048, 0), (257, 768, 512, 128), (2200, 4096, 1024, 512),
+                                       (700, 1016, 256, 4096 * 2 + 64)])
+def test_gemm_gelu_without_the_pre_activation(M, N, K, blk):
+    """Bias + GELU without its pre-activation gives the same bits as with it: every kernel of the family, ragged edges."""
+    torch.manual_seed(M)
+    a, b, bias, aux = _rand(M, K, scale=0.5), _rand(N, K, scale=0.1), _rand(N), torch.empty(M, N, device=DEV, dtype=torch.bfloat16)
+    want, out = torch.empty(M, N, device=DEV, dtype=torch.bfloat16), torch.empty(M, N, device=DEV, dtype=torch.bfloat16)
+    ops.gemm(a, b, want, epi=ops.EPI_BIAS_GELU, bias=bias, aux=aux, block_n=blk)
+    ops.gemm(a, b, out, epi=ops.EPI_GELU, bias=bias, block_n=blk)
+    assert torch.equal(out, want)
+    if M <= ops.SKINNY_MAX_ROWS:
+        scratch = torch.zeros(ops.gemm_skinny_scratch_elems(M, N, K), device=DEV)
+        ops.gemm_skinny(a, b, want, scratch, epi=ops.EPI_BIAS_GELU, bias=bias, aux=aux)
+        ops.gemm_skinny(a, b, out, scratch, epi=ops.EPI_GELU, bias=bias)
+        assert torch.equal(out, want)
+    assert ops.error_word() == 0
