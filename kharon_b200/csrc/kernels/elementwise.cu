@@ -437,14 +437,155 @@ extern "C" int kh_layernorm_fwd(const void* x, const void* w, const void* b, voi
   return 0;
 }
 
-// Backward, two kernels.
-//  (1) dx = rstd * (g - mean(g) - xhat * mean(g * xhat)), g = dy * w, optionally + dres (the
-//      residual-stream gradient that bypasses the norm): one warp per row, the second sweep
-//      over the row hits L1.
-//  (2) dw[j] += sum_r dy * xhat, db[j] += sum_r dy: column-oriented like colsum -- CTA (64
-//      columns, row split) accumulates in registers with 16-byte loads and writes one partial
-//      row per split to `partials` ([splits, 2, d] fp32, caller-supplied scratch); a last
-//      kernel adds the splits in index order into the fp32 gradient buffers.
+// Backward: dx = rstd * (g - mean(g) - xhat * mean(g * xhat)), g = dy * w, optionally + dres (the residual-stream gradient that
+// bypasses the norm); dw[j] += sum_r dy * xhat, db[j] += sum_r dy.
+// Widths up to 4096: one pass over dy and x.  WPR warps share a row, a lane holds 16 columns of it (two 16-byte pieces), requests those of the CTA's next row
+// before it works on this one, and keeps the column sums of all rows of its CTA in registers; a CTA writes one partial
+// row of sums, and a second, small kernel adds them in index order into the fp32 gradients.  What bounds it is memory for many rows, the
+// trips to it for few.  us, this form / two kernels before, one by rows and one by columns (back to back, captured): 16384 x 2048 55.5 (0.74 of the copy
+// rate) / 78.3, 8192 x 512 10.1 / 14.5, 4096 x 256 6.4 / 9.8, 8192 x 1024 16.5 / 17.9, 4096 x 4096 33.0 / 53.4, 512 x 256 4.6 / 5.2.
+template <int WPR>
+__global__ void __launch_bounds__(WPR == 8 ? 256 : 128, WPR == 8 ? 2 : 4)
+layernorm_bwd_k(const bf16* __restrict__ dy, const bf16* __restrict__ x, const bf16* __restrict__ w, const float* __restrict__ mean,
+                const float* __restrict__ rstd, const bf16* __restrict__ dres, bf16* __restrict__ dx, float* __restrict__ partials, int rows, int d) {
+  pdl_wait();
+  pdl_launch_dependents();
+  constexpr int T = WPR == 8 ? 256 : 128, RPI = T / (32 * WPR);      // threads, rows at a time
+  __shared__ float2 s_stat[2][T / 32];
+  __shared__ float s_sum[RPI > 1 ? RPI - 1 : 1][2][WPR * 512];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, slot = warp / WPR, part = warp % WPR;
+  const int nv = d / 8;
+  int piece[2];
+  bool in[2];
+  uint4 wv[2];
+#pragma unroll
+  for (int j = 0; j < 2; j++) {
+    const int c = part * 64 + j * 32 + lane;
+    in[j] = c < nv;
+    piece[j] = in[j] ? c : 0;
+    wv[j] = __ldg(reinterpret_cast<const uint4*>(w) + piece[j]);
+  }
+  float aw[16], ab[16];
+#pragma unroll
+  for (int i = 0; i < 16; i++) aw[i] = ab[i] = 0.f;
+  uint4 gv[2], xv[2], rv[2], ng[2], nx[2], nr[2];
+  float mu = 0.f, rs = 0.f, nmu = 0.f, nrs = 0.f;
+  auto request = [&](int row) {
+#pragma unroll
+    for (int j = 0; j < 2; j++) ng[j] = nx[j] = nr[j] = make_uint4(0, 0, 0, 0);
+    if (row >= rows) return;
+    nmu = mean[row]; nrs = rstd[row];
+#pragma unroll
+    for (int j = 0; j < 2; j++)
+      if (in[j]) {
+        const size_t at = (size_t)row * nv + piece[j];
+        ng[j] = reinterpret_cast<const uint4*>(dy)[at];
+        nx[j] = reinterpret_cast<const uint4*>(x)[at];
+        if (dres) nr[j] = reinterpret_cast<const uint4*>(dres)[at];
+      }
+  };
+  int flip = 0;
+  request((int)blockIdx.x * RPI + slot);
+  for (int r0 = (int)blockIdx.x * RPI; r0 < rows; r0 += (int)gridDim.x * RPI) {      // uniform over the CTA
+    const int row = r0 + slot;
+#pragma unroll
+    for (int j = 0; j < 2; j++) { gv[j] = ng[j]; xv[j] = nx[j]; rv[j] = nr[j]; }
+    mu = nmu; rs = nrs;
+    request(row + (int)gridDim.x * RPI);
+    float s1 = 0.f, s2 = 0.f;
+#pragma unroll
+    for (int j = 0; j < 2; j++) {
+      const uint32_t* gi = &gv[j].x; const uint32_t* xi = &xv[j].x; const uint32_t* wi = &wv[j].x;
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        const float2 g = unpack_bf16(gi[k]), xx = unpack_bf16(xi[k]), ww = unpack_bf16(wi[k]);
+        const float g0 = g.x * ww.x, g1 = g.y * ww.y, h0 = (xx.x - mu) * rs, h1 = (xx.y - mu) * rs;
+        s1 += g0 + g1;
+        s2 += g0 * h0 + g1 * h1;
+        aw[8 * j + 2 * k] += g.x * h0; aw[8 * j + 2 * k + 1] += g.y * h1;
+        ab[8 * j + 2 * k] += g.x; ab[8 * j + 2 * k + 1] += g.y;
+      }
+    }
+    s1 = warp_sum(s1);
+    s2 = warp_sum(s2);
+    if (WPR > 1) {
+      if (lane == 0) s_stat[flip][warp] = make_float2(s1, s2);
+      __syncthreads();
+      s1 = s2 = 0.f;
+#pragma unroll
+      for (int k = 0; k < WPR; k++) { const float2 f = s_stat[flip][slot * WPR + k]; s1 += f.x; s2 += f.y; }
+      flip ^= 1;                     // the next row's sums go to the other buffer; its barrier frees this one
+    }
+    s1 /= d;
+    s2 /= d;
+    if (row < rows)
+#pragma unroll
+      for (int j = 0; j < 2; j++) {
+        uint4 o;
+        const uint32_t* gi = &gv[j].x; const uint32_t* xi = &xv[j].x; const uint32_t* wi = &wv[j].x; const uint32_t* ri = &rv[j].x;
+        uint32_t* oi = &o.x;
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+          const float2 g = unpack_bf16(gi[k]), xx = unpack_bf16(xi[k]), ww = unpack_bf16(wi[k]), rr = unpack_bf16(ri[k]);
+          const float xh0 = (xx.x - mu) * rs, xh1 = (xx.y - mu) * rs;
+          oi[k] = pack_bf16(rs * (g.x * ww.x - s1 - xh0 * s2) + rr.x, rs * (g.y * ww.y - s1 - xh1 * s2) + rr.y);
+        }
+        if (in[j]) reinterpret_cast<uint4*>(dx)[(size_t)row * nv + piece[j]] = o;
+      }
+  }
+  // the CTA's rows side by side -> one partial row, in order of the slots
+  if (RPI > 1) {
+    if (slot > 0)
+#pragma unroll
+      for (int j = 0; j < 2; j++)
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+          s_sum[slot - 1][0][((part * 2 + j) * 8 + i) * 32 + lane] = aw[8 * j + i];
+          s_sum[slot - 1][1][((part * 2 + j) * 8 + i) * 32 + lane] = ab[8 * j + i];
+        }
+    __syncthreads();
+  }
+  if (slot == 0)
+#pragma unroll
+    for (int j = 0; j < 2; j++)
+      if (in[j]) {
+        float* pw = partials + (size_t)blockIdx.x * 2 * d + piece[j] * 8;
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+          float* a = (h ? ab : aw) + 8 * j;
+#pragma unroll
+          for (int k = 0; k < RPI - 1; k++)
+#pragma unroll
+            for (int i = 0; i < 8; i++) a[i] += s_sum[k][h][((part * 2 + j) * 8 + i) * 32 + lane];
+#pragma unroll
+          for (int i = 0; i < 8; i += 4) *reinterpret_cast<float4*>(pw + (size_t)h * d + i) = make_float4(a[i], a[i + 1], a[i + 2], a[i + 3]);
+        }
+      }
+}
+// dw, db += the partial rows in order: a CTA takes 32 columns of the 2 d, its 32 warps every 32nd row
+__global__ void __launch_bounds__(1024)
+layernorm_bwd_sum_k(const float* __restrict__ partials, float* __restrict__ dw, float* __restrict__ db, int parts, int d) {
+  pdl_wait();
+  pdl_launch_dependents();
+  __shared__ float s[32][33];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c = blockIdx.x * 32 + lane;
+  float v = 0.f;
+  if (c < 2 * d)
+#pragma unroll 8
+    for (int k = warp; k < parts; k += 32) v += __ldcg(partials + (size_t)k * 2 * d + c);
+  s[warp][lane] = v;
+  __syncthreads();
+  if (warp == 0 && c < 2 * d) {
+    float* dst = c < d ? dw + c : db + c - d;
+    float t = 0.f;
+#pragma unroll
+    for (int k = 0; k < 32; k++) t += s[k][lane];
+    *dst += t;
+  }
+}
+// Wider rows, two kernels: dx with a warp per row, the second sweep over the row hits L1; dw and db column-oriented like colsum -- CTA (64
+// columns, row split) accumulates in registers with 16-byte loads and writes one partial row per split to `partials`; the
+// last CTA of a column block adds the splits in index order.
 __global__ void layernorm_bwd_dx_k(const bf16* __restrict__ dy, const bf16* __restrict__ x, const bf16* __restrict__ w,
                                    const float* __restrict__ mean, const float* __restrict__ rstd,
                                    const bf16* __restrict__ dres, bf16* __restrict__ dx, int rows, int d) {
@@ -486,60 +627,6 @@ __global__ void layernorm_bwd_dx_k(const bf16* __restrict__ dy, const bf16* __re
       oi[k] = pack_bf16(rs * (g.x * ww.x - s1 - xh0 * s2) + rr.x, rs * (g.y * ww.y - s1 - xh1 * s2) + rr.y);
     }
     op[i] = o;
-  }
-}
-template <int NPL>
-__global__ void __launch_bounds__(256)
-layernorm_bwd_dx_reg_k(const bf16* __restrict__ dy, const bf16* __restrict__ x, const bf16* __restrict__ w,
-                       const float* __restrict__ mean, const float* __restrict__ rstd,
-                       const bf16* __restrict__ dres, bf16* __restrict__ dx, int rows) {
-  pdl_wait();
-  pdl_launch_dependents();
-  constexpr int d = NPL * 256;
-  const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  const int lane = threadIdx.x & 31;
-  if (row >= rows) return;
-  const uint4* dyp = reinterpret_cast<const uint4*>(dy + (size_t)row * d);
-  const uint4* xp = reinterpret_cast<const uint4*>(x + (size_t)row * d);
-  const uint4* wp = reinterpret_cast<const uint4*>(w);
-  const uint4* rp = dres ? reinterpret_cast<const uint4*>(dres + (size_t)row * d) : nullptr;
-  const float mu = mean[row], rs = rstd[row];
-  uint4 gv[NPL], xv[NPL], rv[NPL];
-#pragma unroll
-  for (int j = 0; j < NPL; j++) {
-    gv[j] = dyp[lane + 32 * j];
-    xv[j] = xp[lane + 32 * j];
-    rv[j] = rp ? rp[lane + 32 * j] : make_uint4(0, 0, 0, 0);
-  }
-  float s1 = 0.f, s2 = 0.f;
-#pragma unroll
-  for (int j = 0; j < NPL; j++) {
-    const uint4 wv = __ldg(wp + lane + 32 * j);
-    const uint32_t* gi = &gv[j].x; const uint32_t* xi = &xv[j].x; const uint32_t* wi = &wv.x;
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-      float2 g = unpack_bf16(gi[k]), xx = unpack_bf16(xi[k]), ww = unpack_bf16(wi[k]);
-      float g0 = g.x * ww.x, g1 = g.y * ww.y;
-      s1 += g0 + g1;
-      s2 += g0 * ((xx.x - mu) * rs) + g1 * ((xx.y - mu) * rs);
-    }
-  }
-  s1 = warp_sum(s1) / d;
-  s2 = warp_sum(s2) / d;
-  uint4* op = reinterpret_cast<uint4*>(dx + (size_t)row * d);
-#pragma unroll
-  for (int j = 0; j < NPL; j++) {
-    const uint4 wv = __ldg(wp + lane + 32 * j);
-    uint4 o;
-    const uint32_t* gi = &gv[j].x; const uint32_t* xi = &xv[j].x; const uint32_t* wi = &wv.x; const uint32_t* ri = &rv[j].x;
-    uint32_t* oi = &o.x;
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-      float2 g = unpack_bf16(gi[k]), xx = unpack_bf16(xi[k]), ww = unpack_bf16(wi[k]), rr = unpack_bf16(ri[k]);
-      float xh0 = (xx.x - mu) * rs, xh1 = (xx.y - mu) * rs;
-      oi[k] = pack_bf16(rs * (g.x * ww.x - s1 - xh0 * s2) + rr.x, rs * (g.y * ww.y - s1 - xh1 * s2) + rr.y);
-    }
-    op[lane + 32 * j] = o;
   }
 }
 __global__ void layernorm_bwd_dwdb_k(const bf16* __restrict__ dy, const bf16* __restrict__ x,
@@ -595,8 +682,24 @@ __global__ void layernorm_bwd_dwdb_k(const bf16* __restrict__ dy, const bf16* __
   }
   if (threadIdx.x == 0) counters[blockIdx.x] = 0;
 }
-// Number of row splits layernorm_bwd uses; its scratch is KH_COUNTER_SLOTS + splits * 2 * d floats, zeroed once.
+static int ln_bwd_sms() {
+  static int n = 0;
+  if (!n) {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n < 1) n = 148;
+  }
+  return n;
+}
+// Partial rows that layernorm_bwd uses; its scratch is KH_COUNTER_SLOTS + parts * 2 * d floats, zeroed once.  Up to width 4096: one per CTA.  Up to 256
+// CTAs take two rows of a slot each, beyond four and more, up to what is resident (us with two / four / eight rows: 512 x 1024 5.4 / 6.6 /
+// 9.2, 2048 x 512 6.2 / 7.2 / 9.0, 4096 x 256 8.5 / 7.2 / 8.3, 2048 x 2048 12.3 / 12.0 / 13.2).
 extern "C" int kh_layernorm_bwd_parts(int rows, int d) {
+  if (d <= 4096) {
+    const int rpi = d <= 512 ? 4 : (d <= 1024 ? 2 : 1), most = ln_bwd_sms() * (d <= 2048 ? 4 : 2);
+    const int two = cdiv(rows, rpi * 2), four = cdiv(rows, rpi * 4), few = two < 256 ? two : 256, parts = few > four ? few : four;
+    return parts < 1 ? 1 : (parts < most ? parts : most);
+  }
   const int cb = (d + 63) / 64;
   int parts = (592 + cb - 1) / cb;
   const int by_rows = (rows + 63) / 64;
@@ -613,16 +716,22 @@ extern "C" int kh_layernorm_bwd(const void* dy, const void* x, const void* w, co
   if ((d + 63) / 64 > KH_COUNTER_SLOTS) { kh_set_error("layernorm_bwd: d=%d is too wide", d); return -1; }
   cudaStream_t st = (cudaStream_t)stream;
   const int parts = kh_layernorm_bwd_parts(rows, d);
+  if (d <= 4096) {
+    float* sums = (float*)partials + KH_COUNTER_SLOTS;
+#define KH_LN_BWD(WPR) KH_LAUNCH((layernorm_bwd_k<WPR>), parts, WPR == 8 ? 256 : 128, 0, st, (const bf16*)dy, (const bf16*)x, (const bf16*)w, \
+                                 (const float*)mean, (const float*)rstd, (const bf16*)dres, (bf16*)dx, sums, rows, d)
+    if (d <= 512) KH_LN_BWD(1);
+    else if (d <= 1024) KH_LN_BWD(2);
+    else if (d <= 2048) KH_LN_BWD(4);
+    else KH_LN_BWD(8);
+#undef KH_LN_BWD
+    KH_LAUNCH(layernorm_bwd_sum_k, cdiv(2 * d, 32), 1024, 0, st, (const float*)sums, (float*)dw, (float*)db, parts, d);
+    KH_LAUNCH_CHECK("layernorm_bwd");
+    return 0;
+  }
   const int rps = (rows + parts - 1) / parts;
-  if (d == 2048)
-    KH_LAUNCH((layernorm_bwd_dx_reg_k<8>), cdiv(rows, 8), 256, 0, st, (const bf16*)dy, (const bf16*)x, (const bf16*)w, (const float*)mean,
-                                                            (const float*)rstd, (const bf16*)dres, (bf16*)dx, rows);
-  else if (d == 1024)
-    KH_LAUNCH((layernorm_bwd_dx_reg_k<4>), cdiv(rows, 8), 256, 0, st, (const bf16*)dy, (const bf16*)x, (const bf16*)w, (const float*)mean,
-                                                            (const float*)rstd, (const bf16*)dres, (bf16*)dx, rows);
-  else
-    KH_LAUNCH(layernorm_bwd_dx_k, cdiv(rows, 8), 256, 0, st, (const bf16*)dy, (const bf16*)x, (const bf16*)w, (const float*)mean,
-                                                     (const float*)rstd, (const bf16*)dres, (bf16*)dx, rows, d);
+  KH_LAUNCH(layernorm_bwd_dx_k, cdiv(rows, 8), 256, 0, st, (const bf16*)dy, (const bf16*)x, (const bf16*)w, (const float*)mean,
+                                                   (const float*)rstd, (const bf16*)dres, (bf16*)dx, rows, d);
   dim3 grid(cdiv(d, 64), parts);
   KH_LAUNCH(layernorm_bwd_dwdb_k, grid, 256, 0, st, (const bf16*)dy, (const bf16*)x, (const float*)mean, (const float*)rstd,
                                               (int*)partials, (float*)partials + KH_COUNTER_SLOTS, (float*)dw,

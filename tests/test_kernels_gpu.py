@@ -694,3 +694,32 @@ def test_gemm_gelu_without_the_pre_activation(M, N, K, blk):
         ops.gemm_skinny(a, b, out, scratch, epi=ops.EPI_GELU, bias=bias)
         assert torch.equal(out, want)
     assert ops.error_word() == 0
+
+
+@pytest.mark.parametrize("rows,d", [(1, 8), (3, 128), (31, 264), (33, 512), (4737, 520), (1000, 1024), (5, 1032), (2400, 2040), (700, 2048), (9, 4096), (600, 3080), (70, 4104)])
+def test_layernorm_backward_against_fp64(rows, d):
+    """Ragged rows and widths on both sides of 512, 1024, 2048 and 4096 columns (one to eight warps per row, the two kernels beyond), with and
+    without the residual gradient: column sums to fp32 rounding (n additions of terms below 8: 1e-5 of their norm), dx to bf16 rounding."""
+    torch.manual_seed(rows + d)
+    x, w, dy, dres = _rand(rows, d), _rand(d), _rand(rows, d), _rand(rows, d)
+    X, G = x.double(), dy.double()
+    mean, rstd = X.mean(1).float(), (X.var(1, unbiased=False) + 1e-5).rsqrt().float()
+    xh = (X - mean.double()[:, None]) * rstd.double()[:, None]
+    g = G * w.double()
+    base = rstd.double()[:, None] * (g - g.mean(1, keepdim=True) - xh * (g * xh).mean(1, keepdim=True))
+    for res in (dres, None):
+        dx = torch.full((rows + 1, d), 7.0, device=DEV, dtype=torch.bfloat16)
+        dw, db = torch.ones(d, device=DEV), torch.full((d,), 2.0, device=DEV)
+        part = torch.zeros(ops.layernorm_bwd_scratch_elems(rows, d), device=DEV)
+        for k in (1, 2):               # the scratch is ready for another call
+            ops.layernorm_bwd(dy, x, w, mean, rstd, res, dx[:rows], dw, db, part)
+            want = base + (res.double() if res is not None else 0)
+            assert ((dx[:rows].double() - want).norm() / want.norm()).item() < 2.0 ** -8
+            for got, one, sums in ((dw, 1.0, (G * xh).sum(0)), (db, 2.0, G.sum(0))):
+                assert ((got.double() - one - k * sums).norm() / (k * sums.norm() + one)).item() < 1e-5
+        assert (dx[rows] == 7).all()
+    again = torch.ones(d, device=DEV)
+    ops.layernorm_bwd(dy, x, w, mean, rstd, dres, dx[:rows], again, db, part)
+    once = torch.ones(d, device=DEV)
+    ops.layernorm_bwd(dy, x, w, mean, rstd, dres, dx[:rows], once, db, part)
+    assert torch.equal(again, once) and ops.error_word() == 0
