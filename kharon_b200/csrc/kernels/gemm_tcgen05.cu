@@ -646,8 +646,11 @@ gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ C
 // partial tile in its own shared memory (the operand stages are free by then), and after a cluster barrier every CTA adds
 // its 128 / split rows over the CTAs in rank order through distributed shared memory and runs the epilogue on them.  No
 // workspace and no atomics; the order of the additions is fixed, so results are reproducible.
-// Measured (dW with column sums, K = 9216): 512 x 512 62.2 -> 21.1 us, 1536 x 512 63.6 -> 37.3, 256 x 512 62.1 -> 14.9;
-// K = 4096: 1024 x 256 30.2 -> 15.6; forward 128 x 1024 x 4096: 27.9 -> 13.8.
+// PAIR: the 2, 3 or 4 members of the cluster are CTA pairs with a 256 x 256 tile (cta_group::2).  A k-block takes a pair as long as a
+// CTA with its 128 x 128 tile (0.36 and 0.34 us, bound by the operands' way from L2) and covers four times the output.
+// Measured (dW with column sums, one CTA per tile / CTAs share K / pairs share K, us, K = 9216): 512 x 512 49.1 / 18.2 / 20.2, 1536 x 512 49.7 / 30.9 / 21.8, 2048 x
+// 512 50.2 / 31.6 / 27.3; K = 8192: 1024 x 1024 44.8 / 28.6 / 25.0; K = 4096: 1024 x 256 30.2 / 15.6, 2048 x 1024 26.7 / - / 21.8, 1536 x 512 25.0 / 18.1 /
+// 15.0; forward 128 x 1024 x 4096: 27.9 / 13.8.
 __device__ __forceinline__ float4 ld_cluster_v4(uint32_t a) {
   float4 v;
   asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a));
@@ -699,14 +702,16 @@ __device__ __forceinline__ void epilogue4(const GemmParams& p, int row, int col,
   }
 }
 
-template <int BN>
+template <int BN, bool PAIR>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_splitk_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b, const GemmParams p,
                    int split) {
-  using Cfg = GemmCfg<BN>;
+  using Cfg = GemmCfg<BN, PAIR>;
   constexpr int PITCH = BN + 4;                      // floats per row of the partial tile: conflict-free 16-byte rows
   static_assert((BM * PITCH + BM) * 4 <= Cfg::STAGES * Cfg::STAGE_BYTES, "the partial tile reuses the operand stages");
-  const uint32_t rank = cluster_ctarank();
+  const uint32_t ctarank = cluster_ctarank(), rank = PAIR ? ctarank >> 1 : ctarank;      // slice of K
+  const uint32_t crank = PAIR ? ctarank & 1u : 0u, leader = ctarank & ~1u;                // half of the pair's tile
+  constexpr int TM = PAIR ? 2 * BM : BM;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* smem_al = smem_raw + (smem_base - smem_u32(smem_raw));
@@ -717,8 +722,8 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_const
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   const bool csum = p.colsum != nullptr;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int tiles_m = (p.M + BM - 1) / BM, tile = (int)blockIdx.x / split;
-  const int m0 = (tile % tiles_m) * BM, tn = tile / tiles_m, n0 = tn * BN;
+  const int tiles_m = (p.M + TM - 1) / TM, tile = (int)blockIdx.x / (PAIR ? 2 * split : split);
+  const int m0 = (tile % tiles_m) * TM + (int)crank * BM, tn = tile / tiles_m, n0 = tn * BN, nb0 = n0 + (int)crank * Cfg::BN_CTA;
   const int num_kb = (p.K + BK - 1) / BK, per = (num_kb + split - 1) / split;
   const int kb0 = min(num_kb, (int)rank * per), nkb = min(num_kb, kb0 + per) - kb0;       // the launcher leaves no slice empty
 
@@ -730,9 +735,13 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_const
     tma_prefetch_desc(&tma_a);
     tma_prefetch_desc(&tma_b);
   }
-  if (warp == 1) { tmem_alloc(smem_u32(tmem_slot), BN); tmem_relinquish(); }
+  if (warp == 1) {
+    if (PAIR) { tmem_alloc_pair(smem_u32(tmem_slot), BN); tmem_relinquish_pair(); }
+    else { tmem_alloc(smem_u32(tmem_slot), BN); tmem_relinquish(); }
+  }
   tc_fence_before();
   __syncthreads();
+  if (PAIR) cluster_sync_all();      // the barriers of the pair are initialised before anyone signals them
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
   pdl_wait();
@@ -750,18 +759,31 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_const
         if (!mbar_wait(bar_empty + 8 * s, ph ^ 1, abort_flag, 2, p.err)) break;
         if (csum && !mbar_wait(bar_free + 8 * s, ph ^ 1, abort_flag, 2, p.err)) break;
         const uint32_t sa = smem_base + s * Cfg::STAGE_BYTES, sb = sa + Cfg::A_BYTES;
-        mbar_expect_tx(bar_full + 8 * s, Cfg::STAGE_BYTES);
-        if (!p.a_mn) tma_load_2d(sa, &tma_a, bar_full + 8 * s, kb * BK, m0);
-        else
-          for (int j = 0; j < BM / 64; j++) tma_load_2d(sa + j * (BK * 128), &tma_a, bar_full + 8 * s, m0 + j * 64, kb * BK);
-        if (!p.b_mn) tma_load_2d(sb, &tma_b, bar_full + 8 * s, kb * BK, n0);
-        else
-          for (int j = 0; j < BN / 64; j++) tma_load_2d(sb + j * (BK * 128), &tma_b, bar_full + 8 * s, n0 + j * 64, kb * BK);
+        if (PAIR) {
+          // both CTAs credit the leader's barrier; the leader expects the bytes of the pair
+          const uint32_t lbar = mapa_shared(bar_full + 8 * s, leader);
+          if (crank == 0) mbar_expect_tx(bar_full + 8 * s, 2 * Cfg::STAGE_BYTES);
+          if (!p.a_mn) tma_load_2d_pair(sa, &tma_a, lbar, kb * BK, m0);
+          else
+            for (int j = 0; j < BM / 64; j++) tma_load_2d_pair(sa + j * (BK * 128), &tma_a, lbar, m0 + j * 64, kb * BK);
+          if (!p.b_mn) tma_load_2d_pair(sb, &tma_b, lbar, kb * BK, nb0);
+          else
+            for (int j = 0; j < Cfg::BN_CTA / 64; j++) tma_load_2d_pair(sb + j * (BK * 128), &tma_b, lbar, nb0 + j * 64, kb * BK);
+        } else {
+          mbar_expect_tx(bar_full + 8 * s, Cfg::STAGE_BYTES);
+          if (!p.a_mn) tma_load_2d(sa, &tma_a, bar_full + 8 * s, kb * BK, m0);
+          else
+            for (int j = 0; j < BM / 64; j++) tma_load_2d(sa + j * (BK * 128), &tma_a, bar_full + 8 * s, m0 + j * 64, kb * BK);
+          if (!p.b_mn) tma_load_2d(sb, &tma_b, bar_full + 8 * s, kb * BK, n0);
+          else
+            for (int j = 0; j < BN / 64; j++) tma_load_2d(sb + j * (BK * 128), &tma_b, bar_full + 8 * s, n0 + j * 64, kb * BK);
+        }
       }
     }
   } else if (warp == 1) {
-    if (elect_one()) {
-      const uint32_t idesc = umma_idesc_bf16(BM, BN, p.a_mn, p.b_mn);
+    if (crank == 0 && elect_one()) {
+      const uint32_t idesc = umma_idesc_bf16(TM, BN, p.a_mn, p.b_mn);
+      const uint16_t mask = (uint16_t)(3u << leader);
       const uint32_t a_lbo = p.a_mn ? BK * 128 : 16, b_lbo = p.b_mn ? BK * 128 : 16;
       const uint32_t a_kstep = p.a_mn ? (UMMA_K * 128) >> 4 : (UMMA_K * 2) >> 4;
       const uint32_t b_kstep = p.b_mn ? (UMMA_K * 128) >> 4 : (UMMA_K * 2) >> 4;
@@ -773,10 +795,11 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_const
         const uint64_t adesc = umma_desc_sw128(sa, a_lbo, 1024), bdesc = umma_desc_sw128(sb, b_lbo, 1024);
 #pragma unroll
         for (int k = 0; k < BK / UMMA_K; k++)
-          umma_f16_ss(tmem, adesc + (uint64_t)(k * a_kstep), bdesc + (uint64_t)(k * b_kstep), idesc, (i > 0 || k > 0) ? 1u : 0u);
-        umma_commit(bar_empty + 8 * s);
+          if (PAIR) umma_f16_ss_pair(tmem, adesc + (uint64_t)(k * a_kstep), bdesc + (uint64_t)(k * b_kstep), idesc, (i > 0 || k > 0) ? 1u : 0u);
+          else umma_f16_ss(tmem, adesc + (uint64_t)(k * a_kstep), bdesc + (uint64_t)(k * b_kstep), idesc, (i > 0 || k > 0) ? 1u : 0u);
+        if (PAIR) umma_commit_pair(bar_empty + 8 * s, mask); else umma_commit(bar_empty + 8 * s);
       }
-      if (ok) umma_commit(bar_tfull);
+      if (ok) { if (PAIR) umma_commit_pair(bar_tfull, mask); else umma_commit(bar_tfull); }
     }
   } else if (csum && warp >= 6) {
     // column sums of this CTA's A tiles, see gemm_kernel
@@ -834,30 +857,33 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_const
   tc_fence_before();
   cluster_sync_all();
   bool all_ok = true;
-  for (int s = 0; s < split; s++) all_ok = all_ok && ld_cluster_u32(mapa_shared(smem_u32((const void*)abort_flag), s)) == 0;
+  for (int s = 0; s < (PAIR ? 2 * split : split); s++) all_ok = all_ok && ld_cluster_u32(mapa_shared(smem_u32((const void*)abort_flag), s)) == 0;
   if (all_ok) {
-    const int rows = BM / split;
+    const int first = (int)rank * BM / split, rows = ((int)rank + 1) * BM / split - first;
     for (int i = tid; i < rows * (BN / 4); i += blockDim.x) {
-      const int r = (int)rank * rows + i / (BN / 4), c = (i % (BN / 4)) * 4;
+      const int r = first + i / (BN / 4), c = (i % (BN / 4)) * 4;
       if (m0 + r >= p.M || n0 + c >= p.N) continue;
       const uint32_t at = tile_smem + (uint32_t)(r * PITCH + c) * 4u;
       float v[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll 4
       for (int s = 0; s < split; s++) {
-        const float4 f = ld_cluster_v4(mapa_shared(at, s));
+        const float4 f = ld_cluster_v4(mapa_shared(at, PAIR ? 2 * s + crank : s));
         v[0] += f.x; v[1] += f.y; v[2] += f.z; v[3] += f.w;
       }
       epilogue4(p, m0 + r, n0 + c, v);
     }
     if (csum && tn == 0 && tid < rows) {
-      const int r = (int)rank * rows + tid;
+      const int r = first + tid;
       float v = 0.f;
-      for (int s = 0; s < split; s++) v += __uint_as_float(ld_cluster_u32(mapa_shared(csum_smem + (uint32_t)r * 4u, s)));
+      for (int s = 0; s < split; s++) v += __uint_as_float(ld_cluster_u32(mapa_shared(csum_smem + (uint32_t)r * 4u, PAIR ? 2 * s + crank : s)));
       if (m0 + r < p.M) p.colsum[m0 + r] = p.accumulate ? p.colsum[m0 + r] + v : v;
     }
   }
   cluster_sync_all();                // no CTA leaves while another reads its partial tile
-  if (warp == 1) { tc_fence_after(); tmem_dealloc(tmem, BN); }
+  if (warp == 1) {
+    tc_fence_after();
+    if (PAIR) tmem_dealloc_pair(tmem, BN); else tmem_dealloc(tmem, BN);
+  }
 }
 
 // ------------------------------------------------------------------------------- launcher
@@ -927,39 +953,41 @@ static int launch_gemm(const CUtensorMap* ta, const CUtensorMap* tb, const GemmP
   return 0;
 }
 
-// Clusters of `split` CTAs that can be resident together (0: not available).
-template <int BN>
+// Clusters of `split` CTAs (pairs: 2 split) that can be resident together (0: not available).
+template <int BN, bool PAIR>
 static int splitk_clusters(int split) {
-  static int known[3] = {-1, -1, -1};
-  int& n = known[split == 2 ? 0 : (split == 4 ? 1 : 2)];
+  static int known[9] = {-1, -1, -1, -1, -1, -1, -1, -1, -1};
+  int& n = known[split];
   if (n >= 0) return n;
-  auto kern = gemm_splitk_kernel<BN>;
+  auto kern = gemm_splitk_kernel<BN, PAIR>;
+  const int ctas = PAIR ? 2 * split : split;
   int got = 0;
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, GemmCfg<BN>::SMEM) == cudaSuccess) {
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, GemmCfg<BN, PAIR>::SMEM) == cudaSuccess) {
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = split; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-    cfg.gridDim = dim3(split * (num_sms() / split)); cfg.blockDim = dim3(GEMM_THREADS); cfg.dynamicSmemBytes = GemmCfg<BN>::SMEM;
+    attr[0].val.clusterDim.x = ctas; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    cfg.gridDim = dim3(ctas * (num_sms() / ctas)); cfg.blockDim = dim3(GEMM_THREADS); cfg.dynamicSmemBytes = GemmCfg<BN, PAIR>::SMEM;
     cfg.attrs = attr; cfg.numAttrs = 1;
     if (cudaOccupancyMaxActiveClusters(&got, kern, &cfg) != cudaSuccess) got = 0;
   }
   cudaGetLastError();
   return n = got;
 }
-template <int BN>
+template <int BN, bool PAIR>
 static int launch_splitk(const CUtensorMap* ta, const CUtensorMap* tb, const GemmParams& p, int split, cudaStream_t st) {
-  if (splitk_clusters<BN>(split) < 1) { kh_set_error("gemm: clusters of %d CTAs are not available", split); return -1; }
+  if (splitk_clusters<BN, PAIR>(split) < 1) { kh_set_error("gemm: clusters of %d CTAs are not available", split); return -1; }
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = split; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+  const int ctas = PAIR ? 2 * split : split, tm = PAIR ? 2 * BM : BM;
+  attr[0].val.clusterDim.x = ctas; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[1].val.programmaticStreamSerializationAllowed = 1;
-  cfg.gridDim = dim3(((p.M + BM - 1) / BM) * ((p.N + BN - 1) / BN) * split);
-  cfg.blockDim = dim3(GEMM_THREADS); cfg.dynamicSmemBytes = GemmCfg<BN>::SMEM; cfg.stream = st;
+  cfg.gridDim = dim3(((p.M + tm - 1) / tm) * ((p.N + BN - 1) / BN) * ctas);
+  cfg.blockDim = dim3(GEMM_THREADS); cfg.dynamicSmemBytes = GemmCfg<BN, PAIR>::SMEM; cfg.stream = st;
   cfg.attrs = attr; cfg.numAttrs = kh_pdl_enabled() ? 2 : 1;
-  cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_splitk_kernel<BN>, *ta, *tb, p, split);
+  cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_splitk_kernel<BN, PAIR>, *ta, *tb, p, split);
   if (e != cudaSuccess) { kh_set_error("gemm split-K launch failed: %s", cudaGetErrorString(e)); return -1; }
   return 0;
 }
@@ -968,22 +996,33 @@ static int launch_splitk(const CUtensorMap* ta, const CUtensorMap* tb, const Gem
 // long as one of 16 to 18); only splits whose tiles are all resident at once are taken (a second wave of clusters costs more
 // than it saves: 1024 x 256 x 4096 in 4 x 64 12.2 us, in 8 x 64 25.7).
 static int pick_splitk(int M, int N, int num_kb, int chain, int* bn_out) {
-  constexpr int SPLIT_COST = 8;
+  constexpr int SPLIT_COST = 8, PAIR_COST = 14;
   const int tm = (M + BM - 1) / BM;
   int best = chain * 4 / 5, pick = 0;
   for (int bn = 128; bn >= 64; bn >>= 1)
     for (int split = 2; split <= 8; split <<= 1) {
       const int per = (num_kb + split - 1) / split, tiles = tm * ((N + bn - 1) / bn);
       if ((split - 1) * per >= num_kb || tiles * split > num_sms() || per + SPLIT_COST >= best) continue;
-      if (tiles > (bn == 128 ? splitk_clusters<128>(split) : splitk_clusters<64>(split))) continue;
+      if (tiles > (bn == 128 ? splitk_clusters<128, false>(split) : splitk_clusters<64, false>(split))) continue;
       best = per + SPLIT_COST; pick = split; *bn_out = bn;
+    }
+  // Pairs cover four times the output in a k-block; their launch and the sum of the larger tiles cost 6 k-blocks more (K = 9216: 1536 x 512 in 4 x 36
+  // 21.8 us against 30.9 in 2 x 72, but 512 x 512 in 4 x 36 20.2 against 18.2 in 4 x 36 single CTAs).  Clusters of eight fit 15 times at most: 2048 x
+  // 512, sixteen tiles, 27.3 in three slices, 39.1 in four.
+  const int tiles2 = ((M + 255) / 256) * ((N + 255) / 256);
+  if (M > 128 && N > 128)
+    for (int split = 2; split <= 4; split++) {
+      const int per = (num_kb + split - 1) / split;
+      if ((split - 1) * per >= num_kb || tiles2 * 2 * split > num_sms() || per + PAIR_COST >= best) continue;
+      if (tiles2 > splitk_clusters<256, true>(split)) continue;
+      best = per + PAIR_COST; pick = split; *bn_out = 512;
     }
   return pick;
 }
 
 // C[M,N] = alpha * op(A) op(B) with a fused epilogue.  lda/ldb/ldc/ldaux are row pitches in
 // elements of the row-major buffers described at the top of this file.  block_n = 0 lets the
-// launcher pick the tile width (or a split of K over a cluster; 4096 * split + width asks for one); max_ctas > 0 caps the grid (used to leave SMs to a
+// launcher pick the tile width (or a split of K over a cluster; 4096 * split + width asks for one, width 512 for pairs); max_ctas > 0 caps the grid (used to leave SMs to a
 // concurrently running communication kernel).  Returns 0 or -1 (see kh_cuda_last_error).
 //
 // kh_gemm_bf16_colsum: same product with `colsum` [M] fp32 receiving colsum[m] (+)= sum_k op(A)[m, k]
@@ -1000,8 +1039,8 @@ extern "C" int kh_gemm_bf16_colsum(const void* A, int lda, int a_mn, const void*
   if ((epi == EPI_BIAS || epi == EPI_BIAS_GELU || epi == EPI_BIAS_RESID || epi == EPI_GELU) && (!bias || ((uintptr_t)bias & 15))) { kh_set_error("gemm: bias missing or misaligned"); return -1; }
   if ((epi == EPI_BIAS_GELU || epi == EPI_BIAS_RESID || epi == EPI_DGELU || epi == EPI_RESID) && (!aux || (ldaux % 8) || ((uintptr_t)aux & 15))) { kh_set_error("gemm: aux operand missing or misaligned"); return -1; }
   int bn = block_n & 4095, split = block_n >> 12;
-  if (split && ((split != 2 && split != 4 && split != 8) || (bn != 64 && bn != 128) ||
-                (split - 1) * (((K + BK - 1) / BK + split - 1) / split) >= (K + BK - 1) / BK)) {
+  const bool known_split = bn == 512 ? split >= 2 && split <= 4 : (split == 2 || split == 4 || split == 8) && (bn == 64 || bn == 128);
+  if (split && (!known_split || (split - 1) * (((K + BK - 1) / BK + split - 1) / split) >= (K + BK - 1) / BK)) {
     kh_set_error("gemm: K split %d with tile width %d is not supported for K = %d", split, bn, K);
     return -1;
   }
@@ -1036,7 +1075,7 @@ extern "C" int kh_gemm_bf16_colsum(const void* A, int lda, int a_mn, const void*
       split = pick_splitk(M, N, num_kb, (tiles + workers - 1) / workers * num_kb, &bn);
     }
   }
-  const bool pair = (bn == 512 && !split);      // 256 x 256 tiles on CTA pairs (cta_group::2)
+  const bool pair = bn == 512;                  // 256 x 256 tiles on CTA pairs (cta_group::2)
   if (pair) bn = 256;
   if (bn != 64 && bn != 128 && bn != 256) { kh_set_error("gemm: block_n must be 64, 128, 256 or 512 (CTA pairs)"); return -1; }
   const CUtensorMap* ta = a_mn ? kh_tmap_2d_bf16(A, K, M, lda, BK, 64) : kh_tmap_2d_bf16(A, M, K, lda, BM, BK);
@@ -1049,7 +1088,8 @@ extern "C" int kh_gemm_bf16_colsum(const void* A, int lda, int a_mn, const void*
   p.colsum = (float*)colsum;
   p.err = kh_error_word_dev();
   cudaStream_t st = (cudaStream_t)stream;
-  if (split) return bn == 128 ? launch_splitk<128>(ta, tb, p, split, st) : launch_splitk<64>(ta, tb, p, split, st);
+  if (split && pair) return launch_splitk<256, true>(ta, tb, p, split, st);
+  if (split) return bn == 128 ? launch_splitk<128, false>(ta, tb, p, split, st) : launch_splitk<64, false>(ta, tb, p, split, st);
   if (pair) return launch_gemm_pair(ta, tb, p, max_ctas, st);
   if (bn == 256) return launch_gemm<256>(ta, tb, p, max_ctas, st);
   if (bn == 128) return launch_gemm<128>(ta, tb, p, max_ctas, st);

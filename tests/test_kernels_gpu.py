@@ -723,3 +723,41 @@ def test_layernorm_backward_against_fp64(rows, d):
     once = torch.ones(d, device=DEV)
     ops.layernorm_bwd(dy, x, w, mean, rstd, dres, dx[:rows], once, db, part)
     assert torch.equal(again, once) and ops.error_word() == 0
+
+
+@pytest.mark.parametrize("split", [2, 3, 4])
+@pytest.mark.parametrize("M,N,K", [(256, 256, 1024), (264, 248, 600), (8, 520, 1000), (1000, 136, 4096), (1536, 512, 900)])
+def test_gemm_split_k_on_cta_pairs(M, N, K, split):
+    """256 x 256 tiles of CTA pairs whose K is shared by two to four pairs of a cluster: edges of the tiles, a last slice that is shorter, every
+    operand order, column sums and epilogues, against fp64 and against the form without a split."""
+    torch.manual_seed(M + N + K + split)
+    if (split - 1) * -(-(-(-K // 64)) // split) >= -(-K // 64):
+        pytest.skip("a slice would be empty")
+    pad = lambda n: (n + 7) // 8 * 8
+    r = lambda *s: _rand(*s, scale=0.5)
+    blk = 4096 * split + 512
+    for a_mn, b_mn in ((1, 1), (0, 0), (0, 1), (1, 0)):
+        a, b = (r(K, pad(M))[:, :M] if a_mn else r(M, pad(K))[:, :K]), (r(K, pad(N))[:, :N] if b_mn else r(N, pad(K))[:, :K])
+        want = (a.double().t() if a_mn else a.double()) @ (b.double() if b_mn else b.double().t())
+        big = torch.full((M + 1, pad(N)), 3.0, device=DEV)
+        db = torch.ones(M, device=DEV) if a_mn else None
+        ops.gemm(a, b, big[:M, :N], a_mn=bool(a_mn), b_mn=bool(b_mn), accumulate=True, colsum=db, block_n=blk)
+        assert ((big[:M, :N].double() - 3 - want).norm() / want.norm()).item() < 1e-5
+        assert (big[M] == 3).all() and (big[:, N:] == 3).all()
+        if a_mn:
+            cs = a.double().sum(0)
+            assert ((db.double() - 1 - cs).norm() / cs.norm()).item() < 2e-4
+        again = torch.full((M, pad(N)), 3.0, device=DEV)
+        ops.gemm(a, b, again[:, :N], a_mn=bool(a_mn), b_mn=bool(b_mn), accumulate=True, colsum=db, block_n=blk)
+        assert torch.equal(again, big[:M])
+    bias, res = r(pad(N))[:N], r(M, pad(N))[:, :N]
+    a, b = r(M, pad(K))[:, :K], r(N, pad(K))[:, :K]
+    for epi in (ops.EPI_NONE, ops.EPI_BIAS, ops.EPI_BIAS_GELU, ops.EPI_BIAS_RESID, ops.EPI_DGELU, ops.EPI_RESID, ops.EPI_GELU):
+        out = {}
+        for w in (blk, 512):
+            o, aux = torch.full((M, pad(N)), 7.0, device=DEV).bfloat16(), res.clone().contiguous() if N % 8 == 0 else torch.zeros(M, pad(N), device=DEV).bfloat16()[:, :N].copy_(res)
+            ops.gemm(a, b, o[:, :N], epi=epi, bias=bias if epi in (1, 2, 3, 6) else None, aux=aux if epi in (2, 3, 4, 5) else None, block_n=w)
+            out[w] = o
+        x, y = out[blk].double(), out[512].double()
+        assert ((x - y).norm() / y.norm()).item() < 2.0 ** -8 and torch.equal(out[blk][:, N:], out[512][:, N:])
+    assert ops.error_word() == 0
