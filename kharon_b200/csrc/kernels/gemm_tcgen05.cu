@@ -252,6 +252,30 @@ struct GemmParams {
   int* err;                // library error word
 };
 
+// ---- epilogue arithmetic on pairs of columns (fp32, one instruction for both; the same rounding as one by one)
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 mk2(float a, float b) { f32x2 r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b)); return r; }
+__device__ __forceinline__ float lo2(f32x2 v) { return __uint_as_float((uint32_t)v); }
+__device__ __forceinline__ float hi2(f32x2 v) { return __uint_as_float((uint32_t)(v >> 32)); }
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) { f32x2 r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) { f32x2 r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) { f32x2 r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c)); return r; }
+__device__ __forceinline__ f32x2 un2(uint32_t w) { return mk2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u)); }      // bf16 pair
+__device__ __forceinline__ uint32_t pack2(f32x2 v) { return pack_bf16(lo2(v), hi2(v)); }
+// gelu_tanh and its derivative (common.cuh) with u = x (k + k c x^2)
+__device__ __forceinline__ f32x2 gelu_tanh2(f32x2 x) {
+  constexpr float k = 0.79788456f, c = 0.044715f;
+  const f32x2 u = mul2(x, fma2(mul2(x, x), mk2(k * c, k * c), mk2(k, k))), h = mul2(x, mk2(0.5f, 0.5f));
+  return fma2(h, mk2(tanhf(lo2(u)), tanhf(hi2(u))), h);
+}
+__device__ __forceinline__ f32x2 gelu_tanh_grad2(f32x2 x) {
+  constexpr float k = 0.79788456f, c = 0.044715f;
+  const f32x2 x2 = mul2(x, x), u = mul2(x, fma2(x2, mk2(k * c, k * c), mk2(k, k))), half = mk2(0.5f, 0.5f);
+  const f32x2 t = mk2(tanhf(lo2(u)), tanhf(hi2(u)));
+  const f32x2 s = fma2(mul2(t, mk2(-1.f, -1.f)), t, mk2(1.f, 1.f));                      // 1 - t^2
+  return fma2(mul2(x, s), fma2(x2, mk2(1.5f * k * c, 1.5f * k * c), mk2(0.5f * k, 0.5f * k)), fma2(t, half, half));
+}
+
 constexpr int BM = 128, BK = 64, UMMA_K = 16;
 constexpr int GEMM_THREADS = 320;          // TMA, MMA and eight epilogue warps (or four and four column-sum warps); 192: four epilogue warps
 
@@ -476,19 +500,19 @@ gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ C
     // 23.6 us plain, 30 with a residual, 38 with GELU and its pre-activation; cuBLAS plain 14.1).
     const uint32_t stg = smem_base + Cfg::STAGES * Cfg::STAGE_BYTES + 256 + (warp - 2) * EPI_BYTES;
     const int prow = lane >> 2, pcol = (lane & 3) * 8;          // this lane's piece: row 8 j + prow, columns pcol ..
-    auto put_row = [&](const float (&v)[32]) {                   // own row, bf16 -> staging
+    auto put_row = [&](const uint32_t (&w)[16]) {                // own row, bf16 pairs -> staging
 #pragma unroll
       for (int j = 0; j < 4; j++)
-        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(stg + lane * EPI_PITCH + j * 16), "r"(pack_bf16(v[8 * j], v[8 * j + 1])),
-                     "r"(pack_bf16(v[8 * j + 2], v[8 * j + 3])), "r"(pack_bf16(v[8 * j + 4], v[8 * j + 5])), "r"(pack_bf16(v[8 * j + 6], v[8 * j + 7])) : "memory");
+        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(stg + lane * EPI_PITCH + j * 16), "r"(w[4 * j]), "r"(w[4 * j + 1]), "r"(w[4 * j + 2]),
+                     "r"(w[4 * j + 3]) : "memory");
     };
     auto lds = [&](uint32_t a) {
       uint4 u;
       asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(u.x), "=r"(u.y), "=r"(u.z), "=r"(u.w) : "r"(a) : "memory");
       return u;
     };
-    auto store_rows = [&](bf16* base, int ld, int r0, int col, const float (&v)[32]) {      // 32 rows from r0, columns col ..
-      put_row(v);
+    auto store_rows = [&](bf16* base, int ld, int r0, int col, const uint32_t (&w)[16]) {      // 32 rows from r0, columns col ..
+      put_row(w);
       __syncwarp();
 #pragma unroll
       for (int j = 0; j < 4; j++) {
@@ -545,32 +569,34 @@ gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ C
         for (int j = 0; j < 4; j++) { cb[j] = nb[j]; cx[j] = nx[j]; }
         fetch(c0 + 32);
         tmem_ld_wait();
-        float v[32];
+        if (col + 32 <= p.N) {                 // uniform over the warp: rows past the end take part without memory accesses
+          // With K of a few hundred this arithmetic and the stores bound a tile, not its MMAs: columns in pairs, and one rounding to bf16 for the
+          // stored pre-activation and the argument of its GELU (8192 x 2048 x 512: GELU with pre-activation 31.4 us column by column, 27.4 so; times
+          // GELU' 34.3 and 28.8; without either 18.9).
+          f32x2 v[16];
+          uint32_t w[16];
 #pragma unroll
-        for (int i = 0; i < 32; i++) v[i] = __uint_as_float(r[i]) * p.alpha;
-        const bool full = (col + 32 <= p.N);
-        if (use_bias) {
-          if (full) {
+          for (int i = 0; i < 16; i++) v[i] = mk2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]));
+          if (p.alpha != 1.f) {
+#pragma unroll
+            for (int i = 0; i < 16; i++) v[i] = mul2(v[i], mk2(p.alpha, p.alpha));
+          }
+          if (use_bias) {
 #pragma unroll
             for (int j = 0; j < 4; j++) {
-              uint4 b = cb[j];
-              float2 f0 = unpack_bf16(b.x), f1 = unpack_bf16(b.y), f2 = unpack_bf16(b.z), f3 = unpack_bf16(b.w);
-              v[8 * j + 0] += f0.x; v[8 * j + 1] += f0.y; v[8 * j + 2] += f1.x; v[8 * j + 3] += f1.y;
-              v[8 * j + 4] += f2.x; v[8 * j + 5] += f2.y; v[8 * j + 6] += f3.x; v[8 * j + 7] += f3.y;
+              v[4 * j] = add2(v[4 * j], un2(cb[j].x)); v[4 * j + 1] = add2(v[4 * j + 1], un2(cb[j].y));
+              v[4 * j + 2] = add2(v[4 * j + 2], un2(cb[j].z)); v[4 * j + 3] = add2(v[4 * j + 3], un2(cb[j].w));
             }
-          } else {
-#pragma unroll
-            for (int i = 0; i < 32; i++) if (col + i < p.N) v[i] += __bfloat162float(p.bias[col + i]);
           }
-        }
-        if (full) {                            // uniform over the warp: rows past the end take part without memory accesses
           if (p.epi == EPI_BIAS_GELU || p.epi == EPI_GELU) {
-            // (without a backward pass nobody reads the pre-activation: 4200 x 4096 x 1024 57.6 us with its store, 52.6 without)
-            if (p.epi == EPI_BIAS_GELU) store_rows(p.aux, p.ldaux, row0, col, v);
             // the stored pre-activation is bf16; apply GELU to the rounded value so that the
             // backward pass (which only sees the bf16 copy) differentiates the same function
 #pragma unroll
-            for (int i = 0; i < 32; i++) v[i] = gelu_tanh(__bfloat162float(__float2bfloat16(v[i])));
+            for (int i = 0; i < 16; i++) w[i] = pack2(v[i]);
+            // (without a backward pass nobody reads the pre-activation: 4200 x 4096 x 1024 57.6 us with its store, 52.6 without)
+            if (p.epi == EPI_BIAS_GELU) store_rows(p.aux, p.ldaux, row0, col, w);
+#pragma unroll
+            for (int i = 0; i < 16; i++) v[i] = gelu_tanh2(un2(w[i]));
           } else if (use_aux) {
 #pragma unroll
             for (int j = 0; j < 4; j++)
@@ -580,30 +606,38 @@ gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ C
 #pragma unroll
             for (int j = 0; j < 4; j++) {
               const uint4 b = lds(stg + lane * EPI_PITCH + j * 16);
-              const float2 f0 = unpack_bf16(b.x), f1 = unpack_bf16(b.y), f2 = unpack_bf16(b.z), f3 = unpack_bf16(b.w);
-              const float x[8] = {f0.x, f0.y, f1.x, f1.y, f2.x, f2.y, f3.x, f3.y};
+              w[4 * j] = b.x; w[4 * j + 1] = b.y; w[4 * j + 2] = b.z; w[4 * j + 3] = b.w;
+            }
+            if (p.epi == EPI_DGELU) {
 #pragma unroll
-              for (int i = 0; i < 8; i++) v[8 * j + i] = p.epi == EPI_DGELU ? v[8 * j + i] * gelu_tanh_grad(x[i]) : v[8 * j + i] + x[i];
+              for (int i = 0; i < 16; i++) v[i] = mul2(v[i], gelu_tanh_grad2(un2(w[i])));
+            } else {
+#pragma unroll
+              for (int i = 0; i < 16; i++) v[i] = add2(v[i], un2(w[i]));
             }
             __syncwarp();
           }
-          if (!p.out_fp32) store_rows(reinterpret_cast<bf16*>(p.C), p.ldc, row0, col, v);
-          else if (row_ok) {
+          if (!p.out_fp32) {
+#pragma unroll
+            for (int i = 0; i < 16; i++) w[i] = pack2(v[i]);
+            store_rows(reinterpret_cast<bf16*>(p.C), p.ldc, row0, col, w);
+          } else if (row_ok) {
             float* cp = reinterpret_cast<float*>(p.C) + (size_t)row * p.ldc + col;
             if (p.accumulate) {
 #pragma unroll
-              for (int j = 0; j < 8; j++) red_add_v4_f32(cp + 4 * j, v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+              for (int j = 0; j < 8; j++) red_add_v4_f32(cp + 4 * j, lo2(v[2 * j]), hi2(v[2 * j]), lo2(v[2 * j + 1]), hi2(v[2 * j + 1]));
             } else {
 #pragma unroll
               for (int j = 0; j < 8; j++)
-                reinterpret_cast<float4*>(cp)[j] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+                reinterpret_cast<float4*>(cp)[j] = make_float4(lo2(v[2 * j]), hi2(v[2 * j]), lo2(v[2 * j + 1]), hi2(v[2 * j + 1]));
             }
           }
         } else if (row_ok) {                   // ragged last columns
 #pragma unroll
           for (int i = 0; i < 32; i++) {
             if (col + i >= p.N) break;
-            float x = v[i];
+            float x = __uint_as_float(r[i]) * p.alpha;
+            if (use_bias) x += __bfloat162float(p.bias[col + i]);
             if (p.epi == EPI_BIAS_GELU || p.epi == EPI_GELU) {
               const bf16 pre = __float2bfloat16(x);
               if (p.epi == EPI_BIAS_GELU) p.aux[(size_t)row * p.ldaux + col + i] = pre;
