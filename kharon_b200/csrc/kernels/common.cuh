@@ -326,6 +326,17 @@ __device__ __forceinline__ float2 unpack_bf16(uint32_t u) {
   return __bfloat1622float2(v);
 }
 
+// Pairs of fp32 values: one instruction for both, each rounded as by itself.
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 mk2(float a, float b) { f32x2 r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b)); return r; }
+__device__ __forceinline__ float lo2(f32x2 v) { return __uint_as_float((uint32_t)v); }
+__device__ __forceinline__ float hi2(f32x2 v) { return __uint_as_float((uint32_t)(v >> 32)); }
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) { f32x2 r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) { f32x2 r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) { f32x2 r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c)); return r; }
+__device__ __forceinline__ f32x2 un2(uint32_t w) { return mk2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u)); }      // bf16 pair
+__device__ __forceinline__ uint32_t pack2(f32x2 v) { return pack_bf16(lo2(v), hi2(v)); }
+
 // ---- host side -------------------------------------------------------------------------
 // Encodes a 2-D bf16 tensor map: inner extent `cols` (contiguous), outer extent `rows` with
 // a row pitch of `ld` elements; box = box_cols x box_rows, 128-byte swizzle.  Results are

@@ -151,19 +151,7 @@ __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_
 }
 __device__ __forceinline__ void compute_sync() { asm volatile("bar.sync 1, %0;" ::"n"(CT) : "memory"); }
 
-// ---- pairs of fp32 values in one instruction (same rounding as the scalar ones)
-typedef unsigned long long f2;
-__device__ __forceinline__ f2 mk2(float a, float b) {
-  f2 r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-  return r;
-}
-__device__ __forceinline__ float lo2(f2 v) { return __uint_as_float((uint32_t)v); }
-__device__ __forceinline__ float hi2(f2 v) { return __uint_as_float((uint32_t)(v >> 32)); }
-__device__ __forceinline__ f2 add2(f2 a, f2 b) { f2 r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
-__device__ __forceinline__ f2 mul2(f2 a, f2 b) { f2 r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
-__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) { f2 r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c)); return r; }
-__device__ __forceinline__ f2 un2(uint32_t w) { return mk2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u)); }
+typedef f32x2 f2;
 __device__ __forceinline__ void un8(f2* f, const uint4& v) { f[0] = un2(v.x); f[1] = un2(v.y); f[2] = un2(v.z); f[3] = un2(v.w); }
 __device__ __forceinline__ f2 sum8(const uint4& v) {
   f2 f[4];

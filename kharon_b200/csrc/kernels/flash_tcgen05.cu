@@ -55,6 +55,11 @@ __device__ __forceinline__ void load_tile(uint32_t dst, const CUtensorMap* m, ui
 #pragma unroll
   for (int s = 0; s < HD / 64; s++) tma_load_2d(dst + s * rows * 128, m, bar, col0 + s * 64, row0);
 }
+// The items of a persistent CTA, longest first: round r hands them out from the first CTA to the last, the next one from the last to the
+// first, so that the longest of a round and the longest of the next do not meet on one CTA: with two or three rounds of causal tiles the
+// slowest CTA had 1.7 times the mean (B 2 H 16 T 1777, head width 64: 38 key tiles of 22.7; forward 43.6 us and backward 135, in this order 30.5
+// and 97; B 1 H 16 T 4096: 93 and 299, 62 and 200; head width 128 T 1777: 49 and 164, 34 and 131).  In one round, or with equal items, nothing changes.
+__device__ __forceinline__ int next_item(int& round, int w) { return 2 * ++round * (int)gridDim.x - 1 - w; }
 // UMMA descriptors.  Contraction over the tile's columns (K-major): k-step kk of 16 columns starts
 // (kk >> 2) slabs + (kk & 3) * 32 bytes into the tile.  Contraction over the tile's rows (MN-major):
 // k-step kk of 16 rows starts kk * 2048 bytes in, slabs are `rows * 128` bytes apart (LBO).
@@ -174,7 +179,7 @@ flash_fwd_ws_kernel(const __grid_constant__ FwdMaps<NSEG> maps, const __grid_con
     if (live && elect_one()) {
       int ic = 0, kvc = 0;
       bool ok = true;
-      for (int w = blockIdx.x; ok && w < n_items; w += gridDim.x, ic++) {
+      for (int round = 0, w = blockIdx.x; ok && w < n_items; w = next_item(round, w), ic++) {
         int b, h, q0, n;
         const int sg = decode(w, b, h, q0, n);
         if (!mbar_wait(bar_qfree, (ic & 1) ^ 1, abort_flag, 6, p.err)) break;
@@ -201,7 +206,7 @@ flash_fwd_ws_kernel(const __grid_constant__ FwdMaps<NSEG> maps, const __grid_con
       int ic = 0, pc = 0, kvc = 0;
       bool ok = true;
       const uint64_t dQ0 = dk0(sQ), dP0 = dk0(sP);
-      for (int w = blockIdx.x; ok && w < n_items; w += gridDim.x, ic++) {
+      for (int round = 0, w = blockIdx.x; ok && w < n_items; w = next_item(round, w), ic++) {
         int b, h, q0, n;
         decode(w, b, h, q0, n);
         if (!mbar_wait(bar_qfull, ic & 1, abort_flag, 6, p.err)) break;
@@ -247,75 +252,82 @@ flash_fwd_ws_kernel(const __grid_constant__ FwdMaps<NSEG> maps, const __grid_con
     const uint32_t lane_off = (uint32_t)(warp * 32) << 16;
     const uint32_t tO = tmem + 128 + lane_off;
     const float sl2 = p.scale * LOG2E;
-    int sfc[2] = {0, 0}, odc = 0, epc = 0;
+    uint32_t sph = 0;                          // parity of each S buffer
+    int odc = 0, epc = 0;
     bool ok = true;
-    for (int w = blockIdx.x; ok && w < n_items; w += gridDim.x) {
+    for (int round = 0, w = blockIdx.x; ok && w < n_items; w = next_item(round, w)) {
       int b, h, q0, n;
       const int sg = decode(w, b, h, q0, n);
       const int qpos = q0 + row;
       float m_ref = -INFINITY, l_run = 0.f;     // reference maximum (scaled to log2 units) and normaliser
       for (int j = 0; j < n; j++) {
         const int buf = j & 1;
-        if (!mbar_wait(bar_sfull + 8 * buf, sfc[buf] & 1, abort_flag, 6, p.err)) { ok = false; break; }
-        sfc[buf]++;
+        if (!mbar_wait(bar_sfull + 8 * buf, (sph >> buf) & 1, abort_flag, 6, p.err)) { ok = false; break; }
+        sph ^= 1u << buf;
         tc_fence_after();
-        uint32_t r[64];
-        const uint32_t tS = tmem + buf * 64 + lane_off;
-        tmem_ld32(tS, r);
-        tmem_ld32(tS + 32, r + 32);
-        tmem_ld_wait();
         const int k0 = j * BKV;
-        if (k0 + BKV - 1 > q0) {               // tile touches the diagonal: mask keys after the query
-#pragma unroll
-          for (int i = 0; i < 64; i++)
-            if (k0 + i > qpos) r[i] = 0xff800000u;
-        }
-        // maximum of the raw scores over four independent chains (the scale is positive)
-        float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-#pragma unroll
-        for (int i = 0; i < 64; i += 4) {
-          mx[0] = fmaxf(mx[0], __uint_as_float(r[i])); mx[1] = fmaxf(mx[1], __uint_as_float(r[i + 1]));
-          mx[2] = fmaxf(mx[2], __uint_as_float(r[i + 2])); mx[3] = fmaxf(mx[3], __uint_as_float(r[i + 3]));
-        }
-        const float mt = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * sl2;
         bool waited = false;
-        if (j == 0) {
-          m_ref = mt;
-        } else {
-          const bool grow = mt > m_ref + 8.f;
-          if (__any_sync(0xffffffffu, grow)) {
-            // rescale O in place: PV(j-1) must have retired, PV(j) is issued only after P(j) below
-            if (!mbar_wait(bar_odone, odc & 1, abort_flag, 6, p.err)) { ok = false; break; }
-            odc++;
-            waited = true;
-            tc_fence_after();
-            const float alpha = grow ? exp2f(m_ref - mt) : 1.f;
-#pragma unroll 1
-            for (int c = 0; c < HD; c += 32) {
-              uint32_t o[32];
-              tmem_ld32(tO + c, o);
-              tmem_ld_wait();
-#pragma unroll
-              for (int i = 0; i < 32; i++) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
-              tmem_st32(tO + c, o);
-            }
-            tmem_st_wait();
-            l_run *= alpha;
-            if (grow) m_ref = mt;
-          }
-        }
-        float rs[4] = {0.f, 0.f, 0.f, 0.f};
         uint32_t pk[32];
-        const float nm = -m_ref;
+        if (k0 > qpos - lane + 31) {           // all keys come after the queries of this warp (never the first tile)
 #pragma unroll
-        for (int i = 0; i < 64; i += 4) {
-          const float p0 = exp2f(fmaf(__uint_as_float(r[i]), sl2, nm)), p1 = exp2f(fmaf(__uint_as_float(r[i + 1]), sl2, nm));
-          const float p2 = exp2f(fmaf(__uint_as_float(r[i + 2]), sl2, nm)), p3 = exp2f(fmaf(__uint_as_float(r[i + 3]), sl2, nm));
-          rs[0] += p0; rs[1] += p1; rs[2] += p2; rs[3] += p3;
-          pk[i >> 1] = pack_bf16(p0, p1);
-          pk[(i >> 1) + 1] = pack_bf16(p2, p3);
+          for (int i = 0; i < 32; i++) pk[i] = 0u;
+        } else {
+          uint32_t r[64];
+          const uint32_t tS = tmem + buf * 64 + lane_off;
+          tmem_ld32(tS, r);
+          tmem_ld32(tS + 32, r + 32);
+          tmem_ld_wait();
+          if (k0 + BKV - 1 > qpos - lane) {      // the diagonal: mask keys after the query
+#pragma unroll
+            for (int i = 0; i < 64; i++)
+              if (k0 + i > qpos) r[i] = 0xff800000u;
+          }
+          // maximum of the raw scores over four independent chains (the scale is positive)
+          float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+          for (int i = 0; i < 64; i += 4) {
+            mx[0] = fmaxf(mx[0], __uint_as_float(r[i])); mx[1] = fmaxf(mx[1], __uint_as_float(r[i + 1]));
+            mx[2] = fmaxf(mx[2], __uint_as_float(r[i + 2])); mx[3] = fmaxf(mx[3], __uint_as_float(r[i + 3]));
+          }
+          const float mt = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * sl2;
+          if (j == 0) {
+            m_ref = mt;
+          } else {
+            const bool grow = mt > m_ref + 8.f;
+            if (__any_sync(0xffffffffu, grow)) {
+              // rescale O in place: PV(j-1) must have retired, PV(j) is issued only after P(j) below
+              if (!mbar_wait(bar_odone, odc & 1, abort_flag, 6, p.err)) { ok = false; break; }
+              odc++;
+              waited = true;
+              tc_fence_after();
+              const float alpha = grow ? exp2f(m_ref - mt) : 1.f;
+#pragma unroll 1
+              for (int c = 0; c < HD; c += 32) {
+                uint32_t o[32];
+                tmem_ld32(tO + c, o);
+                tmem_ld_wait();
+#pragma unroll
+                for (int i = 0; i < 32; i++) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+                tmem_st32(tO + c, o);
+              }
+              tmem_st_wait();
+              l_run *= alpha;
+              if (grow) m_ref = mt;
+            }
+          }
+          f32x2 rs0 = 0, rs1 = 0;
+          const f32x2 sl = mk2(sl2, sl2), nm = mk2(-m_ref, -m_ref);
+#pragma unroll
+          for (int i = 0; i < 64; i += 4) {
+            const f32x2 e0 = fma2(mk2(__uint_as_float(r[i]), __uint_as_float(r[i + 1])), sl, nm);
+            const f32x2 e1 = fma2(mk2(__uint_as_float(r[i + 2]), __uint_as_float(r[i + 3])), sl, nm);
+            const f32x2 p0 = mk2(exp2f(lo2(e0)), exp2f(hi2(e0))), p1 = mk2(exp2f(lo2(e1)), exp2f(hi2(e1)));
+            rs0 = add2(rs0, p0); rs1 = add2(rs1, p1);
+            pk[i >> 1] = pack2(p0);
+            pk[(i >> 1) + 1] = pack2(p1);
+          }
+          l_run += (lo2(rs0) + hi2(rs0)) + (lo2(rs1) + hi2(rs1));
         }
-        l_run += (rs[0] + rs[1]) + (rs[2] + rs[3]);
         if (j >= 1 && !waited) {      // PV(j-1) no longer reads the P buffer
           if (!mbar_wait(bar_odone, odc & 1, abort_flag, 6, p.err)) { ok = false; break; }
           odc++;
@@ -417,7 +429,7 @@ __global__ void flash_delta_kernel(const bf16* __restrict__ o, const bf16* __res
 // whole item.  Work items are handed out longest first.
 // TWO (head width 64): S, dP and the gradients take half of the tensor memory when S and dP are held once, and two ring stages
 // half of the shared memory, so two CTAs share an SM and fill each other's gaps in the chain S -> tcgen05.ld -> exponentials ->
-// shared memory -> accumulating products.  B2 H16 T1777: dK/dV 82.5 -> 75 us, dQ 68 -> 58; B32 H8 T256: 26.8 -> 21.5 and 20.6 -> 16.7.
+// shared memory -> accumulating products.  B32 H8 T256: dK/dV 26.8 -> 21.5 us, dQ 20.6 -> 16.7.
 // Head width 128, or no more items than SMs (B32 H4 T128: 7.6 us with one CTA, 8.3 with this form): one CTA with two S / dP buffers.
 template <int HD, bool TWO>
 struct BwdWs {
@@ -497,7 +509,7 @@ flash_dkv_ws_kernel(const __grid_constant__ CUtensorMap map_kv, const __grid_con
     if (live && elect_one()) {
       int ic = 0, qc = 0;
       bool ok = true;
-      for (int w = blockIdx.x; ok && w < n_items; w += gridDim.x, ic++) {
+      for (int round = 0, w = blockIdx.x; ok && w < n_items; w = next_item(round, w), ic++) {
         int b, h, k0, n;
         decode(w, b, h, k0, n);
         if (!mbar_wait(bar_kvfree, (ic & 1) ^ 1, abort_flag, 6, p.err)) break;
@@ -521,7 +533,7 @@ flash_dkv_ws_kernel(const __grid_constant__ CUtensorMap map_kv, const __grid_con
       int ic = 0, qc = 0, rc = 0;
       bool ok = true;
       const uint64_t dK0 = dk0(sK), dV0 = dk0(sV), dP0 = dk0(sP), dDS0 = dk0(sDS);
-      for (int w = blockIdx.x; ok && w < n_items; w += gridDim.x, ic++) {
+      for (int round = 0, w = blockIdx.x; ok && w < n_items; w = next_item(round, w), ic++) {
         int b, h, k0, n;
         decode(w, b, h, k0, n);
         if (!mbar_wait(bar_kvfull, ic & 1, abort_flag, 6, p.err)) break;
@@ -574,16 +586,18 @@ flash_dkv_ws_kernel(const __grid_constant__ CUtensorMap map_kv, const __grid_con
     const int row = tid & 127, half = tid >> 7;          // this thread: key row `row`, columns [32 half, 32 half + 32) of a sub-tile
     const uint32_t lane_off = (uint32_t)((warp & 3) * 32) << 16;
     const float sl2 = p.scale * LOG2E;
-    int sfc[2] = {0, 0}, uses = 0, obs = 0, stc = 0;
+    uint32_t sph = 0;                          // parity of each S buffer
+    int uses = 0, obs = 0, stc = 0;
     bool ok = true;
-    for (int w = blockIdx.x; ok && w < n_items; w += gridDim.x) {
+    for (int round = 0, w = blockIdx.x; ok && w < n_items; w = next_item(round, w)) {
       int b, h, k0, n;
       decode(w, b, h, k0, n);
       const int kpos = k0 + row;
       const size_t stat0 = ((size_t)b * p.H + h) * p.T;
       // threads 0-63 fetch the lse of query tid of sub-tile t, threads 64-127 its delta.  The value is only
       // touched (scaled, stored) at the end of the iteration, so the load is in flight during the sub-tile.
-      const float stat_mul = tid < 64 ? LOG2E : 1.f;
+      // They are kept negated: -lse in log2 units (-inf past the end, so that P is 0 there), -delta.
+      const float stat_mul = tid < 64 ? -LOG2E : -1.f;
       auto fetch_stat = [&](int t) -> float {
         const int qp = k0 + t * BS + (tid & 63);
         if (tid >= 128 || t >= n || qp >= p.T) return tid < 64 ? INFINITY : 0.f;
@@ -597,36 +611,44 @@ flash_dkv_ws_kernel(const __grid_constant__ CUtensorMap map_kv, const __grid_con
         const int sb = t & 1, buf = t & (BUFS - 1);
         const float next_stat = fetch_stat(t + 1);
         const float* st = s_stat + sb * 128;
-        if (!mbar_wait(bar_sfull + 8 * buf, sfc[buf] & 1, abort_flag, 6, p.err)) { ok = false; break; }
-        sfc[buf]++;
+        if (!mbar_wait(bar_sfull + 8 * buf, (sph >> buf) & 1, abort_flag, 6, p.err)) { ok = false; break; }
+        sph ^= 1u << buf;
         tc_fence_after();
         const int q0s = k0 + t * BS;
-        const bool diag = k0 + BT - 1 > q0s;
         const int c = half * 32;
+        // what this warp sees of the sub-tile: 32 keys and 32 queries, all before the keys, across the diagonal or all after
+        const int ahead = kpos - lane - (q0s + c);
+        const bool none = ahead > 31, diag = ahead > -31;
+        const f32x2 sl = mk2(sl2, sl2), sc = mk2(p.scale, p.scale);
         uint32_t pp[16], ds[16];
+        if (none) {
 #pragma unroll
-        for (int w = 0; w < 32; w += CW) {
-          uint32_t rs[CW], rd[CW];
-          tmem_cols<CW>(tmem + buf * 64 + lane_off + c + w, rs);
-          tmem_cols<CW>(tmem + BUFS * 64 + buf * 64 + lane_off + c + w, rd);
-          tmem_ld_wait();
+          for (int e = 0; e < 16; e++) pp[e] = ds[e] = 0u;
+        } else {
 #pragma unroll
-          for (int e = 0; e < CW; e += 4) {
-            const int q0 = c + w + e;
-            const float4 l4 = *reinterpret_cast<const float4*>(st + q0), d4 = *reinterpret_cast<const float4*>(st + 64 + q0);
-            const float lv[4] = {l4.x, l4.y, l4.z, l4.w}, dl[4] = {d4.x, d4.y, d4.z, d4.w};
-            float pv[4], dv[4];
+          for (int w = 0; w < 32; w += CW) {
+            uint32_t rs[CW], rd[CW];
+            tmem_cols<CW>(tmem + buf * 64 + lane_off + c + w, rs);
+            tmem_cols<CW>(tmem + BUFS * 64 + buf * 64 + lane_off + c + w, rd);
+            tmem_ld_wait();
+            if (diag) {
 #pragma unroll
-            for (int u = 0; u < 4; u++) {
-              float pr = exp2f(fmaf(__uint_as_float(rs[e + u]), sl2, -lv[u]));
-              if (diag && kpos > q0s + q0 + u) pr = 0.f;
-              pv[u] = pr;
-              dv[u] = pr * (__uint_as_float(rd[e + u]) - dl[u]) * p.scale;
+              for (int e = 0; e < CW; e++)
+                if (kpos > q0s + c + w + e) rs[e] = 0xff800000u;        // -inf: P and dS are 0
             }
-            pp[(w + e) >> 1] = pack_bf16(pv[0], pv[1]);
-            pp[((w + e) >> 1) + 1] = pack_bf16(pv[2], pv[3]);
-            ds[(w + e) >> 1] = pack_bf16(dv[0], dv[1]);
-            ds[((w + e) >> 1) + 1] = pack_bf16(dv[2], dv[3]);
+#pragma unroll
+            for (int e = 0; e < CW; e += 4) {
+              const int q0 = c + w + e;
+              const ulonglong2 nl = *reinterpret_cast<const ulonglong2*>(st + q0), nd = *reinterpret_cast<const ulonglong2*>(st + 64 + q0);
+#pragma unroll
+              for (int u = 0; u < 4; u += 2) {
+                const f32x2 x = fma2(mk2(__uint_as_float(rs[e + u]), __uint_as_float(rs[e + u + 1])), sl, u ? nl.y : nl.x);
+                const f32x2 pr = mk2(exp2f(lo2(x)), exp2f(hi2(x)));
+                const f32x2 dp = add2(mk2(__uint_as_float(rd[e + u]), __uint_as_float(rd[e + u + 1])), u ? nd.y : nd.x);
+                pp[(w + e + u) >> 1] = pack2(pr);
+                ds[(w + e + u) >> 1] = pack2(mul2(mul2(pr, dp), sc));
+              }
+            }
           }
         }
         // the products that read P^T / dS^T of the previous sub-tile have retired
@@ -751,7 +773,7 @@ flash_dq_ws_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
     if (live && elect_one()) {
       int ic = 0, kvc = 0;
       bool ok = true;
-      for (int w = blockIdx.x; ok && w < n_items; w += gridDim.x, ic++) {
+      for (int round = 0, w = blockIdx.x; ok && w < n_items; w = next_item(round, w), ic++) {
         int b, h, q0, n;
         decode(w, b, h, q0, n);
         if (!mbar_wait(bar_qfree, (ic & 1) ^ 1, abort_flag, 6, p.err)) break;
@@ -775,7 +797,7 @@ flash_dq_ws_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
       int ic = 0, kvc = 0, rc = 0;
       bool ok = true;
       const uint64_t dQ0 = dk0(sQ), dDO0 = dk0(sDO), dDS0 = dk0(sDS);
-      for (int w = blockIdx.x; ok && w < n_items; w += gridDim.x, ic++) {
+      for (int round = 0, w = blockIdx.x; ok && w < n_items; w = next_item(round, w), ic++) {
         int b, h, q0, n;
         decode(w, b, h, q0, n);
         if (!mbar_wait(bar_qfull, ic & 1, abort_flag, 6, p.err)) break;
@@ -825,9 +847,10 @@ flash_dq_ws_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
     const int row = tid & 127, half = tid >> 7;
     const uint32_t lane_off = (uint32_t)((warp & 3) * 32) << 16;
     const float sl2 = p.scale * LOG2E;
-    int sfc[2] = {0, 0}, uses = 0, obs = 0, epc = 0;
+    uint32_t sph = 0;                          // parity of each S buffer
+    int uses = 0, obs = 0, epc = 0;
     bool ok = true;
-    for (int w = blockIdx.x; ok && w < n_items; w += gridDim.x) {
+    for (int round = 0, w = blockIdx.x; ok && w < n_items; w = next_item(round, w)) {
       int b, h, q0, n;
       decode(w, b, h, q0, n);
       const int qpos = q0 + row;
@@ -837,29 +860,36 @@ flash_dq_ws_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
       const float my_delta = qvalid ? p.delta[sidx] : 0.f;
       for (int j = 0; j < n; j++) {
         const int buf = j & (BUFS - 1);
-        if (!mbar_wait(bar_sfull + 8 * buf, sfc[buf] & 1, abort_flag, 6, p.err)) { ok = false; break; }
-        sfc[buf]++;
+        if (!mbar_wait(bar_sfull + 8 * buf, (sph >> buf) & 1, abort_flag, 6, p.err)) { ok = false; break; }
+        sph ^= 1u << buf;
         tc_fence_after();
         const int k0 = j * BS;
-        const bool diag = k0 + BS - 1 > q0;
         const int c = half * 32;
+        const int ahead = k0 + c - (qpos - lane);        // as in the dK / dV kernel
+        const bool none = ahead > 31, diag = ahead > -31;
+        const f32x2 sl = mk2(sl2, sl2), sc = mk2(p.scale, p.scale), nl = mk2(-my_lse, -my_lse), nd = mk2(-my_delta, -my_delta);
         uint32_t ds[16];
+        if (none) {
 #pragma unroll
-        for (int w = 0; w < 32; w += CW) {
-          uint32_t rs[CW], rd[CW];
-          tmem_cols<CW>(tmem + buf * 64 + lane_off + c + w, rs);
-          tmem_cols<CW>(tmem + BUFS * 64 + buf * 64 + lane_off + c + w, rd);
-          tmem_ld_wait();
+          for (int e = 0; e < 16; e++) ds[e] = 0u;
+        } else {
 #pragma unroll
-          for (int e = 0; e < CW; e += 2) {
-            float dv[2];
+          for (int w = 0; w < 32; w += CW) {
+            uint32_t rs[CW], rd[CW];
+            tmem_cols<CW>(tmem + buf * 64 + lane_off + c + w, rs);
+            tmem_cols<CW>(tmem + BUFS * 64 + buf * 64 + lane_off + c + w, rd);
+            tmem_ld_wait();
+            if (diag) {
 #pragma unroll
-            for (int u = 0; u < 2; u++) {
-              float pr = exp2f(fmaf(__uint_as_float(rs[e + u]), sl2, -my_lse));
-              if (diag && k0 + c + w + e + u > qpos) pr = 0.f;
-              dv[u] = pr * (__uint_as_float(rd[e + u]) - my_delta) * p.scale;
+              for (int e = 0; e < CW; e++)
+                if (k0 + c + w + e > qpos) rs[e] = 0xff800000u;         // -inf: dS is 0
             }
-            ds[(w + e) >> 1] = pack_bf16(dv[0], dv[1]);
+#pragma unroll
+            for (int e = 0; e < CW; e += 2) {
+              const f32x2 x = fma2(mk2(__uint_as_float(rs[e]), __uint_as_float(rs[e + 1])), sl, nl);
+              const f32x2 pr = mk2(exp2f(lo2(x)), exp2f(hi2(x)));
+              ds[(w + e) >> 1] = pack2(mul2(mul2(pr, add2(mk2(__uint_as_float(rd[e]), __uint_as_float(rd[e + 1])), nd)), sc));
+            }
           }
         }
         while (obs < uses) {

@@ -252,17 +252,7 @@ struct GemmParams {
   int* err;                // library error word
 };
 
-// ---- epilogue arithmetic on pairs of columns (fp32, one instruction for both; the same rounding as one by one)
-typedef unsigned long long f32x2;
-__device__ __forceinline__ f32x2 mk2(float a, float b) { f32x2 r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b)); return r; }
-__device__ __forceinline__ float lo2(f32x2 v) { return __uint_as_float((uint32_t)v); }
-__device__ __forceinline__ float hi2(f32x2 v) { return __uint_as_float((uint32_t)(v >> 32)); }
-__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) { f32x2 r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
-__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) { f32x2 r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
-__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) { f32x2 r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c)); return r; }
-__device__ __forceinline__ f32x2 un2(uint32_t w) { return mk2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u)); }      // bf16 pair
-__device__ __forceinline__ uint32_t pack2(f32x2 v) { return pack_bf16(lo2(v), hi2(v)); }
-// gelu_tanh and its derivative (common.cuh) with u = x (k + k c x^2)
+// ---- epilogue arithmetic on pairs of columns (f32x2 of common.cuh): gelu_tanh and its derivative (common.cuh) with u = x (k + k c x^2)
 __device__ __forceinline__ f32x2 gelu_tanh2(f32x2 x) {
   constexpr float k = 0.79788456f, c = 0.044715f;
   const f32x2 u = mul2(x, fma2(mul2(x, x), mk2(k * c, k * c), mk2(k, k))), h = mul2(x, mk2(0.5f, 0.5f));

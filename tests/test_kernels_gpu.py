@@ -402,6 +402,13 @@ def test_flash_backward_with_two_ctas_per_sm(B, T, H, hd):
     test_flash_fwd_bwd(B, T, H, hd)
 
 
+@pytest.mark.parametrize("B,T,H,hd", [(1, 200, 150, 64), (2, 129, 160, 64), (1, 385, 151, 64), (2, 257, 50, 128), (3, 130, 74, 128)])
+def test_flash_items_handed_out_there_and_back(B, T, H, hd):
+    """Items of unequal length in two to five rounds over the CTAs, odd rounds from the last CTA to the first, the last round with a few
+    items, one short of full and exactly full (148 CTAs, 296 where two share an SM); warps all of whose keys come after their queries."""
+    test_flash_fwd_bwd(B, T, H, hd)
+
+
 def test_flash_large_scores_rescale():
     """Scores that keep growing along the keys force the in-place rescaling of the output accumulator."""
     torch.manual_seed(21)
