@@ -313,6 +313,37 @@ def test_xent():
         assert logits[3].abs().max().item() == 0
 
 
+@pytest.mark.parametrize("R,V,ld", [(1, 1, 8), (9, 7, 8), (17, 250, 256), (8, 256, 256), (33, 257, 264), (7, 512, 520), (40, 1023, 1024), (25, 1030, 1032),
+                                    (11, 2041, 2048), (6, 2048, 2056)])
+def test_xent_short_rows(R, V, ld):
+    """A warp per row up to 2048 columns (the last shape is past the line): every number of pieces a lane, odd vocabularies, NaN in the
+    padding, masked (-inf) logits, rows without a target; loss, probability and gradient against fp64, the gradient rounded once to bf16."""
+    torch.manual_seed(R + V)
+    x = torch.full((R, ld), float("nan"), device=DEV).bfloat16()
+    x[:, :V] = _rand(R, V, scale=3.0)
+    if V > 16 and ld <= 2048:                              # (a thread of the kernel for longer rows wants a finite logit)
+        x[:, V // 2:V // 2 + 9] = float("-inf")
+    t = torch.randint(0, max(V // 2, 1), (R,), device=DEV, dtype=torch.int32)
+    if R > 5:
+        t[5], t[4] = -1, V
+    coef = torch.randn(R, device=DEV)
+    rl, pr, g = torch.empty(R, device=DEV), torch.empty(R, device=DEV), x.clone()
+    ops.xent(g, V, t, coef=coef, rowloss=rl, prob=pr, write_grad=False)
+    assert torch.equal(g.view(torch.int16), x.view(torch.int16))
+    rl2, pr2 = torch.empty_like(rl), torch.empty_like(pr)
+    ops.xent(g, V, t, coef=coef, rowloss=rl2, prob=pr2)
+    assert torch.equal(rl, rl2) and torch.equal(pr, pr2)
+    ok = (t >= 0) & (t < V)
+    p = x[:, :V].double().softmax(1)
+    pt = p.gather(1, t.clamp(0, V - 1).long()[:, None])[:, 0]
+    assert relerr(rl, torch.where(ok, -pt.log(), 0.)) < 1e-5 and relerr(pr, torch.where(ok, pt, 0.)) < 1e-5       # fp32 sums of up to 2048 terms
+    want = p.clone()
+    want[torch.arange(R, device=DEV)[ok], t[ok].long()] -= 1
+    want *= torch.where(ok, coef.double(), 0.)[:, None]
+    assert ((g[:, :V].double() - want).abs() <= want.abs() * 2 ** -8 + 1e-5 * coef.abs()[:, None]).all()
+    assert not g[:, V:].any()
+
+
 def test_adamw_matches_torch_and_emits_bf16():
     torch.manual_seed(6)
     n = 100003
