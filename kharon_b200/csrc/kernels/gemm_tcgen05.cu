@@ -685,15 +685,27 @@ __device__ __forceinline__ uint32_t ld_cluster_u32(uint32_t a) {
   asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(a));
   return v;
 }
-// Epilogue of four adjacent columns (col % 4 == 0) of one row; the arithmetic and rounding points of gemm_kernel.
-__device__ __forceinline__ void epilogue4(const GemmParams& p, int row, int col, float (&v)[4]) {
-  const int n = min(4, p.N - col);
-  const bool use_bias = (p.epi == EPI_BIAS || p.epi == EPI_BIAS_GELU || p.epi == EPI_BIAS_RESID || p.epi == EPI_GELU);
+// Epilogue of four adjacent columns (col % 4 == 0) of one row; the arithmetic and rounding points of gemm_kernel.  Its operands are read by
+// epilogue4_fetch, ahead of the sum (0 where there are none).
+struct Epi4 { uint2 bias, aux; };
+__device__ __forceinline__ uint2 load4(const bf16* a, int n) {
+  if (n >= 4) return *reinterpret_cast<const uint2*>(a);
+  uint32_t w[3] = {0u, 0u, 0u};
 #pragma unroll
-  for (int i = 0; i < 4; i++) {
-    v[i] *= p.alpha;
-    if (use_bias && i < n) v[i] += __bfloat162float(p.bias[col + i]);
-  }
+  for (int i = 0; i < 3; i++)
+    if (i < n) w[i] = *reinterpret_cast<const uint16_t*>(a + i);
+  return make_uint2(w[0] | w[1] << 16, w[2]);
+}
+__device__ __forceinline__ void epilogue4_fetch(const GemmParams& p, int row, int col, Epi4& e) {
+  const int n = p.N - col;
+  e.bias = e.aux = make_uint2(0u, 0u);
+  if (p.epi == EPI_BIAS || p.epi == EPI_BIAS_GELU || p.epi == EPI_BIAS_RESID || p.epi == EPI_GELU) e.bias = load4(p.bias + col, n);
+  if (p.epi == EPI_BIAS_RESID || p.epi == EPI_RESID || p.epi == EPI_DGELU) e.aux = load4(p.aux + (size_t)row * p.ldaux + col, n);
+}
+__device__ __forceinline__ void epilogue4(const GemmParams& p, int row, int col, float (&v)[4], const Epi4& e) {
+  const int n = min(4, p.N - col);
+  const float2 b0 = unpack_bf16(e.bias.x), b1 = unpack_bf16(e.bias.y);
+  v[0] = v[0] * p.alpha + b0.x; v[1] = v[1] * p.alpha + b0.y; v[2] = v[2] * p.alpha + b1.x; v[3] = v[3] * p.alpha + b1.y;
   if (p.epi == EPI_BIAS_GELU || p.epi == EPI_GELU) {
     if (p.epi == EPI_BIAS_GELU) {
       bf16* ap = p.aux + (size_t)row * p.ldaux + col;
@@ -703,13 +715,8 @@ __device__ __forceinline__ void epilogue4(const GemmParams& p, int row, int col,
 #pragma unroll
     for (int i = 0; i < 4; i++) v[i] = gelu_tanh(__bfloat162float(__float2bfloat16(v[i])));
   } else if (p.epi == EPI_BIAS_RESID || p.epi == EPI_RESID || p.epi == EPI_DGELU) {
-    const bf16* ap = p.aux + (size_t)row * p.ldaux + col;
-    float x[4] = {0.f, 0.f, 0.f, 0.f};
-    if (n == 4) {
-      const uint2 u = *reinterpret_cast<const uint2*>(ap);
-      const float2 a = unpack_bf16(u.x), b = unpack_bf16(u.y);
-      x[0] = a.x; x[1] = a.y; x[2] = b.x; x[3] = b.y;
-    } else for (int i = 0; i < n; i++) x[i] = __bfloat162float(ap[i]);
+    const float2 a = unpack_bf16(e.aux.x), b = unpack_bf16(e.aux.y);
+    const float x[4] = {a.x, a.y, b.x, b.y};
 #pragma unroll
     for (int i = 0; i < 4; i++) v[i] = p.epi == EPI_DGELU ? v[i] * gelu_tanh_grad(x[i]) : v[i] + x[i];
   }
@@ -861,10 +868,11 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_const
   tc_fence_after();
   __syncthreads();                   // every MMA has retired and the column-sum warps are done: the stages are free
   const uint32_t tile_smem = smem_base, csum_smem = smem_base + BM * PITCH * 4;
-  if (warp >= 2 && warp < 6) {
-    const int q = warp & 3, row = q * 32 + lane;
+  tc_fence_after();
+  if (warp >= 2) {                   // two warps to a TMEM quadrant, half of the columns each
+    const int q = warp & 3, row = q * 32 + lane, half = warp >= 6 ? BN / 2 : 0;
 #pragma unroll 1
-    for (int c = 0; c < BN; c += 32) {
+    for (int c = half; c < half + BN / 2; c += 32) {
       uint32_t r[32];
       tmem_ld32(tmem + ((uint32_t)(q * 32) << 16) + c, r);
       tmem_ld_wait();
@@ -873,33 +881,58 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_const
         asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(tile_smem + (uint32_t)(row * PITCH + c + 4 * j) * 4u),
                      "r"(r[4 * j]), "r"(r[4 * j + 1]), "r"(r[4 * j + 2]), "r"(r[4 * j + 3]) : "memory");
     }
-  } else if (csum && warp >= 6 && lane < 4) {
+  }
+  if (csum && warp >= 6 && lane < 4) {
 #pragma unroll
     for (int j = 0; j < 8; j++)
       asm volatile("st.shared.f32 [%0], %1;" ::"r"(csum_smem + (uint32_t)((warp - 6) * 32 + lane * 8 + j) * 4u), "f"(cs[j]) : "memory");
   }
   tc_fence_before();
+  // The tail is a chain of latencies: the reads of all partial tiles (and of the abort flags) go out together, the epilogue's operands before
+  // the barrier (128 x 1024 x 4096 with bias and residual 9.2 us with one read after the other and four warps leaving the tile, 8.0 so;
+  // 18 x 256 x 1024 6.3 and 5.2; dW 768 x 256 x 4096 10.1 and 9.2).
+  const int first = (int)rank * BM / split, rows = ((int)rank + 1) * BM / split - first, items = rows * (BN / 4);
+  auto place = [&](int i, int& r, int& c) {
+    r = first + i / (BN / 4); c = (i % (BN / 4)) * 4;
+    return i < items && m0 + r < p.M && n0 + c < p.N;
+  };
+  int r, c;
+  Epi4 e;
+  if (place(tid, r, c)) epilogue4_fetch(p, m0 + r, n0 + c, e);
   cluster_sync_all();
-  bool all_ok = true;
-  for (int s = 0; s < (PAIR ? 2 * split : split); s++) all_ok = all_ok && ld_cluster_u32(mapa_shared(smem_u32((const void*)abort_flag), s)) == 0;
+  const uint32_t bad = lane < (PAIR ? 2 * split : split) ? ld_cluster_u32(mapa_shared(smem_u32((const void*)abort_flag), lane)) : 0u;
+  float4 f[8];
+  auto partials = [&](int r, int c) {
+    const uint32_t at = tile_smem + (uint32_t)(r * PITCH + c) * 4u;
+#pragma unroll
+    for (int s = 0; s < 8; s++)
+      if (s < split) f[s] = ld_cluster_v4(mapa_shared(at, PAIR ? 2 * s + crank : s));
+  };
+  bool in = place(tid, r, c);
+  if (in) partials(r, c);
+  const bool all_ok = !__any_sync(0xffffffffu, bad != 0);
   if (all_ok) {
-    const int first = (int)rank * BM / split, rows = ((int)rank + 1) * BM / split - first;
-    for (int i = tid; i < rows * (BN / 4); i += blockDim.x) {
-      const int r = first + i / (BN / 4), c = (i % (BN / 4)) * 4;
-      if (m0 + r >= p.M || n0 + c >= p.N) continue;
-      const uint32_t at = tile_smem + (uint32_t)(r * PITCH + c) * 4u;
-      float v[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll 4
-      for (int s = 0; s < split; s++) {
-        const float4 f = ld_cluster_v4(mapa_shared(at, PAIR ? 2 * s + crank : s));
-        v[0] += f.x; v[1] += f.y; v[2] += f.z; v[3] += f.w;
+    for (int i = tid; i < items; i += GEMM_THREADS) {
+      if (i != tid) {
+        in = place(i, r, c);
+        if (in) { epilogue4_fetch(p, m0 + r, n0 + c, e); partials(r, c); }
       }
-      epilogue4(p, m0 + r, n0 + c, v);
+      if (!in) continue;
+      float v[4] = {f[0].x, f[0].y, f[0].z, f[0].w};
+#pragma unroll
+      for (int s = 1; s < 8; s++)
+        if (s < split) { v[0] += f[s].x; v[1] += f[s].y; v[2] += f[s].z; v[3] += f[s].w; }
+      epilogue4(p, m0 + r, n0 + c, v, e);
     }
     if (csum && tn == 0 && tid < rows) {
       const int r = first + tid;
-      float v = 0.f;
-      for (int s = 0; s < split; s++) v += __uint_as_float(ld_cluster_u32(mapa_shared(csum_smem + (uint32_t)r * 4u, PAIR ? 2 * s + crank : s)));
+      float w[8], v = 0.f;
+#pragma unroll
+      for (int s = 0; s < 8; s++)
+        w[s] = s < split ? __uint_as_float(ld_cluster_u32(mapa_shared(csum_smem + (uint32_t)r * 4u, PAIR ? 2 * s + crank : s))) : 0.f;
+#pragma unroll
+      for (int s = 0; s < 8; s++)
+        if (s < split) v += w[s];
       if (m0 + r < p.M) p.colsum[m0 + r] = p.accumulate ? p.colsum[m0 + r] + v : v;
     }
   }
