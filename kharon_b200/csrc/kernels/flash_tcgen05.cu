@@ -110,10 +110,7 @@ template <int NSEG> struct FwdMaps { CUtensorMap q[NSEG], kv[NSEG], o[NSEG]; };
 template <int NSEG> struct FwdSegs { int T[NSEG]; uint16_t pair[MAX_PAIRS]; };      // pair = query tile * MAX_SEGS + sequence
 template <> struct FwdSegs<1> {};
 
-// ONE_TILE (head width 128, one sequence length of up to 128 positions, more than four items per SM): the MMA role is entered by
-// lane 0, as in the dK / dV kernel below (T 40, 4800 items: 53.9 us, 56.8 with the elected lane; T 66, 32 items: 6.4 and 6.2;
-// T 512, 256 items: 40.0 and 39.4).
-template <int HD, int NSEG, bool ONE_TILE>
+template <int HD, int NSEG>
 __global__ void __launch_bounds__(192, 2)
 flash_fwd_ws_kernel(const __grid_constant__ FwdMaps<NSEG> maps, const __grid_constant__ FwdSegs<NSEG> seg, const AttnParams p,
                     int n_items, int n_qt) {
@@ -200,7 +197,7 @@ flash_fwd_ws_kernel(const __grid_constant__ FwdMaps<NSEG> maps, const __grid_con
     }
   } else if (warp == 5) {
     // ------------------------------------------------------------------ MMA issuer
-    if (live && (ONE_TILE ? lane == 0 : elect_one())) {
+    if (live && elect_one()) {
       constexpr uint32_t idesc_s = umma_idesc_bf16(128, BKV, 0, 0);
       constexpr uint32_t idesc_o = umma_idesc_bf16(128, HD, 0, 1);
       int ic = 0, pc = 0, kvc = 0;
@@ -965,13 +962,13 @@ static int num_sms_attn() {
   return sms > 0 ? sms : 148;
 }
 
-template <int HD, int NSEG, bool ONE_TILE>
+template <int HD, int NSEG>
 int launch_fwd_items(const FwdMaps<NSEG>& maps, const FwdSegs<NSEG>& seg, const AttnParams& p, int n_items, int n_qt, cudaStream_t st) {
   using C = FwdWs<HD>;
   static bool once = false;
-  if (!once) { if (set_smem(flash_fwd_ws_kernel<HD, NSEG, ONE_TILE>, C::SMEM, "flash_fwd")) return -1; once = true; }
+  if (!once) { if (set_smem(flash_fwd_ws_kernel<HD, NSEG>, C::SMEM, "flash_fwd")) return -1; once = true; }
   const int ctas = 2 * num_sms_attn();                  // two CTAs per SM
-  KH_LAUNCH((flash_fwd_ws_kernel<HD, NSEG, ONE_TILE>), n_items < ctas ? n_items : ctas, C::THREADS, C::SMEM, st, maps, seg, p, n_items, n_qt);
+  KH_LAUNCH((flash_fwd_ws_kernel<HD, NSEG>), n_items < ctas ? n_items : ctas, C::THREADS, C::SMEM, st, maps, seg, p, n_items, n_qt);
   KH_LAUNCH_CHECK("flash_fwd");
   return 0;
 }
@@ -990,8 +987,7 @@ int launch_fwd(const void* qkv, const AttnParams& p, cudaStream_t st) {
   FwdMaps<1> maps;
   if (fwd_maps(maps, 0, qkv, p.out, p.B, p.T, p.H, HD, p.ld)) return -1;
   const int n_qt = (p.T + 127) / 128;
-  if (HD == 128 && n_qt == 1 && p.B * p.H > 4 * num_sms_attn()) return launch_fwd_items<HD, 1, HD == 128>(maps, FwdSegs<1>{}, p, p.B * p.H, n_qt, st);
-  return launch_fwd_items<HD, 1, false>(maps, FwdSegs<1>{}, p, p.B * p.H * n_qt, n_qt, st);
+  return launch_fwd_items<HD, 1>(maps, FwdSegs<1>{}, p, p.B * p.H * n_qt, n_qt, st);
 }
 // Sequences of rows [row0[i], row0[i] + len[i]) of qkv and out, as many per launch as the maps and the list of pairs hold.
 template <int HD>
@@ -1021,7 +1017,7 @@ int launch_fwd_varlen(const bf16* qkv, AttnParams p, const int* row0, const int*
       for (int i = 0; i < n; i++)
         if (qt < (seg.T[i] + 127) / 128) seg.pair[at++] = (uint16_t)(qt * MAX_SEGS + i);
     p.B = 1; p.T = 0;
-    if (launch_fwd_items<HD, MAX_SEGS, false>(maps, seg, p, pairs * p.H, most, st)) return -1;
+    if (launch_fwd_items<HD, MAX_SEGS>(maps, seg, p, pairs * p.H, most, st)) return -1;
     s0 += n;
   }
   return 0;
@@ -1060,23 +1056,18 @@ int launch_bwd(const void* qkv, const AttnParams& p, cudaStream_t st) {
   return launch_bwd_as<HD, false>(qkv, p, st);
 }
 
-// Whether flash_short.cu takes sequences of T <= 64 positions.  Its cost is the arithmetic of mma.sync on the rows that are there,
-// that of the kernels here the latency of an item per resident CTA.  Head width 64: always (B 32-1000 H8 T 33-64: 0.4 to 0.93 of the
-// time forward, 0.3 to 0.91 backward).  Head width 128, forward, us (short / tcgen05): T 64, 592 items 9.3 / 10.7, 1536 31.8 / 23.5;
-// T 48, 1536 21.1 / 22.2, 2048 30.8 / 26.9; T 40, 2048 24.4 / 26.1, 3200 47.5 / 38.1; T 32, 4096 39.7 / 46.1.  Backward: T 64,
-// 384 items 29.1 / 31.0, 768 71.6 / 56.6; T 48, 4800 218 / 277.
-static bool use_short(bool backward, int T, int hd, long items) {
-  if (T < 1 || T > KH_FLASH_SHORT_T) return false;
-  if (hd == 64 || T <= 32 || (backward && T <= 48)) return true;
-  return items <= (backward ? 3L : T <= 40 ? 14L : T <= 48 ? 10L : 4L) * num_sms_attn();
-}
+// Whether flash_short.cu takes the sequences: up to 64 positions always.  Its cost is the arithmetic of mma.sync on the rows that are there, that of
+// the kernels here the latency of an item per resident CTA.  Head width 64: B 32-1000 H8 T 33-64 0.4 to 0.93 of the time forward, 0.3 to 0.91
+// backward, before its loads were asynchronous.  Head width 128, us (short / tcgen05): forward T 33, 2080 items 16.1 / 28.3; T 48, 8000 65.0 / 86.6;
+// T 64, 960 12.7 / 17.0 and 8000 84.5 / 89.9; backward T 56, 592 items 20.9 / 38.8; T 64, 8000 318 / 475.
+static bool use_short(int T) { return T >= 1 && T <= KH_FLASH_SHORT_T; }
 
 }  // namespace
 
 extern "C" int kh_flash_fwd(const void* qkv, void* out, void* lse, int B, int T, int H, int hd, int ld, float scale,
                             void* stream) {
   if (hd != 64 && hd != 128) { kh_set_error("flash: head dim %d is not supported (64 or 128)", hd); return -1; }
-  if (use_short(false, T, hd, (long)B * H)) return kh_flash_short_fwd(qkv, out, lse, B, T, H, hd, ld, scale, stream);
+  if (use_short(T)) return kh_flash_short_fwd(qkv, out, lse, B, T, H, hd, ld, scale, stream);
   AttnParams p = {};
   p.B = B; p.T = T; p.H = H; p.ld = ld; p.scale = scale; p.out = (bf16*)out; p.lse = (float*)lse;
   p.err = kh_error_word_dev();
@@ -1100,7 +1091,7 @@ extern "C" int kh_flash_fwd_varlen(const void* qkv, void* out, const void* row0,
 extern "C" int kh_flash_bwd(const void* qkv, const void* out, const void* dout, const void* lse, void* dqkv,
                             void* delta, int B, int T, int H, int hd, int ld, float scale, void* stream) {
   if (hd != 64 && hd != 128) { kh_set_error("flash: head dim %d is not supported (64 or 128)", hd); return -1; }
-  if (use_short(true, T, hd, (long)B * H)) return kh_flash_short_bwd(qkv, out, dout, lse, dqkv, delta, B, T, H, hd, ld, scale, stream);
+  if (use_short(T)) return kh_flash_short_bwd(qkv, out, dout, lse, dqkv, delta, B, T, H, hd, ld, scale, stream);
   AttnParams p = {};
   p.B = B; p.T = T; p.H = H; p.ld = ld; p.scale = scale; p.lse = (float*)lse; p.o = (const bf16*)out;
   p.dout = (const bf16*)dout; p.delta = (float*)delta; p.dqkv = (bf16*)dqkv;

@@ -421,8 +421,8 @@ def test_flash_fwd_bwd(B, T, H, hd):
                                       (186, 48, 8, 128), (259, 40, 8, 128), (260, 33, 8, 128), (74, 128, 8, 128), (75, 128, 8, 128),
                                       (80, 65, 16, 128)])
 def test_flash_short_sequences_of_many_items(B, T, H, hd):
-    """Up to 128 positions at head width 128, on both sides of the item counts at which the kernel for short sequences hands over
-    to the 128-row tiles, forward and backward independently, and the kernels for one tile per item come in."""
+    """Up to 128 positions at head width 128 and many items: the kernel for short sequences up to 64 positions, beyond them the 128-row
+    tiles with one tile per item, on both sides of the line at which the backward kernel for those comes in."""
     test_flash_fwd_bwd(B, T, H, hd)
 
 
