@@ -746,75 +746,6 @@ extern "C" int kh_layernorm_bwd(const void* dy, const void* x, const void* w, co
 //   rowloss[r] = lse - logit[target]            prob[r] = softmax[target]
 //   logits[r, :] <- scale_r * (softmax - onehot) in place, scale_r = coef ? coef[r] : uniform
 // Rows whose target is negative contribute nothing (loss 0, zero gradient).
-__global__ void xent_k(bf16* __restrict__ logits, int ld, int V, const int* __restrict__ target,
-                       const float* __restrict__ coef, float uniform, float* __restrict__ rowloss,
-                       float* __restrict__ prob, int write_grad) {
-  pdl_wait();
-  pdl_launch_dependents();
-  __shared__ float s_m[32], s_s[32];
-  __shared__ float s_max, s_sum;
-  const int r = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
-  bf16* row = logits + (size_t)r * ld;
-  const uint4* rp = reinterpret_cast<const uint4*>(row);
-  float m = -INFINITY, s = 0.f;
-  const int nv = V / 8;
-  for (int i = tid; i < nv; i += blockDim.x) {
-    uint4 v = rp[i];
-    float2 a = unpack_bf16(v.x), b = unpack_bf16(v.y), c = unpack_bf16(v.z), e = unpack_bf16(v.w);
-    float mx = fmaxf(fmaxf(fmaxf(a.x, a.y), fmaxf(b.x, b.y)), fmaxf(fmaxf(c.x, c.y), fmaxf(e.x, e.y)));
-    if (mx > m) { s *= __expf(m - mx); m = mx; }
-    s += __expf(a.x - m) + __expf(a.y - m) + __expf(b.x - m) + __expf(b.y - m) + __expf(c.x - m) + __expf(c.y - m) +
-         __expf(e.x - m) + __expf(e.y - m);
-  }
-  for (int i = nv * 8 + tid; i < V; i += blockDim.x) {
-    float x = __bfloat162float(row[i]);
-    if (x > m) { s *= __expf(m - x); m = x; }
-    s += __expf(x - m);
-  }
-  // combine (m, s) pairs in a fixed tree
-  float wm = warp_max(m);
-  s *= (m == -INFINITY) ? 0.f : __expf(m - wm);
-  s = warp_sum(s);
-  if (lane == 0) { s_m[warp] = wm; s_s[warp] = s; }
-  __syncthreads();
-  if (warp == 0) {
-    float mm = lane < nw ? s_m[lane] : -INFINITY;
-    float ss = lane < nw ? s_s[lane] : 0.f;
-    float gm = warp_max(mm);
-    ss *= (mm == -INFINITY) ? 0.f : __expf(mm - gm);
-    ss = warp_sum(ss);
-    if (lane == 0) { s_max = gm; s_sum = ss; }
-  }
-  __syncthreads();
-  const float gmax = s_max, gsum = s_sum;
-  const int t = target[r];
-  if (tid == 0) {
-    const bool valid = t >= 0 && t < V;
-    const float xt = valid ? __bfloat162float(row[t]) : 0.f;
-    if (rowloss) rowloss[r] = valid ? (logf(gsum) + gmax - xt) : 0.f;
-    if (prob) prob[r] = valid ? __expf(xt - gmax) / gsum : 0.f;
-  }
-  if (!write_grad) return;
-  __syncthreads();   // the target logit has been read
-  const float sc = (t >= 0 && t < V) ? (coef ? coef[r] : uniform) : 0.f;
-  const float inv = sc / gsum;
-  uint4* wp = reinterpret_cast<uint4*>(row);
-  const int nvl = ld / 8;
-  for (int i = tid; i < nvl; i += blockDim.x) {
-    uint4 v = wp[i], o;
-    const uint32_t* vi = &v.x; uint32_t* oi = &o.x;
-    const int c0 = i * 8;
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-      float2 xv = unpack_bf16(vi[k]);
-      const int c = c0 + 2 * k;
-      float g0 = c < V ? __expf(xv.x - gmax) * inv - (c == t ? sc : 0.f) : 0.f;
-      float g1 = c + 1 < V ? __expf(xv.y - gmax) * inv - (c + 1 == t ? sc : 0.f) : 0.f;
-      oi[k] = pack_bf16(g0, g1);
-    }
-    wp[i] = o;
-  }
-}
 __device__ __forceinline__ uint32_t max_bf16x2(uint32_t a, uint32_t b) {      // a NaN gives way to a number
   const __nv_bfloat162 m = __hmax2(*reinterpret_cast<const __nv_bfloat162*>(&a), *reinterpret_cast<const __nv_bfloat162*>(&b));
   return *reinterpret_cast<const uint32_t*>(&m);
@@ -850,6 +781,86 @@ __device__ __forceinline__ uint4 xent_grad8(f32x2 (&e)[4], int c, int t, float s
     w[k] = pack2(g);
   }
   return o;
+}
+// XK
+__global__ void xent_k(bf16* __restrict__ logits, int ld, int V, const int* __restrict__ target,
+                       const float* __restrict__ coef, float uniform, float* __restrict__ rowloss,
+                       float* __restrict__ prob, int write_grad) {
+  pdl_wait();
+  pdl_launch_dependents();
+  __shared__ float s_m[32], s_s[32];
+  __shared__ float s_max, s_sum;
+  const int r = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
+  bf16* row = logits + (size_t)r * ld;
+  const uint4* rp = reinterpret_cast<const uint4*>(row);
+  float m = -INFINITY, s = 0.f;
+  const int nv = V / 8;
+  f32x2 s0 = 0, s1 = 0;
+#pragma unroll 2
+  for (int i = tid; i < nv; i += blockDim.x) {
+    const uint4 v = rp[i];
+    const f32x2 m2 = un2(xent_max8(v, 0, 8));
+    const float mx = fmaxf(lo2(m2), hi2(m2));
+    if (mx > m) {
+      const float c = __expf(m - mx);
+      s0 = mul2(s0, mk2(c, c)); s1 = mul2(s1, mk2(c, c));
+      m = mx;
+    }
+    const float nm = m == -INFINITY ? 0.f : -m;      // a masked run: its exponentials are 0
+    f32x2 e[4];
+    xent_exp8(v, 0, 8, mk2(nm, nm), e);
+    s0 = add2(s0, add2(e[0], e[1])); s1 = add2(s1, add2(e[2], e[3]));
+  }
+  s0 = add2(s0, s1);
+  s = lo2(s0) + hi2(s0);
+  for (int i = nv * 8 + tid; i < V; i += blockDim.x) {
+    float x = __bfloat162float(row[i]);
+    if (x > m) { s *= __expf(m - x); m = x; }
+    s += m == x && x == -INFINITY ? 0.f : __expf(x - m);
+  }
+  // combine (m, s) pairs in a fixed tree
+  float wm = warp_max(m);
+  s *= (m == -INFINITY) ? 0.f : __expf(m - wm);
+  s = warp_sum(s);
+  if (lane == 0) { s_m[warp] = wm; s_s[warp] = s; }
+  __syncthreads();
+  if (warp == 0) {
+    float mm = lane < nw ? s_m[lane] : -INFINITY;
+    float ss = lane < nw ? s_s[lane] : 0.f;
+    float gm = warp_max(mm);
+    ss *= (mm == -INFINITY) ? 0.f : __expf(mm - gm);
+    ss = warp_sum(ss);
+    if (lane == 0) { s_max = gm; s_sum = ss; }
+  }
+  __syncthreads();
+  const float gmax = s_max, gsum = s_sum;
+  const int t = target[r];
+  if (tid == 0) {
+    const bool valid = t >= 0 && t < V;
+    const float xt = valid ? __bfloat162float(row[t]) : 0.f;
+    if (rowloss) rowloss[r] = valid ? (logf(gsum) + gmax - xt) : 0.f;
+    if (prob) prob[r] = valid ? __expf(xt - gmax) / gsum : 0.f;
+  }
+  if (!write_grad) return;
+  __syncthreads();   // the target logit has been read
+  const float sc = (t >= 0 && t < V) ? (coef ? coef[r] : uniform) : 0.f;
+  const float inv = sc / gsum;
+  uint4* wp = reinterpret_cast<uint4*>(row);
+  const int nvl = ld / 8;
+  const bool valid = t >= 0 && t < V;
+  const int tp = valid ? t >> 3 : -1;
+  const f32x2 nmax = mk2(-gmax, -gmax), inv2 = mk2(inv, inv);
+#pragma unroll 2
+  for (int i = tid; i < nvl; i += blockDim.x) {
+    f32x2 e[4];
+    if (i < nv && i != tp) {
+      xent_exp8(wp[i], 0, 8, nmax, e);
+      wp[i] = make_uint4(pack2(mul2(e[0], inv2)), pack2(mul2(e[1], inv2)), pack2(mul2(e[2], inv2)), pack2(mul2(e[3], inv2)));
+    } else {
+      xent_exp8(wp[i], i * 8, V, nmax, e);
+      wp[i] = xent_grad8(e, i * 8, valid ? t : -2, sc, inv);
+    }
+  }
 }
 // Up to 256 NC columns: a warp per row, the row read once and kept in registers.
 template <int NC>
