@@ -269,9 +269,9 @@ __device__ __forceinline__ f32x2 gelu_tanh_grad2(f32x2 x) {
 constexpr int BM = 128, BK = 64, UMMA_K = 16;
 constexpr int GEMM_THREADS = 320;          // TMA, MMA and eight epilogue warps (or four and four column-sum warps); 192: four epilogue warps
 
-// Staging buffer of an epilogue warp: 32 rows of 64 bytes (32 bf16 columns), pitch 80 bytes (conflict-free 16-byte accesses both
-// by row and by piece).
-constexpr int EPI_PITCH = 80, EPI_BYTES = 32 * EPI_PITCH;
+// Staging buffer of an epilogue warp: 32 rows of 64 bytes (32 bf16 columns), the 16-byte pieces of a row exchanged by its index (conflict-free
+// accesses both by row and by piece).
+constexpr int EPI_BYTES = 32 * 64;
 
 // PAIR: two CTAs of a cluster form one 256 x BN tile (tcgen05 cta_group::2).  Each CTA stages its
 // own 128 rows of A and its own half of B, so a pair moves and re-reads 2/3 of the shared-memory
@@ -306,7 +306,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ C
   const uint32_t bar_free = bar_tempty + 16;         // column-sum warps are done with the stage
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 3 * Cfg::STAGES + 4);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  const bool csum = p.colsum != nullptr, wide = !csum && blockDim.x == GEMM_THREADS;      // wide: eight epilogue warps
+  const bool csum = p.colsum != nullptr;
+  const int parts = !csum && blockDim.x == GEMM_THREADS ? 2 : 1;      // epilogue warps to a TMEM quadrant
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int tiles_m = (p.M + TM - 1) / TM, tiles_n = (p.N + BN - 1) / BN;
@@ -318,7 +319,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ C
       mbar_init(bar_full + 8 * s, 1); mbar_init(bar_empty + 8 * s, 1); mbar_init(bar_free + 8 * s, 4);
     }
     // accumulator-free barrier: one arrival per epilogue warp of every CTA that reads the accumulator
-    for (int a = 0; a < 2; a++) { mbar_init(bar_tfull + 8 * a, 1); mbar_init(bar_tempty + 8 * a, (PAIR ? 2 : 1) * (wide ? 8 : 4)); }
+    for (int a = 0; a < 2; a++) { mbar_init(bar_tfull + 8 * a, 1); mbar_init(bar_tempty + 8 * a, (PAIR ? 2 : 1) * 4 * parts); }
     *abort_flag = 0;
     mbar_fence_init();
   }
@@ -481,19 +482,23 @@ gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ C
     }
   } else {
     // ------------------------------------------------------------------ epilogue warps
-    // Four warps with all columns of a tile, or eight, two per TMEM quadrant, with half of the columns each (see epilogue_threads).
+    // Four warps with all columns of a tile, or eight, two per TMEM quadrant, with every second 32 columns each (see gemm_threads): the two
+    // halves of a line are then written at about the same time.  With half of the tile's columns each, 8192 x 2048 x 512 took 18.2 us plain, 23.7 with
+    // GELU and 27.3 with its pre-activation too, 28.4 times GELU'; so 17.4, 21.7, 25.3, 26.7; 8192 x 1536 x 512 15.3 and 14.6.  (Sixteen warps: 20.3
+    // plain; steps of 64 columns in whole lines 17.6, but 29 with GELU and pre-activation: fewer steps overlap.)
     const int q = warp & 3;                    // TMEM lane quadrant this warp may access
-    const int col_lo = (wide && warp >= 6) ? BN / 2 : 0, col_hi = (wide && warp < 6) ? BN / 2 : BN;
+    const int part = (warp - 2) >> 2, step = 32 * parts;
     // A thread owns a row of the accumulator, but global memory is read and written in pieces of 16 bytes, four neighbouring
     // lanes to a row of the 32-column chunk: the warp turns the chunk around in its staging buffer.  With every lane on its own row an
     // access touched 32 lines, and the load / store unit bounded the products of narrow models (9216 x 1536 x 512:
     // 23.6 us plain, 30 with a residual, 38 with GELU and its pre-activation; cuBLAS plain 14.1).
     const uint32_t stg = smem_base + Cfg::STAGES * Cfg::STAGE_BYTES + 256 + (warp - 2) * EPI_BYTES;
     const int prow = lane >> 2, pcol = (lane & 3) * 8;          // this lane's piece: row 8 j + prow, columns pcol ..
+    auto staged = [&](int r, int piece) { return stg + r * 64 + ((piece ^ ((r >> 1) & 3)) << 4); };
     auto put_row = [&](const uint32_t (&w)[16]) {                // own row, bf16 pairs -> staging
 #pragma unroll
       for (int j = 0; j < 4; j++)
-        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(stg + lane * EPI_PITCH + j * 16), "r"(w[4 * j]), "r"(w[4 * j + 1]), "r"(w[4 * j + 2]),
+        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(staged(lane, j)), "r"(w[4 * j]), "r"(w[4 * j + 1]), "r"(w[4 * j + 2]),
                      "r"(w[4 * j + 3]) : "memory");
     };
     auto lds = [&](uint32_t a) {
@@ -506,7 +511,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ C
       __syncwarp();
 #pragma unroll
       for (int j = 0; j < 4; j++) {
-        const uint4 u = lds(stg + (j * 8 + prow) * EPI_PITCH + (lane & 3) * 16);
+        const uint4 u = lds(staged(j * 8 + prow, lane & 3));
         if (r0 + j * 8 + prow < p.M) *reinterpret_cast<uint4*>(base + (size_t)(r0 + j * 8 + prow) * ld + col + pcol) = u;
       }
       __syncwarp();
@@ -524,10 +529,10 @@ gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ C
       const bool use_aux = (p.epi == EPI_BIAS_RESID || p.epi == EPI_RESID || p.epi == EPI_DGELU);
       // Operands of the epilogue are fetched one 32-column chunk ahead (the first chunk before the
       // accumulator is even complete), so their DRAM latency is not paid once per chunk.
-      uint4 nb[4], nx[4];
+      uint4 nb[4] = {}, nx[4] = {};
       auto fetch = [&](int c0) {
         const int col = tn * BN + c0;
-        if (c0 >= col_hi || col + 32 > p.N) return;
+        if (c0 >= BN || col + 32 > p.N) return;
         if (use_bias) {
           const uint4* bp = reinterpret_cast<const uint4*>(p.bias + col);
 #pragma unroll
@@ -541,28 +546,24 @@ gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ C
       };
       if (use_aux && row_ok) {
         const char* ap = reinterpret_cast<const char*>(p.aux + (size_t)row * p.ldaux + tn * BN);
-        const int nbytes = min(col_hi, p.N - tn * BN) * 2;
-        for (int b = col_lo * 2 + 128; b < nbytes; b += 128) prefetch_l2(ap + b);
+        const int nbytes = min(BN, p.N - tn * BN) * 2;
+        for (int b = 128 * (1 + part); b < nbytes; b += 128 * parts) prefetch_l2(ap + b);
       }
-      fetch(col_lo);
+      fetch(32 * part);
       if (!mbar_wait(bar_tfull + 8 * acc, aph, abort_flag, 3, p.err)) { ok = false; break; }
       tc_fence_after();
       const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + acc * BN;
 #pragma unroll 1
-      for (int c0 = col_lo; c0 < col_hi; c0 += 32) {
+      for (int c0 = 32 * part; c0 < BN; c0 += step) {
         const int col = tn * BN + c0;
         if (col >= p.N) break;                 // uniform across the warp
         uint32_t r[32];
         tmem_ld32(taddr + c0, r);
-        uint4 cb[4], cx[4];
-#pragma unroll
-        for (int j = 0; j < 4; j++) { cb[j] = nb[j]; cx[j] = nx[j]; }
-        fetch(c0 + 32);
         tmem_ld_wait();
         if (col + 32 <= p.N) {                 // uniform over the warp: rows past the end take part without memory accesses
           // With K of a few hundred this arithmetic and the stores bound a tile, not its MMAs: columns in pairs, and one rounding to bf16 for the
           // stored pre-activation and the argument of its GELU (8192 x 2048 x 512: GELU with pre-activation 31.4 us column by column, 27.4 so; times
-          // GELU' 34.3 and 28.8; without either 18.9).
+          // GELU' 34.3 and 28.8).
           f32x2 v[16];
           uint32_t w[16];
 #pragma unroll
@@ -574,10 +575,11 @@ gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ C
           if (use_bias) {
 #pragma unroll
             for (int j = 0; j < 4; j++) {
-              v[4 * j] = add2(v[4 * j], un2(cb[j].x)); v[4 * j + 1] = add2(v[4 * j + 1], un2(cb[j].y));
-              v[4 * j + 2] = add2(v[4 * j + 2], un2(cb[j].z)); v[4 * j + 3] = add2(v[4 * j + 3], un2(cb[j].w));
+              v[4 * j] = add2(v[4 * j], un2(nb[j].x)); v[4 * j + 1] = add2(v[4 * j + 1], un2(nb[j].y));
+              v[4 * j + 2] = add2(v[4 * j + 2], un2(nb[j].z)); v[4 * j + 3] = add2(v[4 * j + 3], un2(nb[j].w));
             }
           }
+          if (!use_aux) fetch(c0 + step);
           if (p.epi == EPI_BIAS_GELU || p.epi == EPI_GELU) {
             // the stored pre-activation is bf16; apply GELU to the rounded value so that the
             // backward pass (which only sees the bf16 copy) differentiates the same function
@@ -590,12 +592,13 @@ gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ C
           } else if (use_aux) {
 #pragma unroll
             for (int j = 0; j < 4; j++)
-              asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(stg + (j * 8 + prow) * EPI_PITCH + (lane & 3) * 16), "r"(cx[j].x), "r"(cx[j].y),
-                           "r"(cx[j].z), "r"(cx[j].w) : "memory");
+              asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(staged(j * 8 + prow, lane & 3)), "r"(nx[j].x), "r"(nx[j].y),
+                           "r"(nx[j].z), "r"(nx[j].w) : "memory");
+            fetch(c0 + step);
             __syncwarp();
 #pragma unroll
             for (int j = 0; j < 4; j++) {
-              const uint4 b = lds(stg + lane * EPI_PITCH + j * 16);
+              const uint4 b = lds(staged(lane, j));
               w[4 * j] = b.x; w[4 * j + 1] = b.y; w[4 * j + 2] = b.z; w[4 * j + 3] = b.w;
             }
             if (p.epi == EPI_DGELU) {
