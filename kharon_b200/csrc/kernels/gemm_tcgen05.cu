@@ -958,10 +958,11 @@ static int num_sms() {
   return g_num_sms;
 }
 
-// Threads of a gemm_kernel CTA.  Up to K = 1024 the main loop of a tile is shorter than the epilogue of four warps, which then
-// bounds the product: eight warps.  Beyond, the epilogue hides behind the main loop and the second set of warps only takes
-// power and issue slots from it (1.2B training step, K = 2048 and more: 147.3 ms with eight, 144.5 with four).
-static int gemm_threads(const GemmParams& p) { return p.colsum || p.K <= 1024 ? GEMM_THREADS : 192; }
+// Threads of a gemm_kernel CTA (or pair) that takes `turns` tiles.  Up to K = 1024 the main loop of a tile is shorter than the epilogue of four warps,
+// which then bounds the product, and with one or two turns the last epilogue is a good part of it: eight warps (8192 x 512 x 2048 with
+// residual 16.2 us, 17.1 with four; 4200 x 1024 x 4096 26.9, 27.3).  Beyond, the epilogue hides behind the main loop and the second set of warps only
+// takes power and issue slots from it (1.2B training step, K = 2048 and more: 147.3 ms with eight, 144.5 with four).
+static int gemm_threads(const GemmParams& p, int turns) { return p.colsum || p.K <= 1024 || turns <= 2 ? GEMM_THREADS : 192; }
 
 // 256-row tiles on CTA pairs.  Returns the number of clusters that can be resident (0: unsupported).
 static int g_pair_clusters = -1;
@@ -974,7 +975,7 @@ static int launch_gemm_pair(const CUtensorMap* ta, const CUtensorMap* tb, const 
   attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[1].val.programmaticStreamSerializationAllowed = 1;
-  cfg.blockDim = dim3(gemm_threads(p)); cfg.dynamicSmemBytes = Cfg::SMEM; cfg.stream = st; cfg.attrs = attr;
+  cfg.blockDim = dim3(GEMM_THREADS); cfg.dynamicSmemBytes = Cfg::SMEM; cfg.stream = st; cfg.attrs = attr;
   cfg.numAttrs = kh_pdl_enabled() ? 2 : 1;
   if (g_pair_clusters < 0) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM);
@@ -990,6 +991,7 @@ static int launch_gemm_pair(const CUtensorMap* ta, const CUtensorMap* tb, const 
   int clusters = tiles < g_pair_clusters ? tiles : g_pair_clusters;
   if (max_ctas > 0 && 2 * clusters > max_ctas) clusters = max_ctas / 2 > 0 ? max_ctas / 2 : 1;
   cfg.gridDim = dim3(2 * clusters);
+  cfg.blockDim = dim3(gemm_threads(p, (tiles + clusters - 1) / clusters));
   cudaError_t e = cudaLaunchKernelEx(&cfg, kern, *ta, *tb, p);
   if (e != cudaSuccess) { kh_set_error("gemm pair launch failed: %s", cudaGetErrorString(e)); return -1; }
   return 0;
@@ -1008,7 +1010,7 @@ static int launch_gemm(const CUtensorMap* ta, const CUtensorMap* tb, const GemmP
   const int tiles = ((p.M + BM - 1) / BM) * ((p.N + BN - 1) / BN);
   int grid = tiles < num_sms() ? tiles : num_sms();
   if (max_ctas > 0 && grid > max_ctas) grid = max_ctas;
-  cudaError_t e = KH_LAUNCH((gemm_kernel<BN, false>), grid, gemm_threads(p), Cfg::SMEM, st, *ta, *tb, p);
+  cudaError_t e = KH_LAUNCH((gemm_kernel<BN, false>), grid, gemm_threads(p, (tiles + grid - 1) / grid), Cfg::SMEM, st, *ta, *tb, p);
   if (e != cudaSuccess) { kh_set_error("gemm launch failed: %s", cudaGetErrorString(e)); return -1; }
   return 0;
 }
