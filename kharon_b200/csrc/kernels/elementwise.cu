@@ -682,7 +682,7 @@ __global__ void layernorm_bwd_dwdb_k(const bf16* __restrict__ dy, const bf16* __
   }
   if (threadIdx.x == 0) counters[blockIdx.x] = 0;
 }
-static int ln_bwd_sms() {
+static int ew_sms() {
   static int n = 0;
   if (!n) {
     int dev = 0;
@@ -696,7 +696,7 @@ static int ln_bwd_sms() {
 // 9.2, 2048 x 512 6.2 / 7.2 / 9.0, 4096 x 256 8.5 / 7.2 / 8.3, 2048 x 2048 12.3 / 12.0 / 13.2).
 extern "C" int kh_layernorm_bwd_parts(int rows, int d) {
   if (d <= 4096) {
-    const int rpi = d <= 512 ? 4 : (d <= 1024 ? 2 : 1), most = ln_bwd_sms() * (d <= 2048 ? 4 : 2);
+    const int rpi = d <= 512 ? 4 : (d <= 1024 ? 2 : 1), most = ew_sms() * (d <= 2048 ? 4 : 2);
     const int two = cdiv(rows, rpi * 2), four = cdiv(rows, rpi * 4), few = two < 256 ? two : 256, parts = few > four ? few : four;
     return parts < 1 ? 1 : (parts < most ? parts : most);
   }
@@ -927,7 +927,11 @@ extern "C" int kh_xent(void* logits, int ld, int V, const void* target, const vo
     else if (ld <= 1024) KH_XENT(xent_warp_k<4>, grid, 256, 0, rows);
     else KH_XENT(xent_warp_k<8>, grid, 256, 0, rows);
   } else {
-    KH_XENT(xent_k, rows, 512, 0);
+    // Eight CTAs of 256 threads an SM wait for less than four of 512 (8192 x 4000 38.4 / 51.9 us, 8192 x 8192 59.8 / 76.4; loss only, 8192 x 50257
+    // 136.8 / 148.0), but the gradient's second pass finds its row in L2 only while the rows in flight fit there (4096 x 32000 109.4 / 102.6,
+    // 8192 x 50257 382 / 321; 16000 columns, 38 MB, 103.0 / 118.9), and rows
+    // that are all resident with 512 threads want them (100 x 16000 6.7 / 5.4).
+    KH_XENT(xent_k, rows, rows > 4 * ew_sms() && (!write_grad || ld <= 16384) ? 256 : 512, 0);
   }
 #undef KH_XENT
   KH_LAUNCH_CHECK("xent");

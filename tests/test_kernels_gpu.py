@@ -314,9 +314,9 @@ def test_xent():
 
 
 @pytest.mark.parametrize("R,V,ld", [(1, 1, 8), (9, 7, 8), (17, 250, 256), (8, 256, 256), (33, 257, 264), (7, 512, 520), (40, 1023, 1024), (25, 1030, 1032),
-                                    (11, 2041, 2048), (6, 2048, 2056), (7, 9001, 9008)])
+                                    (11, 2041, 2048), (6, 2048, 2056), (7, 9001, 9008), (600, 2500, 2504)])
 def test_xent_short_rows(R, V, ld):
-    """A warp per row up to 2048 columns, a CTA per row past them (the last two shapes): every number of pieces a lane, odd vocabularies, NaN in the
+    """A warp per row up to 2048 columns, a CTA per row past them (the last three shapes; the last with 256 threads): every number of pieces a lane, odd vocabularies, NaN in the
     padding, masked (-inf) logits, rows without a target; loss, probability and gradient against fp64, the gradient rounded once to bf16."""
     torch.manual_seed(R + V)
     x = torch.full((R, ld), float("nan"), device=DEV).bfloat16()
