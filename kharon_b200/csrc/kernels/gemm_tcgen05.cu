@@ -563,7 +563,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ C
         if (col + 32 <= p.N) {                 // uniform over the warp: rows past the end take part without memory accesses
           // With K of a few hundred this arithmetic and the stores bound a tile, not its MMAs: columns in pairs, and one rounding to bf16 for the
           // stored pre-activation and the argument of its GELU (8192 x 2048 x 512: GELU with pre-activation 31.4 us column by column, 27.4 so; times
-          // GELU' 34.3 and 28.8).
+          // GELU' 34.3 and 28.8; then see the order of the steps above).
           f32x2 v[16];
           uint32_t w[16];
 #pragma unroll
@@ -585,7 +585,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ C
             // backward pass (which only sees the bf16 copy) differentiates the same function
 #pragma unroll
             for (int i = 0; i < 16; i++) w[i] = pack2(v[i]);
-            // (without a backward pass nobody reads the pre-activation: 4200 x 4096 x 1024 57.6 us with its store, 52.6 without)
+            // (without a backward pass nobody reads the pre-activation: 4200 x 4096 x 1024 34.3 us with its store, 29.2 without)
             if (p.epi == EPI_BIAS_GELU) store_rows(p.aux, p.ldaux, row0, col, w);
 #pragma unroll
             for (int i = 0; i < 16; i++) v[i] = gelu_tanh2(un2(w[i]));
@@ -1110,10 +1110,10 @@ extern "C" int kh_gemm_bf16_colsum(const void* A, int lda, int a_mn, const void*
     // waves x relative tile time; narrower tiles reuse the A panel less and run at lower efficiency
     const int tm = (M + BM - 1) / BM, sms = num_sms();
     auto waves = [&](int w) { return (tm * ((N + w - 1) / w) + sms - 1) / sms; };
-    // (up to K = 512 the epilogue weighs more and a 128-wide wave costs less: 8192 x 768 x 256 9.2 us in three waves of 128,
-    // 10.0 in two of 256; 4096 x 1536 x 512 11.7 and 11.9; but with up to 64 rows half of the epilogue warps have nothing to do, and
-    // at K = 512 the main loop counts again: 16 x 50257 x 512 13.5 us in two waves of 256, 15.4 in three of 128; K = 256 10.2, 10.1)
-    const float c256 = waves(256) * 1.0f, c128 = waves(128) * (K <= (M > 64 ? 512 : 256) ? 0.62f : 0.7f), c64 = waves(64) * 0.5f;
+    // (up to K = 512 the epilogue weighs more and a 128-wide wave costs less: 8192 x 768 x 256 8.0 us in three waves of 128,
+    // 8.8 in two of 256; 4096 x 1536 x 512 10.4 and 10.6; but with up to 64 rows half of the epilogue warps have nothing to do and
+    // the main loop counts again: 16 x 50257 x 512 12.4 us in two waves of 256, 14.4 in three of 128; K = 256 8.6, 9.1 (64 rows 8.2, 8.1), K = 128 7.2, 7.0)
+    const float c256 = waves(256) * 1.0f, c128 = waves(128) * (K <= (M > 64 ? 512 : 128) ? 0.62f : 0.7f), c64 = waves(64) * 0.5f;
     bn = 256;
     float best = c256;
     if (c128 < best) { best = c128; bn = 128; }
@@ -1123,8 +1123,8 @@ extern "C" int kh_gemm_bf16_colsum(const void* A, int lda, int a_mn, const void*
     // 256 x 256 tiles on CTA pairs: a wave of pairs takes about 0.93 of a wave of single tiles
     // (measured 6-19 % faster on large shapes), so prefer it unless wave quantisation eats the gain.  A pair also pays about
     // 1 us for its cluster, which short main loops do not earn back: single tiles in up to four waves at K = 512
-    // (9216 x 1536 16.5 us against 18.3; 8192 x 50257 in 86 waves 450 against 416), and up to K = 4096 where one wave does
-    // (4200 x 1024, single tiles / pairs: K = 1024 11.0 / 11.9, 2048 17.2 / 17.9, 4096 26.9 / 27.5, 6144 40.9 / 38.1)
+    // (9216 x 1536 14.3 us against 16.4; 8192 x 50257 in 86 waves 420 against 385), and up to K = 4096 where one wave does
+    // (4200 x 1024, single tiles / pairs: K = 1024 11.2 / 12.2, 4096 26.8 / 27.5, 6144 42.8 / 40.1)
     if (bn == 256 && M >= 512 && g_pair_clusters != 0 && (waves(256) > (K <= 512 ? 4 : 1) || K > 4096)) {
       const int clusters = g_pair_clusters > 0 ? g_pair_clusters : sms / 2;
       const int tiles2 = ((M + 255) / 256) * ((N + 255) / 256);
