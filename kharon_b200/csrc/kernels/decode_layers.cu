@@ -22,7 +22,9 @@
 // layers use in turn: when a CTA is done with a phase of layer l - 1, a helper warp empties the words that it will write in
 // that phase of layer l + 1 (last used at l - 2; whoever has seen all inputs of the phase at l - 1 knows that their readers are
 // done, since every output of a phase depends on all outputs of the one before), and its fence precedes the CTA's outputs of
-// layer l, so the words are empty before anybody can come to poll them.
+// layer l, so the words are empty before anybody can come to poll them: a reader of layer l + 1 has read that writer's words of
+// layer l.  The head's readers need not have (a width of 256 has 96, 32 and 128 groups of rows for 148 CTAs, so some take part in the head
+// alone and come to it at once), so the output of the last layer has words of its own, written once in a launch.
 // Launches alternate between two halves of the workspace and empty the other half for the next launch, which also
 // repairs what a launch that gave up has left.
 //
@@ -93,7 +95,7 @@ struct DecodeParams {
   int slots;                              // chunks in the ring
   const LayerW* layers;
   bf16* x;                                // [G, d] in: embedded tokens, out: last layer's output
-  uint32_t* words;                        // activations: [2 halves][3 slots][x d/2 | mid d/2 | att d/2 | qkv 3d/2 | act 4d/2][32 rows]
+  uint32_t* words;                        // activations: [2 halves]([3 slots][x d/2 | mid d/2 | att d/2 | qkv 3d/2 | act 4d/2][32 rows], last layer's x)
   bf16 *kc, *vc;                          // [L, blocks, bs, H, hd]
   size_t layer_elems;
   const int *pos, *slot, *btab;
@@ -112,6 +114,8 @@ struct DecodeParams {
   // j / bs by multiplication: exact for j < max_ctx, since max_ctx * bs stays below 2^32
   __device__ __forceinline__ int block_of(int j) const { return bs == 1 ? j : (int)__umulhi((uint32_t)j, bs_mul); }
 };
+__host__ __device__ constexpr size_t slot_words(int d) { return (size_t)MAX_ROWS * 5 * d; }
+__host__ __device__ constexpr size_t half_words(int d) { return 3 * slot_words(d) + (size_t)MAX_ROWS * (d / 2); }
 constexpr int CTL_BYTES = 512;                // 64 bytes of counters, and zeros that stand in for cache rows that do not exist
 
 struct Shared {               // small control block behind the data regions
@@ -681,16 +685,16 @@ __device__ __forceinline__ void empty_words(const DecodeParams& p, uint32_t* wor
   }
 }
 // The other half of the workspace is emptied for the next launch.
-__device__ __forceinline__ void empty_half(const DecodeParams& p, uint32_t half, size_t block) {
+__device__ __forceinline__ void empty_half(const DecodeParams& p, uint32_t half) {
   const int used = min((int)*reinterpret_cast<volatile uint32_t*>(p.ctl + 3 + (half ^ 1u)) + 7 & ~7, MAX_ROWS), d = p.d;
   const int me = (int)blockIdx.x * 64 + (int)threadIdx.x % 64, all = (int)gridDim.x * 64;
-  uint32_t* w = p.words + (half ^ 1u) * 3 * block;
+  uint32_t* w = p.words + (half ^ 1u) * half_words(d);
 #pragma unroll 1
-  for (int s = 0; s < 3; s++)
+  for (int s = 0; s < 4; s++)                  // three slots, and the last layer's x
 #pragma unroll 1
-    for (int f = 0; f < 5; f++) {
+    for (int f = 0; f < (s < 3 ? 5 : 1); f++) {
       const int width = (f < 3 ? d : (f == 3 ? 3 * d : 4 * d)) / 2, from = f < 4 ? f * d / 2 : 3 * d;
-      uint4* q = reinterpret_cast<uint4*>(w + s * block + (size_t)MAX_ROWS * from);
+      uint4* q = reinterpret_cast<uint4*>(w + s * slot_words(d) + (size_t)MAX_ROWS * from);
 #pragma unroll 1
       for (int i = me; i < used * width / 4; i += all) q[i] = make_uint4(0u, 0u, 0u, 0u);
     }
@@ -961,15 +965,15 @@ __global__ void __launch_bounds__(THREADS, 1) decode_layers_k(const __grid_const
   __syncthreads();
   // launches before this one: constant while it runs (only its last CTA to leave advances the word)
   const uint32_t launch = *reinterpret_cast<volatile uint32_t*>(p.ctl), half = launch & 1u;
-  const size_t block = (size_t)MAX_ROWS * 5 * d;         // words of a slot
-  uint32_t* const words = p.words + half * 3 * block;
+  const size_t block = slot_words(d);
+  uint32_t* const words = p.words + half * half_words(d);
 
   if (warp >= NW) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
     if (warp == NW) produce(p, ring, sh);
     else if (warp == NW + 1) empty_words<HD>(p, words, block, sh);
     else {
-      empty_half(p, half, block);
+      empty_half(p, half);
       if (blockIdx.x == 0 && threadIdx.x == CT + 64) p.ctl[3 + half] = (uint32_t)p.G;
     }
   } else {
@@ -1001,7 +1005,8 @@ __global__ void __launch_bounds__(THREADS, 1) decode_layers_k(const __grid_const
     for (int k = 0; k < 4 * p.L + (p.head_w ? 1 : 0); k++) {
       const int l = k >> 2, j = k & 3, d = fresh(p.d);
       const uint32_t row = (uint32_t)MAX_ROWS * (d / 2);    // words: x at 0, mid at row, att at 2 row, qkv at 3 row, act at 6 row
-      const bool head = k == 4 * p.L, ln = (j & 1) == 0;
+      const bool head = k == 4 * p.L, ln = (j & 1) == 0, last = j == 3 && l + 1 == p.L;
+      uint32_t* const out = words + 3 * block;              // the last layer's x
       if (j == 1) attention_phase<MT, HD>(p, l, 5 * l + 1, cur + 3 * row, cur + 2 * row, satt, sh);
       Lin L;
       L.bias = ptr(rec, j == 0 ? 3 : j == 1 ? 5 : j == 2 ? 9 : 11);
@@ -1009,11 +1014,11 @@ __global__ void __launch_bounds__(THREADS, 1) decode_layers_k(const __grid_const
       L.N = j == 0 ? 3 * d : j == 2 ? 4 * d : d;
       L.kind = j == 0 ? PA : j == 1 ? PC : j == 2 ? PD : PE;
       L.seq = 5 * l + (j == 0 ? 0 : j + 1);
-      L.src = j == 0 ? (l ? prv : nullptr) : cur + (j == 1 ? 2 : j == 2 ? 1 : 6) * row;
+      L.src = j == 0 ? (l ? (head ? out : prv) : nullptr) : cur + (j == 1 ? 2 : j == 2 ? 1 : 6) * row;
       L.res = j == 1 ? (l ? prv : nullptr) : j == 3 ? cur + row : nullptr;
-      L.dst = cur + (j == 0 ? 3 : j == 1 ? 1 : j == 2 ? 6 : 0) * row;
+      L.dst = last ? out : cur + (j == 0 ? 3 : j == 1 ? 1 : j == 2 ? 6 : 0) * row;
       if (head) { L.bias = nullptr; L.N = p.V; L.kind = PH; L.dst = nullptr; }
-      product<MT, LEFT>(p, L, ln, head ? p.n_rows : p.G, j == 3 && l + 1 == p.L, xs, red, flip, ring, sh);
+      product<MT, LEFT>(p, L, ln, head ? p.n_rows : p.G, last, xs, red, flip, ring, sh);
       if (j == 3) {
         uint32_t* t = prv;
         prv = cur; cur = nxt; nxt = t;
@@ -1098,7 +1103,7 @@ extern "C" int kh_decode_layers_ok(int G, int d, int H, int hd, int max_ctx) {
 extern "C" int kh_decode_layers_rows(int d) { return 8 * max_mt(d); }
 
 // Bytes of the workspace of activations (zero-initialised once, then only used by launches that follow one another).
-extern "C" long kh_decode_layers_work_bytes(int d) { return CTL_BYTES + 2l * 3 * MAX_ROWS * 5 * d * 4; }
+extern "C" long kh_decode_layers_work_bytes(int d) { return CTL_BYTES + 2l * half_words(d) * 4; }
 
 // x [G, d] holds the embedded tokens on entry and the last layer's output on return.  `layers`: device
 // array of L records of twelve bf16 pointers (ln1_w, ln1_b, qkv_w, qkv_b, proj_w, proj_b, ln2_w, ln2_b,

@@ -532,6 +532,30 @@ def test_persistent_decode_workspace_between_steps_of_other_sizes(d, heads):
     assert ops.error_word() == 0
 
 
+@pytest.mark.parametrize("L,heads", [(4, 8), (7, 4), (5, 2)])
+@pytest.mark.parametrize("V", [257, 1000, 50257])
+def test_persistent_decode_head_waits_for_the_last_layer(L, heads, V):
+    """At width 256 some CTAs of a 148-CTA grid have columns of the head and no part in any layer: they come to the head when the kernel starts, and
+    layers before the last have used the words of its slot.  Logits against the kernel chain, per eight columns (one CTA's share): the norm of
+    a block's difference over the mean block's norm.  Two bf16 paths lie 3e-2 apart (the tests above); the worst of 6283 blocks of eight such differences
+    is 2.4 times their mean, below 0.2; logits of another layer would be off by about 1."""
+    cfg = Config(L, 256, heads, V, 64, 1)
+    m = GPT(cfg, "cuda", torch.bfloat16); m.init_weights_device(5); m.params.w.mul_(3.0); m.sync_bf16()
+    e = InferEngine(m, block_size=5, max_seqs=33, max_tokens=320, use_graphs=False)
+    c = InferEngine(m, block_size=5, max_seqs=33, max_tokens=320, persistent_decode=False, use_graphs=False)
+    e.persistent_max = 32
+    prompts = [[(7 * g + i) % V for i in range(2 + g % 7)] for g in range(32)]
+    for G in (1, 8, 32, 1):
+        got = []
+        for eng in (c, e):
+            eng.generate(prompts[:G], 2)                     # one decode step
+            got.append(torch.nn.functional.pad(eng.logits[:G, :V].double(), (0, -V % 8)).view(G, -1, 8))
+        assert e._fused and not c._fused
+        per = (got[0] - got[1]).pow(2).sum((0, 2)).sqrt()
+        assert (per / got[0].pow(2).sum((0, 2)).mean().sqrt()).max().item() < 0.2, (G, per.argmax().item())
+    assert ops.error_word() == 0
+
+
 @pytest.mark.parametrize("G", [1, 8, 20])
 def test_persistent_decode_hands_zeros_on(G):
     """An empty activation word is zero, so results that are zero travel as {-0.0, +0.0}: a model whose every product is zero neither
