@@ -627,21 +627,21 @@ __device__ __forceinline__ void produce(const DecodeParams& p, Ring ring, Shared
     }
     ok = stream(W, head ? p.V : j == 0 ? 3 * d : j == 2 ? 4 * d : d, j == 3 ? 4 * d : d, j & 1 ? 1 : LN_GROUPS, range, ring, sh, p);
   }
-  if (!ok) {                     // given up: no copy may be in flight when the CTA leaves
+  // No copy may be in flight when the CTA leaves, not even where all have been issued and computing warps gave up before they took them: every
+  // slot's last copy is waited for, backwards over the rings (a slot that was never filled passes at once).
 #pragma unroll 1
-    for (int k = 0; k < ring.n_ln; k++) {
-      if (ring.ln_slot == 0) { ring.ln_slot = ring.n_ln; ring.ln_par ^= 1u; }
-      ring.ln_slot--;
-      const uint64_t t0 = kh_globaltimer();
-      while (!mbar_try(ring.ln_full + 8 * ring.ln_slot, ring.ln_par) && kh_globaltimer() - t0 < 100000000ull) {}
-    }
+  for (int k = 0; k < ring.n_ln; k++) {
+    if (ring.ln_slot == 0) { ring.ln_slot = ring.n_ln; ring.ln_par ^= 1u; }
+    ring.ln_slot--;
+    const uint64_t t0 = kh_globaltimer();
+    while (!mbar_try(ring.ln_full + 8 * ring.ln_slot, ring.ln_par) && kh_globaltimer() - t0 < 100000000ull) {}
+  }
 #pragma unroll 1
-    for (int k = 0; k < ring.n; k++) {
-      if (ring.slot == 0) { ring.slot = ring.n; ring.par ^= 1u; }
-      ring.slot--;               // backwards over the ring (a slot that was never filled passes at once)
-      const uint64_t t0 = kh_globaltimer();
-      while (!mbar_try(ring.full + 8 * ring.slot, ring.par) && kh_globaltimer() - t0 < 100000000ull) {}
-    }
+  for (int k = 0; k < ring.n; k++) {
+    if (ring.slot == 0) { ring.slot = ring.n; ring.par ^= 1u; }
+    ring.slot--;
+    const uint64_t t0 = kh_globaltimer();
+    while (!mbar_try(ring.full + 8 * ring.slot, ring.par) && kh_globaltimer() - t0 < 100000000ull) {}
   }
 }
 // Empties this CTA's words of the slot that the next layer writes, as soon as the CTA is done with the same phase of the last layer; the

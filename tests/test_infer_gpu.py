@@ -556,6 +556,30 @@ def test_persistent_decode_head_waits_for_the_last_layer(L, heads, V):
     assert ops.error_word() == 0
 
 
+@pytest.mark.parametrize("d,heads,V,G", [(512, 8, 300, 3), (1024, 16, 20000, 9)])
+def test_persistent_decode_gives_up_and_recovers(d, heads, V, G):
+    """A wait that runs out: the head is asked for a row that is not part of the step, whose words nobody writes.  The launch ends by itself with
+    code 9, whether all of its weight copies have been issued by then (few columns) or not, and the launches after it, one for each half of the
+    workspace, give the bits of the one before."""
+    cfg = Config(5, d, heads, V, 64, 1)
+    m = GPT(cfg, "cuda", torch.bfloat16); m.init_weights_device(5); m.sync_bf16()
+    e = InferEngine(m, block_size=5, max_seqs=33, max_tokens=320, use_graphs=False)
+    e.persistent_max = 32
+    e.generate([[(7 * g + i) % V for i in range(2 + g)] for g in range(G)], 2)
+    assert e._fused and ops.error_word() == 0
+    want, rows = e.logits[:G, :V].clone(), e.d_rows.clone()
+    e.d_rows[G - 1] = G                                      # a row of the workspace, but of no sequence
+    e._forward(G, G, 1)
+    torch.cuda.synchronize()
+    assert ops.error_word() == 9
+    e.d_rows.copy_(rows)
+    for _ in range(3):
+        e.logits.fill_(7.0)
+        e._forward(G, G, 1)
+        assert torch.equal(e.logits[:G, :V], want)
+    assert ops.error_word() == 0
+
+
 @pytest.mark.parametrize("G", [1, 8, 20])
 def test_persistent_decode_hands_zeros_on(G):
     """An empty activation word is zero, so results that are zero travel as {-0.0, +0.0}: a model whose every product is zero neither
