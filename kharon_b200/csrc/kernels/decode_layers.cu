@@ -17,14 +17,16 @@
 // from store to successful poll) and the instructions between two trips.  There is no grid barrier: activations are 32-bit words
 // of two bf16 columns in a workspace whose empty words are zero, and a reader polls the words that it needs until none of
 // them is zero (a result of two +0.0 is written as {-0.0, +0.0}).  A word is a single-copy atomic unit, so a word that is not zero
-// is the result; there are no flags, no extra bytes and no fences on the way.  The words are laid out so that a 128-byte line has
-// one writer (word_at).  Every activation has three slots that the
-// layers use in turn: when a CTA is done with a phase of layer l - 1, a helper warp empties the words that it will write in
-// that phase of layer l + 1 (last used at l - 2; whoever has seen all inputs of the phase at l - 1 knows that their readers are
-// done, since every output of a phase depends on all outputs of the one before), and its fence precedes the CTA's outputs of
-// layer l, so the words are empty before anybody can come to poll them: a reader of layer l + 1 has read that writer's words of
-// layer l.  The head's readers need not have (a width of 256 has 96, 32 and 128 groups of rows for 148 CTAs, so some take part in the head
-// alone and come to it at once), so the output of the last layer has words of its own, written once in a launch.
+// is the result; there are no flags and no extra bytes.  The words are laid out so that a 128-byte line has
+// one writer (word_at).  Every activation has four slots that the layers use in turn.  A slot's second use:
+//  - when a CTA is done with layer m - SLOTS + 1, a helper warp empties the words that it will write in layer m (last used at m - SLOTS;
+//    whoever has seen all inputs of a phase at m - SLOTS + 1 knows that the readers of its own outputs of the layer before are done, since every output of
+//    a phase depends on all outputs of the one before);
+//  - the helpers count each other (a release and an acquire at a global word) and hand the outcome to their own CTA's computing warps, which wait for
+//    it before layer m.  It has been there for a layer or two by then, and those warps execute no fence, which would cost
+//    each of them 0.5 to 1 us a layer (with the stores of a phase in flight; L12 d1024 G = 1 203 us a step with one, 184 so).
+// Every CTA waits so before every layer, also one that takes part in the head alone (a width of 256 has 96, 32 and 128 groups of rows for 148
+// CTAs): it comes to the last layer's output when that is all that can be there.
 // Launches alternate between two halves of the workspace and empty the other half for the next launch, which also
 // repairs what a launch that gave up has left.
 //
@@ -95,7 +97,7 @@ struct DecodeParams {
   int slots;                              // chunks in the ring
   const LayerW* layers;
   bf16* x;                                // [G, d] in: embedded tokens, out: last layer's output
-  uint32_t* words;                        // activations: [2 halves]([3 slots][x d/2 | mid d/2 | att d/2 | qkv 3d/2 | act 4d/2][32 rows], last layer's x)
+  uint32_t* words;                        // activations: [2 halves][4 slots][x d/2 | mid d/2 | att d/2 | qkv 3d/2 | act 4d/2][32 rows]
   bf16 *kc, *vc;                          // [L, blocks, bs, H, hd]
   size_t layer_elems;
   const int *pos, *slot, *btab;
@@ -104,7 +106,7 @@ struct DecodeParams {
   bf16* logits;
   int ld_logits, V, n_rows;
   const int* rows;
-  uint32_t* ctl;                          // [0] launches so far, [2] CTAs that left, [3 + half] rows that the half was last used for, [16..] zeros
+  uint32_t* ctl;                          // [0] launches so far, [2] CTAs that left, [3 + half] rows that the half was last used for, [5 + half] CTAs that have emptied words for a layer, [16..] zeros
   float scale, inv_d;
   uint64_t wait_ns;
   int* err;
@@ -115,7 +117,8 @@ struct DecodeParams {
   __device__ __forceinline__ int block_of(int j) const { return bs == 1 ? j : (int)__umulhi((uint32_t)j, bs_mul); }
 };
 __host__ __device__ constexpr size_t slot_words(int d) { return (size_t)MAX_ROWS * 5 * d; }
-__host__ __device__ constexpr size_t half_words(int d) { return 3 * slot_words(d) + (size_t)MAX_ROWS * (d / 2); }
+constexpr int SLOTS = 4;                      // of every activation: layers that lie between two uses of a word
+__host__ __device__ constexpr size_t half_words(int d) { return SLOTS * slot_words(d); }
 constexpr int CTL_BYTES = 512;                // 64 bytes of counters, and zeros that stand in for cache rows that do not exist
 
 struct Shared {               // small control block behind the data regions
@@ -124,7 +127,8 @@ struct Shared {               // small control block behind the data regions
   int share[4][2];                                  // this CTA's groups of eight weight rows of 3d, d, 4d and V rows
   int item_row[NW][8][4];                           // cache rows of its first keys, per lane group
   volatile int abort_flag;
-  volatile int phase, cleared;                      // phases that the computing warps have entered / whose words of the next layer are empty
+  volatile uint32_t launch;                         // launches before this one
+  volatile int phase, cleared;                      // phases that the computing warps have entered / layer whose words are empty in every CTA
 };
 
 __device__ __forceinline__ uint4 ldg_stream(const void* p) {      // read-once data: do not keep it in L1
@@ -184,6 +188,19 @@ __device__ __forceinline__ void wait_bar(uint32_t bar, uint32_t parity, Shared* 
   const uint64_t t0 = kh_globaltimer();
 #pragma unroll 1
   while (!mbar_try(bar, parity))
+    if (sh->abort_flag || kh_globaltimer() - t0 > limit_ns) { sh->abort_flag = 1; return; }
+}
+// until the words of layer n are empty in every CTA
+__device__ __forceinline__ int ld_cleared(Shared* sh) {
+  int v;
+  asm volatile("ld.acquire.cta.shared.s32 %0, [%1];" : "=r"(v) : "r"(smem_u32(const_cast<int*>(&sh->cleared))) : "memory");
+  return v;
+}
+__device__ __forceinline__ void wait_cleared(int n, Shared* sh, uint64_t limit_ns) {
+  if (ld_cleared(sh) >= n) return;
+  const uint64_t t0 = kh_globaltimer();
+#pragma unroll 1
+  while (ld_cleared(sh) < n)
     if (sh->abort_flag || kh_globaltimer() - t0 > limit_ns) { sh->abort_flag = 1; return; }
 }
 // after an unsuccessful round of a poll: true when the wait is over
@@ -567,9 +584,6 @@ __device__ __forceinline__ void product(const DecodeParams& p, const Lin& L, boo
       }
       const uint32_t pk = pack_bf16(v0, v1);
       if (L.dst) {
-        it = 0;
-#pragma unroll 1
-        while (sh->cleared <= L.seq && !expired(it, sh)) {}       // the next layer's words are empty before these are there
         st_word(L.dst + at, full_word(pk));
         if (last) reinterpret_cast<uint32_t*>(p.x)[(uint32_t)(row * L.N + col) / 2] = pk;
       } else {
@@ -644,44 +658,56 @@ __device__ __forceinline__ void produce(const DecodeParams& p, Ring ring, Shared
     while (!mbar_try(ring.full + 8 * ring.slot, ring.par) && kh_globaltimer() - t0 < 100000000ull) {}
   }
 }
-// Empties this CTA's words of the slot that the next layer writes, as soon as the CTA is done with the same phase of the last layer; the
-// fence and the `cleared` count order that before the phase's own outputs.
+// Empties this CTA's words of layer m, where layer m - SLOTS has used them, and waits for the other CTAs to have done so.
 template <int HD>
-__device__ __forceinline__ void empty_words(const DecodeParams& p, uint32_t* words, size_t block, Shared* sh) {
-  const int d = p.d, lane = threadIdx.x & 31, per = NW >> p.lgw, items = p.G * p.H;
-  const size_t row = (size_t)MAX_ROWS * (d / 2);
+__device__ __forceinline__ void empty_words(const DecodeParams& p, uint32_t* words, Shared* sh) {
+  const int lane = threadIdx.x & 31;
   const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll 1
-  for (int k = 0; k < 5 * p.L; k++) {
-    const int l = k / 5, j = k - 5 * l;
-    uint32_t* nxt = words + (size_t)((l + 1) % 3) * block;
-    const uint64_t t0 = kh_globaltimer();
-    while (sh->phase <= k - 4) {       // until this CTA is done with the same phase of the layer before
+  for (int m = SLOTS; m < p.L; m++) {
+    uint64_t t0 = kh_globaltimer();
+    while (sh->phase <= 5 * (m - SLOTS + 2)) {           // until the CTA has entered the layer after m - SLOTS + 1
       if (sh->abort_flag || kh_globaltimer() - t0 > 2 * p.wait_ns) { sh->abort_flag = 1; return; }
       __nanosleep(50);
     }
-    if (j == 1) {
+    const int d = fresh(p.d), row = MAX_ROWS * (d / 2);
+    uint32_t* const nxt = words + m % SLOTS * (uint32_t)slot_words(d);
+    {
+      const int per = NW >> p.lgw, items = p.G * p.H;
       uint32_t* a = nxt + 2 * row;
 #pragma unroll 1
       for (int it0 = (int)blockIdx.x * per; it0 < items; it0 += (int)gridDim.x * per)
 #pragma unroll 1
         for (int i = lane; i < per * (HD / 8); i += 32) {
           const int it = it0 + i / (HD / 8), t = p.seq_of(it);
-          if (it < items) *reinterpret_cast<uint4*>(a + ((size_t)t * d + (it - t * p.H) * HD) / 2 + (i % (HD / 8)) * 4) = zero;
+          if (it < items) *reinterpret_cast<uint4*>(a + (t * d + (it - t * p.H) * HD) / 2 + (i % (HD / 8)) * 4) = zero;
         }
-    } else {
-      const int N = j == 0 ? 3 * d : j == 3 ? 4 * d : d;
-      uint32_t* a = nxt + (j == 0 ? 3 : j == 2 ? 1 : j == 3 ? 6 : 0) * row;
-      const int* range = sh->share[j == 0 ? 0 : j == 3 ? 2 : 1];
-      const int pitch = j == 3 ? act_pitch(p.G) : GROUP;
+    }
+#pragma unroll 1
+    for (int j = 0; j < 4; j++) {              // qkv, mid, act, x
+      const int N = j == 0 ? 3 * d : j == 2 ? 4 * d : d;
+      uint32_t* a = nxt + (j == 0 ? 3 : j == 1 ? 1 : j == 2 ? 6 : 0) * row;
+      const int* range = sh->share[j == 0 ? 0 : j == 2 ? 2 : 1];
+      const int pitch = j == 2 ? act_pitch(p.G) : GROUP;
 #pragma unroll 1
       for (int r = 0; r < p.G; r += 8)
 #pragma unroll 1
         for (int i = range[0] * pitch + lane * 4; i < range[1] * pitch; i += 128) *reinterpret_cast<uint4*>(a + r / 8 * (4 * N) + i) = zero;
     }
-    __threadfence();
     __syncwarp();
-    if (lane == 0) sh->cleared = k + 1;
+    // Nobody counts for layer m + 1 before all have for m, so that one counter serves all layers
+    uint32_t* const count = p.ctl + 5 + (sh->launch & 1u);
+    if (lane == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(count) : "memory");
+    t0 = kh_globaltimer();
+    while (true) {
+      uint32_t n;
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(n) : "l"(count) : "memory");
+      if (n >= gridDim.x * (uint32_t)(m - SLOTS + 1)) break;
+      if (sh->abort_flag || kh_globaltimer() - t0 > 2 * p.wait_ns) { sh->abort_flag = 1; return; }
+      __nanosleep(100);
+    }
+    __syncwarp();
+    if (lane == 0) asm volatile("st.release.cta.shared.s32 [%0], %1;" ::"r"(smem_u32(const_cast<int*>(&sh->cleared))), "r"(m) : "memory");
   }
 }
 // The other half of the workspace is emptied for the next launch.
@@ -690,9 +716,9 @@ __device__ __forceinline__ void empty_half(const DecodeParams& p, uint32_t half)
   const int me = (int)blockIdx.x * 64 + (int)threadIdx.x % 64, all = (int)gridDim.x * 64;
   uint32_t* w = p.words + (half ^ 1u) * half_words(d);
 #pragma unroll 1
-  for (int s = 0; s < 4; s++)                  // three slots, and the last layer's x
+  for (int s = 0; s < SLOTS; s++)
 #pragma unroll 1
-    for (int f = 0; f < (s < 3 ? 5 : 1); f++) {
+    for (int f = 0; f < 5; f++) {
       const int width = (f < 3 ? d : (f == 3 ? 3 * d : 4 * d)) / 2, from = f < 4 ? f * d / 2 : 3 * d;
       uint4* q = reinterpret_cast<uint4*>(w + s * slot_words(d) + (size_t)MAX_ROWS * from);
 #pragma unroll 1
@@ -922,9 +948,6 @@ __device__ __forceinline__ void attention_phase(const DecodeParams& p, int layer
       }
       const float inv = 1.f / den;
       const int tt = p.seq_of(it);
-      uint32_t wt = 0;
-#pragma unroll 1
-      while (sh->cleared <= seq && !expired(wt, sh)) {}
       if (it < items) st_word(attw + ((size_t)tt * d + (it - tt * H) * HD + e) / 2, full_word(pack_bf16(v0 * inv, v1 * inv)));
     }
     compute_sync();                // satt is reused by the next turn or layer
@@ -952,7 +975,8 @@ __global__ void __launch_bounds__(THREADS, 1) decode_layers_k(const __grid_const
   Ring ring = {smem_u32(smem), smem_u32(sh->full), smem_u32(sh->empty), smem_u32(sh->ln_full), smem_u32(sh->ln_empty), p.slots, 0, 0u, sln, n_ln(d), 0, 0u};
   if (threadIdx.x == 0) {
     sh->abort_flag = 0;
-    sh->phase = sh->cleared = 0;
+    sh->phase = 0;
+    sh->cleared = SLOTS - 1;             // (the launch starts with empty slots)
     for (int s = 0; s < p.slots; s++) { mbar_init(ring.full + 8 * s, 1); mbar_init(ring.empty + 8 * s, NW); }
     for (int s = 0; s < 2; s++) { mbar_init(ring.ln_full + 8 * s, 1); mbar_init(ring.ln_empty + 8 * s, NW); }
     mbar_fence_init();
@@ -962,19 +986,21 @@ __global__ void __launch_bounds__(THREADS, 1) decode_layers_k(const __grid_const
     const unsigned groups = (unsigned)(k == 0 ? 3 * d : k == 1 ? d : k == 2 ? 4 * d : p.V + 7) / 8;
     sh->share[k][e] = (int)(groups * (blockIdx.x + e) / gridDim.x);
   }
-  __syncthreads();
   // launches before this one: constant while it runs (only its last CTA to leave advances the word)
-  const uint32_t launch = *reinterpret_cast<volatile uint32_t*>(p.ctl), half = launch & 1u;
-  const size_t block = slot_words(d);
-  uint32_t* const words = p.words + half * half_words(d);
+  if (threadIdx.x == 0) sh->launch = *reinterpret_cast<volatile uint32_t*>(p.ctl);
+  __syncthreads();
 
   if (warp >= NW) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
+    const uint32_t half = sh->launch & 1u;
     if (warp == NW) produce(p, ring, sh);
-    else if (warp == NW + 1) empty_words<HD>(p, words, block, sh);
+    else if (warp == NW + 1) empty_words<HD>(p, p.words + half * half_words(d), sh);
     else {
       empty_half(p, half);
-      if (blockIdx.x == 0 && threadIdx.x == CT + 64) p.ctl[3 + half] = (uint32_t)p.G;
+      if (blockIdx.x == 0 && threadIdx.x == CT + 64) {
+        p.ctl[3 + half] = (uint32_t)p.G;
+        p.ctl[5 + (half ^ 1u)] = 0u;
+      }
     }
   } else {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 232;");
@@ -1000,13 +1026,14 @@ __global__ void __launch_bounds__(THREADS, 1) decode_layers_k(const __grid_const
     unsigned long long rec = record(0), nrec = record(1);
     auto ptr = [&](unsigned long long r, int i) { return reinterpret_cast<const bf16*>(__shfl_sync(0xffffffffu, r, i)); };
     int flip = 0;
-    uint32_t *cur = words, *nxt = words + block, *prv = words + 2 * block;      // slots of this layer, the next and the last
+    const uint32_t block = (uint32_t)slot_words(p.d);
+    uint32_t *cur = p.words + (sh->launch & 1u) * half_words(p.d), *nxt = cur + block, *nx2 = nxt + block, *prv = nx2 + block;
 #pragma unroll 1
     for (int k = 0; k < 4 * p.L + (p.head_w ? 1 : 0); k++) {
       const int l = k >> 2, j = k & 3, d = fresh(p.d);
       const uint32_t row = (uint32_t)MAX_ROWS * (d / 2);    // words: x at 0, mid at row, att at 2 row, qkv at 3 row, act at 6 row
-      const bool head = k == 4 * p.L, ln = (j & 1) == 0, last = j == 3 && l + 1 == p.L;
-      uint32_t* const out = words + 3 * block;              // the last layer's x
+      const bool head = k == 4 * p.L, ln = (j & 1) == 0;
+      if (j == 0 && !head) wait_cleared(l, sh, p.wait_ns);
       if (j == 1) attention_phase<MT, HD>(p, l, 5 * l + 1, cur + 3 * row, cur + 2 * row, satt, sh);
       Lin L;
       L.bias = ptr(rec, j == 0 ? 3 : j == 1 ? 5 : j == 2 ? 9 : 11);
@@ -1014,14 +1041,14 @@ __global__ void __launch_bounds__(THREADS, 1) decode_layers_k(const __grid_const
       L.N = j == 0 ? 3 * d : j == 2 ? 4 * d : d;
       L.kind = j == 0 ? PA : j == 1 ? PC : j == 2 ? PD : PE;
       L.seq = 5 * l + (j == 0 ? 0 : j + 1);
-      L.src = j == 0 ? (l ? (head ? out : prv) : nullptr) : cur + (j == 1 ? 2 : j == 2 ? 1 : 6) * row;
+      L.src = j == 0 ? (l ? prv : nullptr) : cur + (j == 1 ? 2 : j == 2 ? 1 : 6) * row;
       L.res = j == 1 ? (l ? prv : nullptr) : j == 3 ? cur + row : nullptr;
-      L.dst = last ? out : cur + (j == 0 ? 3 : j == 1 ? 1 : j == 2 ? 6 : 0) * row;
+      L.dst = cur + (j == 0 ? 3 : j == 1 ? 1 : j == 2 ? 6 : 0) * row;
       if (head) { L.bias = nullptr; L.N = p.V; L.kind = PH; L.dst = nullptr; }
-      product<MT, LEFT>(p, L, ln, head ? p.n_rows : p.G, last, xs, red, flip, ring, sh);
+      product<MT, LEFT>(p, L, ln, head ? p.n_rows : p.G, j == 3 && l + 1 == p.L, xs, red, flip, ring, sh);
       if (j == 3) {
         uint32_t* t = prv;
-        prv = cur; cur = nxt; nxt = t;
+        prv = cur; cur = nxt; nxt = nx2; nx2 = t;
         rec = nrec;                    // (layer l + 2 is requested two layers ahead of its first use)
         nrec = record(l + 2);
       }
@@ -1030,6 +1057,7 @@ __global__ void __launch_bounds__(THREADS, 1) decode_layers_k(const __grid_const
   __syncthreads();
   if (threadIdx.x == 0) {
     if (sh->abort_flag) atomicCAS(p.err, 0, 9);
+    const uint32_t launch = sh->launch;
     __threadfence();
     if (atomicAdd(p.ctl + 2, 1u) == gridDim.x - 1) {
       p.ctl[2] = 0;

@@ -532,14 +532,13 @@ def test_persistent_decode_workspace_between_steps_of_other_sizes(d, heads):
     assert ops.error_word() == 0
 
 
-@pytest.mark.parametrize("L,heads", [(4, 8), (7, 4), (5, 2)])
-@pytest.mark.parametrize("V", [257, 1000, 50257])
-def test_persistent_decode_head_waits_for_the_last_layer(L, heads, V):
-    """At width 256 some CTAs of a 148-CTA grid have columns of the head and no part in any layer: they come to the head when the kernel starts, and
-    layers before the last have used the words of its slot.  Logits against the kernel chain, per eight columns (one CTA's share): the norm of
+@pytest.mark.parametrize("L,d,heads,V", [(L, 256, h, V) for L, h in ((4, 8), (5, 2), (7, 4)) for V in (257, 1000, 50257)] + [(13, 512, 8, 1000), (9, 1024, 16, 1000)])
+def test_persistent_decode_slots_of_many_layers(L, d, heads, V):
+    """Models with more layers than an activation has slots.  At width 256 some CTAs of a 148-CTA grid have columns of the head and no part in any layer: without a
+    wait they come to the head when the kernel starts, and layers before the last have used the words of its slot.  Logits against the kernel chain, per eight columns (one CTA's share): the norm of
     a block's difference over the mean block's norm.  Two bf16 paths lie 3e-2 apart (the tests above); the worst of 6283 blocks of eight such differences
     is 2.4 times their mean, below 0.2; logits of another layer would be off by about 1."""
-    cfg = Config(L, 256, heads, V, 64, 1)
+    cfg = Config(L, d, heads, V, 64, 1)
     m = GPT(cfg, "cuda", torch.bfloat16); m.init_weights_device(5); m.params.w.mul_(3.0); m.sync_bf16()
     e = InferEngine(m, block_size=5, max_seqs=33, max_tokens=320, use_graphs=False)
     c = InferEngine(m, block_size=5, max_seqs=33, max_tokens=320, persistent_decode=False, use_graphs=False)
