@@ -93,7 +93,7 @@ struct LayerW {               // bf16 pointers of one layer (device array, one e
 
 struct DecodeParams {
   int G, d, H, L, bs, max_lb, max_ctx;
-  int lgw;                                // log2 of the warps per attention item
+  int lgw;                                // log2 of the warps per attention item that keep all items in one turn
   int slots;                              // chunks in the ring
   const LayerW* layers;
   bf16* x;                                // [G, d] in: embedded tokens, out: last layer's output
@@ -128,6 +128,7 @@ struct Shared {               // small control block behind the data regions
   int item_row[NW][8][4];                           // cache rows of its first keys, per lane group
   volatile int abort_flag;
   volatile uint32_t launch;                         // launches before this one
+  volatile int lgw;                                 // log2 of the warps per attention item
   volatile int phase, cleared;                      // phases that the computing warps have entered / layer whose words are empty in every CTA
 };
 
@@ -673,7 +674,7 @@ __device__ __forceinline__ void empty_words(const DecodeParams& p, uint32_t* wor
     const int d = fresh(p.d), row = MAX_ROWS * (d / 2);
     uint32_t* const nxt = words + m % SLOTS * (uint32_t)slot_words(d);
     {
-      const int per = NW >> p.lgw, items = p.G * p.H;
+      const int per = NW >> sh->lgw, items = p.G * p.H;
       uint32_t* a = nxt + 2 * row;
 #pragma unroll 1
       for (int it0 = (int)blockIdx.x * per; it0 < items; it0 += (int)gridDim.x * per)
@@ -726,21 +727,38 @@ __device__ __forceinline__ void empty_half(const DecodeParams& p, uint32_t half)
     }
 }
 
+// log2 of the warps per attention item (whole warp, the same in every CTA).  All items in one turn leave many CTAs without one where they do not
+// divide well (G = 24, 16 heads: 96 of 148 with two warps to an item); more warps to an item then take less time over long contexts, in spite of
+// what a turn costs beside its positions, which is what a warp does in 30 of them.
+__device__ __forceinline__ int item_warps(const DecodeParams& p) {
+  const int lane = threadIdx.x & 31, items = p.G * p.H;
+  int far = lane < p.G ? p.pos[lane] : 0;
+  far = min(__reduce_max_sync(0xffffffffu, far), p.max_ctx);
+  int best = p.lgw, cost = 0x7fffffff;
+#pragma unroll 1
+  for (int lg = p.lgw; lg <= 3; lg++) {
+    const int per = (int)gridDim.x * (NW >> lg), c = (items + per - 1) / per * (30 + (far >> lg));
+    if (c < cost) { cost = c; best = lg; }
+  }
+  return best;
+}
 // ------------------------------------------------------------------------------------------------
 // Positions that a lane group (four lanes) holds at a time: the 16 rows of a score product; twice as many for many sequences with narrow heads,
 // whose rows are short (L4 d512 H16 G = 32, contexts of 20 / 200 / 900: 116 / 131 / 194 us a step, 105 / 125 / 216 with two; d256 H8 100 / 108 /
-// 135 and 93 / 103 / 142), but not elsewhere (head width 64, L12 d1024 G = 8, 160: 205 us with two, 222 with four).
-template <int MT, int HD> constexpr int keys_ahead() { return HD == 32 && MT == 4 ? 4 : 2; }
+// 135 and 93 / 103 / 142), and for such heads in models of long contexts (L4 d512 H16, G = 1 at 20 / 1000 / 4000 / 16000 positions 57 / 76 / 156 / 507 us with
+// two, 59 / 73 / 131 / 391 with four), but not elsewhere (head width 64, L12 d1024 G = 8, 160: 205 us with two, 222 with four; L4 G = 8, 16000: 839
+// and 824).
+constexpr int LONG_CTX = 2048;
 // Bytes of a layer's keys and values up to which the next layer's are prefetched into L2; beyond, they are gone before they are used and
 // come from memory twice (G = 32, 900 positions, 118 MB: L12 d1024 977 us with, 889 without; 59 MB, G = 16: 492 and 500; 65 MB, L4 d2048 G = 8: 252 and 240).
 constexpr float FETCH_LIMIT = 60e6f;
 // Phase B.  Appends the new k, v to the paged cache and attends over positions 0..pos.
 // The W warps of an item hold 8 W lane groups; group i takes positions i, i + 8 W, i + 16 W, ...; the group that would take `pos` starts with
 // the new key and value.
-template <int MT, int HD>
+template <int MT, int HD, int NB>
 __device__ __forceinline__ void attention_phase(const DecodeParams& p, int layer, int seq, const uint32_t* qkvw, uint32_t* attw, float* satt, Shared* sh) {
-  constexpr int NB = keys_ahead<MT, HD>(), NC = HD / 32;      // 16-byte pieces of a row per lane
-  const int tid = tid_fresh(), warp = tid >> 5, lane = tid & 31, lgw = fresh(p.lgw), H = fresh(p.H), bid = fresh(blockIdx.x);
+  constexpr int NC = HD / 32;      // 16-byte pieces of a row per lane
+  const int tid = tid_fresh(), warp = tid >> 5, lane = tid & 31, lgw = sh->lgw, H = fresh(p.H), bid = fresh(blockIdx.x);
   if (tid == 0) sh->phase = seq + 1;
   const int W = 1 << lgw, slots = NW >> lgw, ST = W * 8;
   const int first = (warp & (W - 1)) * 8, kg = first + (lane >> 2), e0 = (lane & 3) * 8;       // (first: uniform over the warp)
@@ -956,7 +974,7 @@ __device__ __forceinline__ void attention_phase(const DecodeParams& p, int layer
 
 __host__ __device__ constexpr int n_ln(int d) { return d <= 1536 ? 2 : 1; }     // buffers of LayerNorm gain and bias (wide models: the ring is no deeper than a phase)
 
-template <int MT, int HD, int LEFT>
+template <int MT, int HD, int NB, int LEFT>
 __global__ void __launch_bounds__(THREADS, 1) decode_layers_k(const __grid_constant__ DecodeParams p) {
   extern __shared__ __align__(128) uint8_t smem[];
   const int d = p.d;
@@ -988,6 +1006,7 @@ __global__ void __launch_bounds__(THREADS, 1) decode_layers_k(const __grid_const
   }
   // launches before this one: constant while it runs (only its last CTA to leave advances the word)
   if (threadIdx.x == 0) sh->launch = *reinterpret_cast<volatile uint32_t*>(p.ctl);
+  if (warp == 1) sh->lgw = item_warps(p);
   __syncthreads();
 
   if (warp >= NW) {
@@ -1006,8 +1025,8 @@ __global__ void __launch_bounds__(THREADS, 1) decode_layers_k(const __grid_const
     asm volatile("setmaxnreg.inc.sync.aligned.u32 232;");
     const int lane = threadIdx.x & 31;
     if (p.L > 0) {                  // this warp's first attention item and the cache rows of its first keys
-      const int W = 1 << p.lgw, ST = W * 8;
-      const int item = (int)blockIdx.x * (NW >> p.lgw) + (warp >> p.lgw), kg = (warp & (W - 1)) * 8 + (lane >> 2);
+      const int lgw = sh->lgw, W = 1 << lgw, ST = W * 8;
+      const int item = (int)blockIdx.x * (NW >> lgw) + (warp >> lgw), kg = (warp & (W - 1)) * 8 + (lane >> 2);
       if (item < p.G * p.H) {
         const int pos = p.pos[item / p.H], slot = p.slot[item / p.H];
         auto row_at = [&](int j) {
@@ -1017,7 +1036,7 @@ __global__ void __launch_bounds__(THREADS, 1) decode_layers_k(const __grid_const
         const bool good = pos >= 0 && slot >= 0 && pos < p.max_ctx && p.block_of(pos) < p.max_lb;
         if (lane == 0) { sh->item_pos[warp] = pos; sh->item_slot[warp] = slot; sh->pos_row[warp] = good ? row_at(pos) : 0; }
         const int i = lane & 3;
-        if (good && i < keys_ahead<MT, HD>() && kg + i * ST < pos) sh->item_row[warp][lane >> 2][i] = row_at(kg + i * ST);
+        if (good && i < NB && kg + i * ST < pos) sh->item_row[warp][lane >> 2][i] = row_at(kg + i * ST);
       }
       __syncwarp();
     }
@@ -1034,7 +1053,7 @@ __global__ void __launch_bounds__(THREADS, 1) decode_layers_k(const __grid_const
       const uint32_t row = (uint32_t)MAX_ROWS * (d / 2);    // words: x at 0, mid at row, att at 2 row, qkv at 3 row, act at 6 row
       const bool head = k == 4 * p.L, ln = (j & 1) == 0;
       if (j == 0 && !head) wait_cleared(l, sh, p.wait_ns);
-      if (j == 1) attention_phase<MT, HD>(p, l, 5 * l + 1, cur + 3 * row, cur + 2 * row, satt, sh);
+      if (j == 1) attention_phase<MT, HD, NB>(p, l, 5 * l + 1, cur + 3 * row, cur + 2 * row, satt, sh);
       Lin L;
       L.bias = ptr(rec, j == 0 ? 3 : j == 1 ? 5 : j == 2 ? 9 : 11);
       L.K = j == 3 ? 4 * d : d;
@@ -1079,13 +1098,13 @@ constexpr int ring_slots(int MT, int d) {
 constexpr int max_mt(int d) { return d <= 1536 ? 4 : (d <= 3328 ? 2 : 1); }
 static_assert(ring_slots(4, 1024) >= 4 && ring_slots(4, 1536) >= 4 && ring_slots(2, 3328) >= 4 && ring_slots(1, 4096) >= 4, "a turn's chunks fit");
 
-template <int MT, int HD, int LEFT>
+template <int MT, int HD, int NB, int LEFT>
 int launch(DecodeParams& p, int grid, cudaStream_t st) {
   p.slots = ring_slots(MT, p.d);
   const int smem = p.slots * SLOT + fixed_bytes(MT, p.d);
   p.lgw = 3;                                    // as many warps per (sequence, head) as keep all items in one turn
   while (p.lgw > 0 && (long)p.G * p.H << p.lgw > (long)grid * NW) p.lgw--;
-  cudaError_t e = cudaFuncSetAttribute(decode_layers_k<MT, HD, LEFT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  cudaError_t e = cudaFuncSetAttribute(decode_layers_k<MT, HD, NB, LEFT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) { kh_set_error("decode_layers: shared memory opt-in failed: %s", cudaGetErrorString(e)); return -1; }
   // cooperative launch: the driver guarantees that all CTAs are resident together (or refuses the launch)
   cudaLaunchConfig_t cfg = {};
@@ -1094,15 +1113,18 @@ int launch(DecodeParams& p, int grid, cudaStream_t st) {
   at[0].id = cudaLaunchAttributeCooperative;
   at[0].val.cooperative = 1;
   cfg.attrs = at; cfg.numAttrs = 1;
-  e = cudaLaunchKernelEx(&cfg, decode_layers_k<MT, HD, LEFT>, p);
+  e = cudaLaunchKernelEx(&cfg, decode_layers_k<MT, HD, NB, LEFT>, p);
   if (e != cudaSuccess) { kh_set_error("decode_layers launch failed: %s", cudaGetErrorString(e)); return -1; }
   return 0;
 }
 template <int HD, int LEFT>
 int launch_rows(DecodeParams& p, int rows, int grid, cudaStream_t st) {
-  if (rows <= 8) return launch<1, HD, LEFT>(p, grid, st);
-  if (rows <= 16) return launch<2, HD, LEFT>(p, grid, st);
-  return launch<4, HD, LEFT>(p, grid, st);
+  if constexpr (HD == 32) {
+    if (rows <= 16 && p.max_ctx > LONG_CTX) return rows <= 8 ? launch<1, HD, 4, LEFT>(p, grid, st) : launch<2, HD, 4, LEFT>(p, grid, st);
+  }
+  if (rows <= 8) return launch<1, HD, 2, LEFT>(p, grid, st);
+  if (rows <= 16) return launch<2, HD, 2, LEFT>(p, grid, st);
+  return launch<4, HD, HD == 32 ? 4 : 2, LEFT>(p, grid, st);
 }
 template <int HD>
 int launch_width(DecodeParams& p, int rows, int grid, cudaStream_t st) {

@@ -280,13 +280,14 @@ class InferEngine:
         return (runs, rest) if runs and ntok * self.Hl >= least else None
 
     def _one_kernel(self, ntok, nseq):
-        """Whether this step runs in the persistent kernel.  Beyond 4096 positions its W warps per (sequence, head) lose to the
-        chain's split-KV attention once the sequences fill the SMs (L4 d1024, us a step, persistent / chain: context 4000 of 4096
-        G = 17 503 / 562, 32 879 / 713; 8100 G = 16 837 / 957, 17 880 / 819, 24 1586 / 1011; 16300 G = 17 1650 / 1389, 32 3164 / 2179; 200 of
-        4096 G = 17 144 / 223, 32 170 / 234; eight heads, context 8000, G = 17 845 / 988, 32 1549 / 1388)."""
+        """Whether this step runs in the persistent kernel.  Over long contexts its W warps per (sequence, head) lose to the chain's
+        attention (split-KV where the model has more than 2048 positions) once the sequences fill the SMs.  L4 d1024, 4200 positions, us a step, persistent / chain:
+        sixteen heads, contexts 200 / 2000 / 3000 / 4000: G = 17 143 / 213, 319 / 437, 413 / 477, 511 / 501; 24 161 / 219, 436 / 480, 575 / 543, 715 / 571; 32 170 / 223,
+        521 / 525, 701 / 621, 885 / 674; eight heads, 2000 / 3000 / 4000: 24 484 / 575, 652 / 636, 826 / 674; 32 501 / 639, 673 / 742, 848 / 791.  Context 8100 of
+        16400: sixteen heads, G = 17 895 / 818, 24 1290 / 936; eight heads, 17 (136 items for 148 SMs) 849 / 960, 24 1527 / 1133."""
         if not (self.persistent and ntok == nseq and ntok <= self.persistent_max and ntok <= 32):
             return False
-        return ntok <= 16 or ntok * self.Hl <= 148 or int(self.np_meta[self._o_pos:self._o_pos + ntok].max()) < 4096
+        return ntok <= 16 or ntok * self.Hl <= 148 or int(self.np_meta[self._o_pos:self._o_pos + ntok].max()) < (4096 if ntok <= 20 else 2560)
 
     def _run(self, ntok, nseq, rep=1):
         """Metadata is already in ``h_meta``; runs one step and returns the sampled ids (host)."""

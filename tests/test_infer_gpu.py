@@ -249,6 +249,31 @@ def test_persistent_decode_steps_against_the_chain(d, heads, G, ctx):
     assert ops.error_word() == 0
 
 
+@pytest.mark.parametrize("d,heads,G,ctx,seq", [(512, 16, 24, 1500, 2000), (512, 8, 31, 900, 1000), (1024, 8, 30, 40, 100), (256, 8, 3, 2100, 4096),
+                                               (512, 16, 12, 70, 4096), (512, 16, 16, 2500, 4096), (256, 8, 32, 700, 4096)])
+def test_persistent_decode_attention_over_long_contexts(d, heads, G, ctx, seq):
+    """More warps to an attention item than one turn has room for (17 to 32 sequences whose longest context outweighs another turn, and not), and
+    four positions a lane group for heads of 32 in models of more than 2048 positions, at short and long contexts.  Bounds of the test above."""
+    cfg = Config(2, d, heads, 601, seq, 1)
+    m = GPT(cfg, "cuda", torch.bfloat16)
+    m.init_weights_device(5)
+    m.params.w.mul_(3.0); m.sync_bf16()
+    gen = torch.Generator().manual_seed(d + G)
+    prompts = [torch.randint(0, 601, (int(n),), generator=gen).tolist() for n in torch.randint(max(1, ctx // 9), ctx + 1, (G,), generator=gen)]
+    out = {}
+    for flag in (False, True):
+        e = InferEngine(m, block_size=16, max_seqs=G + 1, n_blocks=G * (ctx // 16 + 2) + 8, max_tokens=G * ctx + 64, persistent_decode=flag, use_graphs=False)
+        e.persistent_max = 32
+        e.generate(prompts, 2)                           # prefill, then one decode step
+        assert e._fused == flag
+        out[flag] = (e.logits[:G, :601].float().clone(), e.kc[0].float().clone(), e.vc[0].float().clone())
+    for i, tol in ((0, 3e-2), (1, 2.0 ** -7), (2, 2.0 ** -7)):
+        x, y = out[False][i], out[True][i]
+        err = ((x - y).norm() / x.norm()).item()
+        assert err < tol, (i, err)
+    assert ops.error_word() == 0
+
+
 def test_fp32_engine_on_gpu_is_token_exact():
     """The fp32 configuration on the GPU (fp32 weights, activations and KV pool; products on the
     CUDA-core fp32 kernel) reproduces the fp32 CPU engine token for token -- staggered continuous
