@@ -312,15 +312,17 @@ __device__ __forceinline__ void out_pair(int o, int& g, int& row, int& c) {
 }
 constexpr int n_red(int MT) { return MT == 4 ? 1 : 2; }        // buffers of partial sums (shared memory for a second one lacks at 32 rows)
 
-// Steps of a quad that exist, known at compile time for widths 256 and 512 (LEFT = 1, 2: a LayerNorm's only quad) and multiples of 1024 (LEFT = 4,
-// every quad): without the branches of the general form (LEFT = 0) the pieces of a row are worked on together.
+// Steps of a quad that exist, known at compile time where a row is one partial quad (widths below 1024: LEFT = 1, 2, 3, a LayerNorm's only quad) and
+// for multiples of 1024 (LEFT = 4, every quad): without the branches of the general form (LEFT = 0) the pieces of a row are worked on together.  us a
+// step, four layers, general form / this: d256 H8 G = 1 57.4 / 51.6, 32 114.5 / 96.7; d512 H8 G = 1 61.5 / 55.8, 16 83.1 / 74.0; d768 H12 G = 1
+// 63.8 / 59.5, 32 139.7 / 122.5; d512 H4 G = 32 131 / 113.5.
 template <int LEFT> __device__ __forceinline__ int steps_left(int st, int first) { return LEFT ? LEFT : st - first; }
 
 // LayerNorm of rows [0, n) -> xs [8 MT][K + PAD]: the warps fetch the fragments that they will multiply, then a warp takes a row, pieces
 // lane, lane + 32, ... of 16 bytes in blocks of four.
 template <int MT, int LEFT>
 __device__ __forceinline__ void normalise(const DecodeParams& p, const Lin& L, int n, bf16* xs, Ring& ring, Shared* sh) {
-  const int tid = tid_fresh(), warp = tid >> 5, lane = tid & 31, d = L.K, st = LEFT == 1 || LEFT == 2 ? LEFT : d >> 8;
+  const int tid = tid_fresh(), warp = tid >> 5, lane = tid & 31, d = L.K, st = LEFT && LEFT < 4 ? LEFT : d >> 8;
   const uint32_t pitch = (d + PAD) * 2, ln = smem_u32(ring.ln) + ring.ln_slot * (4 * d) + lane * 16;
   {
     const uint32_t to = smem_u32(xs) + (lane >> 2) * pitch + warp * 64 + (lane & 3) * 16;
@@ -363,7 +365,7 @@ __device__ __forceinline__ void normalise(const DecodeParams& p, const Lin& L, i
       for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
       return a;
     };
-    const bool one = (LEFT == 1 || LEFT == 2) || st <= 4;       // one block: it stays in registers
+    const bool one = (LEFT && LEFT < 4) || st <= 4;       // one block: it stays in registers
     load(0);
     int b = 0;
 #pragma unroll 1
@@ -1129,10 +1131,7 @@ int launch_rows(DecodeParams& p, int rows, int grid, cudaStream_t st) {
 template <int HD>
 int launch_width(DecodeParams& p, int rows, int grid, cudaStream_t st) {
   if (p.d % 1024 == 0) return launch_rows<HD, 4>(p, rows, grid, st);
-  if constexpr (HD < 128) {
-    if (p.d == 256) return launch_rows<HD, 1>(p, rows, grid, st);
-    if (p.d == 512) return launch_rows<HD, 2>(p, rows, grid, st);
-  }
+  if (p.d < 1024) return p.d == 256 ? launch_rows<HD, 1>(p, rows, grid, st) : p.d == 512 ? launch_rows<HD, 2>(p, rows, grid, st) : launch_rows<HD, 3>(p, rows, grid, st);
   return launch_rows<HD, 0>(p, rows, grid, st);
 }
 int launch_any(DecodeParams& p, int hd, int rows, int grid, cudaStream_t st) {
