@@ -782,51 +782,57 @@ __device__ __forceinline__ uint4 xent_grad8(f32x2 (&e)[4], int c, int t, float s
   }
   return o;
 }
-// XK
-__global__ void xent_k(bf16* __restrict__ logits, int ld, int V, const int* __restrict__ target,
-                       const float* __restrict__ coef, float uniform, float* __restrict__ rowloss,
-                       float* __restrict__ prob, int write_grad) {
+// A CTA per row: 512 threads (VT = 1), or 256 that do the work of two each (VT = 2), so that loss and probability of a row have the same bits
+// in both forms.
+template <int VT>
+__global__ void __launch_bounds__(512 / VT) xent_k(bf16* __restrict__ logits, int ld, int V, const int* __restrict__ target,
+                                                   const float* __restrict__ coef, float uniform, float* __restrict__ rowloss,
+                                                   float* __restrict__ prob, int write_grad) {
   pdl_wait();
   pdl_launch_dependents();
-  __shared__ float s_m[32], s_s[32];
+  constexpr int T = 512 / VT;
+  __shared__ float s_m[16], s_s[16];
   __shared__ float s_max, s_sum;
-  const int r = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
+  const int r = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   bf16* row = logits + (size_t)r * ld;
   const uint4* rp = reinterpret_cast<const uint4*>(row);
-  float m = -INFINITY, s = 0.f;
   const int nv = V / 8;
-  f32x2 s0 = 0, s1 = 0;
+#pragma unroll 1
+  for (int vt = tid; vt < 512; vt += T) {
+    float m = -INFINITY, s = 0.f;
+    f32x2 s0 = 0, s1 = 0;
 #pragma unroll 2
-  for (int i = tid; i < nv; i += blockDim.x) {
-    const uint4 v = rp[i];
-    const f32x2 m2 = un2(xent_max8(v, 0, 8));
-    const float mx = fmaxf(lo2(m2), hi2(m2));
-    if (mx > m) {
-      const float c = __expf(m - mx);
-      s0 = mul2(s0, mk2(c, c)); s1 = mul2(s1, mk2(c, c));
-      m = mx;
+    for (int i = vt; i < nv; i += 512) {
+      const uint4 v = rp[i];
+      const f32x2 m2 = un2(xent_max8(v, 0, 8));
+      const float mx = fmaxf(lo2(m2), hi2(m2));
+      if (mx > m) {
+        const float c = __expf(m - mx);
+        s0 = mul2(s0, mk2(c, c)); s1 = mul2(s1, mk2(c, c));
+        m = mx;
+      }
+      const float nm = m == -INFINITY ? 0.f : -m;      // a masked run: its exponentials are 0
+      f32x2 e[4];
+      xent_exp8(v, 0, 8, mk2(nm, nm), e);
+      s0 = add2(s0, add2(e[0], e[1])); s1 = add2(s1, add2(e[2], e[3]));
     }
-    const float nm = m == -INFINITY ? 0.f : -m;      // a masked run: its exponentials are 0
-    f32x2 e[4];
-    xent_exp8(v, 0, 8, mk2(nm, nm), e);
-    s0 = add2(s0, add2(e[0], e[1])); s1 = add2(s1, add2(e[2], e[3]));
+    s0 = add2(s0, s1);
+    s = lo2(s0) + hi2(s0);
+    if (nv * 8 + vt < V) {
+      const float x = __bfloat162float(row[nv * 8 + vt]);
+      if (x > m) { s *= __expf(m - x); m = x; }
+      s += m == x && x == -INFINITY ? 0.f : __expf(x - m);
+    }
+    // combine (m, s) pairs in a fixed tree
+    const float wm = warp_max(m);
+    s *= (m == -INFINITY) ? 0.f : __expf(m - wm);
+    s = warp_sum(s);
+    if (lane == 0) { s_m[vt >> 5] = wm; s_s[vt >> 5] = s; }
   }
-  s0 = add2(s0, s1);
-  s = lo2(s0) + hi2(s0);
-  for (int i = nv * 8 + tid; i < V; i += blockDim.x) {
-    float x = __bfloat162float(row[i]);
-    if (x > m) { s *= __expf(m - x); m = x; }
-    s += m == x && x == -INFINITY ? 0.f : __expf(x - m);
-  }
-  // combine (m, s) pairs in a fixed tree
-  float wm = warp_max(m);
-  s *= (m == -INFINITY) ? 0.f : __expf(m - wm);
-  s = warp_sum(s);
-  if (lane == 0) { s_m[warp] = wm; s_s[warp] = s; }
   __syncthreads();
   if (warp == 0) {
-    float mm = lane < nw ? s_m[lane] : -INFINITY;
-    float ss = lane < nw ? s_s[lane] : 0.f;
+    float mm = lane < 16 ? s_m[lane] : -INFINITY;
+    float ss = lane < 16 ? s_s[lane] : 0.f;
     float gm = warp_max(mm);
     ss *= (mm == -INFINITY) ? 0.f : __expf(mm - gm);
     ss = warp_sum(ss);
@@ -927,11 +933,11 @@ extern "C" int kh_xent(void* logits, int ld, int V, const void* target, const vo
     else if (ld <= 1024) KH_XENT(xent_warp_k<4>, grid, 256, 0, rows);
     else KH_XENT(xent_warp_k<8>, grid, 256, 0, rows);
   } else {
-    // Eight CTAs of 256 threads an SM wait for less than four of 512 (8192 x 4000 38.4 / 51.9 us, 8192 x 8192 59.8 / 76.4; loss only, 8192 x 50257
-    // 136.8 / 148.0), but the gradient's second pass finds its row in L2 only while the rows in flight fit there (4096 x 32000 109.4 / 102.6,
-    // 8192 x 50257 382 / 321; 16000 columns, 38 MB, 103.0 / 118.9), and rows
-    // that are all resident with 512 threads want them (100 x 16000 6.7 / 5.4).
-    KH_XENT(xent_k, rows, rows > 4 * ew_sms() && (!write_grad || ld <= 16384) ? 256 : 512, 0);
+    // Eight CTAs of 256 threads an SM wait for less than four of 512 (8192 x 4000 43.1 / 50.2 us, 8192 x 8192 62.9 / 73.1, 8192 x 16000 105.4 / 115.8; loss only,
+    // 4096 x 8192 19.6 / 21.2, 8192 x 50257 151.8 / 154.8), but the gradient's second pass finds its row in L2 only while the rows in flight fit there
+    // (4096 x 32000 109.4 / 102.6, 8192 x 50257 382 / 321), and rows that are all resident with 512 threads want them (100 x 16000 6.7 / 5.4).
+    if (rows > 4 * ew_sms() && (!write_grad || ld <= 16384)) KH_XENT(xent_k<2>, rows, 256, 0);
+    else KH_XENT(xent_k<1>, rows, 512, 0);
   }
 #undef KH_XENT
   KH_LAUNCH_CHECK("xent");

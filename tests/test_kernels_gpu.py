@@ -344,6 +344,29 @@ def test_xent_short_rows(R, V, ld):
     assert not g[:, V:].any()
 
 
+@pytest.mark.parametrize("V", [16390, 9001, 5000])
+def test_xent_bits_of_a_row_do_not_depend_on_the_call(V):
+    """Loss, probability and gradient of a row have the same bits with and without the gradient and beside few or many rows: past 592 rows a row
+    is summed by 256 threads, without the gradient or up to 16384 columns, else by 512."""
+    torch.manual_seed(V)
+    ld, rows = (V + 7) // 8 * 8, 700
+    x = torch.zeros(rows, ld, device=DEV).bfloat16()
+    x[:, :V] = _rand(rows, V, scale=4.0)
+    x[3, :V // 2] = float("-inf")
+    t = torch.randint(V // 2, V, (rows,), device=DEV, dtype=torch.int32)
+    out = []
+    for n, grad in ((rows, True), (rows, False), (40, True), (40, False)):
+        g, rl, pr = x[:n].clone(), torch.empty(n, device=DEV), torch.empty(n, device=DEV)
+        ops.xent(g, V, t[:n], rowloss=rl, prob=pr, write_grad=grad)
+        out.append((rl, pr, g))
+    for i, (rl, pr, g) in enumerate(out):
+        n = rl.numel()
+        assert torch.equal(rl, out[0][0][:n]) and torch.equal(pr, out[0][1][:n])
+        assert torch.equal(g, (x if i & 1 else out[0][2])[:n])
+    want = -x[:, :V].double().log_softmax(1).gather(1, t.long()[:, None])[:, 0]
+    assert relerr(out[0][0], want) < 1e-5
+
+
 def test_adamw_matches_torch_and_emits_bf16():
     torch.manual_seed(6)
     n = 100003
