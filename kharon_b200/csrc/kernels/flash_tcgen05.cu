@@ -628,11 +628,6 @@ flash_dkv_ws_kernel(const __grid_constant__ CUtensorMap map_kv, const __grid_con
             tmem_cols<CW>(tmem + buf * 64 + lane_off + c + w, rs);
             tmem_cols<CW>(tmem + BUFS * 64 + buf * 64 + lane_off + c + w, rd);
             tmem_ld_wait();
-            if (diag) {
-#pragma unroll
-              for (int e = 0; e < CW; e++)
-                if (kpos > q0s + c + w + e) rs[e] = 0xff800000u;        // -inf: P and dS are 0
-            }
 #pragma unroll
             for (int e = 0; e < CW; e += 4) {
               const int q0 = c + w + e;
@@ -644,6 +639,15 @@ flash_dkv_ws_kernel(const __grid_constant__ CUtensorMap map_kv, const __grid_con
                 const f32x2 dp = add2(mk2(__uint_as_float(rd[e + u]), __uint_as_float(rd[e + u + 1])), u ? nd.y : nd.x);
                 pp[(w + e + u) >> 1] = pack2(pr);
                 ds[(w + e + u) >> 1] = pack2(mul2(mul2(pr, dp), sc));
+              }
+            }
+            if (diag) {                        // 0 whatever the statistics of a query that comes before the key (NaN, -inf)
+#pragma unroll
+              for (int e = 0; e < CW; e += 2) {
+                const int q = q0s + c + w + e;
+                const uint32_t keep = (kpos > q ? 0u : 0xffffu) | (kpos > q + 1 ? 0u : 0xffff0000u);
+                pp[(w + e) >> 1] &= keep;
+                ds[(w + e) >> 1] &= keep;
               }
             }
           }

@@ -463,6 +463,28 @@ def test_flash_items_handed_out_there_and_back(B, T, H, hd):
     test_flash_fwd_bwd(B, T, H, hd)
 
 
+@pytest.mark.parametrize("B,T,H,hd", [(1, 200, 2, 64), (4, 200, 80, 64), (1, 200, 2, 128), (2, 50, 2, 64)])
+@pytest.mark.parametrize("bad", [float("nan"), 3e38])
+def test_flash_backward_of_a_query_without_a_softmax(B, T, H, hd, bad):
+    """A query whose scores are NaN, or all -inf, has no softmax and no gradient, but the keys after it do not see it: their dV has the bits of
+    a call without that query's fault, in the tile of the diagonal too."""
+    torch.manual_seed(T + hd)
+    d, at = H * hd, 37
+    qkv, dout = _rand(B * T, 3 * d), _rand(B * T, d)
+    dv = []
+    for value in (None, bad):
+        x = qkv.clone()
+        x[:, d:2 * d] = x[:, d:2 * d].abs() + 0.1            # positive keys: a query of -3e38 scores -inf everywhere
+        if value is not None:
+            x[at, :d] = -value                               # in the first sequence
+        out, lse, delta, dqkv = torch.empty(B * T, d, device=DEV).bfloat16(), torch.empty(B, H, T, device=DEV), torch.empty(B, H, T, device=DEV), torch.empty_like(x)
+        ops.flash_fwd(x, out, lse, B, T, H, hd)
+        ops.flash_bwd(x, out, dout, lse, dqkv, delta, B, T, H, hd)
+        assert value is None or out[at].isnan().all()
+        dv.append(dqkv[:, 2 * d:])
+    assert dv[1][:at + 1].isnan().all() and torch.equal(dv[0][at + 1:], dv[1][at + 1:]) and not dv[0].isnan().any()
+
+
 def test_flash_large_scores_rescale():
     """Scores that keep growing along the keys force the in-place rescaling of the output accumulator."""
     torch.manual_seed(21)
