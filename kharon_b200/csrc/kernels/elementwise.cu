@@ -716,7 +716,7 @@ extern "C" int kh_layernorm_bwd(const void* dy, const void* x, const void* w, co
   if ((d + 63) / 64 > KH_COUNTER_SLOTS) { kh_set_error("layernorm_bwd: d=%d is too wide", d); return -1; }
   cudaStream_t st = (cudaStream_t)stream;
   const int parts = kh_layernorm_bwd_parts(rows, d);
-  if (d <= 4096) {
+  if (d <= 4096 && !((uintptr_t)partials & 15)) {         // (the two kernels add to single elements)
     float* sums = (float*)partials + KH_COUNTER_SLOTS;
 #define KH_LN_BWD(WPR) KH_LAUNCH((layernorm_bwd_k<WPR>), parts, WPR == 8 ? 256 : 128, 0, st, (const bf16*)dy, (const bf16*)x, (const bf16*)w, \
                                  (const float*)mean, (const float*)rstd, (const bf16*)dres, (bf16*)dx, sums, rows, d)

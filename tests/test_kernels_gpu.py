@@ -844,3 +844,22 @@ def test_gemm_split_k_on_cta_pairs(M, N, K, split):
         x, y = out[blk].double(), out[512].double()
         assert ((x - y).norm() / y.norm()).item() < 2.0 ** -8 and torch.equal(out[blk][:, N:], out[512][:, N:])
     assert ops.error_word() == 0
+
+
+def test_layernorm_backward_takes_any_scratch():
+    """A scratch that starts on any fp32 element serves (off 16 bytes by the two kernels of wide rows: 1e-5 for another order of the sums, a bf16 step for
+    dx), and its counters stay zero."""
+    torch.manual_seed(3)
+    for rows, d in ((300, 264), (300, 1024), (130, 2048), (40, 4096)):
+        x, w, dy = _rand(rows, d), _rand(d), _rand(rows, d)
+        mean, rstd = x.float().mean(1), (x.float().var(1, unbiased=False) + 1e-5).rsqrt()
+        n = ops.layernorm_bwd_scratch_elems(rows, d)
+        out = []
+        for off in (0, 1, 2):
+            part = torch.zeros(n + off, device=DEV)[off:]
+            dx, dw, db = torch.empty_like(x), torch.zeros(d, device=DEV), torch.zeros(d, device=DEV)
+            ops.layernorm_bwd(dy, x, w, mean, rstd, None, dx, dw, db, part)
+            out.append((dx, dw, db))
+            assert off == 0 or not part[:1024].any()
+        for o in out[1:]:
+            assert all(relerr(a, b) < t for a, b, t in zip(o, out[0], (2.0 ** -8, 1e-5, 1e-5)))
