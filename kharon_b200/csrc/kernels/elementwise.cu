@@ -712,6 +712,7 @@ extern "C" long kh_layernorm_bwd_scratch_elems(int rows, int d) {
 extern "C" int kh_layernorm_bwd(const void* dy, const void* x, const void* w, const void* mean, const void* rstd,
                                 const void* dres, void* dx, void* dw, void* db, void* partials, int rows, int d,
                                 void* stream) {
+  if (rows < 1 || d < 1) { kh_set_error("layernorm_bwd: empty problem %d x %d", rows, d); return -1; }
   if (d % 8) { kh_set_error("layernorm_bwd: d must be a multiple of 8"); return -1; }
   if ((d + 63) / 64 > KH_COUNTER_SLOTS) { kh_set_error("layernorm_bwd: d=%d is too wide", d); return -1; }
   cudaStream_t st = (cudaStream_t)stream;

@@ -863,3 +863,11 @@ def test_layernorm_backward_takes_any_scratch():
             assert off == 0 or not part[:1024].any()
         for o in out[1:]:
             assert all(relerr(a, b) < t for a, b, t in zip(o, out[0], (2.0 ** -8, 1e-5, 1e-5)))
+
+
+@pytest.mark.parametrize("d", [256, 4096, 4104])
+def test_layernorm_backward_refuses_an_empty_problem(d):
+    x, v = torch.zeros(1, d, device=DEV).bfloat16(), torch.zeros(d, device=DEV)
+    part = torch.zeros(ops.layernorm_bwd_scratch_elems(1, d), device=DEV)
+    with pytest.raises(ops.KernelError):
+        ops.layernorm_bwd(x[:0], x[:0], x[0], v, v, None, x[:0], v, v, part)
