@@ -959,10 +959,12 @@ static int num_sms() {
 }
 
 // Threads of a gemm_kernel CTA (or pair) that takes `turns` tiles.  Up to K = 1024 the main loop of a tile is shorter than the epilogue of four warps,
-// which then bounds the product, and with one or two turns the last epilogue is a good part of it: eight warps (8192 x 512 x 2048 with
-// residual 16.2 us, 17.1 with four; 4200 x 1024 x 4096 26.9, 27.3).  Beyond, the epilogue hides behind the main loop and the second set of warps only
-// takes power and issue slots from it (1.2B training step, K = 2048 and more: 147.3 ms with eight, 144.5 with four).
-static int gemm_threads(const GemmParams& p, int turns) { return p.colsum || p.K <= 1024 || turns <= 2 ? GEMM_THREADS : 192; }
+// which then bounds the product, and with one or two turns the last epilogue is a good part of it: eight warps.  us with eight / four, plain and with
+// residual: K = 2048: 8192 x 512 14.5 / 14.9, 16.4 / 17.3; 8192 x 1024 24.8 / 25.0, 27.4 / 28.3; K = 4096: 4200 x 1024 25.4 / 27.3, 28.2 / 31.5; 4096 x 2048
+// 46.2 / 46.5, 49.9 / 50.6; K = 6144: 1024 x 4096 35.5 / 35.8, 38.3 / 39.2.  Beyond, the epilogue hides behind the main loop and the second set of warps only
+// takes power and issue slots from it (K = 8192: 8192 x 1024 100.2 / 97.7, 4200 x 1024 54.6 / 50.5, 1024 x 4096 48.2 / 48.5; 1.2B training step, K = 2048 and more
+// in many turns: 147.3 ms with eight, 144.5 with four).
+static int gemm_threads(const GemmParams& p, int turns) { return p.colsum || p.K <= 1024 || (turns <= 2 && p.K <= 6144) ? GEMM_THREADS : 192; }
 
 // 256-row tiles on CTA pairs.  Returns the number of clusters that can be resident (0: unsupported).
 static int g_pair_clusters = -1;
