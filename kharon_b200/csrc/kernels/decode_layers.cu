@@ -1008,7 +1008,7 @@ __global__ void __launch_bounds__(THREADS, 1) decode_layers_k(const __grid_const
   }
   // launches before this one: constant while it runs (only its last CTA to leave advances the word)
   if (threadIdx.x == 0) sh->launch = *reinterpret_cast<volatile uint32_t*>(p.ctl);
-  if (warp == 1) sh->lgw = item_warps(p);
+  if (warp == 1 && p.L > 0) sh->lgw = item_warps(p);      // (a launch for the head alone has no positions)
   __syncthreads();
 
   if (warp >= NW) {
