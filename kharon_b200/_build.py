@@ -28,7 +28,7 @@ NVCC_FLAGS = [
     "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr",
 ]
 # --use_fast_math (approximate division / sqrt / tanh, flush-to-zero) only where exponentials and
-# tanh sit in a hot loop: GEMM epilogues (GELU), attention, the decode kernels.  The optimizer
+# tanh sit in a hot loop: GEMM epilogues (GELU), attention.  The persistent decode kernel, the optimizer
 # (fp32 master weights, Adam moments), LayerNorm statistics, the loss and the ZeRO step are
 # compiled with IEEE division and square root; their softmax exponentials call __expf explicitly.
 FAST_MATH_FILES = {"gemm_tcgen05.cu", "gemm_skinny.cu", "flash_tcgen05.cu", "flash_short.cu", "paged.cu", "fused_tp.cu"}

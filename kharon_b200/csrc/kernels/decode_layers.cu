@@ -51,9 +51,9 @@
 //
 // Every wait is bounded: status code 9 in the library error word.
 //
-// Measured (L24 d1024 V50257, a captured step with embedding and sampler, this form / epoch-tagged 8-byte packets, cp.async weights and rows
-// of activations before): context 160, G = 1 / 8 / 16 366 / 402 / 557 us (468 / 518 / 737), context 200, G = 32 926 (1206); L24 d2048 G = 4 935
-// (1143); L8 d4096 G = 8 1068 (1606); L4 d256 G = 1 51 (58).  Of the 28 000 cycles of a layer at G = 1, 1000 each are the trips, 2000 a
+// Measured (L24 d1024 V50257, a captured step with embedding and sampler, on one part; in brackets epoch-tagged 8-byte packets, cp.async weights and
+// rows of activations, the form before): context 160, G = 1 / 8 / 16 374 / 407 / 562 us (463 / 515 / 734), context 200, G = 32 936 (1213); L24 d2048
+// context 300, G = 4 956 (1182); L8 d4096 context 200, G = 8 1070 (1603); L4 d256 G = 1 53 (57).  Of the 28 000 cycles of a layer at G = 1, 1000 each are the trips, 2000 a
 // LayerNorm, 900 the products of qkv and fc, 1500 those of fcproj, 6000 the attention, 600 each the sums and epilogues.
 // Numerics follow the five-kernel path: bf16 activations between phases, fp32 accumulation, GELU applied to the bf16-rounded
 // pre-activation.
@@ -72,7 +72,7 @@ constexpr int MAX_SLOTS = 13;
 constexpr int MAX_ROWS = 32;
 constexpr int ATT_PITCH = 128 + 4;            // floats per warp of the attention hand-off: 128 outputs, maximum, sum
 constexpr int SMEM_LIMIT = 227 * 1024;
-constexpr uint32_t POLL_LIMIT = 1u << 23;     // rounds of at least 290 cycles: 1.3 s and more
+constexpr uint32_t POLL_LIMIT = 1u << 23;     // rounds of an L2 load, 290 cycles and more: 1.3 s at least
 
 // Thread index, read anew in every phase: index arithmetic derived from it would otherwise be kept in registers across the layer loop.
 __device__ __forceinline__ int tid_fresh() {

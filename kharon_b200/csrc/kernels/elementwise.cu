@@ -443,7 +443,8 @@ extern "C" int kh_layernorm_fwd(const void* x, const void* w, const void* b, voi
 // before it works on this one, and keeps the column sums of all rows of its CTA in registers; a CTA writes one partial
 // row of sums, and a second, small kernel adds them in index order into the fp32 gradients.  What bounds it is memory for many rows, the
 // trips to it for few.  us, this form / two kernels before, one by rows and one by columns (back to back, captured): 16384 x 2048 55.5 (0.74 of the copy
-// rate) / 78.3, 8192 x 512 10.1 / 14.5, 4096 x 256 6.4 / 9.8, 8192 x 1024 16.5 / 17.9, 4096 x 4096 33.0 / 53.4, 512 x 256 4.6 / 5.2.
+// rate) / 78.3, 8192 x 512 10.1 / 14.5, 4096 x 256 6.4 / 9.8, 8192 x 1024 16.5 / 17.9, 4096 x 4096 33.0 / 53.4, 512 x 256 4.6 / 5.2.  Four CTAs an SM (two of
+// eight warps) leave 128 registers a thread, at which the instances spill 24 to 40 bytes.
 template <int WPR>
 __global__ void __launch_bounds__(WPR == 8 ? 256 : 128, WPR == 8 ? 2 : 4)
 layernorm_bwd_k(const bf16* __restrict__ dy, const bf16* __restrict__ x, const bf16* __restrict__ w, const float* __restrict__ mean,

@@ -89,9 +89,9 @@ class InferEngine:
         self.logits = torch.zeros(ms_, model.Vp, dtype=self.dt, **z)
         self.d_out = torch.zeros(ms_ * 64, dtype=torch.int32, **z)
         self.h_out = torch.zeros(ms_ * 64, dtype=torch.int32, pin_memory=pin)
-        # bf16 engines on a GPU sample up to this many ids straight into pinned memory: no copy back behind the step (completion of
-        # nine tokens, L4 d256: 1271 us, 1176 with the copy of the metadata in the captured step too; 512 ids over the bus take longer
-        # than the copy: a rollout of 9 x 512 4190 and 4245)
+        # bf16 engines on a GPU sample up to this many ids straight into pinned memory: no copy back behind the step (us a step of a whole
+        # generate call, L4 d256, copied / straight: 1 id 102.0 / 92.6, 8 114.8 / 109.0, 16 129.5 / 123.8, 32 180.0 / 169.5, 64 199.0 / 194.9; from 96 on the bus
+        # takes as long as the copy: 96 227.1 / 226.4, 128 250.8 / 250.7, 256 341.2 / 341.4, 512 515.6 / 511.2)
         self._direct = 64 if pin and self.dt == torch.bfloat16 else 0
         # decode steps (few rows) use the weight-streaming split-K GEMM; its scratch covers every shape used
         self.skinny = None
@@ -102,10 +102,10 @@ class InferEngine:
         # Decode steps of up to ``persistent_max`` sequences run all layers and the head in one persistent kernel
         # when the shape allows it (ops.decode_layers); KHARON_PERSISTENT_DECODE=0 or persistent_decode=False keeps
         # the five-kernel chain.  The limit by width is measured (us a step, persistent / chain):
-        #   L24 d1024, context 200: G = 8 415 / 1633, 16 561 / 1886, 17 772 / 1133, 24 850 / 1155, 32 902 / 1205; context 900: G = 17 1214 /
-        #   1502, 32 1769 / 1779;
-        #   L24 d1280: G = 16 1138 / 2126, 17 1671 / 1285, 32 2068 / 1474 (the chain's tensor-core GEMM starts at 17 rows);
-        #   L24 d2048, context 300: G = 16 1532 / 3471, 17 2454 / 1760 (two launches), 32 3062 / 1981.
+        #   L24 d1024, context 200: G = 8 415 / 1660, 16 573 / 1894, 17 773 / 1063, 24 873 / 1087, 32 936 / 1135; context 900: G = 17 1231 /
+        #   1436, 32 1811 / 1721;
+        #   L24 d1280: G = 16 1139 / 2095, 17 1664 / 1219, 32 2083 / 1436 (the chain's tensor-core GEMM starts at 17 rows);
+        #   L24 d2048, context 300: G = 16 1537 / 3459, 17 2478 / 1832 (two launches), 32 3080 / 1933.
         if persistent_decode is None:
             persistent_decode = os.environ.get("KHARON_PERSISTENT_DECODE", "1") != "0"
         self.persistent = bool(persistent_decode and self.skinny is not None and self.tp == 1 and self.dt == torch.bfloat16
