@@ -626,23 +626,49 @@ gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ C
             }
           }
         } else if (row_ok) {                   // ragged last columns
+          // Everything is read before anything is written: the compiler keeps a load behind the stores of the column before it (bias fetched column
+          // by column / ahead: 455 x 920 x 512 with GELU and pre-activation 16.0 / 11.5 us, 125 x 5848 x 1208 with residual 18.6 / 12.9, 16020 x 144 x 80 times
+          // GELU' 13.5 / 11.5).
+          float* const cf = reinterpret_cast<float*>(p.C) + (size_t)row * p.ldc + col;
+          bf16* const ap = p.aux + (size_t)row * p.ldaux + col;
+          float v[32], a[32];
 #pragma unroll
           for (int i = 0; i < 32; i++) {
-            if (col + i >= p.N) break;
-            float x = __uint_as_float(r[i]) * p.alpha;
-            if (use_bias) x += __bfloat162float(p.bias[col + i]);
-            if (p.epi == EPI_BIAS_GELU || p.epi == EPI_GELU) {
-              const bf16 pre = __float2bfloat16(x);
-              if (p.epi == EPI_BIAS_GELU) p.aux[(size_t)row * p.ldaux + col + i] = pre;
-              x = gelu_tanh(__bfloat162float(pre));
-            } else if (use_aux) {
-              const float a = __bfloat162float(p.aux[(size_t)row * p.ldaux + col + i]);
-              x = p.epi == EPI_DGELU ? x * gelu_tanh_grad(a) : x + a;
+            v[i] = __uint_as_float(r[i]) * p.alpha;
+            a[i] = 0.f;
+          }
+          if (use_bias)
+#pragma unroll
+            for (int i = 0; i < 32; i++)
+              if (col + i < p.N) v[i] += __bfloat162float(p.bias[col + i]);
+          if (use_aux)
+#pragma unroll
+            for (int i = 0; i < 32; i++)
+              if (col + i < p.N) a[i] = __bfloat162float(ap[i]);
+          if (p.epi == EPI_BIAS_GELU || p.epi == EPI_GELU) {
+#pragma unroll
+            for (int i = 0; i < 32; i++) {
+              const bf16 pre = __float2bfloat16(v[i]);
+              if (p.epi == EPI_BIAS_GELU && col + i < p.N) ap[i] = pre;
+              v[i] = gelu_tanh(__bfloat162float(pre));
             }
-            if (p.out_fp32) {
-              float* cp = reinterpret_cast<float*>(p.C) + (size_t)row * p.ldc + col + i;
-              *cp = p.accumulate ? *cp + x : x;
-            } else reinterpret_cast<bf16*>(p.C)[(size_t)row * p.ldc + col + i] = __float2bfloat16(x);
+          } else if (use_aux) {
+#pragma unroll
+            for (int i = 0; i < 32; i++) v[i] = p.epi == EPI_DGELU ? v[i] * gelu_tanh_grad(a[i]) : v[i] + a[i];
+          }
+          if (!p.out_fp32) {
+            bf16* const cp = reinterpret_cast<bf16*>(p.C) + (size_t)row * p.ldc + col;
+#pragma unroll
+            for (int i = 0; i < 32; i++)
+              if (col + i < p.N) cp[i] = __float2bfloat16(v[i]);
+          } else {
+            if (p.accumulate)
+#pragma unroll
+              for (int i = 0; i < 32; i++)
+                if (col + i < p.N) a[i] = cf[i];
+#pragma unroll
+            for (int i = 0; i < 32; i++)
+              if (col + i < p.N) cf[i] = p.accumulate ? a[i] + v[i] : v[i];
           }
         }
       }
