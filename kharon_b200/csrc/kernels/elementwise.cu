@@ -870,54 +870,84 @@ __global__ void __launch_bounds__(512 / VT) xent_k(bf16* __restrict__ logits, in
     }
   }
 }
-// Up to 256 NC columns: a warp per row, the row read once and kept in registers.
-template <int NC>
+// Up to 2048 columns: the row read once and kept in registers, in NP parts of NC pieces of 8 x 32 columns.  SHARE: a warp per part, else one warp has all of
+// them (two parts, many rows).  Sums are formed by part and added in order, so that both forms give a row the same bits.
+template <int NP, int NC, bool SHARE>
 __global__ void __launch_bounds__(256) xent_warp_k(bf16* __restrict__ logits, int ld, int V, const int* __restrict__ target,
                                                    const float* __restrict__ coef, float uniform, float* __restrict__ rowloss,
                                                    float* __restrict__ prob, int write_grad, int rows) {
   pdl_wait();
   pdl_launch_dependents();
-  const int r = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-  if (r >= rows) return;
-  bf16* row = logits + (size_t)r * ld;
-  uint4* rp = reinterpret_cast<uint4*>(row);
-  uint4 v[NC];
+  constexpr int WPR = SHARE ? NP : 1, PW = NP / WPR;      // warps of a row, parts of a warp
+  __shared__ float s_max[SHARE ? 8 : 1], s_sum[SHARE ? 8 : 1];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, part = warp % WPR;
+  const int r = (int)blockIdx.x * (8 / WPR) + warp / WPR;
+  if (!SHARE && r >= rows) return;
+  const bool mine = r < rows;
+  bf16* row = logits + (size_t)(mine ? r : 0) * ld;
+  auto col = [&](int p, int j) { return ((j * NP + part + p) * 32 + lane) * 8; };
+  uint4 v[PW][NC];
   uint32_t m2 = 0xff80ff80u;
 #pragma unroll
-  for (int j = 0; j < NC; j++) {
-    const int i = lane + 32 * j;
-    v[j] = i * 8 < V ? rp[i] : make_uint4(0xff80ff80u, 0xff80ff80u, 0xff80ff80u, 0xff80ff80u);
-  }
-  const int t = target[r];
+  for (int p = 0; p < PW; p++)
+#pragma unroll
+    for (int j = 0; j < NC; j++)
+      v[p][j] = mine && col(p, j) < V ? *reinterpret_cast<const uint4*>(row + col(p, j)) : make_uint4(0xff80ff80u, 0xff80ff80u, 0xff80ff80u, 0xff80ff80u);
+  const int t = mine ? target[r] : -1;
   const bool valid = t >= 0 && t < V;
   const float xt = valid ? __bfloat162float(row[t]) : 0.f;
 #pragma unroll
-  for (int j = 0; j < NC; j++) m2 = max_bf16x2(m2, xent_max8(v[j], (lane + 32 * j) * 8, V));
-  const float gmax = warp_max(fmaxf(lo2(un2(m2)), hi2(un2(m2))));
-  const f32x2 nmax = mk2(-gmax, -gmax);
-  f32x2 s2 = 0;
+  for (int p = 0; p < PW; p++)
 #pragma unroll
-  for (int j = 0; j < NC; j++) {
-    f32x2 e[4];
-    xent_exp8(v[j], (lane + 32 * j) * 8, V, nmax, e);
-    s2 = add2(s2, add2(add2(e[0], e[1]), add2(e[2], e[3])));
+    for (int j = 0; j < NC; j++) m2 = max_bf16x2(m2, xent_max8(v[p][j], col(p, j), V));
+  float gmax = warp_max(fmaxf(lo2(un2(m2)), hi2(un2(m2))));
+  if (SHARE) {
+    if (lane == 0) s_max[warp] = gmax;
+    __syncthreads();                       // (and every warp has the target logit)
+#pragma unroll
+    for (int k = 0; k < WPR; k++) gmax = fmaxf(gmax, s_max[warp - part + k]);
   }
-  const float gsum = warp_sum(lo2(s2) + hi2(s2));
-  if (lane == 0) {
+  const f32x2 nmax = mk2(-gmax, -gmax);
+  float sum[PW];
+#pragma unroll
+  for (int p = 0; p < PW; p++) {
+    f32x2 s2 = 0;
+#pragma unroll
+    for (int j = 0; j < NC; j++) {
+      f32x2 e[4];
+      xent_exp8(v[p][j], col(p, j), V, nmax, e);
+      s2 = add2(s2, add2(add2(e[0], e[1]), add2(e[2], e[3])));
+    }
+    sum[p] = warp_sum(lo2(s2) + hi2(s2));
+  }
+  float gsum = sum[0];
+  if (SHARE) {
+    if (lane == 0) s_sum[warp] = gsum;
+    __syncthreads();
+    gsum = s_sum[warp - part];
+#pragma unroll
+    for (int k = 1; k < WPR; k++) gsum += s_sum[warp - part + k];
+  } else {
+#pragma unroll
+    for (int p = 1; p < PW; p++) gsum += sum[p];
+  }
+  if (lane == 0 && part == 0 && mine) {
     if (rowloss) rowloss[r] = valid ? (logf(gsum) + gmax - xt) : 0.f;
     if (prob) prob[r] = valid ? __expf(xt - gmax) / gsum : 0.f;
   }
-  if (!write_grad) return;
-  __syncwarp();      // every lane has the target logit
+  if (!write_grad || !mine) return;
+  if (!SHARE) __syncwarp();                // every lane has the target logit
   const float sc = valid ? (coef ? coef[r] : uniform) : 0.f, inv = sc / gsum;
 #pragma unroll
-  for (int j = 0; j < NC; j++) {
-    const int i = lane + 32 * j;
-    if (i * 8 >= ld) break;
-    f32x2 e[4];
-    xent_exp8(v[j], i * 8, V, nmax, e);
-    rp[i] = xent_grad8(e, i * 8, valid ? t : -2, sc, inv);
-  }
+  for (int p = 0; p < PW; p++)
+#pragma unroll
+    for (int j = 0; j < NC; j++) {
+      const int c = col(p, j);
+      if (c >= ld) continue;
+      f32x2 e[4];
+      xent_exp8(v[p][j], c, V, nmax, e);
+      *reinterpret_cast<uint4*>(row + c) = xent_grad8(e, c, valid ? t : -2, sc, inv);
+    }
 }
 extern "C" int kh_xent(void* logits, int ld, int V, const void* target, const void* coef, float uniform,
                        void* rowloss, void* prob, int write_grad, int rows, void* stream) {
@@ -926,14 +956,15 @@ extern "C" int kh_xent(void* logits, int ld, int V, const void* target, const vo
 #define KH_XENT(K, GRID, THREADS, SMEM, ...) KH_LAUNCH(K, GRID, THREADS, SMEM, st, (bf16*)logits, ld, V, (const int*)target, (const float*)coef, uniform, \
                                                        (float*)rowloss, (float*)prob, write_grad, ##__VA_ARGS__)
   // A CTA of 512 threads has no work for most of them on a short row, and its reductions take longer than its loads: 9216 rows of 256 columns
-  // 35.2 us, a warp per row 4.6 (bound by latency: 1.4 us of memory traffic); 8192 x 1000 35.8 and 10.6, 8192 x 2000 41.8 and 20.6.  More
-  // columns than that are too many registers for one warp.
+  // 35.2 us, a warp per row 4.6 (bound by latency: 1.4 us of memory traffic).  Longer rows keep one warp busy for microseconds, which few rows wait for
+  // (512 threads / a warp / two or four warps: 16 x 1000 3.2 / 3.3 / 2.7 us, 1000 x 1000 6.5 / 3.6 / 3.4, 8192 x 1000 37.9 / 11.0 / 11.6; 150 x 2000 3.4 / 5.3 / 3.0, 1000 x
+  // 2000 7.1 / 5.5 / 4.9, 8192 x 2000 42.8 / 21.8 / 20.4).
   if (ld <= 2048) {
-    const int grid = (rows + 7) / 8;
-    if (ld <= 256) KH_XENT(xent_warp_k<1>, grid, 256, 0, rows);
-    else if (ld <= 512) KH_XENT(xent_warp_k<2>, grid, 256, 0, rows);
-    else if (ld <= 1024) KH_XENT(xent_warp_k<4>, grid, 256, 0, rows);
-    else KH_XENT(xent_warp_k<8>, grid, 256, 0, rows);
+    if (ld <= 256) KH_XENT((xent_warp_k<1, 1, false>), (rows + 7) / 8, 256, 0, rows);
+    else if (ld <= 512) KH_XENT((xent_warp_k<1, 2, false>), (rows + 7) / 8, 256, 0, rows);
+    else if (ld > 1024) KH_XENT((xent_warp_k<4, 2, true>), (rows + 1) / 2, 256, 0, rows);
+    else if (rows <= 1024) KH_XENT((xent_warp_k<2, 2, true>), (rows + 3) / 4, 256, 0, rows);
+    else KH_XENT((xent_warp_k<2, 2, false>), (rows + 7) / 8, 256, 0, rows);
   } else {
     // Eight CTAs of 256 threads an SM wait for less than four of 512 (8192 x 4000 43.1 / 50.2 us, 8192 x 8192 62.9 / 73.1, 8192 x 16000 105.4 / 115.8; loss only,
     // 4096 x 8192 19.6 / 21.2, 8192 x 50257 151.8 / 154.8), but the gradient's second pass finds its row in L2 only while the rows in flight fit there
