@@ -968,8 +968,10 @@ extern "C" int kh_xent(void* logits, int ld, int V, const void* target, const vo
   } else {
     // Eight CTAs of 256 threads an SM wait for less than four of 512 (8192 x 4000 43.1 / 50.2 us, 8192 x 8192 62.9 / 73.1, 8192 x 16000 105.4 / 115.8; loss only,
     // 4096 x 8192 19.6 / 21.2, 8192 x 50257 151.8 / 154.8), but the gradient's second pass finds its row in L2 only while the rows in flight fit there
-    // (4096 x 32000 109.4 / 102.6, 8192 x 50257 382 / 321), and rows that are all resident with 512 threads want them (100 x 16000 6.7 / 5.4).
-    if (rows > 4 * ew_sms() && (!write_grad || ld <= 16384)) KH_XENT(xent_k<2>, rows, 256, 0);
+    // (4096 x 32000 109.4 / 102.6, 8192 x 50257 382 / 321), and rows that are resident with 512 threads, or little more than that, want them, the more so the
+    // longer they are (600 / 1000 / 1300 / 1800 rows of 6659 columns 9.5 / 8.4, 10.7 / 10.6, 12.7 / 13.4, 15.1 / 17.3; of 16000 15.2 / 11.8, 17.8 / 15.7, 20.6 / 19.6, 26.3 /
+    // 26.5; of 2500 6.5 / 6.5, 7.1 / 7.6, 9.4 / 9.9, 10.6 / 12.4).
+    if (rows > (ld <= 4096 ? 4 : ld <= 8192 ? 7 : 12) * ew_sms() && (!write_grad || ld <= 16384)) KH_XENT(xent_k<2>, rows, 256, 0);
     else KH_XENT(xent_k<1>, rows, 512, 0);
   }
 #undef KH_XENT
